@@ -426,7 +426,7 @@ extern "C" int rsd_per_grpery_inv_fri_dev(rsd_ctx* ctx, int32_t nn, const double
   // (regularized Green's function), added after the Ewald sums
   int nov = 0;
   if (correction_method != 0) RSD_TRY(rsd_count_overlaps(ctx, nn, d_pos, d_radii, lat, &nov));
-  RSD_TRY(rsd_ewald_assemble(ctx, nn, d_pos, d_radii, lat, mu_f, RSD_PREC_FP64, d_M, ldm));
+  RSD_TRY(rsd_ewald_assemble(ctx, nn, d_pos, d_radii, lat, mu_f, RSD_PREC_FP64, radii.data(), d_M, ldm));
   return rsd_overlap_correct(ctx, correction_method, RSD_PREC_FP64, nn, d_pos, d_radii, lat, mu_f, nov, d_M, ldm);
 }
 

@@ -6,21 +6,22 @@
 // ldm) in the reference's order: rows/cols 3a..3a+2 translation of particle
 // a, 3N+3a.. rotation, 6N+5a.. stresslet (Y2 basis).
 //
-// Work split (thread per unordered pair a < b):
-//   ewald_ktable      per reciprocal vector k (half space k > 0): the
-//                     radius-independent weights S(k) k^alpha of the cos and
-//                     sin moments (pair independent, computed once per call)
-//   ewald_trig        per (k, particle): cos(k.x_a), sin(k.x_a), so that
+// Work split:
+//   ewald_weights     per reciprocal vector k (half space k > 0): the weights
+//                     of the pair sums, in the layout [weight][vector]
+//   ewald_trig        per (particle, k): cos(k.x_a), sin(k.x_a), so that
 //                     cos(k.R_ab) = c_a c_b + s_a s_b needs no sincos per pair
-//   ewald_pair_k      per pair: reciprocal moments over the half space (x2),
-//                     epilogue, writes both 11x11 blocks of the pair
-//   ewald_pair_real   per pair: real-space moments over the image cube,
-//                     epilogue, adds into both blocks
-//   ewald_self        per particle: self block (images n != 0, k != 0, and
-//                     the analytic terms of PER_ROTNE_PRAGER_SELF 179-188)
+//   ewald_pair64      FP64 form, a group of lanes per pair a < b: real-space
+//                     and reciprocal sums and the epilogue, both 11x11 blocks
+//                     of the pair written once
+//   ewald_pair_*      mixed form, a thread per pair (below)
+//   ewald_self_sums, ewald_self*  the diagonal blocks (images n != 0, k != 0
+//                     and the analytic terms of PER_ROTNE_PRAGER_SELF 179-188)
 // The closed forms come from ewald_gen.cuh (generated by gen_ewald.py).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "ewald_gen.cuh"
@@ -40,6 +41,9 @@ __host__ __device__ inline void half_space_index(int h, int NI, int* nx, int* ny
   *nz = q % w - NI;
 }
 
+// outputs (gen_ewald.py's order) that the sin sums feed: TR and G
+__host__ __device__ constexpr bool kblock_is_sin(int q) { return (q >= 12 && q < 15) || (q >= 30 && q < 45); }
+
 // S(k) of F_Jk (Ewald_summation.f90:1067-1071): F_Jk = S (delta k^2 - k k)
 template <typename T>
 __device__ inline T kernel_S(T k2, T lam) {
@@ -47,34 +51,57 @@ __device__ inline T kernel_S(T k2, T lam) {
   return T(8.0 * RSD_PI) * (T(1) + k2 / (T(4) * l2) + k2 * k2 / (T(8) * l2 * l2)) * exp(-k2 / (T(4) * l2)) / (k2 * k2);
 }
 
-__global__ void ewald_ktable(rsd_lat_dev L, int Kh, double* __restrict__ tab) {
+// Weights of the listed half-space vectors (kv: 3 doubles each), W[q * Kh + h]:
+// with equal radii (EQ) the 60 block weights -- the epilogue of the moment
+// weights for the common radius a, scaled like the block (ewald_kblock_list);
+// otherwise the 80 moment weights (cos, then sin).  blockIdx.y = 0 forms the
+// cos part, 1 the sin part: one warp issues an FP64 instruction every 64
+// cycles here, so a thread's instruction count is the kernel's time.
+template <bool EQ>
+__global__ void ewald_weights(rsd_lat_dev L, int Kh, const double* __restrict__ kv, double a, double inv_pimu,
+                              double* __restrict__ W) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= Kh) return;
-  int nx, ny, nz;
-  half_space_index(h, L.NI, &nx, &ny, &nz);
-  double k[3];
-  for (int j = 0; j < 3; j++)
-    k[j] = 2.0 * RSD_PI * (nx * L.LI[0 + 3 * j] + ny * L.LI[1 + 3 * j] + nz * L.LI[2 + 3 * j]);
-  const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
-  const double S = kernel_S<double>(k2, L.lam);
-  double* e = tab + (size_t)h * KW;
-  e[0] = k[0];
-  e[1] = k[1];
-  e[2] = k[2];
-  rsd_kcos_weights<double>(k[0], k[1], k[2], S, L.lam, e + 3);
-  rsd_ksin_weights<double>(k[0], k[1], k[2], S, L.lam, e + 3 + RSD_NMOM_KCOS);
+  const double k0 = kv[3 * h], k1 = kv[3 * h + 1], k2v = kv[3 * h + 2];
+  const double S = kernel_S<double>(k0 * k0 + k1 * k1 + k2v * k2v, L.lam);
+  const double f = 2.0 / L.LV, na = f * inv_pimu / (6.0 * a), na3 = na / (a * a);  // EQ: half space counted twice
+  double w[RSD_NMOM_KCOS], v[60];
+  if (blockIdx.y == 0) {
+    rsd_kcos_weights<double>(k0, k1, k2v, S, L.lam, w);
+    if (EQ) {
+      rsd_kcos_epilogue<double>(w, a, a, L.phix, v);
+#pragma unroll
+      for (int q = 0; q < 60; q++) {
+        const bool a3 = (q >= 6 && q < 12) || (q >= 15 && q < 30) || q >= 45;
+        if (!kblock_is_sin(q)) W[(size_t)q * Kh + h] = v[q] * (a3 ? na3 : na);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < RSD_NMOM_KCOS; m++) W[(size_t)m * Kh + h] = w[m];
+    }
+  } else {
+    rsd_ksin_weights<double>(k0, k1, k2v, S, L.lam, w);
+    if (EQ) {
+      rsd_ksin_epilogue<double>(w, a, a, L.phix, v);
+#pragma unroll
+      for (int q = 0; q < 60; q++)
+        if (kblock_is_sin(q)) W[(size_t)q * Kh + h] = v[q] * na;  // TR and G
+    } else {
+#pragma unroll
+      for (int m = 0; m < RSD_NMOM_KSIN; m++) W[(size_t)(RSD_NMOM_KCOS + m) * Kh + h] = w[m];
+    }
+  }
 }
 
-__global__ void ewald_trig(int nn, int Kh, const double* __restrict__ tab, const double* __restrict__ pos,
+// cs[a * Kh + h] = (cos, sin)(k_h . x_a)
+__global__ void ewald_trig(int nn, int Kh, const double* __restrict__ kv, const double* __restrict__ pos,
                            double2* __restrict__ cs) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  const int h = blockIdx.y;
-  if (a >= nn) return;
-  const double* e = tab + (size_t)h * KW;
-  const double kr = e[0] * pos[3 * a] + e[1] * pos[3 * a + 1] + e[2] * pos[3 * a + 2];
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (int64_t)nn * Kh) return;
+  const int a = (int)(t / Kh), h = (int)(t % Kh);
   double s, c;
-  sincos(kr, &s, &c);
-  cs[(size_t)h * nn + a] = make_double2(c, s);
+  sincos(kv[3 * h] * pos[3 * a] + kv[3 * h + 1] * pos[3 * a + 1] + kv[3 * h + 2] * pos[3 * a + 2], &s, &c);
+  cs[t] = make_double2(c, s);
 }
 
 // Weights and trig tables restricted to a list of half-space indices, in
@@ -409,11 +436,6 @@ struct Vec2<float> {
   using type = float4;  // four weights per shared-memory load
   static constexpr int W = 4;
 };
-template <>
-struct Vec2<double> {
-  using type = double2;
-  static constexpr int W = 2;
-};
 
 // Reciprocal-space pair sums: per half-space vector, cos and sin of k.(x_a -
 // x_b) from the per-particle trig table, times the vector's 80 moment
@@ -568,7 +590,6 @@ __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, in
 // FP64.  A pair then costs 60 multiply-adds per vector instead of 80, and
 // its FP32 rounding is no longer amplified by the epilogue's cancellation
 // between moments.
-__host__ __device__ constexpr bool kblock_is_sin(int q) { return (q >= 12 && q < 15) || (q >= 30 && q < 45); }
 constexpr int KBW = 64;  // weights per vector (60 used, padded for 16-byte rows)
 
 template <typename T>
@@ -1037,103 +1058,315 @@ __global__ void __launch_bounds__(REAL_THREADS, MINB) ewald_pair_real_eq(int nn,
 }
 
 
-__global__ void __launch_bounds__(128) ewald_pair_real(int nn, rsd_lat_dev L, const double* __restrict__ pos,
-                                                       const double* __restrict__ radii, double inv_pimu,
-                                                       DenseSink sk) {
-  int a, b;
-  if (!pair_of(nn, &a, &b)) return;
-  double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
-  double dmin;
-  rsd_skew_correction(L.LR, L.LI, R, &dmin);
-  double acc[RSD_NMOM_REAL];
+// ----------------------------------------------------------- FP64 pair sums
+// GB300's FP64 pipe (2 multiply-adds per SM and cycle) bounds the FP64
+// assembly: an image costs ~400 FP64 instructions, a reciprocal vector ~66
+// (equal radii) or ~86, everything else (loads included) hides behind them.
+// So the work per pair is what counts, and it is cut to what FP64 can
+// represent: the Ewald sum does not depend on its splitting parameter, which
+// is moved to EWALD64_SCALE times the reference's, and terms beyond lambda r =
+// EWALD64_XC or k^2 / (4 lambda^2) = EWALD64_YC are left out.  Against long
+// double sums over larger cubes the largest entry of a pair block moves by
+// <= 3e-17 by that (2e-16 at two spheres in a box of 3.5 radii), with FP64
+// rounding of a block at 1e-17 to 1e-16 either way.  A pair then takes ~77
+// images and ~357 vectors instead of 343 to 1331 and 171 to 665.  Measured,
+// pair sums in all, a thread per pair over the whole cubes before: N = 1000
+// at zero strain 122.7 -> 47.4 ms (0.63e12 FP64 instructions/s, the pipe's
+// rate), N = 512 at skew 0.5 76.3 -> 12.5 ms, N = 125 9.8 -> 0.91 ms, N = 64
+// 9.8 -> 0.29 ms.
+//
+// A group of G lanes takes a pair: the group lists the images inside the
+// sphere (an FP32 test; images within rounding of the surface may fall
+// either way), its lanes take them and then the vectors in turn, and the
+// moments are added up by halving exchanges, each lane left with 1/G of them.
+// The lanes of a warp stay on images of the same pairs, so none idles
+// through another's, and a small system still fills the GPU.  The epilogue
+// is spread over the outputs (equal radii) or taken by one thread per pair.
+constexpr double EWALD64_SCALE = 1.45, EWALD64_XC = 6.8, EWALD64_YC = 46.0;
+constexpr int P64_THREADS = 128, P64_CAP = 128;
+
+// Halving exchange over the lanes of a group: N values per lane in, the sums
+// of `n` of them from `off` on out (the rest is with the other lanes).
+template <int H, int N, int G>
+__device__ __forceinline__ void group_halve(double (&v)[G], int gl, int& off, int& n) {
+  if constexpr (H > 0) {
+    constexpr int HN = (N + 1) / 2;
+    const bool up = (gl & H) != 0;
 #pragma unroll
-  for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.0;
-  const double lam = L.lam, lam2 = lam * lam, cd = 2.0 * RSD_PIP5 * lam;
-  const int NR = L.NR;
-  for (int nx = -NR; nx <= NR; nx++)
-    for (int ny = -NR; ny <= NR; ny++) {
-      double x0 = R[0] + L.LR[0] * nx + L.LR[3] * ny - L.LR[6] * NR;
-      double x1 = R[1] + L.LR[1] * nx + L.LR[4] * ny - L.LR[7] * NR;
-      double x2 = R[2] + L.LR[2] * nx + L.LR[5] * ny - L.LR[8] * NR;
-      for (int nz = -NR; nz <= NR; nz++) {
-        const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-        const double r = sqrt(r2), ir = 1.0 / r;
-        const double E0 = erfc(lam * r), Ed = cd * exp(-r2 * lam2);
-        rsd_real_image<double>(x0, x1, x2, r, ir, E0, Ed, lam, acc);
-        x0 += L.LR[6];
-        x1 += L.LR[7];
-        x2 += L.LR[8];
-      }
+    for (int i = 0; i < HN; i++) {
+      const double lo = v[i], hi = i + HN < N ? v[i + HN] : 0.0;
+      v[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, H);
     }
-  double v[60];
-  rsd_real_epilogue<double>(acc, radii[a], radii[b], L.phix, v);
-  scale_block(v, radii[a], inv_pimu);
-  store_pair_d(sk, nn, a, b, v, 1);
+    if (up) {
+      off += HN;
+      n -= HN;
+    } else {
+      n = min(n, HN);
+    }
+    group_halve<H / 2, HN, G>(v, gl, off, n);
+  }
 }
 
-// Self-image moments.  The real-space images n != 0 of a particle and the
-// cos weights of the half space do not depend on the particle (only the
-// epilogue does, through its radius), so one CTA sums them once in FP64:
-// out[0..96] = real moments, out[97..145] = kcos weights.
-constexpr int SELF_NMOM = RSD_NMOM_REAL + RSD_NMOM_KCOS;
-constexpr int SELF_THREADS = 128;
-
-__device__ __forceinline__ double warp_sum(double v) {
+template <int L, int N>
+__device__ __forceinline__ void group_sum(double (&v)[N], int gl, double* dst) {
+  int off = 0, n = N;
+  group_halve<L / 2, N, N>(v, gl, off, n);
+  constexpr int LEFT = (N + L - 1) / L + 1;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int i = 0; i < LEFT; i++)
+    if (i < n) dst[off + i] = v[i];
 }
 
-__global__ void __launch_bounds__(SELF_THREADS) ewald_self_moments(rsd_lat_dev L, int Kh,
-                                                                   const double* __restrict__ tab,
-                                                                   double* __restrict__ out) {
-  __shared__ double part[SELF_THREADS / 32][SELF_NMOM];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const double lam = L.lam, lam2 = lam * lam, cd = 2.0 * RSD_PIP5 * lam;
+// Entry (r, c) of the 11 x 11 block (a, b), a < b, from the pair's 60 values.
+__device__ __forceinline__ double pair_block_entry(const double* v, int r, int c) {
+  const int rs = r < 3 ? 0 : (r < 6 ? 1 : 2), cs = c < 3 ? 0 : (c < 6 ? 1 : 2);
+  const int i = rs == 2 ? r - 6 : r - 3 * rs, j = cs == 2 ? c - 6 : c - 3 * cs;
+  if (rs == cs && rs < 2) {  // TT, RR: symmetric 3 x 3 as 00 01 02 11 12 22
+    const int lo = min(i, j), hi = max(i, j);
+    return v[6 * rs + (lo == 0 ? hi : lo + hi + 1)];
+  }
+  if (rs == 2 && cs == 2) {
+    const int lo = min(i, j), hi = max(i, j);
+    return v[15 + lo * 5 - lo * (lo - 1) / 2 + (hi - lo)];
+  }
+  if (rs < 2 && cs < 2) {  // TR: antisymmetric, odd under a <-> b
+    const int t = rs == 0 ? i : j, q = rs == 0 ? j : i;
+    if (t == q) return 0.0;
+    const double x = v[12 + min(t, q) + max(t, q) - 1];
+    return (t < q) == (rs == 0) ? x : -x;
+  }
+  if (rs < 2) return v[(rs ? 45 : 30) + 5 * i + j];   // G, H
+  const double x = v[(cs ? 45 : 30) + 5 * j + i];
+  return cs == 0 ? -x : x;                             // G is odd under a <-> b
+}
+
+// grand-matrix index of component k (0..10) of particle p
+__device__ __forceinline__ int64_t grand_row(int N, int p, int k) {
+  return k < 3 ? 3 * p + k : (k < 6 ? 3 * N + 3 * p + k - 3 : 6 * N + 5 * p + k - 6);
+}
+
+// cube: every listed image counts, around the exact minimum image of
+// rsd_skew_correction (a sum whose cube the reference cuts visibly).
+template <int G, bool EQ>
+__global__ void __launch_bounds__(P64_THREADS) ewald_pair64(int nn, int64_t npair, rsd_lat_dev L, int cube, int nimg,
+                                                            const double* __restrict__ img,
+                                                            const float4* __restrict__ imgf, float rc2, int Kh,
+                                                            const double* __restrict__ W,
+                                                            const double2* __restrict__ cs,
+                                                            const double* __restrict__ pos,
+                                                            const double* __restrict__ radii, double inv_pimu,
+                                                            const double* __restrict__ coef,
+                                                            const unsigned short* __restrict__ etab, DenseSink sk) {
+  constexpr int PP = P64_THREADS / G, NK = EQ ? 60 : RSD_NMOM_KCOS + RSD_NMOM_KSIN, NR = RSD_NMOM_REAL;
+  __shared__ double mom[PP][NR + NK];
+  __shared__ int list[PP][P64_CAP];
+  __shared__ double sc[EQ ? RSD_REAL_EPI_NC : 1];
+  __shared__ unsigned short st[EQ ? RSD_REAL_EPI_NC : 1], so[EQ ? 61 : 1];
+  const int t = threadIdx.x, g = t / G, gl = t % G, seg = (t & 31) / G * G;
+  if (EQ) {
+    for (int k = t; k < RSD_REAL_EPI_NC; k += P64_THREADS) {
+      sc[k] = coef[k];
+      st[k] = etab[61 + k];
+    }
+    for (int q = t; q < 61; q += P64_THREADS) so[q] = etab[q];
+  }
+  // pair p = b (b - 1) / 2 + a; the groups past the end repeat the last pair
+  const int64_t p0 = (int64_t)blockIdx.x * PP;
+  auto pair_ab = [&](int64_t p, int* pa, int* pb) {
+    int b = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
+    while ((int64_t)b * (b - 1) / 2 > p) b--;
+    while ((int64_t)(b + 1) * b / 2 <= p) b++;
+    *pb = b;
+    *pa = (int)(p - (int64_t)b * (b - 1) / 2);
+  };
+  int a, b;
+  pair_ab(min(p0 + g, npair - 1), &a, &b);
+  double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
+  if (cube) {
+    double dmin;
+    rsd_skew_correction(L.LR, L.LI, R, &dmin);
+  } else {
+    float A[9], LIf[9];
+    for (int k = 0; k < 9; k++) {
+      A[k] = (float)L.LR[k];
+      LIf[k] = (float)L.LI[k];
+    }
+    const float R0[3] = {(float)R[0], (float)R[1], (float)R[2]};
+    int k[3];
+    rsd_skew_shift_f32(A, LIf, R0, k);
+    for (int i = 0; i < 3; i++) R[i] -= k[0] * L.LR[i] + k[1] * L.LR[3 + i] + k[2] * L.LR[6 + i];
+  }
   {
-    double acc[RSD_NMOM_REAL];
+    const float Rf[3] = {(float)R[0], (float)R[1], (float)R[2]};
+    const double lam = L.lam, lam2 = lam * lam, cd = 2.0 * RSD_PIP5 * lam;
+    double acc[NR];
 #pragma unroll
-    for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.0;
-    const int NR = L.NR, w = 2 * NR + 1, nimg = w * w * w;
-    for (int i = tid; i < nimg; i += SELF_THREADS) {
-      const int nx = i / (w * w) - NR, ny = (i / w) % w - NR, nz = i % w - NR;
-      if (!nx && !ny && !nz) continue;  // PER_ROTNE_PRAGER_SELF 61
-      const double x0 = L.LR[0] * nx + L.LR[3] * ny + L.LR[6] * nz;
-      const double x1 = L.LR[1] * nx + L.LR[4] * ny + L.LR[7] * nz;
-      const double x2 = L.LR[2] * nx + L.LR[5] * ny + L.LR[8] * nz;
+    for (int m = 0; m < NR; m++) acc[m] = 0.0;
+    int cnt = 0;
+    auto flush = [&](bool last) {
+      const int nb = last ? (cnt + G - 1) / G : cnt / G;
+      const int mb = __reduce_max_sync(0xffffffffu, nb);
+      __syncwarp();
+      for (int q = 0; q < mb; q++) {
+        const int e = q * G + gl;
+        if (q < nb && e < cnt) {
+          const double* x = img + 3 * (size_t)list[g][e];
+          const double x0 = R[0] + x[0], x1 = R[1] + x[1], x2 = R[2] + x[2];
+          const double r2 = x0 * x0 + x1 * x1 + x2 * x2, r = sqrt(r2);
+          rsd_real_image<double>(x0, x1, x2, r, 1.0 / r, erfc(lam * r), cd * exp(-r2 * lam2), lam, acc);
+        }
+      }
+      if (!last) {  // the images of the last, partly filled round start the next list
+        const int rem = cnt - nb * G;
+        const int v = gl < rem ? list[g][nb * G + gl] : 0;
+        __syncwarp();
+        if (gl < rem) list[g][gl] = v;
+        cnt = rem;
+      }
+      __syncwarp();
+    };
+    for (int c0 = 0; c0 < nimg; c0 += G) {
+      const int i = c0 + gl;
+      bool in = false;
+      if (i < nimg) {
+        const float4 x = imgf[i];
+        const float x0 = Rf[0] + x.x, x1 = Rf[1] + x.y, x2 = Rf[2] + x.z;
+        in = x0 * x0 + x1 * x1 + x2 * x2 < rc2;
+      }
+      unsigned m = __ballot_sync(0xffffffffu, in) >> seg;
+      if (G < 32) m &= (1u << (G & 31)) - 1u;
+      if (in) list[g][cnt + __popc(m & ((1u << gl) - 1u))] = i;
+      cnt += __popc(m);
+      if (__any_sync(0xffffffffu, cnt > P64_CAP - G)) flush(false);
+    }
+    flush(true);
+    group_sum<G, NR>(acc, gl, mom[g]);
+  }
+  {
+    double acc[NK];
+#pragma unroll
+    for (int m = 0; m < NK; m++) acc[m] = 0.0;
+    const double2 *ca = cs + (size_t)a * Kh, *cb = cs + (size_t)b * Kh;
+    for (int h = gl; h < Kh; h += G) {
+      const double2 ua = ca[h], ub = cb[h];
+      const double c = ua.x * ub.x + ua.y * ub.y;   // cos(k.(x_a - x_b))
+      const double sn = ua.y * ub.x - ua.x * ub.y;  // sin(k.(x_a - x_b))
+#pragma unroll
+      for (int m = 0; m < NK; m++)
+        acc[m] = ::fma(W[(size_t)m * Kh + h], (EQ ? kblock_is_sin(m) : m >= RSD_NMOM_KCOS) ? sn : c, acc[m]);
+    }
+    __syncwarp();
+    group_sum<G, NK>(acc, gl, mom[g] + NR);
+  }
+  __syncthreads();
+  const int np = (int)min((int64_t)PP, npair - p0);
+  if (EQ) {
+    for (int e = t; e < np * 60; e += P64_THREADS) {
+      double* m = mom[e / 60];
+      const int q = e % 60;
+      double v = m[NR + q];
+      for (int k = so[q]; k < so[q + 1]; k++) v = ::fma(sc[k], m[st[k]], v);
+      m[NR + q] = v;
+    }
+  } else if (t < np) {
+    pair_ab(p0 + t, &a, &b);
+    const double ai = radii[a], aj = radii[b], f = 2.0 / L.LV;  // half space counted twice
+    double* m = mom[t];
+    double v[60], w[60], o[60];
+    rsd_real_epilogue<double>(m, ai, aj, L.phix, o);
+    rsd_kcos_epilogue<double>(m + NR, ai, aj, L.phix, v);
+    rsd_ksin_epilogue<double>(m + NR + RSD_NMOM_KCOS, ai, aj, L.phix, w);
+#pragma unroll
+    for (int q = 0; q < 60; q++) o[q] += (v[q] + w[q]) * f;
+    scale_block(o, ai, inv_pimu);
+#pragma unroll
+    for (int q = 0; q < 60; q++) m[NR + q] = o[q];
+  }
+  __syncthreads();
+  for (int e = t; e < np * 121; e += P64_THREADS) {
+    const int pr = e % np, en = e / np, r = en % 11, c = en / 11;
+    pair_ab(p0 + pr, &a, &b);
+    const double v = pair_block_entry(mom[pr] + NR, r, c);
+    const int64_t i = grand_row(nn, a, r), j = grand_row(nn, b, c);
+    sk.M[i + j * sk.ld] = v;
+    sk.M[j + i * sk.ld] = v;
+  }
+}
+
+// Self sums.  The real-space images n != 0 of a particle and the cos weights
+// of the half space do not depend on the particle (only the epilogue does,
+// through its radius), so one CTA sums them once in FP64.  EQ: out[0..59] =
+// the whole diagonal block of the common radius ai, scaled; otherwise the
+// moments, out[0..96] real and out[97..145] kcos.
+constexpr int SELF_NMOM = RSD_NMOM_REAL + RSD_NMOM_KCOS;
+constexpr int SELF_THREADS = 256;
+
+// analytic self terms (Ewald_summation.f90:179-188) of output q
+__device__ __forceinline__ double self_analytic(int q, double ai, double lam, double phix) {
+  const double sp = sqrt(RSD_PI), a3 = ai * ai * ai, l3 = lam * lam * lam;
+  if (q == 0 || q == 3 || q == 5) return 1.0 - 6.0 * lam / sp * ai + 40.0 / 3.0 / sp * l3 * a3 * phix;
+  if (q == 6 || q == 9 || q == 11) return 0.75 - 10.0 / sp * a3 * l3;
+  if (q == 15 || q == 20 || q == 24 || q == 27 || q == 29)  // QQ diagonal in the upper-triangle order
+    return 0.9 - l3 * a3 / 25.0 / sp * (50.0 - 126.0 * lam * lam * ai * ai) * 6.0;
+  return 0.0;
+}
+
+template <bool EQ>
+__global__ void __launch_bounds__(SELF_THREADS) ewald_self_sums(rsd_lat_dev L, int nimg,
+                                                                const double* __restrict__ img,
+                                                                const float4* __restrict__ imgf, float rc2, int Kh,
+                                                                const double* __restrict__ W, double ai,
+                                                                double inv_pimu, const double* __restrict__ coef,
+                                                                const unsigned short* __restrict__ etab,
+                                                                double* __restrict__ out) {
+  constexpr int NW = SELF_THREADS / 32, NR = RSD_NMOM_REAL, NQ = EQ ? 60 : RSD_NMOM_KCOS;
+  __shared__ double part[NW][NR], mom[NR], ks[NQ];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  {
+    const double lam = L.lam, lam2 = lam * lam, cd = 2.0 * RSD_PIP5 * lam;
+    double acc[NR];
+#pragma unroll
+    for (int m = 0; m < NR; m++) acc[m] = 0.0;
+    for (int i = t; i < nimg; i += SELF_THREADS) {  // shortest first; n = 0 is left out (PER_ROTNE_PRAGER_SELF 61)
+      const float4 f = imgf[i];
+      const float r2f = f.x * f.x + f.y * f.y + f.z * f.z;
+      if (!(r2f > 0.f && r2f < rc2)) continue;
+      const double x0 = img[3 * i], x1 = img[3 * i + 1], x2 = img[3 * i + 2];
       const double r2 = x0 * x0 + x1 * x1 + x2 * x2, r = sqrt(r2);
       rsd_real_image<double>(x0, x1, x2, r, 1.0 / r, erfc(lam * r), cd * exp(-r2 * lam2), lam, acc);
     }
-#pragma unroll
-    for (int m = 0; m < RSD_NMOM_REAL; m++) {
-      const double v = warp_sum(acc[m]);
-      if (lane == 0) part[warp][m] = v;
-    }
+    __syncwarp();
+    group_sum<32, NR>(acc, lane, part[warp]);
   }
-  {
-    double ac[RSD_NMOM_KCOS];
+  for (int q = warp; q < NQ; q += NW) {  // sin sums vanish: k and -k cancel
+    double v = 0.0;
+    if (!EQ || !kblock_is_sin(q))
+      for (int h = lane; h < Kh; h += 32) v += W[(size_t)q * Kh + h];
 #pragma unroll
-    for (int m = 0; m < RSD_NMOM_KCOS; m++) ac[m] = 0.0;
-    for (int h = tid; h < Kh; h += SELF_THREADS) {
-      const double* e = tab + (size_t)h * KW + 3;
-#pragma unroll
-      for (int m = 0; m < RSD_NMOM_KCOS; m++) ac[m] += e[m];
-    }
-#pragma unroll
-    for (int m = 0; m < RSD_NMOM_KCOS; m++) {
-      const double v = warp_sum(ac[m]);
-      if (lane == 0) part[warp][RSD_NMOM_REAL + m] = v;
-    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) ks[q] = v;
   }
   __syncthreads();
-  for (int m = tid; m < SELF_NMOM; m += SELF_THREADS) {
-    double t = 0.0;
-    for (int q = 0; q < SELF_THREADS / 32; q++) t += part[q][m];
-    out[m] = t;
+  if (t < NR) {
+    double v = 0.0;
+    for (int w = 0; w < NW; w++) v += part[w][t];
+    mom[t] = v;
+  }
+  __syncthreads();
+  if (EQ) {
+    if (t < 60) {
+      const bool a3 = (t >= 6 && t < 12) || (t >= 15 && t < 30) || t >= 45;
+      double v = self_analytic(t, ai, L.lam, L.phix) * inv_pimu / (6.0 * (a3 ? ai * ai * ai : ai)) + ks[t];
+      for (int k = etab[t]; k < etab[t + 1]; k++) v = ::fma(coef[k], mom[etab[61 + k]], v);
+      out[t] = v;
+    }
+  } else {
+    if (t < NR) out[t] = mom[t];
+    if (t < RSD_NMOM_KCOS) out[NR + t] = ks[t];
   }
 }
 
-// Diagonal blocks from the self moments (ewald_self_moments) and the
+// Diagonal blocks from the self sums (ewald_self_sums<false>) and the
 // particle's radius.
 __device__ __forceinline__ void sink_put(const DenseSink& sk, int64_t o, double x) { sk.M[o] = x; }
 __device__ __forceinline__ void sink_put(const PlaneSink& sk, int64_t o, double x) {
@@ -1199,6 +1432,18 @@ __global__ void __launch_bounds__(64) ewald_self(int nn, rsd_lat_dev L, const do
     for (int y = x; y < 5; y++) qq[x][y] = qq[y][x] = v[q++];
   for (int x = 0; x < 5; x++)
     for (int y = 0; y < 5; y++) M((6 * N + 5 * a + x) + (int64_t)(6 * N + 5 * a + y) * ldm, qq[x][y]);
+}
+
+// Diagonal blocks of equal spheres: the one block of ewald_self_sums<true>
+// written for every particle (TT, RR, QQ; TR, G, H are zero,
+// per_GRPY_YZD.f90:63-66), a thread per entry.
+template <typename S>
+__global__ void ewald_self_eq(int nn, const double* __restrict__ v, S sk) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 121 * nn) return;
+  const int a = t % nn, r = t / nn % 11, c = t / nn / 11;
+  const bool same = (r < 3) == (c < 3) && (r < 6) == (c < 6);
+  sink_put(sk, grand_row(nn, a, r) + grand_row(nn, a, c) * sk.ld, same ? pair_block_entry(v, r, c) : 0.0);
 }
 
 __global__ void overlap_count(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
@@ -1353,43 +1598,233 @@ int rsd_mirror_planes(rsd_ctx* ctx, int nn, double* d_M, int64_t ldm) {
   return RSD_OK;
 }
 
+namespace {
+// Lattice vectors and reciprocal vectors of a sum, made on the host.
+struct ewald_lists {
+  std::vector<double> img;  // lattice vectors LR n, shortest first (3 each)
+  std::vector<double> kv;   // half-space reciprocal vectors (3 each)
+  double rc2 = 0.0;         // images beyond rc2 are left out (infinite: none)
+};
+
+// The images within EWALD64_XC / lam of a point of the cell around the
+// origin (self_only: of the origin), and the half-space vectors below
+// EWALD64_YC.
+ewald_lists ewald_sphere_lists(const rsd_lat_dev& L, double lam, bool self_only) {
+  ewald_lists o;
+  const double rc = EWALD64_XC / lam, kmax = 2.0 * lam * sqrt(EWALD64_YC);
+  o.rc2 = rc * rc;
+  double dmax = 0.0;  // a minimum image is no longer than half the longest diagonal of the cell
+  for (int m = 0; m < 4 && !self_only; m++) {
+    double d2 = 0.0;
+    for (int j = 0; j < 3; j++) {
+      const double x = L.LR[j] + (m & 1 ? -L.LR[3 + j] : L.LR[3 + j]) + (m & 2 ? -L.LR[6 + j] : L.LR[6 + j]);
+      d2 += x * x;
+    }
+    dmax = fmax(dmax, 0.5 * sqrt(d2));
+  }
+  const double lim = rc + 1.001 * dmax;
+  int nr[3], ni[3];
+  for (int i = 0; i < 3; i++) {
+    double a2 = 0.0, b2 = 0.0;
+    for (int j = 0; j < 3; j++) {
+      a2 += L.LR[j + 3 * i] * L.LR[j + 3 * i];
+      b2 += L.LI[i + 3 * j] * L.LI[i + 3 * j];
+    }
+    nr[i] = (int)(lim * sqrt(b2)) + 1;
+    ni[i] = (int)(kmax * sqrt(a2) / (2.0 * RSD_PI)) + 1;
+  }
+  std::vector<std::pair<double, int>> key;
+  std::vector<double> x;
+  for (int nx = -nr[0]; nx <= nr[0]; nx++)
+    for (int ny = -nr[1]; ny <= nr[1]; ny++)
+      for (int nz = -nr[2]; nz <= nr[2]; nz++) {
+        double v[3], r2 = 0.0;
+        for (int j = 0; j < 3; j++) {
+          v[j] = L.LR[j] * nx + L.LR[3 + j] * ny + L.LR[6 + j] * nz;
+          r2 += v[j] * v[j];
+        }
+        if (r2 >= lim * lim) continue;
+        key.emplace_back(r2, (int)key.size());
+        x.insert(x.end(), v, v + 3);
+      }
+  std::sort(key.begin(), key.end());
+  for (const auto& q : key) o.img.insert(o.img.end(), x.begin() + 3 * q.second, x.begin() + 3 * q.second + 3);
+  for (int nx = 0; nx <= ni[0]; nx++)
+    for (int ny = -ni[1]; ny <= ni[1]; ny++)
+      for (int nz = -ni[2]; nz <= ni[2]; nz++) {
+        if (nx == 0 && (ny < 0 || (ny == 0 && nz <= 0))) continue;
+        double k[3], k2 = 0.0;
+        for (int j = 0; j < 3; j++) {
+          k[j] = 2.0 * RSD_PI * (nx * L.LI[3 * j] + ny * L.LI[1 + 3 * j] + nz * L.LI[2 + 3 * j]);
+          k2 += k[j] * k[j];
+        }
+        if (k2 < kmax * kmax) o.kv.insert(o.kv.end(), k, k + 3);
+      }
+  return o;
+}
+
+// The reference's cubes, whole.
+ewald_lists ewald_cube_lists(const rsd_lat_dev& L) {
+  ewald_lists o;
+  o.rc2 = INFINITY;
+  for (int nx = -L.NR; nx <= L.NR; nx++)
+    for (int ny = -L.NR; ny <= L.NR; ny++)
+      for (int nz = -L.NR; nz <= L.NR; nz++)
+        for (int j = 0; j < 3; j++) o.img.push_back(L.LR[j] * nx + L.LR[3 + j] * ny + L.LR[6 + j] * nz);
+  const int w = 2 * L.NI + 1, Kh = (w * w * w - 1) / 2;
+  for (int h = 0; h < Kh; h++) {
+    int nx, ny, nz;
+    half_space_index(h, L.NI, &nx, &ny, &nz);
+    for (int j = 0; j < 3; j++)
+      o.kv.push_back(2.0 * RSD_PI * (nx * L.LI[3 * j] + ny * L.LI[1 + 3 * j] + nz * L.LI[2 + 3 * j]));
+  }
+  return o;
+}
+
+// Whether the reference's cubes reach as far as FP64 shows: the nearest image
+// they leave out is at lambda r >= 6, the first vector at k^2 / (4 lambda^2)
+// >= 40 (terms below ~1e-13 of a block).  True for EWS_ERR up to 1e-9 or so
+// in a cell of any skew; a looser EWS_ERR cuts the sum where it shows, and
+// its result is then the reference's cut sum.
+bool cubes_converged(const rsd_lat_dev& L) {
+  for (int i = 0; i < 3; i++) {
+    double a2 = 0.0, b2 = 0.0;
+    for (int j = 0; j < 3; j++) {
+      a2 += L.LR[j + 3 * i] * L.LR[j + 3 * i];
+      b2 += L.LI[i + 3 * j] * L.LI[i + 3 * j];
+    }
+    const double k = 2.0 * RSD_PI * (L.NI + 1) / sqrt(a2);
+    if (L.lam * (L.NR + 0.5) < 6.0 * sqrt(b2) || k * k < 40.0 * 4.0 * L.lam * L.lam) return false;
+  }
+  return true;
+}
+
+struct ewald_dev_lists {
+  int nimg = 0, Kh = 0;
+  float rc2 = 0.f;
+  const double *img = nullptr, *kv = nullptr, *coef = nullptr;
+  const float4* imgf = nullptr;
+  const unsigned short* etab = nullptr;  // rsd_real_epi_off (61), rsd_real_epi_mom
+};
+
+// One copy brings the lists and, for equal radii, the coefficients of the
+// real-space epilogue to the device.
+int upload_lists(rsd_ctx* ctx, const ewald_lists& H, bool equal, double a, const rsd_lat_dev& L, double inv_pimu,
+                 ewald_dev_lists* D) {
+  const size_t ni = H.img.size() / 3, nk = H.kv.size() / 3;
+  const size_t nt = 5 * ni + 3 * nk + RSD_REAL_EPI_NC;  // float4 = two doubles
+  const size_t nd = nt + (61 + RSD_REAL_EPI_NC + 3) / 4;
+  std::vector<double> h(nd, 0.0);
+  float* f = reinterpret_cast<float*>(h.data());
+  for (size_t i = 0; i < ni; i++)
+    for (int j = 0; j < 3; j++) f[4 * i + j] = (float)H.img[3 * i + j];
+  std::copy(H.img.begin(), H.img.end(), h.begin() + 2 * ni);
+  std::copy(H.kv.begin(), H.kv.end(), h.begin() + 5 * ni);
+  if (equal) {
+    const double s1 = inv_pimu / (6.0 * a);
+    rsd_real_epi_coef_scaled<double>(a, a, L.phix, s1, s1 / (a * a), h.data() + 5 * ni + 3 * nk);
+    unsigned short* e = reinterpret_cast<unsigned short*>(h.data() + nt);
+    for (int q = 0; q < 61; q++) e[q] = (unsigned short)rsd_real_epi_off(q);
+    for (int k = 0; k < RSD_REAL_EPI_NC; k++) e[61 + k] = (unsigned short)rsd_real_epi_mom(k);
+  }
+  double* d = (double*)rsd_scratch(ctx, "ewald_lists", sizeof(double) * nd);
+  if (!d) return RSD_ENOMEM;
+  RSD_CUDA(ctx, cudaMemcpyAsync(d, h.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, ctx->stream));
+  D->nimg = (int)ni;
+  D->Kh = (int)nk;
+  D->rc2 = (float)H.rc2;
+  D->imgf = reinterpret_cast<const float4*>(d);
+  D->img = d + 2 * ni;
+  D->kv = d + 5 * ni;
+  D->coef = d + 5 * ni + 3 * nk;
+  D->etab = reinterpret_cast<const unsigned short*>(d + nt);
+  return RSD_OK;
+}
+
+// The weights of D's vectors and the diagonal blocks.
+template <typename S>
+int assemble_self(rsd_ctx* ctx, int nn, const double* d_radii, double a0, bool equal, const rsd_lat_dev& L,
+                  double inv_pimu, const ewald_dev_lists& D, const S& sk) {
+  cudaStream_t s = ctx->stream;
+  double* W = (double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
+  double* self = (double*)rsd_scratch(ctx, "ewald_self_sums", sizeof(double) * SELF_NMOM);
+  if (!W || !self) return RSD_ENOMEM;
+  const dim3 wg((unsigned)((D.Kh + 31) / 32), 2);
+  if (equal) {
+    ewald_weights<true><<<wg, 32, 0, s>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    ewald_self_sums<true><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
+                                                     D.etab, self); RSD_LAUNCH_NOTE();
+    ewald_self_eq<<<(121 * nn + 255) / 256, 256, 0, s>>>(nn, self, sk); RSD_LAUNCH_NOTE();
+  } else {
+    ewald_weights<false><<<wg, 32, 0, s>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    ewald_self_sums<false><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
+                                                      D.etab, self); RSD_LAUNCH_NOTE();
+    ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, self, d_radii, inv_pimu, sk); RSD_LAUNCH_NOTE();
+  }
+  RSD_CUDA(ctx, cudaGetLastError());
+  return RSD_OK;
+}
+
+// FP64 form.  Lanes per pair, counted by what the exchanges cost: 8 keep the lanes' shares of ~77 images even and
+// the exchanges at 87 additions per pair; below P64_WIDE pairs (N = 128)
+// there are fewer groups of 8 than the FP64 pipes want warps, and 32 lanes
+// take a pair.
+constexpr int64_t P64_WIDE = 8192;
+int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, double a0, bool equal,
+                  rsd_lat_dev L, double inv_pimu, const DenseSink& sk) {
+  cudaStream_t s = ctx->stream;
+  const bool cube = !cubes_converged(L);
+  if (!cube) L.lam *= EWALD64_SCALE;
+  ewald_dev_lists D;
+  RSD_TRY(upload_lists(ctx, cube ? ewald_cube_lists(L) : ewald_sphere_lists(L, L.lam, false), equal, a0, L, inv_pimu,
+                       &D));
+  RSD_TRY(assemble_self(ctx, nn, d_radii, a0, equal, L, inv_pimu, D, sk));
+  if (nn < 2) return RSD_OK;
+  double2* cs = (double2*)rsd_scratch(ctx, "ewald_trig", sizeof(double2) * (size_t)D.Kh * nn);
+  const double* W = (const double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
+  if (!cs || !W) return RSD_ENOMEM;
+  ewald_trig<<<(unsigned)(((int64_t)nn * D.Kh + 127) / 128), 128, 0, s>>>(nn, D.Kh, D.kv, d_pos, cs); RSD_LAUNCH_NOTE();
+  const int64_t npair = (int64_t)nn * (nn - 1) / 2;
+  auto go = [&](auto lanes, auto eq) {
+    constexpr int G = decltype(lanes)::value;
+    constexpr int PP = P64_THREADS / G;
+    ewald_pair64<G, decltype(eq)::value><<<(unsigned)((npair + PP - 1) / PP), P64_THREADS, 0, s>>>(
+        nn, npair, L, cube, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, cs, d_pos, d_radii, inv_pimu, D.coef, D.etab, sk);
+    RSD_LAUNCH_NOTE();
+  };
+  using wide = std::integral_constant<int, 32>;
+  using narrow = std::integral_constant<int, 8>;
+  if (npair < P64_WIDE) {
+    equal ? go(wide{}, std::true_type{}) : go(wide{}, std::false_type{});
+  } else {
+    equal ? go(narrow{}, std::true_type{}) : go(narrow{}, std::false_type{});
+  }
+  RSD_CUDA(ctx, cudaGetLastError());
+  return RSD_OK;
+}
+}  // namespace
+
 int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
-                       double mu_f, int precision, double* d_M, int64_t ldm) {
+                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm) {
   if (nn < 1 || ldm < 11LL * nn) return rsd_fail(ctx, RSD_EARG, "bad size nn=%d ldm=%lld", nn, (long long)ldm);
   rsd_lat_dev L = rsd_lat_pack(lat);
   if (precision == RSD_PREC_MIXED) L = mixed_lattice(ctx, L);
   if (L.NR > 40 || L.NI > 40) return rsd_fail(ctx, RSD_EARG, "image cubes too large (NR=%d NI=%d)", L.NR, L.NI);
-  const int w = 2 * L.NI + 1;
-  const int Kh = (w * w * w - 1) / 2;
-  double* tab = (double*)rsd_scratch(ctx, "ewald_ktab", sizeof(double) * (size_t)Kh * KW);
-  if (!tab) return RSD_ENOMEM;
-  // FP64 cos/sin per (vector, particle): the FP64 form only (the mixed form
-  // keeps its own FP32 and float-pair lists)
-  double2* cs = nullptr;
-  if (precision != RSD_PREC_MIXED) {
-    cs = (double2*)rsd_scratch(ctx, "ewald_trig", sizeof(double2) * (size_t)Kh * nn);
-    if (!cs) return RSD_ENOMEM;
-  }
   const double inv_pimu = 1.0 / (RSD_PI * mu_f);
   cudaStream_t s = ctx->stream;
-  ewald_ktable<<<(Kh + 127) / 128, 128, 0, s>>>(L, Kh, tab); RSD_LAUNCH_NOTE();
-  if (precision != RSD_PREC_MIXED) {
-    ewald_trig<<<dim3((nn + 127) / 128, Kh), 128, 0, s>>>(nn, Kh, tab, d_pos, cs); RSD_LAUNCH_NOTE();
-  }
-  double* mom = (double*)rsd_scratch(ctx, "ewald_self_mom", sizeof(double) * SELF_NMOM);
-  if (!mom) return RSD_ENOMEM;
-  ewald_self_moments<<<1, SELF_THREADS, 0, s>>>(L, Kh, tab, mom); RSD_LAUNCH_NOTE();
-  // mixed form: M as FP32 planes hi + lo (PlaneSink), in the buffer of the FP64 matrix
-  const DenseSink dsk{d_M, ldm};
+  bool equal = true;
+  for (int i = 1; i < nn && equal; i++) equal = h_radii[i] == h_radii[0];
+  if (precision != RSD_PREC_MIXED)
+    return assemble_fp64(ctx, nn, d_pos, d_radii, h_radii[0], equal, L, inv_pimu, DenseSink{d_M, ldm});
+  // M as FP32 planes hi + lo (PlaneSink), in the buffer of the FP64 matrix
   const PlaneSink psk{reinterpret_cast<float*>(d_M), reinterpret_cast<float*>(d_M) + (size_t)ldm * (11LL * nn), ldm};
-  if (precision == RSD_PREC_MIXED) {
-    ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, mom, d_radii, inv_pimu, psk); RSD_LAUNCH_NOTE();
-  } else {
-    ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, mom, d_radii, inv_pimu, dsk); RSD_LAUNCH_NOTE();
-  }
+  const ewald_lists SL = ewald_sphere_lists(L, L.lam, /*self_only=*/true);
+  ewald_dev_lists D;
+  RSD_TRY(upload_lists(ctx, SL, equal, h_radii[0], L, inv_pimu, &D));
+  RSD_TRY(assemble_self(ctx, nn, d_radii, h_radii[0], equal, L, inv_pimu, D, psk));
   if (nn > 1) {
     dim3 blk(32, 4), grd((nn + 31) / 32, (nn + 3) / 4);
-    if (precision == RSD_PREC_MIXED) {
+    {
       // Double-single: real images with lambda r < mixed_rcut (default 4.5)
       // and reciprocal vectors with k^2/(4 lambda^2) <= 3 pi mixed_kshell^2
       // (default 1); FP32 for the rest.  The FP32 error of a block follows
@@ -1407,6 +1842,7 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       // max|n_i| <= 1); FP32 for the others below the truncation
       const double k2ds = 4.0 * L.lam * L.lam * 3.0 * RSD_PI * ks * ks;
       const double k2max = 4.0 * L.lam * L.lam * ctx->mixed_kexp;
+      const int w = 2 * L.NI + 1, Kh = (w * w * w - 1) / 2;
       std::vector<int> h64, h32;
       for (int h = 0; h < Kh; h++) {
         int nx, ny, nz;
@@ -1432,11 +1868,6 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       all.insert(all.end(), h32.begin(), h32.end());
       RSD_CUDA(ctx, cudaMemcpyAsync(dh, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, s));
       RSD_CUDA(ctx, cudaStreamSynchronize(s));
-      // equal radii: per-vector block weights (ewald_pair_kblock)
-      std::vector<double> hr((size_t)nn);
-      RSD_CUDA(ctx, cudaMemcpy(hr.data(), d_radii, sizeof(double) * nn, cudaMemcpyDeviceToHost));
-      bool equal = true;
-      for (int i = 1; i < nn && equal; i++) equal = hr[i] == hr[0];
       if (K64) {
         ewald_trig_list<float4><<<dim3((nn + 127) / 128, K64), 128, 0, s>>>(nn, L, dh, d_pos, c64); RSD_LAUNCH_NOTE();
       }
@@ -1448,10 +1879,10 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         float* w32 = (float*)rsd_scratch(ctx, "ewald_kblock32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KBW);
         if (!w64 || !w32) return RSD_ENOMEM;
         if (K64) {
-          ewald_kblock_list<dsf><<<(K64 + 127) / 128, 128, 0, s>>>(L, K64, dh, hr[0], inv_pimu, w64); RSD_LAUNCH_NOTE();
+          ewald_kblock_list<dsf><<<(K64 + 127) / 128, 128, 0, s>>>(L, K64, dh, h_radii[0], inv_pimu, w64); RSD_LAUNCH_NOTE();
         }
         if (K32) {
-          ewald_kblock_list<float><<<(K32 + 127) / 128, 128, 0, s>>>(L, K32, dh + K64, hr[0], inv_pimu, w32); RSD_LAUNCH_NOTE();
+          ewald_kblock_list<float><<<(K32 + 127) / 128, 128, 0, s>>>(L, K32, dh + K64, h_radii[0], inv_pimu, w32); RSD_LAUNCH_NOTE();
         }
         ewald_pair_kblock<<<grd, blk, 0, s>>>(nn, K32, w32, c32, K64, w64, c64, psk, 0); RSD_LAUNCH_NOTE();
       } else {
@@ -1468,15 +1899,12 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         dsf* cr = (dsf*)rsd_scratch(ctx, "ewald_real_cr", sizeof(dsf) * RSD_REAL_EPI_NC);
         float* cf = (float*)rsd_scratch(ctx, "ewald_real_cf", sizeof(float) * RSD_REAL_EPI_NC);
         if (!cr || !cf) return RSD_ENOMEM;
-        ewald_real_epi_table<<<1, 32, 0, s>>>(hr[0], L.phix, inv_pimu, cr, cf); RSD_LAUNCH_NOTE();
+        ewald_real_epi_table<<<1, 32, 0, s>>>(h_radii[0], L.phix, inv_pimu, cr, cf); RSD_LAUNCH_NOTE();
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
         ewald_pair_real_near_ds<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, rc2, psk); RSD_LAUNCH_NOTE();
         ewald_pair_real_far<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, rc2, rmax2, psk); RSD_LAUNCH_NOTE();
       }
-    } else {
-      ewald_pair_k<double, double2><<<grd, blk, 0, s>>>(nn, L, Kh, tab, cs, d_radii, inv_pimu, dsk, 0); RSD_LAUNCH_NOTE();
-      ewald_pair_real<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, dsk); RSD_LAUNCH_NOTE();
     }
   }
   RSD_CUDA(ctx, cudaGetLastError());

@@ -501,6 +501,18 @@ def gen():
         L.append("  out[%d] = fma(c[%d], acc[%d], out[%d]);" % (q, kk, m, q))
     L.append("}")
     L.append("")
+    L.append("// The table's shape, for kernels that spread the outputs of a pair over lanes:")
+    L.append("// output q sums entries rsd_real_epi_off(q) .. rsd_real_epi_off(q + 1) - 1, entry k")
+    L.append("// reads moment rsd_real_epi_mom(k).")
+    offs, mts = [0], [m for _, m in keys]
+    for q in range(60):
+        offs.append(offs[-1] + len(byq.get(q, [])))
+    for nm, arg, vals in (("off", "q", offs), ("mom", "k", mts)):
+        L.append("__host__ __device__ inline int rsd_real_epi_%s(int %s) {" % (nm, arg))
+        L.append("  constexpr unsigned short t[%d] = {%s};" % (len(vals), ", ".join(str(v) for v in vals)))
+        L.append("  return t[%s];" % arg)
+        L.append("}")
+    L.append("")
     # ---- reciprocal-space weights: w[m] = S k^alpha for each moment
     for tag, mom, dec in (("kcos", mom_c, dec_c), ("ksin", mom_s, dec_s)):
         L.append("// Per-k weights of the %s moments: w[m] = g_m(S, lam) * k^alpha." % tag)

@@ -170,8 +170,9 @@ __host__ __device__ inline void rsd_skew_shift_f32(const float* LR, const float*
 // (float*)d_M and lo at (float*)d_M + ldm * 11 nn, both with ld ldm, and
 // only the entries whose row's particle is at most the column's are written
 // (M is symmetric); rsd_mirror_planes fills the others.
+// h_radii: the radii on the host.
 int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
-                       double mu_f, int precision, double* d_M, int64_t ldm);
+                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm);
 int rsd_mirror_planes(rsd_ctx* ctx, int nn, double* d_M, int64_t ldm);
 int rsd_count_overlaps(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
                        int* count);

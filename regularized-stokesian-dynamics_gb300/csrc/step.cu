@@ -238,7 +238,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   {
     // grand mobility
     rsd_range r("rsd_assembly");
-    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, M, n));
+    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, radii.data(), M, n));
     if (ctx->correction_method) {  // overlap corrections (per_GRPY_YZD.f90:98-116)
       int nov = 0;
       RSD_TRY(rsd_count_overlaps(ctx, nn, d_conf, d_radii, &lat, &nov));
