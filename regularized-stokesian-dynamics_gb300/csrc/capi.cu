@@ -11,6 +11,10 @@
 
 #include "rsd_internal.cuh"
 
+template <typename T>
+int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t lda, const T* X, int64_t ldx,
+             int nrhs, T beta, T* y, int64_t ldy);
+
 std::atomic<long long> rsd_launches{0};
 extern "C" long long rsd_launch_count(void) { return rsd_launches.load(); }
 
@@ -563,8 +567,8 @@ int dmdx_dev(rsd_ctx* ctx, int32_t nn, const double* conf, const double* radii, 
   if (!M1 || !M2) return RSD_ENOMEM;
   RSD_TRY(rsd_per_grpery_inv_fri_dev(ctx, nn, d1, dr, lat, ews_err, mu_f, correction_method, M1, n));
   RSD_TRY(rsd_per_grpery_inv_fri_dev(ctx, nn, d2, dr, lat, ews_err, mu_f, correction_method, M2, n));
-  rsd_gemm_f64(ctx->stream, (int)t, 1, (int)t, 1.0 / DMDX_DETA, M1, n, 0, dz, t, 0, 0.0, d_out, t);
-  rsd_gemm_f64(ctx->stream, (int)t, 1, (int)t, -1.0 / DMDX_DETA, M2, n, 0, dz, t, 0, 1.0, d_out, t);
+  RSD_TRY(rsd_gemv<double>(ctx, 0, (int)t, (int)t, 1.0 / DMDX_DETA, M1, n, dz, t, 1, 0.0, d_out, t));
+  RSD_TRY(rsd_gemv<double>(ctx, 0, (int)t, (int)t, -1.0 / DMDX_DETA, M2, n, dz, t, 1, 1.0, d_out, t));
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -610,7 +614,7 @@ extern "C" int rsd_brownian_velocity(rsd_ctx* ctx, int32_t nn, const double* APP
   double* vb = (double*)rsd_scratch(ctx, "brown_vb", sizeof(double) * 2 * (size_t)t);
   if (!vb) return RSD_ENOMEM;
   // VB = sqrt(2 kBT) L Z / DT (stepper.f90:79)
-  rsd_gemm_f64(ctx->stream, (int)t, 1, (int)t, std::sqrt(2.0 * kBT) / dt, dA, t, 1, dz, t, 0, 0.0, vb, t);
+  RSD_TRY(rsd_gemv<double>(ctx, 1, (int)t, (int)t, std::sqrt(2.0 * kBT) / dt, dA, t, dz, t, 1, 0.0, vb, t));
   RSD_CUDA(ctx, cudaGetLastError());
   RSD_TRY(dmdx_dev(ctx, nn, conf, radii, lat, ews_err, mu_f, correction_method, Z, vb + t));
   std::vector<double> h(2 * (size_t)t);
@@ -692,72 +696,60 @@ static int nogmres_impl(rsd_ctx* ctx, int32_t nn, const double* APP, const doubl
   const int64_t n = 11LL * nn, p = 6LL * nn, q = 5LL * nn;
   double* M = (double*)rsd_scratch(ctx, "M", sizeof(double) * n * n);
   double* Lb = (double*)rsd_scratch(ctx, "L", sizeof(double) * n * n);
-  double* V = (double*)rsd_scratch(ctx, "nog_vec", sizeof(double) * (3 * p + 2 * q + 8 * p));
-  if (!M || !Lb || !V) return RSD_ENOMEM;
-  // MobToResist_FTS
+  double* RP = (double*)rsd_scratch(ctx, "nog_RPP", sizeof(double) * p * p);
+  double* V = (double*)rsd_scratch(ctx, "nog_vec", sizeof(double) * (8 * p + 4 * q));
+  if (!M || !Lb || !RP || !V) return RSD_ENOMEM;
+  // MobToResist_FTS, through the Schur complement (resist64.cu)
   RSD_TRY(put_block(ctx, M, n, APP, p, p));
   RSD_TRY(put_block(ctx, M + p * n, n, APQ, p, q));
   RSD_TRY(put_block(ctx, M + p + p * n, n, AQQ, q, q));
-  int inf_m = 0;
-  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)n, M, n, &inf_m, "mob"));
-  if (inf_m) {
-    *info = inf_m;
+  rsd_r64 h;
+  int inf = 0;
+  RSD_TRY(rsd_r64_factor(ctx, nn, M, n, &h, &inf));
+  if (inf) {
+    *info = inf;
     return RSD_OK;
   }
-  RSD_TRY(rsd_potri_upper_tag(ctx, (int)n, M, n, "mob"));
-  RSD_TRY(rsd_mirror_upper(ctx, (int)n, M, n));
-  // arrangResist: R = R0 + [rfu rfe; . rse] on the blocks used below
-  RSD_TRY(put_block(ctx, Lb, n, rfu, p, p));
-  RSD_TRY(put_block(ctx, Lb + p * n, n, rfe, p, q));
-  RSD_TRY(put_block(ctx, Lb + p + p * n, n, rse, q, q));
-  // R += L on the P-P, P-Q and Q-Q blocks
-  {
-    RSD_TRY(rsd_axpy_block(ctx, p, p, Lb, n, M, n));
-    RSD_TRY(rsd_axpy_block(ctx, p, q, Lb + p * n, n, M + p * n, n));
-    RSD_TRY(rsd_axpy_block(ctx, q, q, Lb + p + p * n, n, M + p + p * n, n));
-  }
-  // RHS: [Fe + RPQ EIN, RPQ EIN, Fe_inter]
-  double* X = V;                  // p x 3
-  double* ein = V + 3 * p;        // q
-  double* UB = V + 3 * p + q;     // p
-  double* tmp = V + 4 * p + q;    // 3 q
+  // arrangResist: R = R0 + [rfu rfe; . rse]; RPP formed, the rest applied
+  double *drfu = Lb, *drfe = Lb + p * p, *drse = drfe + p * q;
+  RSD_CUDA(ctx, cudaMemcpyAsync(drfu, rfu, sizeof(double) * p * p, cudaMemcpyHostToDevice, s));
+  RSD_CUDA(ctx, cudaMemcpyAsync(drfe, rfe, sizeof(double) * p * q, cudaMemcpyHostToDevice, s));
+  RSD_CUDA(ctx, cudaMemcpyAsync(drse, rse, sizeof(double) * q * q, cudaMemcpyHostToDevice, s));
+  RSD_CUDA(ctx, cudaMemcpyAsync(RP, h.Ai, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, s));
+  RSD_TRY(rsd_axpy_block(ctx, p, p, drfu, p, RP, p));
+  // right-hand sides [Fe + RPQ EIN, RPQ EIN, Fe_inter] in X; Y = [X2, X3, UB]
+  double *X = V, *Y = V + 3 * p, *f0 = V + 6 * p, *ein = V + 7 * p, *S = ein + q;
   RSD_CUDA(ctx, cudaMemcpyAsync(ein, EIN, sizeof(double) * q, cudaMemcpyHostToDevice, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(X, Fe, sizeof(double) * p, cudaMemcpyHostToDevice, s));
-  RSD_CUDA(ctx, cudaMemsetAsync(X + p, 0, sizeof(double) * p, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(X + 2 * p, Fe_inter, sizeof(double) * p, cudaMemcpyHostToDevice, s));
-  RSD_CUDA(ctx, cudaMemsetAsync(UB, 0, sizeof(double) * p, s));
-  if (u_brown) RSD_CUDA(ctx, cudaMemcpyAsync(UB, u_brown, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, s));
-  const double* RPQd = M + p * n;
-  rsd_gemm_f64(s, (int)p, 1, (int)q, 1.0, RPQd, n, 0, ein, q, 0, 1.0, X, p);
-  rsd_gemm_f64(s, (int)p, 1, (int)q, 1.0, RPQd, n, 0, ein, q, 0, 0.0, X + p, p);
-  // RPP (factor and inverse on a copy so RPQ/RQQ stay intact)
-  double* P = (double*)rsd_scratch(ctx, "nog_RPP", sizeof(double) * p * p);
-  if (!P) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemcpy2DAsync(P, p * sizeof(double), M, n * sizeof(double), p * sizeof(double), p,
-                                  cudaMemcpyDeviceToDevice, s));
+  RSD_TRY(rsd_r64_pq(ctx, &h, ein, f0));
+  RSD_CUDA(ctx, cudaMemcpyAsync(X + p, f0, sizeof(double) * p, cudaMemcpyDeviceToDevice, s));
+  RSD_TRY(rsd_gemv<double>(ctx, 0, (int)p, (int)q, 1.0, drfe, p, ein, q, 1, 1.0, X + p, p));
+  RSD_TRY(rsd_axpy_block(ctx, p, 1, X + p, p, X, p));
+  // RPP factored in place
   int inf_r = 0;
-  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)p, P, p, &inf_r, "rpp"));
+  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)p, RP, p, &inf_r, "rpp"));
   if (inf_r) {
     *info = inf_r;
     return RSD_OK;
   }
-  RSD_TRY(rsd_potrs_upper_tag(ctx, (int)p, P, p, X, p, 3, "rpp"));
-  // S_hyd = RPQ^T X1 - RQQ EIN ; S_FP(part) = RPQ^T X2 ; S_B = RPQ^T UB
-  double* S = tmp;  // 3 q
-  rsd_gemm_f64(s, (int)q, 1, (int)p, 1.0, RPQd, n, 1, X + p, p, 0, 0.0, S, q);
-  rsd_gemm_f64(s, (int)q, 1, (int)q, -1.0, M + p + p * n, n, 0, ein, q, 0, 1.0, S, q);
-  rsd_gemm_f64(s, (int)q, 1, (int)p, 1.0, RPQd, n, 1, X + 2 * p, p, 0, 0.0, S + q, q);
-  rsd_gemm_f64(s, (int)q, 1, (int)p, 1.0, RPQd, n, 1, UB, p, 0, 0.0, S + 2 * q, q);
-  RSD_CUDA(ctx, cudaGetLastError());
+  RSD_TRY(rsd_potrs_upper_tag(ctx, (int)p, RP, p, X, p, 3, "rpp"));
+  // S_hyd = RPQ^T X2 - RQQ EIN ; S_FP(part) = RPQ^T X3 ; S_B = RPQ^T UB
+  RSD_CUDA(ctx, cudaMemcpyAsync(Y, X + p, sizeof(double) * 2 * p, cudaMemcpyDeviceToDevice, s));
+  RSD_CUDA(ctx, cudaMemsetAsync(Y + 2 * p, 0, sizeof(double) * p, s));
+  if (u_brown) RSD_CUDA(ctx, cudaMemcpyAsync(Y + 2 * p, u_brown, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, s));
+  RSD_TRY(rsd_r64_stresslet(ctx, &h, Y, 3, f0, S));
+  RSD_TRY(rsd_gemv<double>(ctx, 1, (int)q, (int)p, 1.0, drfe, p, Y, p, 3, 1.0, S, q));
+  RSD_TRY(rsd_gemv<double>(ctx, 1, (int)q, (int)q, -1.0, drse, q, ein, q, 1, 1.0, S, q));
   RSD_CUDA(ctx, cudaMemcpyAsync(U_par, X, sizeof(double) * p, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(SijN_hyd, S, sizeof(double) * q, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(SijN_FP, S + q, sizeof(double) * q, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(SijN_B, S + 2 * q, sizeof(double) * q, cudaMemcpyDeviceToHost, s));
   // Rheology leaves RPP inverted
   if (RPP) {
-    RSD_TRY(rsd_potri_upper_tag(ctx, (int)p, P, p, "rpp"));
-    RSD_TRY(rsd_mirror_upper(ctx, (int)p, P, p));
-    RSD_CUDA(ctx, cudaMemcpyAsync(RPP, P, sizeof(double) * p * p, cudaMemcpyDeviceToHost, s));
+    RSD_TRY(rsd_potri_upper_tag(ctx, (int)p, RP, p, "rpp"));
+    RSD_TRY(rsd_mirror_upper(ctx, (int)p, RP, p));
+    RSD_CUDA(ctx, cudaMemcpyAsync(RPP, RP, sizeof(double) * p * p, cudaMemcpyDeviceToHost, s));
   }
   RSD_TRY(sync(ctx));
   // stresslet dipole of the interparticle forces (Rheology 425-444)

@@ -1,8 +1,7 @@
 // Kernel 3: dense SPD factorisation, inverse and solves for the grand
 // resistance (MATREV, src/matrices.f90:4-34, which calls LAPACK DPOTRF('U')
-// and DPOTRI('U') and mirrors the upper triangle).  Column-major throughout,
-// templated on the element type: FP64 for the plain form, FP32 for the
-// factorisations of the mixed form.
+// and DPOTRI('U') and mirrors the upper triangle), FP32 for the mixed form
+// (the FP64 factorisations are in dense64.cu).  Column-major throughout.
 //
 //   potrf_upper   blocked right-looking Cholesky A = U^T U: per block column
 //                 one CTA factors the nb x nb diagonal block in shared memory
@@ -16,7 +15,7 @@
 //                 block substitution (diagonal blocks by their inverses, the
 //                 updates as wide GEMVs).
 //   gemv          y = alpha op(A) X + beta y for 1..4 columns, split over k
-//                 with a fixed-order second pass (deterministic).
+//                 with a fixed-order second pass (deterministic); FP32, FP64.
 #include <cuda_runtime.h>
 
 #include <string>
@@ -368,54 +367,6 @@ GemmP gp(int m, int n, int k, double alpha, const void* A, int64_t lda, int ta, 
 }
 
 constexpr int NB = 128;  // block size of the blocked factorisations
-
-// One CTA: Cholesky (upper) of the jb x jb diagonal block in shared memory.
-// The trailing update of each column step is spread over a 16 x 16 thread
-// grid.  info: first failing global index + 1 (DPOTRF's INFO).
-template <typename T>
-__global__ void __launch_bounds__(256) potf2_upper(T* __restrict__ A, int64_t lda, int jb, int* __restrict__ info,
-                                                   int j0) {
-  extern __shared__ unsigned char smraw[];
-  T* S = (T*)smraw;  // jb x jb, column-major, ld = jb
-  T* rowk = S + jb * jb;  // scaled pivot row, read without bank conflicts
-  __shared__ int failed;
-  const int t = threadIdx.x, tx = t % 16, ty = t / 16;
-  for (int e = t; e < jb * jb; e += blockDim.x) {
-    const int i = e % jb, j = e / jb;
-    S[e] = (i <= j) ? A[i + (int64_t)j * lda] : T(0);
-  }
-  if (t == 0) failed = 0;
-  __syncthreads();
-  for (int k = 0; k < jb; k++) {
-    if (t == 0) {
-      const T d = S[k + k * jb];
-      if (!(d > T(0)) || !isfinite(d)) {
-        failed = 1;
-        atomicCAS(info, 0, j0 + k + 1);
-      } else {
-        S[k + k * jb] = sqrt(d);
-      }
-    }
-    __syncthreads();
-    if (failed) break;
-    const T rk = T(1) / S[k + k * jb];
-    for (int j = k + 1 + t; j < jb; j += blockDim.x) {
-      const T v = S[k + j * jb] * rk;
-      S[k + j * jb] = v;
-      rowk[j] = v;
-    }
-    __syncthreads();
-    for (int j = k + 1 + ty; j < jb; j += 16) {
-      const T skj = rowk[j];
-      for (int i = k + 1 + tx; i <= j; i += 16) S[i + j * jb] -= rowk[i] * skj;
-    }
-    __syncthreads();
-  }
-  for (int e = t; e < jb * jb; e += blockDim.x) {
-    const int i = e % jb, j = e / jb;
-    if (i <= j) A[i + (int64_t)j * lda] = S[e];
-  }
-}
 
 // FP32 diagonal block (jb <= 128): upper Cholesky factor U and its inverse
 // W = U^-1 in one CTA of 8 warps.  Right-looking over 32-wide sub-blocks D:
@@ -787,38 +738,6 @@ __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int6
   }
 }
 
-// Panel solve U_jj^T X = B in place (B = A(j0:j0+jb, j0+jb:n)): the factor
-// block and 64 columns of B in shared memory, one thread per column
-// (forward substitution), coalesced loads and stores of the columns.
-constexpr int TRSM_COLS = 64;
-template <typename T>
-__global__ void __launch_bounds__(TRSM_COLS) trsm_panel(const T* __restrict__ Ujj, int64_t lda, int jb, int rest,
-                                                        T* __restrict__ B) {
-  extern __shared__ unsigned char smraw[];
-  T* S = (T*)smraw;        // jb x jb
-  T* Xs = S + jb * jb;     // row i, column c at Xs[i * TRSM_COLS + c]
-  const int t = threadIdx.x, c0 = blockIdx.x * TRSM_COLS;
-  for (int e = t; e < jb * jb; e += TRSM_COLS) {
-    const int i = e % jb, j = e / jb;
-    S[e] = (i <= j) ? Ujj[i + (int64_t)j * lda] : T(0);
-  }
-  for (int e = t; e < jb * TRSM_COLS; e += TRSM_COLS) {
-    const int i = e % jb, c = e / jb;
-    Xs[i * TRSM_COLS + c] = (c0 + c < rest) ? B[i + (int64_t)(c0 + c) * lda] : T(0);
-  }
-  __syncthreads();
-  for (int i = 0; i < jb; i++) {
-    T s = Xs[i * TRSM_COLS + t];
-    for (int p = 0; p < i; p++) s -= S[p + i * jb] * Xs[p * TRSM_COLS + t];
-    Xs[i * TRSM_COLS + t] = s / S[i + i * jb];
-  }
-  __syncthreads();
-  for (int e = t; e < jb * TRSM_COLS; e += TRSM_COLS) {
-    const int i = e % jb, c = e / jb;
-    if (c0 + c < rest) B[i + (int64_t)(c0 + c) * lda] = Xs[i * TRSM_COLS + c];
-  }
-}
-
 // Inverses of all diagonal blocks of an upper triangular U (one CTA each).
 template <typename T>
 __global__ void __launch_bounds__(256) trtri_diag(int n, const T* __restrict__ U, int64_t ldu, T* __restrict__ W) {
@@ -966,10 +885,6 @@ int smem_potf2(int jb) {
   return (jb * jb + jb) * (int)sizeof(T);
 }
 template <typename T>
-int smem_trsm() {
-  return (NB * NB + NB * TRSM_COLS) * (int)sizeof(T);
-}
-template <typename T>
 int smem_trsv() {
   return (NB * NB + NB * 4) * (int)sizeof(T);
 }
@@ -996,8 +911,6 @@ template <typename T>
 int ensure_attrs(rsd_ctx* ctx) {
   static bool done = false;
   if (done) return RSD_OK;
-  RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_upper<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_potf2<T>(NB)));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(trsm_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_trsm<T>()));
   RSD_CUDA(ctx, cudaFuncSetAttribute(trsv_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_trsv<T>()));
   RSD_CUDA(ctx, cudaFuncSetAttribute(trtri_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_potf2<T>(NB)));
   RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_inv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_POTF2_INV));
@@ -1268,7 +1181,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
       T* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       // panel j on the side stream, after the first tile row of step j-1's update
       RSD_CUDA(ctx, cudaStreamWaitEvent(s2, ctx->ev_next, 0));
-      if constexpr (F32) {
+      {
         // factor + inverse of the diagonal block, then the panel as W_jj^T B
         T* Wb = W + (size_t)b * NB * NB;
         potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, ctx->d_info, j0, Wb); RSD_LAUNCH_NOTE();
@@ -1276,11 +1189,6 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
           launch_gemm<T>(s2, gp(jb, rest, jb, 1.0, Wb, NB, 1, Apan, lda, 0, 0.0, T1, NB));
           RSD_CUDA(ctx, cudaMemcpy2DAsync(Apan, lda * sizeof(T), T1, NB * sizeof(T), jb * sizeof(T), rest,
                                           cudaMemcpyDeviceToDevice, s2));
-        }
-      } else {
-        potf2_upper<T><<<1, 256, smem_potf2<T>(jb), s2>>>(Ajj, lda, jb, ctx->d_info, j0); RSD_LAUNCH_NOTE();
-        if (rest > 0) {
-          trsm_panel<T><<<(rest + TRSM_COLS - 1) / TRSM_COLS, TRSM_COLS, smem_trsm<T>(), s2>>>(Ajj, lda, jb, rest, Apan); RSD_LAUNCH_NOTE();
         }
       }
       RSD_CUDA(ctx, cudaEventRecord(ctx->ev_panel, s2));
@@ -1296,12 +1204,6 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
                                      A22 + NB + (int64_t)NB * lda, lda, 1));
       }
     }
-  }
-  // diagonal-block inverses for the solves; the FP32 paths made them with
-  // their diagonal blocks, the FP64 one takes them here
-  if (!F32) {
-    const int nblk = (n + NB - 1) / NB;
-    trtri_diag<T><<<nblk, 256, smem_potf2<T>(NB), s>>>(n, d_A, lda, W); RSD_LAUNCH_NOTE();
   }
   RSD_CUDA(ctx, cudaGetLastError());
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1981,34 +1883,9 @@ void rsd_gemm_f64(cudaStream_t s, int m, int n, int k, double alpha, const doubl
                   const double* B, int64_t ldb, int tb, double beta, double* C, int64_t ldc) {
   launch_gemm<double>(s, gp(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc));
 }
-int rsd_zero_lower(rsd_ctx* ctx, int n, double* d_A, int64_t lda) { return rsd_zero_lower_t<double>(ctx, n, d_A, lda); }
 int rsd_mirror_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda) {
   return rsd_mirror_upper_t<double>(ctx, n, d_A, lda);
 }
-int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info, const char* tag) {
-  return rsd_potrf_upper_t<double>(ctx, n, d_A, lda, info, tag, 0);
-}
-int rsd_potrf_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info) {
-  return rsd_potrf_upper_t<double>(ctx, n, d_A, lda, info, "A", 0);
-}
-int rsd_potri_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const char* tag) {
-  return rsd_potri_upper_t<double>(ctx, n, d_A, lda, tag, 0);
-}
-int rsd_potri_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda) {
-  return rsd_potri_upper_t<double>(ctx, n, d_A, lda, "A", 0);
-}
-int rsd_potrs_upper_tag(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, double* d_X, int64_t ldx, int nrhs,
-                        const char* tag) {
-  // the factor's diagonal-block inverses are still in the tag's buffer
-  const double* W = diag_inverses<double>(ctx, n, tag);
-  return rsd_potrs_upper_t<double>(ctx, n, d_U, ldu, d_X, ldx, nrhs, tag, W);
-}
-int rsd_trsv_upper(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, double* d_X, int64_t ldx, int nrhs,
-                   int transpose) {
-  (void)transpose;
-  return rsd_potrs_upper_tag(ctx, n, d_U, ldu, d_X, ldx, nrhs, "A");
-}
-
 // ------------------------------------------------ FP32 exported blocks
 static int check_prec(rsd_ctx* ctx, int prec) {
   if (prec != 0 && prec != 1 && prec != 3) return rsd_fail(ctx, RSD_EARG, "prec must be 0, 1 or 3 (got %d)", prec);

@@ -391,27 +391,29 @@ __global__ void lub_spmv_w(int N, const int* __restrict__ off, const int* __rest
   if (lane < 11) y[gidx(N, u, r) + col * ldy] = vs + vp * scale;
 }
 
-// A (FP32, ld lda) += the force/torque-velocity part L_PP of the sparse
+// A (ld lda) += the force/torque-velocity part L_PP of the sparse
 // operator: pair blocks (each entry of A is touched by at most one pair or
 // self block, so no two threads add to the same entry)
+template <typename T>
 __global__ void lub_pp_pairs(int npair, int N, const int2* __restrict__ pairs, const double* __restrict__ blk,
-                             double scale, float* __restrict__ A, int64_t lda) {
+                             double scale, T* __restrict__ A, int64_t lda) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)npair * 36) return;
   const int p = (int)(t / 36), e = (int)(t % 36);
   const int r = e % 6, c = e / 6;
   const int a = pairs[p].x, b = pairs[p].y;
   const double* B = blk + (size_t)p * PB;
-  A[gidx(N, a, r) + gidx(N, b, c) * lda] += (float)(pair_entry(B, r, c, true) * scale);
-  A[gidx(N, b, r) + gidx(N, a, c) * lda] += (float)(pair_entry(B, r, c, false) * scale);
+  A[gidx(N, a, r) + gidx(N, b, c) * lda] += (T)(pair_entry(B, r, c, true) * scale);
+  A[gidx(N, b, r) + gidx(N, a, c) * lda] += (T)(pair_entry(B, r, c, false) * scale);
 }
 
-__global__ void lub_pp_self(int N, const double* __restrict__ self, float* __restrict__ A, int64_t lda) {
+template <typename T>
+__global__ void lub_pp_self(int N, const double* __restrict__ self, T* __restrict__ A, int64_t lda) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)N * 36) return;
   const int u = (int)(t / 36), e = (int)(t % 36);
   const int r = e % 6, c = e / 6;
-  A[gidx(N, u, r) + gidx(N, u, c) * lda] += (float)self[(size_t)u * 121 + r + 11 * c];
+  A[gidx(N, u, r) + gidx(N, u, c) * lda] += (T)self[(size_t)u * 121 + r + 11 * c];
 }
 
 __global__ void zero_matrix(int64_t rows, int64_t cols, double* __restrict__ A, int64_t ld) {
@@ -565,16 +567,23 @@ int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w
   return RSD_OK;
 }
 
-// A (6N x 6N FP32, ld lda) += L_PP
-int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t lda) {
+// A (6N x 6N, ld lda) += L_PP
+template <typename T>
+static int lub_add_pp(rsd_ctx* ctx, const rsd_lub_sparse* sp, T* A, int64_t lda) {
   cudaStream_t s = ctx->stream;
   if (sp->npair > 0) {
     const int64_t tp = 36LL * sp->npair;
-    lub_pp_pairs<<<(unsigned)((tp + 255) / 256), 256, 0, s>>>(sp->npair, sp->nn, sp->pairs, sp->blk, sp->scale, A,
-                                                              lda); RSD_LAUNCH_NOTE();
+    lub_pp_pairs<T><<<(unsigned)((tp + 255) / 256), 256, 0, s>>>(sp->npair, sp->nn, sp->pairs, sp->blk, sp->scale, A,
+                                                                 lda); RSD_LAUNCH_NOTE();
   }
   const int64_t ts = 36LL * sp->nn;
-  lub_pp_self<<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(sp->nn, sp->self, A, lda); RSD_LAUNCH_NOTE();
+  lub_pp_self<T><<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(sp->nn, sp->self, A, lda); RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
+}
+int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t lda) {
+  return lub_add_pp<float>(ctx, sp, A, lda);
+}
+int rsd_lub_add_pp_f64(rsd_ctx* ctx, const rsd_lub_sparse* sp, double* A, int64_t lda) {
+  return lub_add_pp<double>(ctx, sp, A, lda);
 }

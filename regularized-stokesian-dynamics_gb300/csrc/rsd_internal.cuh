@@ -203,13 +203,10 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, in
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy);
 int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t lda);
+int rsd_lub_add_pp_f64(rsd_ctx* ctx, const rsd_lub_sparse* sp, double* A, int64_t lda);
 // Dense linear algebra (dense.cu)
-int rsd_potrf_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info);
-int rsd_potri_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda);  // after potrf; result upper
 int rsd_mirror_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda);
-int rsd_trsv_upper(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, double* d_X, int64_t ldx, int nrhs,
-                   int transpose);
-// Tagged variants: the diagonal-block inverses of a factorisation are kept
+// FP64 factor, inverse from it and solves (dense64.cu): the diagonal-block inverses of a factorisation are kept
 // in a scratch buffer named by `tag`, so two factorisations can coexist.
 int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info, const char* tag);
 int rsd_potri_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const char* tag);
@@ -217,9 +214,24 @@ int rsd_potrs_upper_tag(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, dou
                         const char* tag);
 void rsd_gemm_f64(cudaStream_t s, int m, int n, int k, double alpha, const double* A, int64_t lda, int ta,
                   const double* B, int64_t ldb, int tb, double beta, double* C, int64_t ldc);
-int rsd_zero_lower(rsd_ctx* ctx, int n, double* d_A, int64_t lda);
-// A(rows x cols) += B, both column-major sub-blocks (step.cu)
-int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, int64_t ldb, double* A, int64_t lda);
+// FP64 grand resistance through the Schur complement (resist64.cu)
+struct rsd_factor64 {
+  double* W = nullptr;  // inverses of the 64-wide diagonal blocks
+  int* dexp = nullptr;  // half the exponents of the factored matrix's diagonal
+};
+struct rsd_r64 {
+  int64_t P = 0, Q = 0, Qp = 0, np = 0;
+  double* Mp = nullptr;  // U' in the upper triangle, np x np
+  double* Ai = nullptr;  // (M^-1)_PP, full
+  rsd_factor64 f;
+  double* z = nullptr;
+};
+int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int* info);
+int rsd_r64_pq(rsd_ctx* ctx, rsd_r64* h, const double* ein, double* f0);
+int rsd_r64_stresslet(rsd_ctx* ctx, rsd_r64* h, const double* Y, int nr, const double* f0, double* S);
+// A(rows x cols) += alpha B, both column-major sub-blocks (step.cu)
+int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, int64_t ldb, double* A, int64_t lda,
+                   double alpha = 1.0);
 
 // Tensor-core (tcgen05) GEMM on K-major FP32 operands (tc_gemm.cu):
 // C = alpha A^T B (store) or C += alpha A^T B (reduce) on 128-tiles, prec 1

@@ -13,12 +13,12 @@
 
 namespace {
 
-__global__ void axpy_block_k(int64_t rows, int64_t cols, const double* __restrict__ B, int64_t ldb,
+__global__ void axpy_block_k(int64_t rows, int64_t cols, double alpha, const double* __restrict__ B, int64_t ldb,
                              double* __restrict__ A, int64_t lda) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= rows * cols) return;
   const int64_t i = t % rows, j = t / rows;
-  A[i + j * lda] += B[i + j * ldb];
+  A[i + j * lda] += alpha * B[i + j * ldb];
 }
 
 __global__ void fill_ein(int nn, const double* __restrict__ ei5, double* __restrict__ ein) {
@@ -138,10 +138,11 @@ __global__ void nan_check(int64_t n, const double* __restrict__ v, int* __restri
 
 }  // namespace
 
-int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, int64_t ldb, double* A, int64_t lda) {
+int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, int64_t ldb, double* A, int64_t lda,
+                   double alpha) {
   const int64_t tot = rows * cols;
   if (tot <= 0) return RSD_OK;
-  axpy_block_k<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(rows, cols, B, ldb, A, lda); RSD_LAUNCH_NOTE();
+  axpy_block_k<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(rows, cols, alpha, B, ldb, A, lda); RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -255,33 +256,46 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   RSD_CUDA(ctx, cudaMemcpyAsync(hred.data(), red, 256 * sizeof(double), cudaMemcpyDeviceToHost, s));
   int info_m = 0;
   if (p->precision == RSD_PREC_FP64) {
-    // MobToResist_FTS: R_inf = M^-1
-    RSD_TRY(rsd_potrf_upper_tag(ctx, (int)n, M, n, &info_m, "mob"));
+    // MobToResist_FTS: R_inf = M^-1 through the Schur complement (resist64.cu)
+    rsd_r64 h;
+    RSD_TRY(rsd_r64_factor(ctx, nn, M, n, &h, &info_m));
     if (info_m) {
       loc.info = info_m;
       if (info) *info = loc;
       return info_m;
     }
-    RSD_TRY(rsd_potri_upper_tag(ctx, (int)n, M, n, "mob"));
-    RSD_TRY(rsd_mirror_upper(ctx, (int)n, M, n));
     cudaEventRecord(ctx->ev[2], s);
-    // arrangResist: R = R_inf + R_lub
+    // arrangResist: RPP = (R_inf)_PP + rfu; the products with rfe and rse
+    // come from the sparse lubrication operator
     int nc = 0;
-    if (p->use_lub) RSD_TRY(rsd_lub_assemble(ctx, tab, nn, p->nb, 1, d_conf, d_radii, &lat, p->mu_f, M, n, 1, &nc));
+    rsd_lub_sparse lub;
+    if (p->use_lub) RSD_TRY(rsd_lub_build_sparse(ctx, tab, nn, p->nb, 1, d_conf, d_radii, &lat, p->mu_f, &lub, &nc));
     loc.n_contact = nc;
+    double* RPP = (double*)rsd_scratch(ctx, "step_RPP", sizeof(double) * P * P);
+    double* f0 = (double*)rsd_scratch(ctx, "step_f0", sizeof(double) * (P + 3 * n));
+    if (!RPP || !f0) return RSD_ENOMEM;
+    RSD_CUDA(ctx, cudaMemcpyAsync(RPP, h.Ai, sizeof(double) * P * P, cudaMemcpyDeviceToDevice, s));
+    if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f64(ctx, &lub, RPP, P));
     if (rpp_out) {
-      RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(double) * rpp_ld, M, sizeof(double) * n, sizeof(double) * P, P,
+      RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(double) * rpp_ld, RPP, sizeof(double) * P, sizeof(double) * P, P,
                                       cudaMemcpyDeviceToDevice, s));
       RSD_CUDA(ctx, cudaStreamSynchronize(s));
       if (info) *info = loc;
       return RSD_OK;
     }
     cudaEventRecord(ctx->ev[3], s);
-    // RHS [Fe + RPQ EIN, RPQ EIN]; RPP factored in place (RPQ, RQQ untouched)
-    const double* RPQ = M + P * n;
+    // RHS [Fe + RPQ EIN, RPQ EIN], RPQ EIN = f0 + rfe EIN
+    double *w = f0 + P, *Lw = w + n;  // w = [0; EIN], then [X2; -EIN]; Lw = L w
+    RSD_TRY(rsd_r64_pq(ctx, &h, ein, f0));
+    RSD_CUDA(ctx, cudaMemcpyAsync(X + P, f0, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
+    if (p->use_lub) {
+      RSD_CUDA(ctx, cudaMemsetAsync(w, 0, sizeof(double) * P, s));
+      RSD_CUDA(ctx, cudaMemcpyAsync(w + P, ein, sizeof(double) * Q, cudaMemcpyDeviceToDevice, s));
+      RSD_TRY(rsd_lub_spmv(ctx, &lub, 1, w, n, Lw, n));
+      RSD_TRY(rsd_axpy_block(ctx, P, 1, Lw, P, X + P, P));
+    }
     RSD_CUDA(ctx, cudaMemcpyAsync(X, Fe, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
-    rsd_gemm_f64(s, (int)P, 1, (int)Q, 1.0, RPQ, n, 0, ein, Q, 0, 1.0, X, P);
-    rsd_gemm_f64(s, (int)P, 1, (int)Q, 1.0, RPQ, n, 0, ein, Q, 0, 0.0, X + P, P);
+    RSD_TRY(rsd_axpy_block(ctx, P, 1, X + P, P, X, P));
     bool solved = false;
     if (ctx->rpp_mode != RSD_PC_NONE) {
       // PCG on RPP with the chosen preconditioner; the factorisation stays
@@ -292,7 +306,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
       const double tol = ctx->rpp_tol > 0 ? ctx->rpp_tol : 1e-12;
       int it = 0;
       double res = 0.0;
-      RSD_TRY(rsd_lp_pcg_internal(ctx, (rsd_lp*)ctx->rpp_net, ctx->rpp_mode, nn, d_conf, d_radii, &lat, M, n, 2, B, X,
+      RSD_TRY(rsd_lp_pcg_internal(ctx, (rsd_lp*)ctx->rpp_net, ctx->rpp_mode, nn, d_conf, d_radii, &lat, RPP, P, 2, B, X,
                                   tol, ctx->rpp_maxit > 0 ? ctx->rpp_maxit : 1000, &it, &res));
       loc.rpp_iterations = it;
       if (res <= tol) {
@@ -304,17 +318,23 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     }
     if (!solved) {
       int info_r = 0;
-      RSD_TRY(rsd_potrf_upper_tag(ctx, (int)P, M, n, &info_r, "rpp"));
+      RSD_TRY(rsd_potrf_upper_tag(ctx, (int)P, RPP, P, &info_r, "rpp"));
       if (info_r) {
         loc.info = info_r;
         if (info) *info = loc;
         return info_r;
       }
-      RSD_TRY(rsd_potrs_upper_tag(ctx, (int)P, M, n, X, P, 2, "rpp"));
+      RSD_TRY(rsd_potrs_upper_tag(ctx, (int)P, RPP, P, X, P, 2, "rpp"));
     }
     // SijN_hyd = RPQ^T RPP^-1 RPQ EIN - RQQ EIN
-    rsd_gemm_f64(s, (int)Q, 1, (int)P, 1.0, RPQ, n, 1, X + P, P, 0, 0.0, S, Q);
-    rsd_gemm_f64(s, (int)Q, 1, (int)Q, -1.0, M + P + P * n, n, 0, ein, Q, 0, 1.0, S, Q);
+    RSD_TRY(rsd_r64_stresslet(ctx, &h, X + P, 1, f0, S));
+    if (p->use_lub) {
+      RSD_CUDA(ctx, cudaMemcpyAsync(w, X + P, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
+      RSD_CUDA(ctx, cudaMemsetAsync(w + P, 0, sizeof(double) * Q, s));
+      RSD_TRY(rsd_axpy_block(ctx, Q, 1, ein, Q, w + P, Q, -1.0));
+      RSD_TRY(rsd_lub_spmv(ctx, &lub, 1, w, n, Lw, n));
+      RSD_TRY(rsd_axpy_block(ctx, Q, 1, Lw + P, Q, S, Q));
+    }
     RSD_CUDA(ctx, cudaGetLastError());
   } else {
     cudaEventRecord(ctx->ev[2], s);
