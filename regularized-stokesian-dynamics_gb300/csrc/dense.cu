@@ -992,11 +992,11 @@ int rsd_mirror_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda) {
 // uplo: only the tiles on and above the diagonal.  Tensor cores (prec tc)
 // where the layout allows, else the SIMT GEMM.
 template <typename T>
-int trailing_update(rsd_ctx* ctx, int tc, const T* P, int64_t ldp, int kb, int m, int nc, T* C, int64_t ldc,
-                    int uplo) {
+int trailing_update(rsd_ctx* ctx, int tc, const T* P, int64_t ldp, int kb, int m, int nc, T* C, int64_t ldc, int uplo,
+                    int* err) {
   if constexpr (std::is_same<T, float>::value) {
     if (tc && ctx->use_tc && rsd_tc_syrk_ok(P, ldp, C, ldc, kb))
-      return rsd_tc_gemm(ctx, tc, m, nc, kb, -1.0f, P, ldp, P, ldp, C, ldc, 1, uplo, 0, ctx->d_info + 1);
+      return rsd_tc_gemm(ctx, tc, m, nc, kb, -1.0f, P, ldp, P, ldp, C, ldc, 1, uplo, 0, err);
   }
   GemmP g = gp(m, nc, kb, -1.0, P, ldp, 1, P, ldp, 0, 1.0, C, ldc);
   g.uplo = uplo;
@@ -1025,7 +1025,7 @@ int trailing_update(rsd_ctx* ctx, int tc, const T* P, int64_t ldp, int kb, int m
 // Events: A (a's near work done), B (the work the next near step reads),
 // M (the previous remainder, which the next diagonal tile reads).
 constexpr int NBO = 512;
-static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W) {
+static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
   cudaStream_t s = ctx->stream, s2 = ctx->side;
   RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
   for (int J0 = 0; J0 < n; J0 += NBO) {
@@ -1037,15 +1037,15 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, ctx->d_info, j0, Wb); RSD_LAUNCH_NOTE();
+      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
       if (rest <= 0) continue;
       // row panel U_jj^-T B = W_jj^T B in place on tensor cores (each output
       // tile reads only its own columns of B)
-      RSD_TRY(rsd_tc_gemm(ctx, tc, jb, rest, jb, 1.0f, Wb, NB, Apan, lda, Apan, lda, 0, 0, 0, ctx->d_info + 1, s2));
+      RSD_TRY(rsd_tc_gemm(ctx, tc, jb, rest, jb, 1.0f, Wb, NB, Apan, lda, Apan, lda, 0, 0, 0, st + 1, s2));
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel still to update
       if (m_in > 0)
         RSD_TRY(rsd_tc_gemm(ctx, tc, m_in, rest, jb, -1.0f, Apan, lda, Apan, lda, Apan + jb, lda, 1, 1, 0,
-                            ctx->d_info + 1, s2));
+                            st + 1, s2));
     }
     RSD_CUDA(ctx, cudaEventRecord(ctx->ev_panel, s2));
     RSD_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_panel, 0));
@@ -1054,21 +1054,21 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const float* PO = d_A + J0 + (int64_t)(J0 + JB) * lda;
       float* C = d_A + (J0 + JB) + (int64_t)(J0 + JB) * lda;
       const int m1 = restO < NBO ? restO : NBO;
-      RSD_TRY(rsd_tc_gemm(ctx, tc, m1, restO, JB, -1.0f, PO, lda, PO, lda, C, lda, 1, 1, 0, ctx->d_info + 1, s));
+      RSD_TRY(rsd_tc_gemm(ctx, tc, m1, restO, JB, -1.0f, PO, lda, PO, lda, C, lda, 1, 1, 0, st + 1, s));
       RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
       if (restO > NBO)
         RSD_TRY(rsd_tc_gemm(ctx, tc, restO - NBO, restO - NBO, JB, -1.0f, PO + (int64_t)NBO * lda, lda,
                             PO + (int64_t)NBO * lda, lda, C + NBO + (int64_t)NBO * lda, lda, 1, 1, 0,
-                            ctx->d_info + 1, s));
+                            st + 1, s));
     }
   }
   return RSD_OK;
 }
 
-static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W) {
+static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
   cudaStream_t s = ctx->stream, sa = ctx->side, sb = ctx->side2;
   cudaEvent_t evA = ctx->ev_la[0], evB = ctx->ev_la[1], evM = ctx->ev_la[2], evS = ctx->ev_la[3];
-  int* err = ctx->d_info + 1;
+  int* err = st + 1;
   // the matrix is ready on the main stream; B and M start out satisfied
   RSD_CUDA(ctx, cudaEventRecord(evS, s));
   RSD_CUDA(ctx, cudaStreamWaitEvent(sa, evS, 0));
@@ -1083,7 +1083,7 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, sa>>>(Ajj, lda, jb, ctx->d_info, j0, Wb); RSD_LAUNCH_NOTE();
+      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, sa>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
       if (rest <= 0) continue;
       RSD_CUDA(ctx, cudaStreamWaitEvent(sa, evB, 0));
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel below block k
@@ -1143,9 +1143,9 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
   return RSD_OK;
 }
 
-int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W) {
-  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W)
-                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W);
+int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
+  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W, st)
+                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W, st);
 }
 
 // Blocked right-looking upper Cholesky with one step of look-ahead: the
@@ -1153,7 +1153,7 @@ int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, fl
 // higher-priority stream as soon as the first tile row of step j's trailing
 // update has landed, while the rest of that update runs on the main stream.
 template <typename T>
-int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc) {
+int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc, int* d_status) {
   if (n < 1 || lda < n) return rsd_fail(ctx, RSD_EARG, "potrf: n=%d lda=%lld", n, (long long)lda);
   RSD_TRY(ensure_attrs<T>(ctx));
   RSD_TRY(rsd_side_stream(ctx));
@@ -1166,11 +1166,13 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
     T1 = (T*)rsd_scratch(ctx, "potrf_panel_s", sizeof(T) * (size_t)NB * n);
     if (!T1) return RSD_ENOMEM;
   }
-  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
+  // d_status (zeroed by the caller, read by it later): info and the timeout code
+  int* st = d_status ? d_status : ctx->d_info;
+  if (!d_status) RSD_CUDA(ctx, cudaMemsetAsync(st, 0, 2 * sizeof(int), s));
   bool two_level = false;
   if constexpr (F32) two_level = tc && ctx->use_tc && rsd_tc_syrk_ok(d_A, lda, d_A, lda, NB);
   if constexpr (F32) {
-    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W));
+    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W, st));
   }
   if (!two_level) {
     RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
@@ -1184,7 +1186,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
       {
         // factor + inverse of the diagonal block, then the panel as W_jj^T B
         T* Wb = W + (size_t)b * NB * NB;
-        potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, ctx->d_info, j0, Wb); RSD_LAUNCH_NOTE();
+        potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
         if (rest > 0) {
           launch_gemm<T>(s2, gp(jb, rest, jb, 1.0, Wb, NB, 1, Apan, lda, 0, 0.0, T1, NB));
           RSD_CUDA(ctx, cudaMemcpy2DAsync(Apan, lda * sizeof(T), T1, NB * sizeof(T), jb * sizeof(T), rest,
@@ -1197,15 +1199,19 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
         // trailing A22 -= Apan^T Apan: first tile row (the next panel's input), then the rest
         T* A22 = d_A + (j0 + jb) + (int64_t)(j0 + jb) * lda;
         const int m1 = rest < NB ? rest : NB;
-        RSD_TRY(trailing_update<T>(ctx, tc, Apan, lda, jb, m1, rest, A22, lda, 0));
+        RSD_TRY(trailing_update<T>(ctx, tc, Apan, lda, jb, m1, rest, A22, lda, 0, st + 1));
         RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
         if (rest > NB)
           RSD_TRY(trailing_update<T>(ctx, tc, Apan + (int64_t)NB * lda, lda, jb, rest - NB, rest - NB,
-                                     A22 + NB + (int64_t)NB * lda, lda, 1));
+                                     A22 + NB + (int64_t)NB * lda, lda, 1, st + 1));
       }
     }
   }
   RSD_CUDA(ctx, cudaGetLastError());
+  if (d_status) {
+    *info = 0;
+    return RSD_OK;
+  }
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
   *info = ctx->h_info[0];
@@ -1264,17 +1270,20 @@ __global__ void put_diag_transposed(int jb, const float* __restrict__ Wb, float*
 // WT(jblk, 0:j0) = -W_jj^T T1^T), and A^-1 = W W^T = WT^T WT over k >= the
 // tile's column.  prec 1 (TF32) or 3 (3xTF32).
 constexpr int POTRI_KSPLIT = 1024;
-int potri_tc_s(rsd_ctx* ctx, int prec, int n, float* d_A, int64_t lda, const char* tag) {
+int potri_tc_s(rsd_ctx* ctx, int prec, int n, float* d_A, int64_t lda, const char* tag, const float* W, int* d_err) {
   cudaStream_t s = ctx->stream;
-  float* W = nullptr;
-  RSD_TRY(rsd_diag_inverses_t<float>(ctx, n, d_A, lda, tag, &W));
+  if (!W) {
+    float* Wn = nullptr;
+    RSD_TRY(rsd_diag_inverses_t<float>(ctx, n, d_A, lda, tag, &Wn));
+    W = Wn;
+  }
   const int64_t ldw = (n + 3) / 4 * 4;
   float* WT = (float*)rsd_scratch(ctx, "potri_WT_s", sizeof(float) * (size_t)ldw * n);
   float* T1 = (float*)rsd_scratch(ctx, "potri_T1t_s", sizeof(float) * (size_t)NB * n);
   if (!WT || !T1) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info + 1, 0, sizeof(int), s));
+  int* err = d_err ? d_err : ctx->d_info + 1;
+  if (!d_err) RSD_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(int), s));
   RSD_CUDA(ctx, cudaMemsetAsync(WT, 0, sizeof(float) * (size_t)ldw * n, s));
-  int* err = ctx->d_info + 1;
   for (int j0 = 0, b = 0; j0 < n; j0 += NB, b++) {
     const int jb = n - j0 < NB ? n - j0 : NB;
     const float* Wb = W + (size_t)b * NB * NB;
@@ -1292,6 +1301,7 @@ int potri_tc_s(rsd_ctx* ctx, int prec, int n, float* d_A, int64_t lda, const cha
     RSD_TRY(rsd_tc_gemm(ctx, prec, jb, j0, jb, -1.0f, Wb, NB, T1, NB, WT + j0, ldw, 0, 0, 0, err));
   }
   RSD_TRY(rsd_tc_gemm(ctx, prec, n, n, n, 1.0f, WT, ldw, WT, ldw, d_A, lda, 0, 1, 1, err));
+  if (d_err) return RSD_OK;  // zeroed and read by the caller
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 1, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
   if (ctx->h_info[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "potri: tensor-core GEMM timed out (code %d)", ctx->h_info[1]);
@@ -1300,13 +1310,18 @@ int potri_tc_s(rsd_ctx* ctx, int prec, int n, float* d_A, int64_t lda, const cha
 
 // A <- A^-1 (upper triangle) from its upper Cholesky factor in A
 template <typename T>
-int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc) {
+// (Wd: its NB diagonal-block inverses, null to form them here)
+int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc, const T* Wd, int* d_err) {
   if constexpr (std::is_same<T, float>::value) {
-    if (tc && ctx->use_tc && rsd_tc_gemm_ok(d_A, lda, d_A, lda, d_A, lda)) return potri_tc_s(ctx, tc, n, d_A, lda, tag);
+    if (tc && ctx->use_tc && rsd_tc_gemm_ok(d_A, lda, d_A, lda, d_A, lda)) return potri_tc_s(ctx, tc, n, d_A, lda, tag, Wd, d_err);
   }
   cudaStream_t s = ctx->stream;
-  T* W = nullptr;
-  RSD_TRY(rsd_diag_inverses_t<T>(ctx, n, d_A, lda, tag, &W));
+  const T* W = Wd;
+  if (!W) {
+    T* Wn = nullptr;
+    RSD_TRY(rsd_diag_inverses_t<T>(ctx, n, d_A, lda, tag, &Wn));
+    W = Wn;
+  }
   T* T1 = (T*)rsd_scratch(ctx, sizeof(T) == 8 ? "potri_T1_d" : "potri_T1_s", sizeof(T) * (size_t)NB * n);
   if (!T1) return RSD_ENOMEM;
   RSD_TRY(rsd_zero_lower_t<T>(ctx, n, d_A, lda));
@@ -1331,27 +1346,21 @@ int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag,
 // wide-block solves: each block copied out (lower part zero) and inverted in
 // place by the blocked triangular inverse.  W2: nblk2 blocks of NB2 x NB2.
 constexpr int NB2 = 512;
-__global__ void copy_upper_block(int jb, const float* __restrict__ U, int64_t ldu, float* __restrict__ D) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= NB2 * NB2) return;
-  const int i = t % NB2, j = t / NB2;
-  D[t] = (i < jb && j < jb && i <= j) ? U[i + (int64_t)j * ldu] : (i == j ? 1.0f : 0.0f);
-}
-
-// The full NB2 diagonal blocks of U (blockIdx.z = block) into D (one
-// NB2 x NB2 block each, lower part zero).
-__global__ void copy_upper_blocks(const float* __restrict__ U, int64_t ldu, float* __restrict__ D) {
+// The NB2 diagonal blocks of U (n x n, blockIdx.z = block) into D (one NB2 x
+// NB2 block each, lower part and what lies past n zero).
+__global__ void copy_upper_blocks(int64_t n, const float* __restrict__ U, int64_t ldu, float* __restrict__ D) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.z;
   if (t >= NB2 * NB2) return;
   const int i = t % NB2, j = t / NB2;
   const int64_t o = (int64_t)b * NB2;
-  D[(size_t)b * NB2 * NB2 + t] = i <= j ? U[(o + i) + (o + j) * ldu] : 0.0f;
+  D[(size_t)b * NB2 * NB2 + t] = i <= j && o + j < n ? U[(o + i) + (o + j) * ldu] : 0.0f;
 }
 
 // D_b(j0:j0+NB, j0:j0+NB) = W_{b NB2/NB + j0/NB} for every block b = blockIdx.z
-__global__ void put_diag_blocks(int j0, const float* __restrict__ W, float* __restrict__ D) {
+// (nb128 blocks W exist; a block past them stays zero)
+__global__ void put_diag_blocks(int j0, int nb128, const float* __restrict__ W, float* __restrict__ D) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.z;
-  if (t >= NB * NB) return;
+  if (t >= NB * NB || b * (NB2 / NB) + j0 / NB >= nb128) return;
   const int i = t % NB, j = t / NB;
   D[(size_t)b * NB2 * NB2 + (j0 + i) + (int64_t)(j0 + j) * NB2] = W[((size_t)b * (NB2 / NB) + j0 / NB) * NB * NB + t];
 }
@@ -1359,7 +1368,7 @@ __global__ void put_diag_blocks(int j0, const float* __restrict__ W, float* __re
 // In-place inverses of nblk upper triangular NB2 x NB2 blocks D_b (ld NB2,
 // stride NB2^2) from their NB diagonal-block inverses: trtri_inplace_t on
 // all blocks at once, one batched GEMM pair per NB column block.
-int trtri_wide_batched_s(rsd_ctx* ctx, int nblk, float* D, const float* W, float* T1) {
+int trtri_wide_batched_s(rsd_ctx* ctx, int nblk, int nb128, float* D, const float* W, float* T1) {
   cudaStream_t s = ctx->stream;
   for (int j0 = 0; j0 < NB2; j0 += NB) {
     if (j0 > 0) {
@@ -1378,45 +1387,27 @@ int trtri_wide_batched_s(rsd_ctx* ctx, int nblk, float* D, const float* W, float
       g2.sC = (int64_t)NB2 * NB2;
       launch_gemm<float>(s, g2);
     }
-    put_diag_blocks<<<dim3(NB * NB / 256, 1, nblk), 256, 0, s>>>(j0, W, D); RSD_LAUNCH_NOTE();
+    put_diag_blocks<<<dim3(NB * NB / 256, 1, nblk), 256, 0, s>>>(j0, nb128, W, D); RSD_LAUNCH_NOTE();
   }
   return RSD_OK;
 }
 
-// W128 (optional): the NB x NB diagonal-block inverses that the FP32 potrf
-// of U left (NB-block b at W128 + b NB^2); the full NB2 blocks then start
-// from them (all blocks in one batched pass) instead of inverting their NB
-// blocks again.
+// W128: the NB x NB diagonal-block inverses that the FP32 potrf of U left
+// (NB-block b at W128 + b NB^2); the NB2 blocks start from them, all blocks in
+// one batched pass.
 int rsd_wide_inverses_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const char* tag, const float* W128,
                         float** W2out) {
-  const int nblk2 = (n + NB2 - 1) / NB2;
+  const int nblk2 = (n + NB2 - 1) / NB2, nb128 = (n + NB - 1) / NB;
   std::string name = std::string("wide_W_") + tag;
   float* W2 = (float*)rsd_scratch(ctx, name.c_str(), sizeof(float) * (size_t)nblk2 * NB2 * NB2);
-  float* Wt = (float*)rsd_scratch(ctx, "wide_Wsmall", sizeof(float) * (size_t)(NB2 / NB) * NB * NB);
-  float* T1 = (float*)rsd_scratch(ctx, "wide_T1", sizeof(float) * (size_t)NB * NB2);
-  if (!W2 || !Wt || !T1) return RSD_ENOMEM;
-  RSD_TRY(ensure_attrs<float>(ctx));
-  int b0 = 0;
-  if (W128 && n >= NB2) {
-    const int full = n / NB2;
-    float* Tb = (float*)rsd_scratch(ctx, "wide_T1b", sizeof(float) * (size_t)full * NB * NB2);
-    if (!Tb) return RSD_ENOMEM;
-    copy_upper_blocks<<<dim3(NB2 * NB2 / 256, 1, full), 256, 0, ctx->stream>>>(U, ldu, W2); RSD_LAUNCH_NOTE();
-    RSD_TRY(trtri_wide_batched_s(ctx, full, W2, W128, Tb));
-    b0 = full;
-  }
-  for (int b = b0; b < nblk2; b++) {
-    const int j0 = b * NB2, jb = n - j0 < NB2 ? n - j0 : NB2;
-    float* D = W2 + (size_t)b * NB2 * NB2;
-    copy_upper_block<<<(NB2 * NB2 + 255) / 256, 256, 0, ctx->stream>>>(jb, U + j0 + (int64_t)j0 * ldu, ldu, D); RSD_LAUNCH_NOTE();
-    const float* Wb = Wt;
-    if (W128 && jb == NB2) {
-      Wb = W128 + (size_t)(j0 / NB) * NB * NB;
-    } else {
-      trtri_diag<float><<<NB2 / NB, 256, smem_potf2<float>(NB), ctx->stream>>>(NB2, D, NB2, Wt); RSD_LAUNCH_NOTE();
-    }
-    RSD_TRY(trtri_inplace_t<float>(ctx, NB2, D, NB2, Wb, T1, NB2));
-  }
+  float* Tb = (float*)rsd_scratch(ctx, "wide_T1b", sizeof(float) * (size_t)nblk2 * NB * NB2);
+  // a whole block of inverses per NB2 block is addressed in the batch
+  float* Wp = (float*)rsd_scratch(ctx, "wide_Wpad", sizeof(float) * (size_t)nblk2 * (NB2 / NB) * NB * NB);
+  if (!W2 || !Tb || !Wp) return RSD_ENOMEM;
+  RSD_CUDA(ctx, cudaMemsetAsync(Wp, 0, sizeof(float) * (size_t)nblk2 * (NB2 / NB) * NB * NB, ctx->stream));
+  RSD_CUDA(ctx, cudaMemcpyAsync(Wp, W128, sizeof(float) * (size_t)nb128 * NB * NB, cudaMemcpyDeviceToDevice, ctx->stream));
+  copy_upper_blocks<<<dim3(NB2 * NB2 / 256, 1, nblk2), 256, 0, ctx->stream>>>(n, U, ldu, W2); RSD_LAUNCH_NOTE();
+  RSD_TRY(trtri_wide_batched_s(ctx, nblk2, nb128, W2, Wp, Tb));
   RSD_CUDA(ctx, cudaGetLastError());
   *W2out = W2;
   return RSD_OK;
@@ -1697,8 +1688,9 @@ __global__ void __launch_bounds__(256) blockdiag_gemv(int n, const float* __rest
 
 // Builds Uh (strict upper block strips, ld ldu, in a buffer of its own) and
 // the G_b blocks from the factor U and its NB2 block inverses W2.
-int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float* W2, const char* tag,
-                   rsd_uhat* out) {
+// err: a status word zeroed and read by the caller.
+int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float* W2, const char* tag, rsd_uhat* out,
+                   int* err) {
   if (ldu % 4 != 0 || ((uintptr_t)U & 15)) return rsd_fail(ctx, RSD_EARG, "uhat: unsupported layout");
   const int nblk2 = (n + NB2 - 1) / NB2;
   std::string nu = std::string("uhat_U_") + tag, ng = std::string("uhat_G_") + tag;
@@ -1708,8 +1700,6 @@ int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float
   if (!Uh || !G || !WT) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;
   transpose_block<<<dim3(NB2 / 32, NB2 / 32, nblk2), dim3(32, 8), 0, s>>>(NB2, W2, WT); RSD_LAUNCH_NOTE();
-  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info + 1, 0, sizeof(int), s));
-  int* err = ctx->d_info + 1;
   // all blocks in two batched launches: G_b = W_b W_b^T, and the strips
   // Uh_b = W_b^T U(block b rows, columns after block b), whose width drops
   // by NB2 from one block to the next
@@ -1722,9 +1712,6 @@ int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float
     RSD_TRY(rsd_tc_gemm_zbatch(ctx, 3, NB2, n - NB2, NB2, 1.0f, WT, NB2, NB2, nw, U1, ldu, n, n - NB2, Uh1, ldu, n,
                                n - NB2, nblk2 - 1, 0, NB2, NB2, NB2, NB2, NB2, NB2, err));
   }
-  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 1, err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaStreamSynchronize(s));
-  if (ctx->h_info[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "uhat: tensor-core GEMM timed out");
   out->n = n;
   out->Uh = Uh;
   out->ld = ldu;
@@ -1732,26 +1719,26 @@ int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float
   return RSD_OK;
 }
 
-// X (n x nrhs, ld ldx) <- (U^T U)^-1 X with the block-scaled factor; Y is
-// n x nrhs scratch (ld ldx).
+// Y (n x nrhs, ld ldx) = (U^T U)^-1 X with the block-scaled factor; X is
+// overwritten.
 int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int nrhs, float* Y, int zero_lead) {
   if (nrhs < 1 || nrhs > 2) return rsd_fail(ctx, RSD_EARG, "uhat solve: 1 or 2 right-hand sides");
   const int n = h->n, nblk2 = (n + NB2 - 1) / NB2;
   cudaStream_t s = ctx->stream;
   const int gsm = ctx->sm_count > 0 ? ctx->sm_count : 148;
   if (nblk2 > TRI_MAX_BLOCKS) return rsd_fail(ctx, RSD_EUNSUP, "uhat solve: order %d above %d", n, TRI_MAX_BLOCKS * NB2);
-  int* sync = rsd_uhat_error_flag(ctx);  // [0] error (cumulative), [1] ticket, ready counts
+  // [0] error (cumulative), [1], [2] tickets, then the ready counts of the two sweeps
+  int* sync = rsd_uhat_error_flag(ctx);
   if (!sync) return RSD_ENOMEM;
   // leading zero blocks of the right-hand side: the forward sweep starts at
   // the first block that can be nonzero (z is zero before it)
   const int b0 = zero_lead > 0 ? min(zero_lead / NB2, nblk2 - 1) : 0;
-  TriArgs A{h->Uh, h->ld, n, nblk2, X, ldx, sync + 2, sync + 1, sync, b0,
+  TriArgs A{h->Uh, h->ld, n, nblk2, X, ldx, sync + 3, sync + 1, sync, b0,
             ctx->tri_spin_polls > 0 ? ctx->tri_spin_polls : TRI_SPIN_LIMIT};
   const int tasks = TRI_Q * (nblk2 - 1);
-  const int grid = max(1, min(tasks, 4 * gsm));
   const int ftasks = TRI_Q * (nblk2 - 1 - b0);
+  if (tasks > 0) RSD_CUDA(ctx, cudaMemsetAsync(sync + 1, 0, sizeof(int) * (size_t)(2 + 2 * nblk2), s));
   if (ftasks > 0) {  // forward, in place on X
-    RSD_CUDA(ctx, cudaMemsetAsync(sync + 1, 0, sizeof(int) * (size_t)(1 + nblk2), s));
     const int fgrid = max(1, min(ftasks, 4 * gsm));
     if (nrhs == 1)
       tri_forward<1><<<fgrid, TRI_THREADS, 0, s>>>(A);
@@ -1767,15 +1754,15 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
   if (tasks > 0) {  // backward, in place on Y
     A.V = Y;
     A.b0 = 0;
-    RSD_CUDA(ctx, cudaMemsetAsync(sync + 1, 0, sizeof(int) * (size_t)(1 + nblk2), s));
+    A.ticket = sync + 2;
+    A.ready = sync + 3 + nblk2;
+    const int grid = max(1, min(tasks, 4 * gsm));
     if (nrhs == 1)
       tri_backward<1><<<grid, TRI_THREADS, 0, s>>>(A);
     else
       tri_backward<2><<<grid, TRI_THREADS, 0, s>>>(A);
     RSD_LAUNCH_NOTE();
   }
-  for (int r = 0; r < nrhs; r++)
-    RSD_CUDA(ctx, cudaMemcpyAsync(X + r * ldx, Y + r * ldx, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -1784,9 +1771,11 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
 // error flag, nonzero once a sweep's wait timed out (the caller zeroes it
 // and reads it after synchronising the stream).
 int* rsd_uhat_error_flag(rsd_ctx* ctx) {
-  return (int*)rsd_scratch(ctx, "tri_sync", sizeof(int) * (size_t)(2 * TRI_MAX_BLOCKS + 2));
+  return (int*)rsd_scratch(ctx, "tri_sync", sizeof(int) * (size_t)(2 * TRI_MAX_BLOCKS + 3));
 }
 
+// The same by blocks on the factor itself (FP32 SIMT form): X is overwritten,
+// the solution is in Y.
 int rsd_potrs_wide_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float* W2, float* X, int64_t ldx,
                      int nrhs, float* Y) {
   const int nblk2 = (n + NB2 - 1) / NB2;
@@ -1807,6 +1796,8 @@ int rsd_potrs_wide_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const flo
     if (j0 > 0)
       RSD_TRY(rsd_gemv<float>(ctx, 0, j0, jb, -1.0f, U + (int64_t)j0 * ldu, ldu, X + j0, ldx, nrhs, 1.0f, Y, ldx));
   }
+  for (int r = 0; r < nrhs; r++)
+    RSD_CUDA(ctx, cudaMemcpyAsync(Y + r * ldx, X + r * ldx, sizeof(float) * n, cudaMemcpyDeviceToDevice, ctx->stream));
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -1871,8 +1862,8 @@ template int rsd_gemv<float>(rsd_ctx*, int, int, int, float, const float*, int64
                              float*, int64_t);
 template int rsd_gemv<double>(rsd_ctx*, int, int, int, double, const double*, int64_t, const double*, int64_t, int,
                               double, double*, int64_t);
-template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int);
-template int rsd_potri_upper_t<float>(rsd_ctx*, int, float*, int64_t, const char*, int);
+template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*);
+template int rsd_potri_upper_t<float>(rsd_ctx*, int, float*, int64_t, const char*, int, const float*, int*);
 template int rsd_potrs_upper_t<float>(rsd_ctx*, int, const float*, int64_t, float*, int64_t, int, const char*,
                                       const float*);
 template int rsd_mirror_upper_t<float>(rsd_ctx*, int, float*, int64_t);
@@ -1921,7 +1912,7 @@ extern "C" int rsd_potrf_f32_dev(rsd_ctx* ctx, int32_t n, float* d_A, int64_t ld
   RSD_TRY(check_prec(ctx, prec));
   RSD_TRY(rsd_set_device(ctx));
   int inf = 0;
-  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec));
+  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec, nullptr));
   *info = inf;
   return RSD_OK;
 }
@@ -1931,7 +1922,7 @@ extern "C" int rsd_potri_f32_dev(rsd_ctx* ctx, int32_t n, float* d_A, int64_t ld
   if (n < 1 || lda < n || !d_A) return rsd_fail(ctx, RSD_EARG, "rsd_potri_f32_dev: bad arguments");
   RSD_TRY(check_prec(ctx, prec));
   RSD_TRY(rsd_set_device(ctx));
-  RSD_TRY(rsd_potri_upper_t<float>(ctx, n, d_A, lda, "f32dev", prec));
+  RSD_TRY(rsd_potri_upper_t<float>(ctx, n, d_A, lda, "f32dev", prec, nullptr, nullptr));
   RSD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return RSD_OK;
 }

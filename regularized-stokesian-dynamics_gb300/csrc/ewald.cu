@@ -296,8 +296,7 @@ __device__ inline void store_pair_t(const S& sk, int N, int a, int b, const V* v
 // Mixed form: only the entries whose row belongs to particle a (a < b) of
 // each pair block are written (121 of 242: the pair's rows of the grand
 // matrix, all coalesced along a); the consumers read the other half at the
-// mirrored position, or mirror_planes fills it by symmetry.  Values as in
-// store_pair_t.
+// mirrored position.  Values as in store_pair_t.
 __device__ inline void store_pair_rows_a(const PlaneSink& sk, int N, int a, int b, const dsf* v, int add) {
   auto at = [&](int r, int c) { return (int64_t)r + (int64_t)c * sk.ld; };
   constexpr int sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
@@ -361,44 +360,6 @@ __device__ inline void store_pair_rows_a(const PlaneSink& sk, int N, int a, int 
         x[5 * xi + y] = v[15 + lo * 5 - lo * (lo - 1) / 2 + (hi - lo)];
       }
     sk.template put<25>(p, x, add);
-  }
-}
-
-// particle of grand-matrix index x
-__device__ __forceinline__ int grand_particle(int N, int x) {
-  return x < 3 * N ? x / 3 : (x < 6 * N ? (x - 3 * N) / 3 : (x - 6 * N) / 5);
-}
-
-// M(r, c) = M(c, r) for every entry whose row's particle is above its
-// column's (the entries store_pair_rows_a leaves out), on both planes:
-// 32 x 32 tiles through shared memory, both the read and the write
-// coalesced; tiles with nothing to fill return at once.
-__global__ void mirror_planes(int N, int64_t n, float* __restrict__ hi, float* __restrict__ lo, int64_t ld) {
-  __shared__ float th[32][33], tl[32][33];
-  __shared__ int skip;
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  if (ty == 0) {  // the particle index is monotonic only within each of the three row sections
-    const int rmax = __reduce_max_sync(0xffffffffu, grand_particle(N, (int)min((int64_t)r0 + tx, n - 1)));
-    const int cmin = __reduce_min_sync(0xffffffffu, grand_particle(N, (int)min((int64_t)c0 + tx, n - 1)));
-    if (tx == 0) skip = rmax <= cmin;
-  }
-  __syncthreads();
-  if (skip) return;
-  for (int k = ty; k < 32; k += blockDim.y) {  // source M(c0 + tx, r0 + k)
-    const int64_t c = c0 + tx, r = r0 + k;
-    if (c < n && r < n) {
-      th[k][tx] = hi[c + r * ld];
-      tl[k][tx] = lo[c + r * ld];
-    }
-  }
-  __syncthreads();
-  for (int k = ty; k < 32; k += blockDim.y) {  // destination M(r0 + tx, c0 + k)
-    const int64_t r = r0 + tx, c = c0 + k;
-    if (r < n && c < n && grand_particle(N, (int)r) > grand_particle(N, (int)c)) {
-      hi[r + c * ld] = th[tx][k];
-      lo[r + c * ld] = tl[tx][k];
-    }
   }
 }
 
@@ -1589,15 +1550,6 @@ int launch_real_eq(rsd_ctx* ctx, int passes, dim3 grd, dim3 blk, int nn, const r
 }
 }  // namespace
 
-int rsd_mirror_planes(rsd_ctx* ctx, int nn, double* d_M, int64_t ldm) {
-  const int64_t n11 = 11LL * nn;
-  float* hi = reinterpret_cast<float*>(d_M);
-  const dim3 mt((unsigned)((n11 + 31) / 32), (unsigned)((n11 + 31) / 32));
-  mirror_planes<<<mt, dim3(32, 8), 0, ctx->stream>>>(nn, n11, hi, hi + (size_t)ldm * n11, ldm); RSD_LAUNCH_NOTE();
-  RSD_CUDA(ctx, cudaGetLastError());
-  return RSD_OK;
-}
-
 namespace {
 // Lattice vectors and reciprocal vectors of a sum, made on the host.
 struct ewald_lists {
@@ -1867,7 +1819,6 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       std::vector<int> all(h64);
       all.insert(all.end(), h32.begin(), h32.end());
       RSD_CUDA(ctx, cudaMemcpyAsync(dh, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, s));
-      RSD_CUDA(ctx, cudaStreamSynchronize(s));
       if (K64) {
         ewald_trig_list<float4><<<dim3((nn + 127) / 128, K64), 128, 0, s>>>(nn, L, dh, d_pos, c64); RSD_LAUNCH_NOTE();
       }

@@ -2,10 +2,10 @@
 // src/hydro_lub.f90:22-308, with lubcalc 310-398 and lubtabcalc 400-525).
 //
 // Pipeline (all FP64, deterministic order):
-//   lub_count     one warp per particle a: near partners b > a (s <= 4 in
+//   lub_near      one warp per particle a: near partners b > a (s <= 4 in
 //                 the minimum image), ballot-compacted -> count[a]
 //   lub_scan      exclusive scan of the counts (one block)
-//   lub_list      the same sweep writes the pair list, sorted by (a, b)
+//   lub_near      the same sweep writes the pair list, sorted by (a, b)
 //   lub_pairs     one thread per near pair: the 19 resistance scalars and
 //                 the projected two-body blocks (139 values per pair)
 //   lub_cross     one thread per (pair, entry): the (a,b) and (b,a) blocks
@@ -24,8 +24,6 @@ constexpr int PB = 139;  // doubles per pair block
 // offsets inside a pair block
 constexpr int O_A11 = 0, O_A12 = 9, O_B11 = 18, O_B12 = 27, O_C11 = 36, O_C12 = 45;
 constexpr int O_G11 = 54, O_G12 = 69, O_H11 = 84, O_H12 = 99, O_M = 114;
-
-__constant__ double c_Y2[45];  // Y2(m,i,j) at m + 5*(i + 3*j), tensors.f90:43-67
 
 struct lub_dev_tab {
   const double *abc, *gh, *m;
@@ -56,12 +54,15 @@ __device__ void lubcalc_dev(const lub_dev_tab& t, double r, double* o) {
     o[18] = 0.00645755 - 0.021142 * xi;
     return;
   }
+#pragma unroll
   for (int q = 0; q < 19; q++) o[q] = 0.0;
   for (int i = 0; i < t.nabc - 1; i++) {
     const double* a = t.abc + 11 * i;
     const double* b = a + 11;
     if (a[0] <= r && b[0] > r) {
-      for (int q = 0; q < 10; q++) o[q] = a[q + 1] + (r - a[0]) * (b[q + 1] - a[q + 1]) / (b[0] - a[0]);
+      const double f = (r - a[0]) / (b[0] - a[0]);
+#pragma unroll
+      for (int q = 0; q < 10; q++) o[q] = a[q + 1] + f * (b[q + 1] - a[q + 1]);
       break;
     }
   }
@@ -69,7 +70,9 @@ __device__ void lubcalc_dev(const lub_dev_tab& t, double r, double* o) {
     const double* a = t.gh + 7 * i;
     const double* b = a + 7;
     if (a[0] <= r && b[0] > r) {
-      for (int q = 0; q < 6; q++) o[10 + q] = a[q + 1] + (r - a[0]) * (b[q + 1] - a[q + 1]) / (b[0] - a[0]);
+      const double f = (r - a[0]) / (b[0] - a[0]);
+#pragma unroll
+      for (int q = 0; q < 6; q++) o[10 + q] = a[q + 1] + f * (b[q + 1] - a[q + 1]);
       break;
     }
   }
@@ -77,59 +80,92 @@ __device__ void lubcalc_dev(const lub_dev_tab& t, double r, double* o) {
     const double* a = t.m + 4 * i;
     const double* b = a + 4;
     if (a[0] <= r && b[0] > r) {
-      for (int q = 0; q < 3; q++) o[16 + q] = (a[q + 1] + (r - a[0]) * (b[q + 1] - a[q + 1]) / (b[0] - a[0])) / 2.0;
+      const double f = (r - a[0]) / (b[0] - a[0]);
+#pragma unroll
+      for (int q = 0; q < 3; q++) o[16 + q] = (a[q + 1] + f * (b[q + 1] - a[q + 1])) / 2.0;
       break;
     }
   }
 }
 
-__device__ inline double eps3(int i, int j, int k) {
-  return (double)((i - j) * (j - k) * (k - i)) / 2.0;  // Levi-Civita for 0..2
+// FP32 screen of a pair: false where it is clearly beyond the cut-off s = 4
+__device__ __forceinline__ bool maybe_near(const float* LR, const float* LI, int is_period, const float R[3], float asum) {
+  float d2;
+  if (is_period) {
+    int k[3];
+    rsd_skew_shift_f32(LR, LI, R, k);
+    d2 = 0.f;
+    for (int i = 0; i < 3; i++) {
+      const float e = R[i] - (LR[i] * k[0] + LR[i + 3] * k[1] + LR[i + 6] * k[2]);
+      d2 += e * e;
+    }
+  } else {
+    d2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+  }
+  const float lim = 2.0f * asum * 1.001f + 1e-3f;
+  return !(d2 > lim * lim);
 }
 
 __device__ inline bool near_pair(const rsd_lat_dev& L, int is_period, const double* pos, const double* radii, int a,
                                  int b) {
   double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
-  {  // FP32 screen: pairs clearly beyond the cut-off need no FP64 test
-    float LRf[9], LIf[9], Rf[3] = {(float)R[0], (float)R[1], (float)R[2]};
-    for (int k = 0; k < 9; k++) {
-      LRf[k] = (float)L.LR[k];
-      LIf[k] = (float)L.LI[k];
-    }
-    float d2;
-    if (is_period) {
-      int k[3];
-      rsd_skew_shift_f32(LRf, LIf, Rf, k);
-      d2 = 0.f;
-      for (int i = 0; i < 3; i++) {
-        const float e = Rf[i] - (LRf[i] * k[0] + LRf[i + 3] * k[1] + LRf[i + 6] * k[2]);
-        d2 += e * e;
-      }
-    } else {
-      d2 = Rf[0] * Rf[0] + Rf[1] * Rf[1] + Rf[2] * Rf[2];
-    }
-    const float lim = 2.0f * (float)(radii[a] + radii[b]) * 1.001f + 1e-3f;  // s = 4 with a margin
-    if (d2 > lim * lim) return false;
-  }
   double r = sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]);
   if (is_period) rsd_skew_correction(L.LR, L.LI, R, &r);
   const double s = r / (0.5 * (radii[a] + radii[b]));
   return !(s > 4.0);
 }
 
-__global__ void lub_count(int nn, int nb, int is_period, rsd_lat_dev L, const double* __restrict__ pos,
-                          const double* __restrict__ radii, int* __restrict__ count) {
-  const int a = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+// The near partners b > a of a particle, ascending, one warp per particle:
+// lanes screen 32 partners at a time in FP32 and the survivors are collected,
+// so that the FP64 test (a warp issues an FP64 instruction every 64 cycles)
+// runs over full warps of them.  LIST: the pairs are written from off[a] on;
+// otherwise they are counted.
+constexpr int LUB_WARPS = 8, LUB_CAND = 64;
+template <bool LIST>
+__global__ void lub_near(int nn, int nb, int is_period, rsd_lat_dev L, const double* __restrict__ pos,
+                         const double* __restrict__ radii, int* __restrict__ count, const int* __restrict__ off,
+                         int2* __restrict__ pairs) {
+  __shared__ int cand[LUB_WARPS][LUB_CAND];
+  const int warp = threadIdx.x / 32, a = blockIdx.x * LUB_WARPS + warp, lane = threadIdx.x & 31;
   if (a >= nn) return;
-  int c = 0;
-  if (a < nn - nb) {
+  float LR[9], LI[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    LR[k] = (float)L.LR[k];
+    LI[k] = (float)L.LI[k];
+  }
+  const double x0 = pos[3 * a], x1 = pos[3 * a + 1], x2 = pos[3 * a + 2];
+  const float ra = (float)radii[a];
+  const unsigned below = (1u << lane) - 1;
+  int found = 0, nc = 0;
+  auto flush = [&](int n) {  // tests the first n <= 32 candidates and drops them
+    __syncwarp();
+    const int b = lane < n ? cand[warp][lane] : -1;
+    const bool nr = b >= 0 && near_pair(L, is_period, pos, radii, a, b);
+    const unsigned m = __ballot_sync(0xffffffffu, nr);
+    if (LIST && nr) pairs[off[a] + found + __popc(m & below)] = make_int2(a, b);
+    found += __popc(m);
+    const int rest = lane + n < nc ? cand[warp][lane + n] : 0;
+    __syncwarp();
+    cand[warp][lane] = rest;
+    nc -= n;
+    __syncwarp();
+  };
+  if (a < nn - nb)
     for (int b0 = a + 1; b0 < nn; b0 += 32) {
       const int b = b0 + lane;
-      const bool nr = b < nn && near_pair(L, is_period, pos, radii, a, b);
-      c += __popc(__ballot_sync(0xffffffffu, nr));
+      bool c = false;
+      if (b < nn) {
+        const float R[3] = {(float)(x0 - pos[3 * b]), (float)(x1 - pos[3 * b + 1]), (float)(x2 - pos[3 * b + 2])};
+        c = maybe_near(LR, LI, is_period, R, ra + (float)radii[b]);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, c);
+      if (c) cand[warp][nc + __popc(m & below)] = b;
+      nc += __popc(m);
+      if (nc >= 32) flush(32);
     }
-  }
-  if (lane == 0) count[a] = c;
+  if (nc > 0) flush(nc);
+  if (!LIST && lane == 0) count[a] = found;
 }
 
 // exclusive scan of count[0..n) into off[0..n], one block of 1024 threads
@@ -156,34 +192,68 @@ __global__ void lub_scan(int n, const int* __restrict__ count, int* __restrict__
   if (t == 1023) off[n] = part[1023];
 }
 
-__global__ void lub_list(int nn, int nb, int is_period, rsd_lat_dev L, const double* __restrict__ pos,
-                         const double* __restrict__ radii, const int* __restrict__ off, int2* __restrict__ pairs) {
-  const int a = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-  if (a >= nn || a >= nn - nb) return;
-  int w = off[a];
-  for (int b0 = a + 1; b0 < nn; b0 += 32) {
-    const int b = b0 + lane;
-    const bool nr = b < nn && near_pair(L, is_period, pos, radii, a, b);
-    const unsigned m = __ballot_sync(0xffffffffu, nr);
-    if (nr) pairs[w + __popc(m & ((1u << lane) - 1))] = make_int2(a, b);
-    w += __popc(m);
-  }
-}
-
-// rtd_front: C(m,c) = sum_ij T3(i,j,c) Y2(m,i,j)   (tensors.f90:966-978)
-__device__ inline void front_y2(const double T3[27], double* C /*5x3, m + 5c*/) {
+// The two-body blocks of a pair (hydro_lub.f90:95-160 with rtd_front and
+// DD_transY2, tensors.f90:966-1023), in closed form.  With v_m = Y_m e and q_m
+// = e.v_m (Y_m the symmetric traceless basis, Y_m : Y_n = delta_mn) the tensor
+// sums of the reference contract to
+//   G(m, c) = x q_m e_c + y (2 v_mc - 2 q_m e_c)
+//   H(m, c) = 2 y (e x v_m)_c
+//   M(m, n) = 3/2 x q_m q_n + 2 y (v_m.v_n - q_m q_n) + z (delta_mn - 2 v_m.v_n + q_m q_n / 2)
+// about 600 FP64 instructions a pair where the sums take 9700.  A warp issues
+// one every 64 cycles, so this is the kernel's time: 300 -> 72 us (N = 512).
+__device__ inline void pair_tensors(const double* o, const double e[3], double* B) {
+  const double x11a = o[0], x12a = o[1], y11a = o[2], y12a = o[3], y11b = o[4], y12b = o[5], x11c = o[6],
+               x12c = o[7], y11c = o[8], y12c = o[9], x11g = o[10], x12g = o[11], y11g = o[12], y12g = o[13],
+               y11h = o[14], y12h = o[15], xm = o[16], ym = o[17], zm = o[18];
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double ee = e[i] * e[j], t = (i == j ? 1.0 : 0.0) - ee;
+      // eps_ijk e_k
+      const double pe = i == j ? 0.0 : ((j - i + 3) % 3 == 1 ? e[3 - i - j] : -e[3 - i - j]);
+      B[O_A11 + i + 3 * j] = x11a * ee + y11a * t;
+      B[O_A12 + i + 3 * j] = x12a * ee + y12a * t;
+      B[O_B11 + i + 3 * j] = y11b * pe;
+      B[O_B12 + i + 3 * j] = y12b * pe;
+      B[O_C11 + i + 3 * j] = x11c * ee + y11c * t;
+      B[O_C12 + i + 3 * j] = x12c * ee + y12c * t;
+    }
+  const double s2 = 0.70710678118654752440, s6 = 0.40824829046386301637;  // 1/sqrt 2, 1/sqrt 6
+  const double v[5][3] = {{s2 * e[1], s2 * e[0], 0.0},
+                          {0.0, -s2 * e[2], -s2 * e[1]},
+                          {-s6 * e[0], -s6 * e[1], 2.0 * s6 * e[2]},
+                          {-s2 * e[2], 0.0, -s2 * e[0]},
+                          {s2 * e[0], -s2 * e[1], 0.0}};
+  double q[5];
+#pragma unroll
+  for (int m = 0; m < 5; m++) q[m] = e[0] * v[m][0] + e[1] * v[m][1] + e[2] * v[m][2];
+#pragma unroll
   for (int m = 0; m < 5; m++)
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-      double v = 0.0;
-      for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) v += T3[i + 3 * j + 9 * c] * c_Y2[m + 5 * (i + 3 * j)];
-      C[m + 5 * c] = v;
+      const double qe = q[m] * e[c], w = 2.0 * (v[m][c] - qe);
+      const double h = 2.0 * (e[(c + 1) % 3] * v[m][(c + 2) % 3] - e[(c + 2) % 3] * v[m][(c + 1) % 3]);
+      B[O_G11 + m + 5 * c] = x11g * qe + y11g * w;
+      B[O_G12 + m + 5 * c] = x12g * qe + y12g * w;
+      B[O_H11 + m + 5 * c] = y11h * h;
+      B[O_H12 + m + 5 * c] = y12h * h;
+    }
+#pragma unroll
+  for (int m = 0; m < 5; m++)
+#pragma unroll
+    for (int n = m; n < 5; n++) {
+      const double qq = q[m] * q[n], vv = v[m][0] * v[n][0] + v[m][1] * v[n][1] + v[m][2] * v[n][2];
+      const double t = 1.5 * xm * qq + 2.0 * ym * (vv - qq) + zm * ((m == n ? 1.0 : 0.0) - 2.0 * vv + 0.5 * qq);
+      B[O_M + m + 5 * n] = t;
+      B[O_M + n + 5 * m] = t;
     }
 }
 
-__global__ void lub_pairs(int npair, lub_dev_tab tab, int is_period, rsd_lat_dev L, const double* __restrict__ pos,
-                          const double* __restrict__ radii, const int2* __restrict__ pairs, double* __restrict__ blk,
-                          int* __restrict__ contacts) {
+__global__ void __launch_bounds__(32) lub_pairs(int npair, lub_dev_tab tab, int is_period, rsd_lat_dev L,
+                                                const double* __restrict__ pos, const double* __restrict__ radii,
+                                                const int2* __restrict__ pairs, double* __restrict__ blk,
+                                                int* __restrict__ contacts) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npair) return;
   const int a = pairs[p].x, b = pairs[p].y;
@@ -197,62 +267,8 @@ __global__ void lub_pairs(int npair, lub_dev_tab tab, int is_period, rsd_lat_dev
   }
   double o[19];
   lubcalc_dev(tab, s, o);
-  const double x11a = o[0], x12a = o[1], y11a = o[2], y12a = o[3], y11b = o[4], y12b = o[5], x11c = o[6],
-               x12c = o[7], y11c = o[8], y12c = o[9], x11g = o[10], x12g = o[11], y11g = o[12], y12g = o[13],
-               y11h = o[14], y12h = o[15], xm = o[16], ym = o[17], zm = o[18];
   const double e[3] = {R[0] / r, R[1] / r, R[2] / r};
-  double* B = blk + (size_t)p * PB;
-  auto kd = [](int i, int j) { return i == j ? 1.0 : 0.0; };
-  for (int j = 0; j < 3; j++)
-    for (int i = 0; i < 3; i++) {
-      const double ee = e[i] * e[j], d = kd(i, j);
-      const double pe = eps3(i, j, 0) * e[0] + eps3(i, j, 1) * e[1] + eps3(i, j, 2) * e[2];
-      B[O_A11 + i + 3 * j] = x11a * ee + y11a * (d - ee);
-      B[O_A12 + i + 3 * j] = x12a * ee + y12a * (d - ee);
-      B[O_B11 + i + 3 * j] = y11b * pe;
-      B[O_B12 + i + 3 * j] = y12b * pe;
-      B[O_C11 + i + 3 * j] = x11c * ee + y11c * (d - ee);
-      B[O_C12 + i + 3 * j] = x12c * ee + y12c * (d - ee);
-    }
-  double g11[27], g12[27], h11[27], h12[27];
-  for (int k = 0; k < 3; k++)
-    for (int j = 0; j < 3; j++)
-      for (int i = 0; i < 3; i++) {
-        const double t1 = (e[i] * e[j] - kd(i, j) / 3.0) * e[k];
-        const double t2 = e[i] * kd(j, k) + e[j] * kd(i, k) - 2 * e[i] * e[j] * e[k];
-        const int q = i + 3 * j + 9 * k;
-        g11[q] = x11g * t1 + y11g * t2;
-        g12[q] = x12g * t1 + y12g * t2;
-        const double pik = eps3(i, k, 0) * e[0] + eps3(i, k, 1) * e[1] + eps3(i, k, 2) * e[2];
-        const double pjk = eps3(j, k, 0) * e[0] + eps3(j, k, 1) * e[1] + eps3(j, k, 2) * e[2];
-        h11[q] = y11h * (pik * e[j] + pjk * e[i]);
-        h12[q] = y12h * (pik * e[j] + pjk * e[i]);
-      }
-  front_y2(g11, B + O_G11);
-  front_y2(g12, B + O_G12);
-  front_y2(h11, B + O_H11);
-  front_y2(h12, B + O_H12);
-  // mlub (hydro_lub.f90:136-142) projected on Y2 x Y2 (DD_transY2)
-  double mm[25];
-  for (int x = 0; x < 25; x++) mm[x] = 0.0;
-  for (int l = 0; l < 3; l++)
-    for (int k = 0; k < 3; k++)
-      for (int j = 0; j < 3; j++)
-        for (int i = 0; i < 3; i++) {
-          const double t = xm * (3.0 * (e[i] * e[j] - kd(i, j) / 3.0) * (e[k] * e[l] - kd(k, l) / 3.0) / 2.0) +
-                           ym * (e[i] * kd(j, l) * e[k] + e[j] * kd(i, l) * e[k] + e[i] * kd(j, k) * e[l] +
-                                 e[j] * kd(i, k) * e[l] - 4.0 * e[i] * e[j] * e[k] * e[l]) / 2.0 +
-                           zm * (kd(i, k) * kd(j, l) + kd(j, k) * kd(i, l) - kd(i, j) * kd(k, l) + e[i] * e[j] * kd(k, l) +
-                                 kd(i, j) * e[k] * e[l] - e[i] * kd(j, l) * e[k] - e[j] * kd(i, l) * e[k] -
-                                 e[i] * kd(j, k) * e[l] - e[j] * kd(i, k) * e[l] + e[i] * e[j] * e[k] * e[l]) / 2.0;
-          if (t == 0.0) continue;
-          for (int x = 0; x < 5; x++) {
-            const double yx = c_Y2[x + 5 * (i + 3 * j)];
-            if (yx == 0.0) continue;
-            for (int y = 0; y < 5; y++) mm[x + 5 * y] += t * yx * c_Y2[y + 5 * (k + 3 * l)];
-          }
-        }
-  for (int x = 0; x < 25; x++) B[O_M + x] = mm[x];
+  pair_tensors(o, e, blk + (size_t)p * PB);
 }
 
 __device__ inline void lput(double* L, int64_t ld, int r, int c, double v, int acc) {
@@ -322,18 +338,16 @@ __global__ void lub_second_fill(int npair, const int2* __restrict__ pairs, const
   list2[off2[b] + atomicAdd(&cur[b], 1)] = p;
 }
 
-__global__ void lub_second_sort(int nn, const int* __restrict__ off2, int* __restrict__ list2) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nn) return;
-  for (int i = off2[u] + 1; i < off2[u + 1]; i++) {
-    const int v = list2[i];
-    int j = i - 1;
-    while (j >= off2[u] && list2[j] > v) {
-      list2[j + 1] = list2[j];
-      j--;
-    }
-    list2[j + 1] = v;
-  }
+// list2 in pair order: an entry's place is the number of smaller ones in its
+// particle's list, a thread per entry
+__global__ void lub_second_rank(int npair, const int2* __restrict__ pairs, const int* __restrict__ off2,
+                                const int* __restrict__ raw, int* __restrict__ list2) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= npair) return;
+  const int u = pairs[p].y, lo = off2[u], hi = off2[u + 1];
+  int k = lo;
+  for (int q = lo; q < hi; q++) k += raw[q] < p;
+  list2[k] = p;
 }
 
 // self block of particle u: its pairs as second particle, then as first,
@@ -355,40 +369,68 @@ __global__ void lub_self(int N, const int* __restrict__ off, const int* __restri
     self[t] = v * scale;
 }
 
-// y = L w for the sparse operator: the particle's self block, then its pairs
-// as first and as second particle.  One warp per (particle, right-hand
-// side): lane r + 11 g (r < 11, g < 2) takes row r and every other
-// neighbour block starting at g; the two halves are added by a shuffle
-// (fixed order)
-__global__ void lub_spmv_w(int N, const int* __restrict__ off, const int* __restrict__ off2,
-                           const int* __restrict__ list2, const int2* __restrict__ pairs,
-                           const double* __restrict__ blk, const double* __restrict__ self, double scale, int nr,
-                           const double* __restrict__ w, int64_t ldw, double* __restrict__ y, int64_t ldy) {
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= (int64_t)N * nr) return;
-  const int u = (int)(wid % N), col = (int)(wid / N);
-  const int r = lane % 11, g = lane / 11;
-  const double* wc = w + col * ldw;
-  double vs = 0.0, vp = 0.0;
-  if (g < 2) {
-    if (g == 0) {
-      const double* S = self + (size_t)u * 121;
-#pragma unroll
-      for (int c = 0; c < 11; c++) vs += S[r + 11 * c] * wc[gidx(N, u, c)];
-    }
-    const int p1 = off[u], n1 = off[u + 1] - p1, q2 = off2[u], n2 = off2[u + 1] - q2;
-    for (int k = g; k < n1 + n2; k += 2) {
-      const bool first = k < n1;
-      const int p = first ? p1 + k : list2[q2 + k - n1];
-      const double* B = blk + (size_t)p * PB;
-      const int o = first ? pairs[p].y : pairs[p].x;
-#pragma unroll
-      for (int c = 0; c < 11; c++) vp += pair_entry(B, r, c, first) * wc[gidx(N, o, c)];
-    }
+// Position and sign of entry (r, c) in a pair block: pair_entry as a table
+// lookup, for the block of the pair's first particle (ab) or its second.
+__device__ inline void pair_pos(int r, int c, bool ab, int* off, double* sgn) {
+  const int R = r < 3 ? 0 : (r < 6 ? 1 : 2), C = c < 3 ? 0 : (c < 6 ? 1 : 2);
+  const int i = R == 2 ? r - 6 : r - 3 * R, j = C == 2 ? c - 6 : c - 3 * C;
+  *sgn = 1.0;
+  if (R == C && R < 2) {
+    *off = (R ? O_C12 : O_A12) + (ab ? i + 3 * j : j + 3 * i);
+  } else if (R == 2 && C == 2) {
+    *off = O_M + i + 5 * j;
+  } else if (R < 2 && C < 2) {
+    *off = O_B12 + (R ? i + 3 * j : j + 3 * i);
+    *sgn = (R == 1) == ab ? 1.0 : -1.0;
+  } else {
+    const int p = R == 2 ? C : R;  // the velocity section: 0 G, 1 H
+    *off = (p ? O_H12 : O_G12) + (R == 2 ? i + 5 * j : j + 5 * i);
+    if (p == 0) *sgn = (R == 2) == ab ? 1.0 : -1.0;
   }
-  vp += __shfl_down_sync(0xffffffffu, vp, 11);
-  if (lane < 11) y[gidx(N, u, r) + col * ldy] = vs + vp * scale;
+}
+
+// y = L w for the sparse operator: the particle's self block, then its pairs
+// as first and as second particle.  One CTA per (particle, right-hand side),
+// a thread per entry (r, c) of its 11 x 11 blocks: the position in the pair
+// block is fixed per thread, a neighbour costs one multiply-add of each, and
+// the 11 columns are added at the end in a fixed order.  Bound by the FP64
+// pipe and the latency of the neighbour loop.
+__global__ void __launch_bounds__(128) lub_spmv_w(int N, const int* __restrict__ off, const int* __restrict__ off2,
+                                                  const int* __restrict__ list2, const int2* __restrict__ pairs,
+                                                  const double* __restrict__ blk, const double* __restrict__ self,
+                                                  double scale, const double* __restrict__ w, int64_t ldw,
+                                                  double* __restrict__ y, int64_t ldy) {
+  __shared__ double sv[121], pv[121];
+  const int u = blockIdx.x, t = threadIdx.x, r = t % 11, c = t / 11;
+  const double* wc = w + blockIdx.y * ldw;
+  if (t < 121) {
+    int oa, ob;
+    double sa, sb;
+    pair_pos(r, c, true, &oa, &sa);
+    pair_pos(r, c, false, &ob, &sb);
+    const int wbase = c < 3 ? c : (c < 6 ? 3 * N + c - 3 : 6 * N + c - 6), wstep = c < 6 ? 3 : 5;
+    sv[t] = self[(size_t)u * 121 + t] * wc[wbase + wstep * u];
+    double va = 0.0, vb = 0.0;
+    const int p1 = off[u + 1], q1 = off2[u + 1];
+#pragma unroll 4
+    for (int p = off[u]; p < p1; p++) va = fma(blk[(size_t)p * PB + oa], wc[wbase + wstep * pairs[p].y], va);
+#pragma unroll 4
+    for (int q = off2[u]; q < q1; q++) {
+      const int p = list2[q];
+      vb = fma(blk[(size_t)p * PB + ob], wc[wbase + wstep * pairs[p].x], vb);
+    }
+    pv[t] = sa * va + sb * vb;
+  }
+  __syncthreads();
+  if (t < 11) {
+    double vs = 0.0, vp = 0.0;
+#pragma unroll
+    for (int k = 0; k < 11; k++) {
+      vs += sv[t + 11 * k];
+      vp += pv[t + 11 * k];
+    }
+    y[gidx(N, u, t) + blockIdx.y * ldy] = vs + vp * scale;
+  }
 }
 
 // A (ld lda) += the force/torque-velocity part L_PP of the sparse
@@ -442,21 +484,6 @@ static double* lubtab_device(rsd_ctx* ctx, const rsd_lubtab* tab) {
 // list, pair blocks (unscaled), second-particle lists and contact count.
 static int lub_pair_stage(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is_period, const double* d_pos,
                           const double* d_radii, const rsd_lattice* lat, rsd_lub_sparse* sp, int* dcon) {
-  static bool y2_ready = false;
-  if (!y2_ready) {
-    double Y[45] = {0};
-    const double s2 = 1.0 / sqrt(2.0), s6 = 1.0 / sqrt(6.0);
-    auto at = [&](int m, int i, int j) -> double& { return Y[m + 5 * (i + 3 * j)]; };
-    at(0, 0, 1) = at(0, 1, 0) = s2;
-    at(1, 1, 2) = at(1, 2, 1) = -s2;
-    at(2, 0, 0) = at(2, 1, 1) = -s6;
-    at(2, 2, 2) = sqrt(2.0 / 3.0);
-    at(3, 0, 2) = at(3, 2, 0) = -s2;
-    at(4, 0, 0) = s2;
-    at(4, 1, 1) = -s2;
-    RSD_CUDA(ctx, cudaMemcpyToSymbol(c_Y2, Y, sizeof Y));
-    y2_ready = true;
-  }
   double* dt = lubtab_device(ctx, tab);
   if (!dt) return rsd_fail(ctx, RSD_ENOMEM, "lub table upload failed");
   lub_dev_tab T{dt, dt + 64 * 11, dt + 64 * 18, tab->nabc, tab->ngh, tab->nm};
@@ -465,8 +492,8 @@ static int lub_pair_stage(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, i
   int* cnt = (int*)rsd_scratch(ctx, "lub_count", sizeof(int) * (nn + 1));
   int* off = (int*)rsd_scratch(ctx, "lub_off", sizeof(int) * (nn + 1));
   if (!cnt || !off) return RSD_ENOMEM;
-  const int wpb = 8;
-  lub_count<<<(nn + wpb - 1) / wpb, 32 * wpb, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, cnt); RSD_LAUNCH_NOTE();
+  const unsigned ng = (unsigned)((nn + LUB_WARPS - 1) / LUB_WARPS);
+  lub_near<false><<<ng, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, cnt, nullptr, nullptr); RSD_LAUNCH_NOTE();
   lub_scan<<<1, 1024, 0, s>>>(nn, cnt, off); RSD_LAUNCH_NOTE();
   int npair = 0;
   RSD_CUDA(ctx, cudaMemcpyAsync(&npair, off + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -476,18 +503,19 @@ static int lub_pair_stage(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, i
   int* cnt2 = (int*)rsd_scratch(ctx, "lub_count2", sizeof(int) * (nn + 1));
   int* off2 = (int*)rsd_scratch(ctx, "lub_off2", sizeof(int) * (nn + 1));
   int* cur = (int*)rsd_scratch(ctx, "lub_cur", sizeof(int) * (nn + 1));
-  int* list2 = (int*)rsd_scratch(ctx, "lub_list2", sizeof(int) * (size_t)(npair > 0 ? npair : 1));
+  int* list2 = (int*)rsd_scratch(ctx, "lub_list2", sizeof(int) * 2 * (size_t)(npair > 0 ? npair : 1));
+  int* raw2 = list2 ? list2 + npair : nullptr;
   if (!pairs || !blk || !cnt2 || !off2 || !cur || !list2) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemsetAsync(dcon, 0, sizeof(int), s));
   RSD_CUDA(ctx, cudaMemsetAsync(cnt2, 0, sizeof(int) * (nn + 1), s));
   RSD_CUDA(ctx, cudaMemsetAsync(cur, 0, sizeof(int) * (nn + 1), s));
   if (npair > 0) {
-    lub_list<<<(nn + wpb - 1) / wpb, 32 * wpb, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, off, pairs); RSD_LAUNCH_NOTE();
-    lub_pairs<<<(npair + 127) / 128, 128, 0, s>>>(npair, T, is_period, Ld, d_pos, d_radii, pairs, blk, dcon); RSD_LAUNCH_NOTE();
+    lub_near<true><<<ng, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, nullptr, off, pairs); RSD_LAUNCH_NOTE();
+    lub_pairs<<<(npair + 31) / 32, 32, 0, s>>>(npair, T, is_period, Ld, d_pos, d_radii, pairs, blk, dcon); RSD_LAUNCH_NOTE();
     lub_second_count<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, cnt2); RSD_LAUNCH_NOTE();
     lub_scan<<<1, 1024, 0, s>>>(nn, cnt2, off2); RSD_LAUNCH_NOTE();
-    lub_second_fill<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, off2, cur, list2); RSD_LAUNCH_NOTE();
-    lub_second_sort<<<(nn + 127) / 128, 128, 0, s>>>(nn, off2, list2); RSD_LAUNCH_NOTE();
+    lub_second_fill<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, off2, cur, raw2); RSD_LAUNCH_NOTE();
+    lub_second_rank<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, off2, raw2, list2); RSD_LAUNCH_NOTE();
   } else {
     RSD_CUDA(ctx, cudaMemsetAsync(off2, 0, sizeof(int) * (nn + 1), s));
   }
@@ -544,6 +572,7 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, in
   cudaStream_t s = ctx->stream;
   RSD_TRY(lub_pair_stage(ctx, tab, nn, nb, is_period, d_pos, d_radii, lat, sp, dcon));
   sp->scale = 6.0 * (RSD_PI * mu_f);
+  sp->contacts = dcon;
   sp->self = self;
   const int64_t ts = 121LL * nn;
   lub_self<<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(nn, sp->off, sp->off2, sp->list2, sp->blk, sp->scale,
@@ -559,10 +588,8 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, in
 // y (11N x nr, grand layout, ld ldy) = L w
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy) {
-  const int64_t tot = 32LL * sp->nn * nr;  // one warp per particle and right-hand side
-  lub_spmv_w<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(sp->nn, sp->off, sp->off2, sp->list2, sp->pairs,
-                                                                      sp->blk, sp->self, sp->scale, nr, w, ldw, y,
-                                                                      ldy); RSD_LAUNCH_NOTE();
+  lub_spmv_w<<<dim3(sp->nn, nr), 128, 0, ctx->stream>>>(sp->nn, sp->off, sp->off2, sp->list2, sp->pairs, sp->blk,
+                                                        sp->self, sp->scale, w, ldw, y, ldy); RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }

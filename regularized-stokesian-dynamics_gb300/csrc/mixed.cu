@@ -30,9 +30,11 @@ template <typename T>
 int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t lda, const T* X, int64_t ldx,
              int nrhs, T beta, T* y, int64_t ldy);
 template <typename T>
-int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc);
+int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc,
+                      int* d_status = nullptr);
 template <typename T>
-int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc);
+int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc, const T* W = nullptr,
+                      int* d_err = nullptr);
 template <typename T>
 int rsd_potrs_upper_t(rsd_ctx* ctx, int n, const T* d_U, int64_t ldu, T* d_X, int64_t ldx, int nrhs, const char* tag,
                       const T* W);
@@ -53,38 +55,48 @@ __device__ __forceinline__ int grand_pid(int N, int x) {
   return x < 3 * N ? x / 3 : (x < 6 * N ? (x - 3 * N) / 3 : (x - 6 * N) / 5);
 }
 
-// M32 = M in [Q, P] order from the hi plane holding only the stored half
-// (entries whose row's particle is at most the column's; the rest is read
-// at the transposed position): 32 x 32 output tiles, the direct and the
-// transposed source tiles staged in shared memory so that reads and writes
-// stay coalesced; a tile loads only the kinds it needs.
-__device__ __forceinline__ int64_t perm_src(int N, int64_t i) {
-  const int64_t Q = 5LL * N;
-  return i < Q ? 6LL * N + i : i - Q;
+// The FP32 matrix M32 is M in [Q, P] order, Q padded to Qp (a multiple of the
+// factorisation's block, so that the diagonal blocks of U_PP are blocks of
+// the factor) and P to Pp (a multiple of 4, for 16-byte columns) with the
+// identity; np = Qp + Pp.
+struct mixed_dims {
+  int64_t P, Q, n, Qp, Pp, np;
+};
+
+// M32 from the hi plane holding only the stored half (entries whose row's
+// particle is at most the column's; the rest is read at the transposed
+// position): 32 x 32 output tiles, the direct and the transposed source tiles
+// staged in shared memory so that reads and writes stay coalesced; a tile
+// loads only the kinds it needs.
+__device__ __forceinline__ int64_t perm_src(const mixed_dims& d, int64_t i) {  // -1: padding
+  if (i < d.Qp) return i < d.Q ? d.P + i : -1;
+  return i < d.Qp + d.P ? i - d.Qp : -1;
 }
 
-__global__ void convert_perm_half(int N, int64_t n, const float* __restrict__ Mh, int64_t ld,
+__global__ void convert_perm_half(int N, mixed_dims d, const float* __restrict__ Mh, int64_t ld,
                                   float* __restrict__ M32) {
   __shared__ float D[32][33], T[32][33];
   __shared__ int64_t si[32], sj[32];
   __shared__ int pi[32], pj[32], need;
-  const int64_t I0 = (int64_t)blockIdx.x * 32, J0 = (int64_t)blockIdx.y * 32;
+  const int64_t I0 = (int64_t)blockIdx.x * 32, J0 = (int64_t)blockIdx.y * 32, n = d.np;
   const int tx = threadIdx.x, ty = threadIdx.y;
   if (ty == 0) {
-    const int64_t i = min(I0 + tx, n - 1), j = min(J0 + tx, n - 1);
-    si[tx] = perm_src(N, i);
-    sj[tx] = perm_src(N, j);
-    pi[tx] = grand_pid(N, (int)si[tx]);
-    pj[tx] = grand_pid(N, (int)sj[tx]);
+    const int64_t i = perm_src(d, I0 + tx), j = perm_src(d, J0 + tx);
+    si[tx] = i;
+    sj[tx] = j;
+    pi[tx] = i >= 0 ? grand_pid(N, (int)i) : -1;
+    pj[tx] = j >= 0 ? grand_pid(N, (int)j) : -1;
     // need: bit 0 = some entry stored directly, bit 1 = some entry transposed
-    const int imin = __reduce_min_sync(0xffffffffu, pi[tx]), imax = __reduce_max_sync(0xffffffffu, pi[tx]);
-    const int jmin = __reduce_min_sync(0xffffffffu, pj[tx]), jmax = __reduce_max_sync(0xffffffffu, pj[tx]);
+    const int big = 1 << 30;
+    const int imin = __reduce_min_sync(0xffffffffu, i >= 0 ? pi[tx] : big), imax = __reduce_max_sync(0xffffffffu, pi[tx]);
+    const int jmin = __reduce_min_sync(0xffffffffu, j >= 0 ? pj[tx] : big), jmax = __reduce_max_sync(0xffffffffu, pj[tx]);
     if (tx == 0) need = (imin <= jmax ? 1 : 0) | (imax > jmin ? 2 : 0);
   }
   __syncthreads();
   const int t = ty * 32 + tx;
-  const bool full = I0 + 32 <= n && J0 + 32 <= n && si[31] - si[0] == 31;  // rows contiguous in the source
-  if (need == 1 && full && (ld & 3) == 0 && (n & 3) == 0 && (si[0] & 3) == 0) {
+  // rows contiguous in the source and no padding in the tile
+  const bool full = si[0] >= 0 && si[31] - si[0] == 31 && sj[0] >= 0 && sj[31] - sj[0] == 31;
+  if (need == 1 && full && (n & 3) == 0 && (si[0] & 3) == 0) {
     // all in place: one 16-byte move per thread (4 rows of one column)
     const int r4 = 4 * (t & 7), k = t >> 3;
     *reinterpret_cast<float4*>(M32 + I0 + r4 + (J0 + k) * n) =
@@ -92,13 +104,20 @@ __global__ void convert_perm_half(int N, int64_t n, const float* __restrict__ Mh
     return;
   }
   for (int k = ty; k < 32; k += blockDim.y) {
-    if (need & 1) D[k][tx] = Mh[si[tx] + sj[k] * ld];  // (I0 + tx, J0 + k) in place
-    if (need & 2) T[k][tx] = Mh[sj[tx] + si[k] * ld];  // (I0 + k, J0 + tx) at the mirrored position
+    // (I0 + tx, J0 + k) in place; (I0 + k, J0 + tx) at the mirrored position
+    if ((need & 1) && si[tx] >= 0 && sj[k] >= 0) D[k][tx] = Mh[si[tx] + sj[k] * ld];
+    if ((need & 2) && sj[tx] >= 0 && si[k] >= 0) T[k][tx] = Mh[sj[tx] + si[k] * ld];
   }
   __syncthreads();
   for (int k = ty; k < 32; k += blockDim.y) {
     const int64_t i = I0 + tx, j = J0 + k;
-    if (i < n && j < n) M32[i + j * n] = pi[tx] <= pj[k] ? D[k][tx] : T[tx][k];
+    if (i >= n || j >= n) continue;
+    float v;
+    if (si[tx] < 0 || sj[k] < 0)
+      v = i == j ? 1.f : 0.f;
+    else
+      v = pi[tx] <= pj[k] ? D[k][tx] : T[tx][k];
+    M32[i + j * n] = v;
   }
 }
 
@@ -110,43 +129,15 @@ __global__ void to_dsf_vec(int64_t n, const double* __restrict__ x, float2* __re
   xs[t] = make_float2(d.hi, d.lo);
 }
 
-// part[c][r][i] = sum over the chunk c of columns p of M(i, p) x(p, r), with
-// M = hi + lo and x as float pairs, in double-single arithmetic on the FP32
-// pipe (the FP64 pipe of GB300 would bound an FP64 product at ~1/60 of the
-// FP32 rate; this one is bound by HBM).  Chunks of GEMV_PL_CHUNK columns
-// keep the double-single rounding of each partial near 2^-48 sqrt(chunk).
-constexpr int GEMV_PL_CHUNK = 512;
-template <int R>
-__global__ void gemv_planes_part(int m, int k, const float* __restrict__ Mh, const float* __restrict__ Ml, int64_t ld,
-                                 const float2* __restrict__ xs, double* __restrict__ part) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  const int p0 = c * GEMV_PL_CHUNK, p1 = min(k, p0 + GEMV_PL_CHUNK);
-  if (i >= m) return;
-  dsf acc[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) acc[r] = dsf(0);
-#pragma unroll 4
-  for (int p = p0; p < p1; p++) {
-    const int64_t o = i + (int64_t)p * ld;
-    const dsf a(Mh[o], Ml[o]);
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const float2 x = xs[p + (int64_t)r * k];
-      acc[r] = fma(a, dsf(x.x, x.y), acc[r]);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < R; r++) part[((size_t)c * R + r) * m + i] = dsf_to(acc[r]);
-}
-
 // Symmetric M f over the stored half of M's planes: the entries whose row's
 // particle is at most the column's (pair blocks in the rows of their first
 // particle, and the whole diagonal particle blocks).  A CTA takes a 128 x 128
 // tile: row products of its stored entries (-> prow[R][C]) and column
 // products of its entries strictly above the particle diagonal
 // (-> pcol[C][R]), in double-single; tiles with no stored entry write zero
-// partials.  About half of M is read.  Needs n % 4 == 0.
+// partials, in double-single arithmetic on the FP32 pipe (the FP64 pipe of
+// GB300 would bound an FP64 product at ~1/60 of the FP32 rate; this one is
+// bound by HBM).  About half of M is read.  Needs ld % 4 == 0.
 constexpr int SYMV_T = 128;
 constexpr int symv_smem(int nr) { return (int)(sizeof(dsf) * 8 * nr * SYMV_T + sizeof(float2) * nr * SYMV_T * 33); }
 template <int NR>
@@ -181,7 +172,7 @@ __global__ void __launch_bounds__(256) symv_planes_part(int N, int n, const floa
     for (int e = t; e < NR * SYMV_T; e += 256) pr[e] = pc[e] = 0.0;
     return;
   }
-  const int rb = r0 + 4 * lane;  // this lane's four rows (one section: boundaries are multiples of 4)
+  const int rb = r0 + 4 * lane;  // this lane's four rows (past n: the padding of the column)
   int prr[4];
   dsf xr[NR][4];
 #pragma unroll
@@ -194,6 +185,7 @@ __global__ void __launch_bounds__(256) symv_planes_part(int N, int n, const floa
       xr[r][k] = dsf(v.x, v.y);
     }
   }
+  const int pmin = min(min(prr[0], prr[1]), min(prr[2], prr[3]));  // a section may end among them
   dsacc racc[NR][4];
 #pragma unroll
   for (int r = 0; r < NR; r++)
@@ -207,7 +199,7 @@ __global__ void __launch_bounds__(256) symv_planes_part(int N, int n, const floa
     for (int r = 0; r < NR; r++) cacc[r] = dsacc(0);
     if (c < n) {
       const int pcn = grand_pid(N, c);
-      if (rb < n && prr[0] <= pcn) {  // the lane's rows hold stored entries of this column
+      if (rb < n && pmin <= pcn) {  // the lane's rows hold stored entries of this column
         const int64_t o = rb + (int64_t)c * ld;
         const float4 h = *reinterpret_cast<const float4*>(Mh + o), l = *reinterpret_cast<const float4*>(Ml + o);
         const dsf m[4] = {dsf(h.x, l.x), dsf(h.y, l.y), dsf(h.z, l.z), dsf(h.w, l.w)};
@@ -267,18 +259,6 @@ __global__ void symv_planes_reduce(int n, int nr, int nbt, const double* __restr
   }
 }
 
-// y(:, r) += alpha * sum_c part[c][r]
-__global__ void gemv_planes_reduce(int m, int nr, int nchunk, const double* __restrict__ part, double alpha,
-                                   double* __restrict__ y, int64_t ldy) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  for (int r = 0; r < nr; r++) {
-    double s = 0.0;
-    for (int c = 0; c < nchunk; c++) s += part[((size_t)c * nr + r) * m + i];
-    y[i + (int64_t)r * ldy] += alpha * s;
-  }
-}
-
 __global__ void copy_block_f(int64_t rows, int64_t cols, const float* __restrict__ S, int64_t lds,
                              float* __restrict__ D, int64_t ldd) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -307,90 +287,120 @@ __global__ void build_r2(int64_t P, int64_t n, int nr, const double* __restrict_
   r2[t] = fe - f[i + c * n] - Lw[i + c * n];
 }
 
-// per-column sums of squares of r1 (n), r2 (P) and of b = ([0; -EIN], Fe)
-__global__ void norms(int64_t P, int64_t n, int nr, const double* __restrict__ r1, const double* __restrict__ r2,
-                      const double* __restrict__ ein, const double* __restrict__ Fe, int have_fe,
-                      double* __restrict__ out) {
+// ---- the stationary iteration's elementwise work, fused into the four
+// kernels between its products and solves (an iteration of a small system is
+// launches and little else)
+
+// w = [U; -EIN], r1 = w, fs = f as float pairs
+__global__ void it_begin(int64_t P, int64_t Q, int nr, const double* __restrict__ U, const double* __restrict__ ein,
+                         const double* __restrict__ f, double* __restrict__ w, double* __restrict__ r1,
+                         float2* __restrict__ fs) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n = P + Q;
+  if (t >= n * nr) return;
+  const int64_t i = t % n, c = t / n;
+  w[t] = r1[t] = i < P ? U[i + c * P] : -ein[i - P];
+  const dsf d = dsf_from(f[t]);
+  fs[t] = make_float2(d.hi, d.lo);
+}
+
+// r2 = Fe_c - f_P - (Lw)_P (Fe only in column 0 when have_fe); t32 = r1 in the
+// padded [Q, P] order; per block of the grid the sums of squares of (r1, r2)
+// and of b = ([0; -EIN], Fe), added up by the host.  blockIdx.y = column.
+constexpr int IT_BLOCKS = 32;
+__global__ void __launch_bounds__(256) it_residual(mixed_dims d, const double* __restrict__ r1,
+                                                   const double* __restrict__ ein, const double* __restrict__ Fe,
+                                                   int have_fe, const double* __restrict__ f,
+                                                   const double* __restrict__ Lw, double* __restrict__ r2,
+                                                   float* __restrict__ t32, double* __restrict__ part) {
   __shared__ double sr[256], sb[256];
-  const int c = blockIdx.x;
-  double a = 0, b = 0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const double v = r1[i + c * n];
-    a += v * v;
-    if (i >= P) {
-      const double e = ein[i - P];
-      b += e * e;
+  const int c = blockIdx.y;
+  const double *r1c = r1 + c * d.n, *fc = f + c * d.n, *lc = Lw + c * d.n;
+  const bool fe = have_fe && c == 0;
+  double a = 0.0, b = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < d.np; i += (int64_t)gridDim.x * 256) {
+    const int64_t q = perm_src(d, i);
+    float o = 0.f;
+    if (q >= 0) {
+      const double v = r1c[q];
+      a += v * v;
+      o = (float)v;
+      if (q >= d.P) {
+        const double e = ein[q - d.P];
+        b += e * e;
+      } else {
+        const double g = fe ? Fe[q] : 0.0, x = g - fc[q] - lc[q];
+        r2[q + c * d.P] = x;
+        a += x * x;
+        b += g * g;
+      }
     }
-  }
-  for (int64_t i = threadIdx.x; i < P; i += blockDim.x) {
-    const double v = r2[i + c * P];
-    a += v * v;
-    if (have_fe && c == 0) b += Fe[i] * Fe[i];
+    t32[i + c * d.np] = o;
   }
   sr[threadIdx.x] = a;
   sb[threadIdx.x] = b;
   __syncthreads();
-  for (int d = 128; d > 0; d >>= 1) {
-    if (threadIdx.x < d) {
-      sr[threadIdx.x] += sr[threadIdx.x + d];
-      sb[threadIdx.x] += sb[threadIdx.x + d];
+  for (int h = 128; h > 0; h >>= 1) {
+    if (threadIdx.x < h) {
+      sr[threadIdx.x] += sr[threadIdx.x + h];
+      sb[threadIdx.x] += sb[threadIdx.x + h];
     }
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    out[2 * c] = sr[0];
-    out[2 * c + 1] = sb[0];
+    part[2 * (c * gridDim.x + blockIdx.x)] = sr[0];
+    part[2 * (c * gridDim.x + blockIdx.x) + 1] = sb[0];
   }
 }
 
-// x32' = perm(x) (FP32, [Q, P] order); x may have a zero Q part (zq)
-__global__ void to32_perm(int64_t P, int64_t Q, int nr, const double* __restrict__ x, int64_t ldx, int zq,
-                          float* __restrict__ y) {
-  const int64_t n = P + Q;
+// y = unperm(x32) (y = M^-1 r1); u32 = r2 - y_P, zero past P
+__global__ void it_velocity(mixed_dims d, int nr, const float* __restrict__ x32, const double* __restrict__ r2,
+                            double* __restrict__ y, float* __restrict__ u32) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * nr) return;
-  const int64_t i = t % n, c = t / n;
-  double v;
-  if (i < Q)
-    v = zq ? 0.0 : x[P + i + c * ldx];
-  else
-    v = x[i - Q + c * ldx];
-  y[t] = (float)v;
+  if (t >= d.np * nr) return;
+  const int64_t i = t % d.np, c = t / d.np, q = perm_src(d, i);
+  double v = 0.0;
+  if (q >= 0) {
+    v = (double)x32[t];
+    y[q + c * d.n] = v;
+  }
+  if (i >= d.Qp) u32[i - d.Qp + c * d.Pp] = q >= 0 ? (float)(r2[q + c * d.P] - v) : 0.f;
 }
 
-// y (FP64, [P, Q] order) (+)= unperm(x32')
-__global__ void from32_perm(int64_t P, int64_t Q, int nr, const float* __restrict__ x, double* __restrict__ y,
-                            int add) {
-  const int64_t n = P + Q;
+// t32 = [0; dU]
+__global__ void it_force(mixed_dims d, int nr, const float* __restrict__ du, float* __restrict__ t32) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * nr) return;
-  const int64_t i = t % n, c = t / n;
-  const double v = (double)(i < P ? x[Q + i + c * n] : x[i - P + c * n]);
-  y[i + c * n] = add ? y[i + c * n] + v : v;
+  if (t >= d.np * nr) return;
+  const int64_t i = t % d.np, c = t / d.np;
+  t32[t] = i < d.Qp ? 0.f : du[i - d.Qp + c * d.Pp];
 }
 
-// u32 = r2 - y_P
-__global__ void rhs_u(int64_t P, int64_t n, int nr, const double* __restrict__ r2, const double* __restrict__ y,
-                      float* __restrict__ u) {
+// f += y + unperm(x32), U += dU
+__global__ void it_update(mixed_dims d, int nr, const float* __restrict__ x32, const double* __restrict__ y,
+                          const float* __restrict__ du, double* __restrict__ f, double* __restrict__ U) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P * nr) return;
-  const int64_t i = t % P, c = t / P;
-  u[t] = (float)(r2[t] - y[i + c * n]);
+  if (t >= d.np * nr) return;
+  const int64_t i = t % d.np, c = t / d.np, q = perm_src(d, i);
+  if (q < 0) return;
+  f[q + c * d.n] += y[q + c * d.n] + (double)x32[t];
+  if (q < d.P) U[q + c * d.P] += (double)du[q + c * d.Pp];
 }
 
-__global__ void update_fu(int64_t P, int64_t n, int nr, const double* __restrict__ df, const float* __restrict__ du,
-                          double* __restrict__ f, double* __restrict__ U) {
+// ---- the same pieces one by one, for the GMRES below (one right-hand side)
+
+// y32 = x in the padded [Q, P] order
+__global__ void to32_perm(mixed_dims d, const double* __restrict__ x, float* __restrict__ y) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n * nr) f[t] += df[t];
-  if (t < P * nr) U[t] += (double)du[t];
+  if (t >= d.np) return;
+  const int64_t q = perm_src(d, t);
+  y[t] = q >= 0 ? (float)x[q] : 0.f;
 }
 
-// dU as an FP64 [dU; 0] vector block for the second M^-1 application
-__global__ void du_vec(int64_t P, int64_t n, int nr, const float* __restrict__ du, double* __restrict__ v) {
+// y (FP64, [P, Q] order) += unperm(x32)
+__global__ void from32_add(mixed_dims d, const float* __restrict__ x, double* __restrict__ y) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * nr) return;
-  const int64_t i = t % n, c = t / n;
-  v[t] = i < P ? (double)du[i + c * P] : 0.0;
+  if (t >= d.np) return;
+  const int64_t q = perm_src(d, t);
+  if (q >= 0) y[q] += (double)x[t];
 }
 
 // S = f_Q + (Lw)_Q of column c; U_par = U column 0
@@ -500,6 +510,16 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
                     int64_t rpp_ld) {
   cudaStream_t s = ctx->stream;
   const int64_t N = nn, n = 11 * N, P = 6 * N, Q = 5 * N;
+  mixed_dims d;
+  d.P = P;
+  d.Q = Q;
+  d.n = n;
+  // An exported RPP32 carries the rounding of its TF32 factors (1e-4), which
+  // moves with the blocks' places: it is formed without the padding, so that
+  // the training data of the learned preconditioner stay what they are.
+  d.Qp = rpp_out ? Q : (Q + 127) / 128 * 128;
+  d.Pp = rpp_out ? P : (P + 3) / 4 * 4;
+  d.np = d.Qp + d.Pp;
   const int have_fe = Fe != nullptr;
   const int nr = have_fe ? 2 : 1;
   const double tol = p->tol > 0 ? p->tol : 1e-12;
@@ -507,36 +527,40 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   // M as FP32 planes hi + lo in the buffer of the FP64 matrix (rsd_ewald_assemble)
   const float* Mh = reinterpret_cast<const float*>(M);
   const float* Ml = Mh + (size_t)ld * n;
-  const unsigned gchunks = (unsigned)((n + GEMV_PL_CHUNK - 1) / GEMV_PL_CHUNK);
-  const bool symv = n % 4 == 0 && ld % 4 == 0;
-  bool mirrored = false;
+  if (ld % 4) return rsd_fail(ctx, RSD_EARG, "mixed solve: the planes' leading dimension must be a multiple of 4");
   const int nbt = (int)((n + SYMV_T - 1) / SYMV_T);
-  if (symv)
-    RSD_CUDA(ctx, cudaFuncSetAttribute(symv_planes_part<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, symv_smem(2)));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(symv_planes_part<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, symv_smem(2)));
   float2* fs = (float2*)rsd_scratch(ctx, "mixed_fs", sizeof(float2) * (size_t)nr * n);
-  double* gpart = symv ? (double*)rsd_scratch(ctx, "mixed_symv_part", sizeof(double) * 2 * 2 * (size_t)nbt * nbt * SYMV_T)
-                       : (double*)rsd_scratch(ctx, "mixed_gemv_part", sizeof(double) * (size_t)gchunks * nr * n);
+  double* gpart = (double*)rsd_scratch(ctx, "mixed_symv_part", sizeof(double) * 2 * 2 * (size_t)nbt * nbt * SYMV_T);
   if (!fs || !gpart) return RSD_ENOMEM;
-  float* M32 = (float*)rsd_scratch(ctx, "mixed_M32", sizeof(float) * n * n);
-  float* A32 = (float*)rsd_scratch(ctx, "mixed_A32", sizeof(float) * P * P);
-  double* V = (double*)rsd_scratch(ctx, "mixed_vec", sizeof(double) * (size_t)nr * (7 * n + 2 * P) + 64 * 8);
-  float* V32 = (float*)rsd_scratch(ctx, "mixed_vec32", sizeof(float) * (size_t)nr * (2 * n + 2 * P));
+  float* M32 = (float*)rsd_scratch(ctx, "mixed_M32", sizeof(float) * d.np * d.np);
+  float* A32 = (float*)rsd_scratch(ctx, "mixed_A32", sizeof(float) * d.Pp * d.Pp);
+  const size_t nvec = (size_t)nr * (5 * n + 2 * P) + 2 * 2 * IT_BLOCKS;
+  double* V = (double*)rsd_scratch(ctx, "mixed_vec", sizeof(double) * nvec);
+  float* V32 = (float*)rsd_scratch(ctx, "mixed_vec32", sizeof(float) * (size_t)nr * (2 * d.np + 2 * d.Pp));
   if (!M32 || !A32 || !V || !V32) return RSD_ENOMEM;
   double *f = V, *U = f + nr * n, *w = U + nr * P, *r1 = w + nr * n, *Lw = r1 + nr * n, *r2 = Lw + nr * n,
-         *y = r2 + nr * P, *y2 = y + nr * n, *dv = y2 + nr * n, *nrm = dv + nr * n;
-  float *t32 = V32, *u32 = V32 + nr * n, *ywork = u32 + nr * P;
+         *y = r2 + nr * P, *nrm = y + nr * n;
+  float *t32 = V32, *x32 = t32 + nr * d.np, *u32 = x32 + nr * d.np, *du32 = u32 + nr * d.Pp;
+  // Status words of the factorisations, read once with the first residual (a
+  // failed factor leaves values that nothing branches on): info and timeout
+  // of the factor of M', timeout of the inverse, info and timeout of the
+  // factor of RPP, timeouts of the block-scaled factors, contacts.
+  int* st = ctx->d_info + 16;
+  RSD_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(int) * 8, s));
   // sparse FP64 lubrication operator (R_lub - R_2B in the grand layout)
-  int nc = 0;
   rsd_lub_sparse lub;
-  if (p->use_lub) RSD_TRY(rsd_lub_build_sparse(ctx, tab, nn, p->nb, 1, d_pos, d_radii, lat, p->mu_f, &lub, &nc));
-  info->n_contact = nc;
+  info->n_contact = 0;
+  if (p->use_lub) {
+    RSD_TRY(rsd_lub_build_sparse(ctx, tab, nn, p->nb, 1, d_pos, d_radii, lat, p->mu_f, &lub, nullptr));
+    RSD_CUDA(ctx, cudaMemcpyAsync(st + 7, lub.contacts, sizeof(int), cudaMemcpyDeviceToDevice, s));
+  }
   cudaEventRecord(ctx->ev[6], s);
   // FP32 factor of M' (stresslets first)
   {
-    const dim3 tg((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32));
-    convert_perm_half<<<tg, dim3(32, 8), 0, s>>>(nn, n, Mh, ld, M32); RSD_LAUNCH_NOTE();
+    const unsigned nt = (unsigned)((d.np + 31) / 32);
+    convert_perm_half<<<dim3(nt, nt), dim3(32, 8), 0, s>>>(nn, d, Mh, ld, M32); RSD_LAUNCH_NOTE();
   }
-  int inf = 0;
   // Tensor-core precision per factor.  The refinement contracts by about the
   // preconditioner's relative error times the condition number it meets:
   // cond(M') is moderate, so TF32 (2^-11) suffices for the factor of M' and
@@ -544,36 +568,64 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   // with 3xTF32 there, for half the inverse's time); the factor of RPP meets
   // cond(RPP), which grows like the inverse lubrication gap, and uses 3xTF32
   // (about 2^-21, close to FP32; TF32 there takes ~17 iterations).
-  RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)n, M32, n, &inf, "m32", ctx->use_tc == 3 ? 3 : 1));
-  if (inf) {
-    info->info = inf;
-    return rsd_fail(ctx, inf, "FP32 factor of the grand mobility: leading minor %d not positive", inf);
-  }
+  int inf = 0;
+  RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)d.np, M32, d.np, &inf, "m32", ctx->use_tc == 3 ? 3 : 1, st));
+  const float* W128 = rsd_potrf_inverses_s(ctx, (int)d.np, "m32");
   float* W_m = nullptr;
-  RSD_TRY(rsd_wide_inverses_s(ctx, (int)n, M32, n, "m32", rsd_potrf_inverses_s(ctx, (int)n, "m32"), &W_m));
-  // block-scaled factors for one-launch-per-block refinement solves (the
-  // tensor-core GEMMs that form them need leading dimensions divisible by 4)
+  if (!rpp_out) RSD_TRY(rsd_wide_inverses_s(ctx, (int)d.np, M32, d.np, "m32", W128, &W_m));
+  // block-scaled factors for one-launch-per-block refinement solves
   rsd_uhat uh_m, uh_r;
-  const bool use_uh = ctx->use_tc && n % 4 == 0 && P % 4 == 0 && !rpp_out;
-  if (use_uh) RSD_TRY(rsd_uhat_build(ctx, (int)n, M32, n, W_m, "m32", &uh_m));
+  const bool use_uh = ctx->use_tc && !rpp_out;
+  if (use_uh) RSD_TRY(rsd_uhat_build(ctx, (int)d.np, M32, d.np, W_m, "m32", &uh_m, st + 5));
   // A^-1 from the trailing factor block, then RPP32 = A^-1 + rfu and its factor
-  copy_block_f<<<nblk(P * P), 256, 0, s>>>(P, P, M32 + Q + Q * n, n, A32, P); RSD_LAUNCH_NOTE();
-  RSD_TRY(rsd_potri_upper_t<float>(ctx, (int)P, A32, P, "a32", ctx->use_tc == 3 ? 3 : 1));
-  RSD_TRY(rsd_mirror_upper_t<float>(ctx, (int)P, A32, P));
-  if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f32(ctx, &lub, A32, P));
-  if (rpp_out) {
-    RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(float) * rpp_ld, A32, sizeof(float) * P, sizeof(float) * P, P,
-                                    cudaMemcpyDeviceToDevice, s));
-    return RSD_OK;
-  }
-  RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)P, A32, P, &inf, "rpp32", 3));
-  if (inf) {
-    info->info = inf;
-    return rsd_fail(ctx, inf, "FP32 factor of RPP: leading minor %d not positive", inf);
-  }
+  copy_block_f<<<nblk(d.Pp * d.Pp), 256, 0, s>>>(d.Pp, d.Pp, M32 + d.Qp * (d.np + 1), d.np, A32, d.Pp); RSD_LAUNCH_NOTE();
+  RSD_TRY(rsd_potri_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp, "a32", ctx->use_tc == 3 ? 3 : 1,
+                                   rpp_out ? nullptr : W128 + (size_t)(d.Qp / 128) * 128 * 128, st + 2));
+  RSD_TRY(rsd_mirror_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp));
+  if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f32(ctx, &lub, A32, d.Pp));
+  if (!rpp_out) RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp, &inf, "rpp32", 3, st + 3));
   float* W_r = nullptr;
-  RSD_TRY(rsd_wide_inverses_s(ctx, (int)P, A32, P, "rpp32", rsd_potrf_inverses_s(ctx, (int)P, "rpp32"), &W_r));
-  if (use_uh) RSD_TRY(rsd_uhat_build(ctx, (int)P, A32, P, W_r, "rpp32", &uh_r));
+  if (!rpp_out)
+    RSD_TRY(rsd_wide_inverses_s(ctx, (int)d.Pp, A32, d.Pp, "rpp32", rsd_potrf_inverses_s(ctx, (int)d.Pp, "rpp32"), &W_r));
+  if (use_uh) RSD_TRY(rsd_uhat_build(ctx, (int)d.Pp, A32, d.Pp, W_r, "rpp32", &uh_r, st + 6));
+  // the status words, once the stream has been waited for
+  auto status = [&]() -> int {
+    const int* h = ctx->h_info + 16;
+    info->n_contact = h[7];
+    if (h[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "potrf: tensor-core update timed out (code %d)", h[1]);
+    if (h[0]) {  // in [Q, P] order without the padding
+      info->info = h[0] > d.Qp ? h[0] - (int)(d.Qp - d.Q) : h[0];
+      return rsd_fail(ctx, info->info, "FP32 factor of the grand mobility: leading minor %d not positive", info->info);
+    }
+    if (h[2]) return rsd_fail(ctx, RSD_ETIMEOUT, "potri: tensor-core GEMM timed out (code %d)", h[2]);
+    if (h[4]) return rsd_fail(ctx, RSD_ETIMEOUT, "potrf: tensor-core update timed out (code %d)", h[4]);
+    if (h[3]) {
+      info->info = h[3];
+      return rsd_fail(ctx, h[3], "FP32 factor of RPP: leading minor %d not positive", h[3]);
+    }
+    if (h[5] || h[6]) return rsd_fail(ctx, RSD_ETIMEOUT, "uhat: tensor-core GEMM timed out");
+    return RSD_OK;
+  };
+  auto read_status = [&]() -> int {
+    RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 16, st, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+    return RSD_OK;
+  };
+  if (rpp_out) {
+    RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(float) * rpp_ld, A32, sizeof(float) * d.Pp, sizeof(float) * P, P,
+                                    cudaMemcpyDeviceToDevice, s));
+    RSD_TRY(read_status());
+    RSD_CUDA(ctx, cudaStreamSynchronize(s));
+    return status();
+  }
+  // the solves with the two factors: X (overwritten) -> Y
+  auto solve_m = [&](float* X, int cols, float* Y, int zero_lead) -> int {
+    if (use_uh) return rsd_uhat_solve(ctx, &uh_m, X, d.np, cols, Y, zero_lead);
+    return rsd_potrs_wide_s(ctx, (int)d.np, M32, d.np, W_m, X, d.np, cols, Y);
+  };
+  auto solve_r = [&](float* X, int cols, float* Y) -> int {
+    if (use_uh) return rsd_uhat_solve(ctx, &uh_r, X, d.Pp, cols, Y);
+    return rsd_potrs_wide_s(ctx, (int)d.Pp, A32, d.Pp, W_r, X, d.Pp, cols, Y);
+  };
   // refinement
   int* tri_err = rsd_uhat_error_flag(ctx);
   if (!tri_err) return RSD_ENOMEM;
@@ -594,21 +646,14 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     if (!hacc || !hbuf || !Lz) return RSD_ENOMEM;
     RSD_CUDA(ctx, cudaMemsetAsync(f, 0, sizeof(double) * nr * n, s));
     RSD_CUDA(ctx, cudaMemsetAsync(U, 0, sizeof(double) * nr * P, s));
+    double* dv = (double*)rsd_scratch(ctx, "gm_dv", sizeof(double) * (size_t)n);
+    if (!dv) return RSD_ENOMEM;
     // the product M v (FP64 v of length n, planes in double-single) into out (added)
     auto symv_add = [&](const double* v, double* out) -> int {
       to_dsf_vec<<<nblk(n), 256, 0, s>>>(n, v, fs); RSD_LAUNCH_NOTE();
-      if (symv) {
-        double* pcol = gpart + (size_t)nbt * nbt * SYMV_T;
-        symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
-        symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, 1, nbt, gpart, pcol, 1.0, out, n); RSD_LAUNCH_NOTE();
-      } else {
-        if (!mirrored) {
-          RSD_TRY(rsd_mirror_planes(ctx, nn, M, ld));
-          mirrored = true;
-        }
-        gemv_planes_part<1><<<dim3((unsigned)((n + 255) / 256), gchunks), 256, 0, s>>>((int)n, (int)n, Mh, Ml, ld, fs, gpart); RSD_LAUNCH_NOTE();
-        gemv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, 1, gchunks, gpart, 1.0, out, n); RSD_LAUNCH_NOTE();
-      }
+      double* pcol = gpart + (size_t)nbt * nbt * SYMV_T;
+      symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
+      symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, 1, nbt, gpart, pcol, 1.0, out, n); RSD_LAUNCH_NOTE();
       return RSD_OK;
     };
     // residual of column c: (r1, r2) = b - A x into out (length n + P);
@@ -629,25 +674,14 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     };
     // z = P v (v, z of length n + P)
     auto precond = [&](const double* v, double* z) -> int {
-      to32_perm<<<nblk(n), 256, 0, s>>>(P, Q, 1, v, n, 0, t32); RSD_LAUNCH_NOTE();
-      if (use_uh)
-        RSD_TRY(rsd_uhat_solve(ctx, &uh_m, t32, n, 1, ywork));
-      else
-        RSD_TRY(rsd_potrs_wide_s(ctx, (int)n, M32, n, W_m, t32, n, 1, ywork));
-      from32_perm<<<nblk(n), 256, 0, s>>>(P, Q, 1, t32, z, 0); RSD_LAUNCH_NOTE();  // y = M^-1 v1
-      rhs_u<<<nblk(P), 256, 0, s>>>(P, n, 1, v + n, z, u32); RSD_LAUNCH_NOTE();
-      if (use_uh)
-        RSD_TRY(rsd_uhat_solve(ctx, &uh_r, u32, P, 1, ywork));
-      else
-        RSD_TRY(rsd_potrs_wide_s(ctx, (int)P, A32, P, W_r, u32, P, 1, ywork));
-      du_vec<<<nblk(n), 256, 0, s>>>(P, n, 1, u32, dv); RSD_LAUNCH_NOTE();
-      to32_perm<<<nblk(n), 256, 0, s>>>(P, Q, 1, dv, n, 1, t32); RSD_LAUNCH_NOTE();
-      if (use_uh)
-        RSD_TRY(rsd_uhat_solve(ctx, &uh_m, t32, n, 1, ywork, (int)Q));
-      else
-        RSD_TRY(rsd_potrs_wide_s(ctx, (int)n, M32, n, W_m, t32, n, 1, ywork));
-      from32_perm<<<nblk(n), 256, 0, s>>>(P, Q, 1, t32, z, 1); RSD_LAUNCH_NOTE();  // df
-      gm_f2d<<<nblk(P), 256, 0, s>>>(P, u32, z + n); RSD_LAUNCH_NOTE();           // dU
+      to32_perm<<<nblk(d.np), 256, 0, s>>>(d, v, t32); RSD_LAUNCH_NOTE();
+      RSD_TRY(solve_m(t32, 1, x32, 0));
+      it_velocity<<<nblk(d.np), 256, 0, s>>>(d, 1, x32, v + n, z, u32); RSD_LAUNCH_NOTE();  // y = M^-1 v1
+      RSD_TRY(solve_r(u32, 1, du32));
+      it_force<<<nblk(d.np), 256, 0, s>>>(d, 1, du32, t32); RSD_LAUNCH_NOTE();
+      RSD_TRY(solve_m(t32, 1, x32, (int)d.Qp));
+      from32_add<<<nblk(d.np), 256, 0, s>>>(d, x32, z); RSD_LAUNCH_NOTE();          // df
+      gm_f2d<<<nblk(P), 256, 0, s>>>(P, du32, z + n); RSD_LAUNCH_NOTE();             // dU
       return RSD_OK;
     };
     // a = A z
@@ -666,11 +700,17 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     // |b_c|: b = ([0; -EIN], Fe_c)
     std::vector<double> bnorm(nr);
     {
-      norms<<<nr, 256, 0, s>>>(P, n, nr, r1, r2, ein, Fe, have_fe, nrm); RSD_LAUNCH_NOTE();  // b part only is used
-      std::vector<double> hb(2 * nr);
-      RSD_CUDA(ctx, cudaMemcpyAsync(hb.data(), nrm, sizeof(double) * 2 * nr, cudaMemcpyDeviceToHost, s));
+      it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();  // b part only is used
+      std::vector<double> hb(2 * nr * IT_BLOCKS);
+      RSD_CUDA(ctx, cudaMemcpyAsync(hb.data(), nrm, sizeof(double) * hb.size(), cudaMemcpyDeviceToHost, s));
+      RSD_TRY(read_status());
       RSD_CUDA(ctx, cudaStreamSynchronize(s));
-      for (int c = 0; c < nr; c++) bnorm[c] = sqrt(hb[2 * c + 1]) > 0 ? sqrt(hb[2 * c + 1]) : 1.0;
+      RSD_TRY(status());
+      for (int c = 0; c < nr; c++) {
+        double b2 = 0.0;
+        for (int k = 0; k < IT_BLOCKS; k++) b2 += hb[2 * (c * IT_BLOCKS + k) + 1];
+        bnorm[c] = b2 > 0 ? sqrt(b2) : 1.0;
+      }
     }
     int total_it = 0;
     double worst = 0.0;
@@ -773,47 +813,38 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   RSD_CUDA(ctx, cudaMemsetAsync(U, 0, sizeof(double) * nr * P, s));
   double worst = 0.0, best_res = INFINITY;
   int it = 0;
-  std::vector<double> hn(2 * nr), hist;
+  std::vector<double> hn(2 * nr * IT_BLOCKS), hist;
   for (;; it++) {
-    build_w<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, U, ein, w); RSD_LAUNCH_NOTE();
-    RSD_CUDA(ctx, cudaMemcpyAsync(r1, w, sizeof(double) * nr * n, cudaMemcpyDeviceToDevice, s));
-    // r1 -= M f, double-single products of the two planes
-    to_dsf_vec<<<nblk(n * nr), 256, 0, s>>>(n * nr, f, fs); RSD_LAUNCH_NOTE();
-    if (symv) {  // both right-hand sides in one pass over the stored half of M
-      double* pcol = gpart + (size_t)nbt * nbt * SYMV_T * nr;
-      if (nr == 2) {
-        symv_planes_part<2><<<dim3(nbt, nbt), 256, symv_smem(2), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
-      } else {
-        symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
-      }
-      symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, nr, nbt, gpart, pcol, -1.0, r1, n); RSD_LAUNCH_NOTE();
+    it_begin<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, U, ein, f, w, r1, fs); RSD_LAUNCH_NOTE();
+    // r1 -= M f, double-single products of the two planes, both right-hand
+    // sides in one pass over the stored half of M
+    double* pcol = gpart + (size_t)nbt * nbt * SYMV_T * nr;
+    if (nr == 2) {
+      symv_planes_part<2><<<dim3(nbt, nbt), 256, symv_smem(2), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
     } else {
-      // full product: the mirrored entries are filled in first
-      if (!mirrored) {
-        RSD_TRY(rsd_mirror_planes(ctx, nn, M, ld));
-        mirrored = true;
-      }
-      if (nr == 1) {
-        gemv_planes_part<1><<<dim3((unsigned)((n + 255) / 256), gchunks), 256, 0, s>>>((int)n, (int)n, Mh, Ml, ld, fs, gpart); RSD_LAUNCH_NOTE();
-      } else {
-        gemv_planes_part<2><<<dim3((unsigned)((n + 255) / 256), gchunks), 256, 0, s>>>((int)n, (int)n, Mh, Ml, ld, fs, gpart); RSD_LAUNCH_NOTE();
-      }
-      gemv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, nr, gchunks, gpart, -1.0, r1, n); RSD_LAUNCH_NOTE();
+      symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
     }
+    symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, nr, nbt, gpart, pcol, -1.0, r1, n); RSD_LAUNCH_NOTE();
     if (p->use_lub) {
       RSD_TRY(rsd_lub_spmv(ctx, &lub, nr, w, n, Lw, n));
     } else {
       RSD_CUDA(ctx, cudaMemsetAsync(Lw, 0, sizeof(double) * nr * n, s));
     }
-    build_r2<<<nblk(P * nr), 256, 0, s>>>(P, n, nr, Fe, have_fe, f, Lw, r2); RSD_LAUNCH_NOTE();
-    norms<<<nr, 256, 0, s>>>(P, n, nr, r1, r2, ein, Fe, have_fe, nrm); RSD_LAUNCH_NOTE();
-    RSD_CUDA(ctx, cudaMemcpyAsync(hn.data(), nrm, sizeof(double) * 2 * nr, cudaMemcpyDeviceToHost, s));
+    it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();
+    RSD_CUDA(ctx, cudaMemcpyAsync(hn.data(), nrm, sizeof(double) * hn.size(), cudaMemcpyDeviceToHost, s));
     RSD_CUDA(ctx, cudaMemcpyAsync(&h_tri_err, tri_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (it == 0) RSD_TRY(read_status());
     RSD_CUDA(ctx, cudaStreamSynchronize(s));
+    if (it == 0) RSD_TRY(status());
     if (h_tri_err) return rsd_fail(ctx, RSD_ETIMEOUT, "refinement: a triangular sweep's wait timed out");
     worst = 0.0;
     for (int c = 0; c < nr; c++) {
-      const double rr = sqrt(hn[2 * c]) / (sqrt(hn[2 * c + 1]) > 0 ? sqrt(hn[2 * c + 1]) : 1.0);
+      double a2 = 0.0, b2 = 0.0;
+      for (int k = 0; k < IT_BLOCKS; k++) {
+        a2 += hn[2 * (c * IT_BLOCKS + k)];
+        b2 += hn[2 * (c * IT_BLOCKS + k) + 1];
+      }
+      const double rr = sqrt(a2) / (sqrt(b2) > 0 ? sqrt(b2) : 1.0);
       worst = std::isfinite(rr) ? fmax(worst, rr) : INFINITY;
     }
     if (worst <= tol || it >= maxit) break;
@@ -830,28 +861,12 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     // further); the reported residual is the one reached.
     hist.push_back(worst);
     if (it >= 2 && worst <= 100.0 * tol && worst > 0.5 * fmin(hist[it - 1], hist[it - 2])) break;
-    // y = M^-1 r1
-    to32_perm<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, r1, n, 0, t32); RSD_LAUNCH_NOTE();
-    if (use_uh)
-      RSD_TRY(rsd_uhat_solve(ctx, &uh_m, t32, n, nr, ywork));
-    else
-      RSD_TRY(rsd_potrs_wide_s(ctx, (int)n, M32, n, W_m, t32, n, nr, ywork));
-    from32_perm<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, t32, y, 0); RSD_LAUNCH_NOTE();
-    // dU = RPP^-1 (r2 - y_P)
-    rhs_u<<<nblk(P * nr), 256, 0, s>>>(P, n, nr, r2, y, u32); RSD_LAUNCH_NOTE();
-    if (use_uh)
-      RSD_TRY(rsd_uhat_solve(ctx, &uh_r, u32, P, nr, ywork));
-    else
-      RSD_TRY(rsd_potrs_wide_s(ctx, (int)P, A32, P, W_r, u32, P, nr, ywork));
-    // df = y + M^-1 [dU; 0]
-    du_vec<<<nblk(n * nr), 256, 0, s>>>(P, n, nr, u32, dv); RSD_LAUNCH_NOTE();
-    to32_perm<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, dv, n, 1, t32); RSD_LAUNCH_NOTE();
-    if (use_uh)
-      RSD_TRY(rsd_uhat_solve(ctx, &uh_m, t32, n, nr, ywork, (int)Q));
-    else
-      RSD_TRY(rsd_potrs_wide_s(ctx, (int)n, M32, n, W_m, t32, n, nr, ywork));
-    from32_perm<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, t32, y, 1); RSD_LAUNCH_NOTE();
-    update_fu<<<nblk(n * nr), 256, 0, s>>>(P, n, nr, y, u32, f, U); RSD_LAUNCH_NOTE();
+    RSD_TRY(solve_m(t32, nr, x32, 0));  // y = M^-1 r1
+    it_velocity<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, x32, r2, y, u32); RSD_LAUNCH_NOTE();
+    RSD_TRY(solve_r(u32, nr, du32));    // dU = RPP^-1 (r2 - y_P)
+    it_force<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, du32, t32); RSD_LAUNCH_NOTE();
+    RSD_TRY(solve_m(t32, nr, x32, (int)d.Qp));
+    it_update<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, x32, y, du32, f, U); RSD_LAUNCH_NOTE();  // df = y + M^-1 [dU; 0]
   }
   if (!(worst <= accept)) {
     // diverged or stalled above the band: flexible GMRES from zero over the

@@ -169,11 +169,10 @@ __host__ __device__ inline void rsd_skew_shift_f32(const float* LR, const float*
 // ldm).  RSD_PREC_MIXED: the same buffer holds it as two FP32 planes, hi at
 // (float*)d_M and lo at (float*)d_M + ldm * 11 nn, both with ld ldm, and
 // only the entries whose row's particle is at most the column's are written
-// (M is symmetric); rsd_mirror_planes fills the others.
+// (M is symmetric; its readers take the others at the mirrored position).
 // h_radii: the radii on the host.
 int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
                        double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm);
-int rsd_mirror_planes(rsd_ctx* ctx, int nn, double* d_M, int64_t ldm);
 int rsd_count_overlaps(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
                        int* count);
 // Adds the overlap correction of correction_method 1 or 2 (GRPY_YZD.f90:
@@ -195,6 +194,7 @@ struct rsd_lub_sparse {
   const double* blk = nullptr;
   const int *off = nullptr, *off2 = nullptr, *list2 = nullptr;
   const double* self = nullptr;
+  const int* contacts = nullptr;  // device word: pairs found at s <= 2
   double scale = 0.0;
 };
 int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is_period, const double* d_pos,
@@ -257,7 +257,8 @@ struct rsd_uhat {
   int64_t ld = 0;
   const float* G = nullptr;
 };
-int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float* W2, const char* tag, rsd_uhat* out);
+int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float* W2, const char* tag, rsd_uhat* out,
+                   int* err);
 // zero_lead: the number of leading entries of X known to be zero (the
 // forward sweep skips the whole zero blocks)
 int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int nrhs, float* Y, int zero_lead = 0);

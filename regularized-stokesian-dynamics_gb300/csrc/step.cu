@@ -216,7 +216,9 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   loc.phi = lat.phi;
   loc.LV = lat.LV;
   if (lat_out) *lat_out = lat;
-  double* M = (double*)rsd_scratch(ctx, "step_M", sizeof(double) * n * n);
+  // the mixed form's planes have 16-byte aligned columns
+  const int64_t ldm = p->precision == RSD_PREC_MIXED ? (n + 3) / 4 * 4 : n;
+  double* M = (double*)rsd_scratch(ctx, "step_M", sizeof(double) * ldm * n);
   double* V = (double*)rsd_scratch(ctx, "step_vec", sizeof(double) * (4 * P + 4 * Q + 1024));
   if (!M || !V) return RSD_ENOMEM;
   double* X = V;               // P x 2
@@ -239,19 +241,19 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   {
     // grand mobility
     rsd_range r("rsd_assembly");
-    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, radii.data(), M, n));
+    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, radii.data(), M, ldm));
     if (ctx->correction_method) {  // overlap corrections (per_GRPY_YZD.f90:98-116)
       int nov = 0;
       RSD_TRY(rsd_count_overlaps(ctx, nn, d_conf, d_radii, &lat, &nov));
       RSD_TRY(rsd_overlap_correct(ctx, ctx->correction_method, p->precision, nn, d_conf, d_radii, &lat, p->mu_f, nov,
-                                  M, n));
+                                  M, ldm));
     }
   }
   cudaEventRecord(ctx->ev[1], s);
   // averageU on APP before it is overwritten
   const bool planes = p->precision == RSD_PREC_MIXED;
   const float* Mh = planes ? reinterpret_cast<const float*>(M) : nullptr;
-  sum_app_xx<<<256, 256, 0, s>>>(nn, M, Mh, planes ? Mh + (size_t)n * n : nullptr, n, red); RSD_LAUNCH_NOTE();
+  sum_app_xx<<<256, 256, 0, s>>>(nn, M, Mh, planes ? Mh + (size_t)ldm * n : nullptr, ldm, red); RSD_LAUNCH_NOTE();
   std::vector<double> hred(256);
   RSD_CUDA(ctx, cudaMemcpyAsync(hred.data(), red, 256 * sizeof(double), cudaMemcpyDeviceToHost, s));
   int info_m = 0;
@@ -340,7 +342,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     cudaEventRecord(ctx->ev[2], s);
     {
       rsd_range r("rsd_solve");
-      RSD_TRY(rsd_mixed_solve(ctx, nn, M, n, d_conf, d_radii, &lat, tab, p, ein, d_Fe ? Fe : nullptr, Upar, S, &loc,
+      RSD_TRY(rsd_mixed_solve(ctx, nn, M, ldm, d_conf, d_radii, &lat, tab, p, ein, d_Fe ? Fe : nullptr, Upar, S, &loc,
                               (float*)rpp_out, rpp_ld));
     }
     if (rpp_out) {
