@@ -114,44 +114,70 @@ __device__ inline bool lp_pair(const rsd_lat_dev& L, const double* pos, const do
   return dmin < (double)LP_CUT * ab;
 }
 
-__global__ void lp_count(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
-                         int* __restrict__ cnt) {
-  const int a = blockIdx.x;
-  int c = 0;
-  for (int b = threadIdx.x; b < nn; b += blockDim.x) {
-    double g;
-    if (b != a && lp_pair(L, pos, radii, a, b, &g)) c++;
-  }
-  __shared__ int red[256];
-  red[threadIdx.x] = c;
-  __syncthreads();
-  for (int d = blockDim.x / 2; d > 0; d >>= 1) {
-    if (threadIdx.x < d) red[threadIdx.x] += red[threadIdx.x + d];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) cnt[a] = red[0];
-}
-
-// one warp per destination: the sources in ascending order (ballot + prefix)
-__global__ void lp_fill(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
-                        const int* __restrict__ off, int* __restrict__ src, int* __restrict__ dst,
-                        float* __restrict__ gap) {
-  const int a = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+// The sources of a destination in ascending order, one warp per destination:
+// lanes screen 32 particles at a time in FP32 (with a margin) and the
+// survivors are collected, so that the FP64 test (a warp issues an FP64
+// instruction every 64 cycles) runs over full warps of them.  FILL: the edges
+// are written from off[a] on; otherwise they are counted.
+constexpr int GR_WARPS = 8, GR_CAND = 64;
+template <bool FILL>
+__global__ void lp_near(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
+                        int* __restrict__ cnt, const int* __restrict__ off, int* __restrict__ src,
+                        int* __restrict__ dst, float* __restrict__ gap) {
+  __shared__ int cand[GR_WARPS][GR_CAND];
+  const int warp = threadIdx.x / 32, a = blockIdx.x * GR_WARPS + warp, lane = threadIdx.x & 31;
   if (a >= nn) return;
-  int o = off[a];
-  for (int b0 = 0; b0 < nn; b0 += 32) {
-    const int b = b0 + lane;
+  float LR[9], LI[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    LR[k] = (float)L.LR[k];
+    LI[k] = (float)L.LI[k];
+  }
+  const double x0 = pos[3 * a], x1 = pos[3 * a + 1], x2 = pos[3 * a + 2];
+  const float ra = (float)radii[a];
+  const unsigned below = (1u << lane) - 1;
+  int found = 0, nc = 0;
+  auto flush = [&](int n) {  // tests the first n <= 32 candidates and drops them
+    __syncwarp();
+    const int b = lane < n ? cand[warp][lane] : -1;
     double g = 0.0;
-    const bool in = b < nn && b != a && lp_pair(L, pos, radii, a, b, &g);
+    const bool in = b >= 0 && lp_pair(L, pos, radii, a, b, &g);
     const unsigned m = __ballot_sync(0xffffffffu, in);
-    if (in) {
-      const int k = o + __popc(m & ((1u << lane) - 1u));
+    if (FILL && in) {
+      const int k = off[a] + found + __popc(m & below);
       src[k] = b;
       dst[k] = a;
       gap[k] = (float)g;
     }
-    o += __popc(m);
+    found += __popc(m);
+    const int rest = lane + n < nc ? cand[warp][lane + n] : 0;
+    __syncwarp();
+    cand[warp][lane] = rest;
+    nc -= n;
+    __syncwarp();
+  };
+  for (int b0 = 0; b0 < nn; b0 += 32) {
+    const int b = b0 + lane;
+    bool c = false;
+    if (b < nn && b != a) {
+      const float R[3] = {(float)(x0 - pos[3 * b]), (float)(x1 - pos[3 * b + 1]), (float)(x2 - pos[3 * b + 2])};
+      int k[3];
+      rsd_skew_shift_f32(LR, LI, R, k);
+      float d2 = 0.f;
+      for (int i = 0; i < 3; i++) {
+        const float e = R[i] - (LR[i] * k[0] + LR[i + 3] * k[1] + LR[i + 6] * k[2]);
+        d2 += e * e;
+      }
+      const float lim = 0.5f * (float)LP_CUT * (ra + (float)radii[b]) * 1.001f + 1e-3f;
+      c = !(d2 > lim * lim);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, c);
+    if (c) cand[warp][nc + __popc(m & below)] = b;
+    nc += __popc(m);
+    if (nc >= 32) flush(32);
   }
+  if (nc > 0) flush(nc);
+  if (!FILL && lane == 0) cnt[a] = found;
 }
 
 // rev[e]: the edge (src <- dst) in src's list (binary search, lists sorted)
@@ -316,40 +342,51 @@ __global__ void __launch_bounds__(FS_THREADS) lp_fsai(int nn, int lower_only_sel
     B[q] = rpp_at(A, ld, nn, i, j) * dinv[i] * dinv[j];
   }
   __syncthreads();
-  // Cholesky B = L L^T (lower, in place), column by column
+  // Cholesky B = L L^T (lower, in place), column by column: warp 0 scales the
+  // column, then the warps take the columns right of it, lanes on the rows
+  // below the diagonal.  FP64 pipe-bound: m^3 / 6 multiply-adds.
+  const int lane = t & 31, warp = t >> 5;
   for (int j = 0; j < m; j++) {
-    if (t == 0) {
-      const double d = B[j + j * m];
-      if (!(d > 0.0)) atomicExch(bad, 2);
-      B[j + j * m] = sqrt(fmax(d, 1e-300));
+    double* Bj = B + (size_t)j * m;
+    if (warp == 0) {
+      const double d = Bj[j];
+      const double piv = sqrt(fmax(d, 1e-300));
+      __syncwarp();
+      if (lane == 0) {
+        if (!(d > 0.0)) atomicExch(bad, 2);
+        Bj[j] = piv;
+      }
+      for (int i = j + 1 + lane; i < m; i += 32) Bj[i] /= piv;
     }
     __syncthreads();
-    const double piv = B[j + j * m];
-    for (int i = j + 1 + t; i < m; i += FS_THREADS) B[i + j * m] /= piv;
-    __syncthreads();
-    for (int q = t; q < (m - j - 1) * (m - j - 1); q += FS_THREADS) {
-      const int i = j + 1 + q % (m - j - 1), c = j + 1 + q / (m - j - 1);
-      if (i >= c) B[i + c * m] -= B[i + j * m] * B[c + j * m];
+    for (int c = j + 1 + warp; c < m; c += FS_THREADS / 32) {
+      const double l = Bj[c];
+      for (int i = c + lane; i < m; i += 32) B[i + (size_t)c * m] -= Bj[i] * l;
     }
     __syncthreads();
   }
-  // Y = B^-1 E_a, E_a the last 6 unit columns: forward then backward
-  // substitution, one thread per right-hand side
+  // Y = B^-1 E_a, E_a the last 6 unit columns: the forward substitution
+  // starts at row m - 6; backward, each solved row is subtracted from the
+  // rows above by all threads
   if (t < 6) {
     double* y = Y + t * m;
     for (int i = 0; i < m; i++) y[i] = (i == m - 6 + t) ? 1.0 : 0.0;
-    for (int i = 0; i < m; i++) {
+    for (int i = m - 6; i < m; i++) {
       double s = y[i];
-      for (int c = 0; c < i; c++) s -= B[i + c * m] * y[c];
-      y[i] = s / B[i + i * m];
-    }
-    for (int i = m - 1; i >= 0; i--) {
-      double s = y[i];
-      for (int r = i + 1; r < m; r++) s -= B[r + i * m] * y[r];
+      for (int c = m - 6; c < i; c++) s -= B[i + c * m] * y[c];
       y[i] = s / B[i + i * m];
     }
   }
   __syncthreads();
+  for (int i = m - 1; i >= 0; i--) {
+    if (t < 6) Y[t * m + i] /= B[i + (size_t)i * m];
+    __syncthreads();
+    for (int q = t; q < 6 * i; q += FS_THREADS) {
+      const int c = q / i, r = q % i;
+      Y[c * m + r] -= B[i + (size_t)r * m] * Y[c * m + i];
+    }
+    __syncthreads();
+  }
   if (t == 0) {
     double Yaa[36];
     for (int r = 0; r < 6; r++)
@@ -513,36 +550,55 @@ struct LayerArgs {
 
 constexpr int LW = 8;  // warps per CTA
 
+constexpr int LR4 = 4;  // rows per warp at a time: a weight read from shared memory serves four rows
+
 __global__ void __launch_bounds__(32 * LW) lp_layer_fwd(LayerArgs A) {
-  extern __shared__ float ls[];
+  extern __shared__ __align__(16) float ls[];
   float* Wt = ls;                       // [kin][kout]
-  float* xs = ls + A.kin * A.kout;      // [LW][kin]
+  float* xs = ls + A.kin * A.kout;      // [LW][kin][LR4]
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int q = t; q < A.kin * A.kout; q += 32 * LW) {
     const int o = q / A.kin, k = q % A.kin;
     Wt[k * A.kout + o] = __bfloat162float(A.W[q]);
   }
   __syncthreads();
-  float* x = xs + warp * A.kin;
-  for (int r = blockIdx.x * LW + warp; r < A.rows; r += gridDim.x * LW) {
-    int k0 = 0;
-    for (int s = 0; s < A.nseg; s++) {
-      const int row = A.s[s].idx ? A.s[s].idx[r] : r;
-      const __nv_bfloat16* p = A.s[s].p + (size_t)row * A.s[s].w;
-      for (int k = lane; k < A.s[s].w; k += 32) x[k0 + k] = __bfloat162float(p[k]);
-      k0 += A.s[s].w;
+  float* x = xs + warp * A.kin * LR4;
+  for (int r0 = (blockIdx.x * LW + warp) * LR4; r0 < A.rows; r0 += gridDim.x * LW * LR4) {
+    const int nr = min(LR4, A.rows - r0);
+    for (int u = 0; u < LR4; u++) {
+      int k0 = 0;
+      for (int s = 0; s < A.nseg; s++) {
+        const int r = r0 + min(u, nr - 1), row = A.s[s].idx ? A.s[s].idx[r] : r;
+        const __nv_bfloat16* p = A.s[s].p + (size_t)row * A.s[s].w;
+        for (int k = lane; k < A.s[s].w; k += 32) x[(k0 + k) * LR4 + u] = __bfloat162float(p[k]);
+        k0 += A.s[s].w;
+      }
     }
     __syncwarp();
     for (int o = lane; o < A.kout; o += 32) {
-      float acc = A.b[o];
-      for (int k = 0; k < A.kin; k++) acc = fmaf(Wt[k * A.kout + o], x[k], acc);
-      if (A.act) acc = fmaxf(acc, 0.f);
-      if (A.add_eye && (o / 6 == o % 6)) acc += 1.f;
-      const size_t yo = (size_t)r * A.kout + o;
-      const __nv_bfloat16 yb = __float2bfloat16(acc);
-      if (A.y) A.y[yo] = yb;
-      if (A.y32) A.y32[yo] = acc;
-      if (A.sum) A.sum[yo] = __float2bfloat16(__bfloat162float(A.res[yo]) + __bfloat162float(yb));
+      float acc[LR4];
+#pragma unroll
+      for (int u = 0; u < LR4; u++) acc[u] = A.b[o];
+#pragma unroll 4
+      for (int k = 0; k < A.kin; k++) {
+        const float w = Wt[k * A.kout + o];
+        const float4 v = *reinterpret_cast<const float4*>(x + k * LR4);
+        acc[0] = fmaf(w, v.x, acc[0]);
+        acc[1] = fmaf(w, v.y, acc[1]);
+        acc[2] = fmaf(w, v.z, acc[2]);
+        acc[3] = fmaf(w, v.w, acc[3]);
+      }
+#pragma unroll
+      for (int u = 0; u < LR4; u++) {
+        if (u >= nr) break;
+        if (A.act) acc[u] = fmaxf(acc[u], 0.f);
+        if (A.add_eye && (o / 6 == o % 6)) acc[u] += 1.f;
+        const size_t yo = (size_t)(r0 + u) * A.kout + o;
+        const __nv_bfloat16 yb = __float2bfloat16(acc[u]);
+        if (A.y) A.y[yo] = yb;
+        if (A.y32) A.y32[yo] = acc[u];
+        if (A.sum) A.sum[yo] = __float2bfloat16(__bfloat162float(A.res[yo]) + __bfloat162float(yb));
+      }
     }
     __syncwarp();
   }
@@ -611,36 +667,51 @@ __global__ void __launch_bounds__(256) lp_layer_bwd(LayerBwdArgs A) {
     xs[q] = v;
   }
   __syncthreads();
-  // input gradients
-  for (int q = t; q < LB_ROWS * A.kin; q += 256) {
-    const int rl = q / A.kin, k = q % A.kin, r = r0 + rl;
-    if (r >= A.rows) continue;
-    float s = 0.f;
-    for (int o = 0; o < A.kout; o++) s = fmaf(Ws[o * A.kin + k], dz[rl * A.kout + o], s);
-    int k0 = 0;
-    for (int sg = 0; sg < A.nseg; sg++) {
-      if (k < k0 + A.s[sg].w) {
-        if (A.dx[sg]) {
-          const int row = A.s[sg].idx ? A.s[sg].idx[r] : r;
-          atomicAdd(A.dx[sg] + (size_t)row * A.s[sg].w + (k - k0), s);
-        }
-        break;
+  // input gradients, eight rows per thread and column k
+  if (A.dx[0] || A.dx[1] || A.dx[2]) {
+    constexpr int RB = 8;
+    for (int q = t; q < LB_ROWS / RB * A.kin; q += 256) {
+      const int k = q % A.kin, rb = q / A.kin * RB;
+      if (r0 + rb >= A.rows) continue;
+      float s[RB];
+#pragma unroll
+      for (int u = 0; u < RB; u++) s[u] = 0.f;
+      for (int o = 0; o < A.kout; o++) {
+        const float w = Ws[o * A.kin + k];
+#pragma unroll
+        for (int u = 0; u < RB; u++) s[u] = fmaf(w, dz[(rb + u) * A.kout + o], s[u]);
       }
-      k0 += A.s[sg].w;
+      int sg = 0, k0 = 0;
+      while (k >= k0 + A.s[sg].w) k0 += A.s[sg++].w;
+      if (!A.dx[sg]) continue;
+#pragma unroll
+      for (int u = 0; u < RB; u++) {
+        const int r = r0 + rb + u;
+        if (r >= A.rows) break;
+        const int row = A.s[sg].idx ? A.s[sg].idx[r] : r;
+        atomicAdd(A.dx[sg] + (size_t)row * A.s[sg].w + (k - k0), s[u]);
+      }
     }
   }
-  // weight and bias partials of this chunk
+  // weight and bias partials of this chunk, four outputs per thread and
+  // column k (kout is a multiple of 4)
   float* p = A.part + (size_t)blockIdx.x * (A.kout * A.kin + A.kout);
-  for (int q = t; q < A.kout * A.kin + A.kout; q += 256) {
-    float s = 0.f;
-    if (q < A.kout * A.kin) {
-      const int o = q / A.kin, k = q % A.kin;
-      for (int rl = 0; rl < LB_ROWS; rl++) s = fmaf(dz[rl * A.kout + o], xs[rl * A.kin + k], s);
-    } else {
-      const int o = q - A.kout * A.kin;
-      for (int rl = 0; rl < LB_ROWS; rl++) s += dz[rl * A.kout + o];
+  for (int q = t; q < A.kout / 4 * A.kin; q += 256) {
+    const int k = q % A.kin, o = q / A.kin * 4;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int rl = 0; rl < LB_ROWS; rl++) {
+      const float x = xs[rl * A.kin + k];
+#pragma unroll
+      for (int u = 0; u < 4; u++) s[u] = fmaf(dz[rl * A.kout + o + u], x, s[u]);
     }
-    p[q] = s;
+#pragma unroll
+    for (int u = 0; u < 4; u++) p[(o + u) * A.kin + k] = s[u];
+  }
+  for (int o = t; o < A.kout; o += 256) {
+    float s = 0.f;
+    for (int rl = 0; rl < LB_ROWS; rl++) s += dz[rl * A.kout + o];
+    p[A.kout * A.kin + o] = s;
   }
 }
 
@@ -742,100 +813,217 @@ __global__ void lp_to_bf16(int64_t n, const float* __restrict__ w, __nv_bfloat16
 }
 
 // ------------------------------------------------------------ preconditioner
-// y = G v, G = D^-1/2 Z^T Z D^-1/2 (mode FSAI / learned), D^-1 (Jacobi) or I
-// t = Z (dinv v): row block a = zd[a] v^_a + sum over lower edges (a <- b) ze[e] v^_b
-__global__ void lp_apply_z(int nn, const int* __restrict__ off, const int* __restrict__ src,
-                           const float* __restrict__ zd, const float* __restrict__ ze, const double* __restrict__ dinv,
-                           const double* __restrict__ v, double* __restrict__ tmp) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * nn) return;
-  const int a = t / 6, r = t % 6;
-  double s = 0.0;
-  for (int c = 0; c < 6; c++) s += (double)zd[(size_t)a * 36 + r * 6 + c] * dinv[6 * a + c] * v[6 * a + c];
-  for (int e = off[a]; e < off[a + 1]; e++) {
-    const int b = src[e];
-    if (b >= a) continue;
-    for (int c = 0; c < 6; c++) s += (double)ze[(size_t)e * 36 + r * 6 + c] * dinv[6 * b + c] * v[6 * b + c];
-  }
-  tmp[t] = s;
-}
+// PCG on RPP x = b in one cooperative launch per right-hand side, everything in
+// the grand layout.  The iteration is three phases between barriers of the
+// whole grid; each CTA adds the others' partial dot products up in a fixed
+// order:
+//   residual   x += alpha p, r' = r - alpha q (r is double-buffered, so that a
+//              row of t = Z D^-1/2 r' can form its neighbours' entries itself)
+//   z          z = D^-1/2 Z^T t (Jacobi: D^-1 r'; none: r'), r'.z
+//   product    p' = z + beta p, formed whole by every CTA in shared memory, q =
+//              A p', p'.q: a warp per column of A
+// Bound by the product: (6N)^2 FP64 multiply-adds at 2 per SM and cycle, 14.5
+// us at N = 500; a launch per operation took 98 us an iteration there.
+struct PcgArgs {
+  int nn, mode;
+  const int *off, *src, *rev;
+  const float *zd, *ze;
+  const double* dinv;  // particle-block layout
+  const double* A;
+  int64_t ld;
+  const double* b;
+  double *x, *r[2], *p[2], *z, *q, *tmp;
+  double* part;  // 3 x gridDim.x
+  int* bar;      // [0] arrivals, [1] error
+  double* out;   // iterations, |r|, |b|
+  double tol;
+  int maxit, staged;
+};
+constexpr int PCG_THREADS = 512;
+constexpr int PCG_STAGE = 200 * 1024;  // p staged in shared memory up to this many bytes
 
-// y = dinv Z^T t: row block b = zd[b]^T t_b + sum over edges (a <- b), a > b,
-// ze[(a <- b)]^T t_a; the edges into b give (b <- a) and rev gives (a <- b)
-__global__ void lp_apply_zt(int nn, const int* __restrict__ off, const int* __restrict__ src,
-                            const int* __restrict__ rev, const float* __restrict__ zd, const float* __restrict__ ze,
-                            const double* __restrict__ dinv, const double* __restrict__ tmp, double* __restrict__ y) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * nn) return;
-  const int b = t / 6, c = t % 6;
-  double s = 0.0;
-  for (int r = 0; r < 6; r++) s += (double)zd[(size_t)b * 36 + r * 6 + c] * tmp[6 * b + r];
-  for (int e = off[b]; e < off[b + 1]; e++) {
-    const int a = src[e];
-    if (a <= b) continue;
-    const int f = rev[e];  // (a <- b)
-    if (f < 0) continue;
-    for (int r = 0; r < 6; r++) s += (double)ze[(size_t)f * 36 + r * 6 + c] * tmp[6 * a + r];
-  }
-  y[t] = dinv[t] * s;
-}
-
-// particle-block layout <-> grand layout of a 6N vector
-__global__ void lp_to_blk(int nn, const double* __restrict__ g, double* __restrict__ b) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 6 * nn) b[t] = g[grand_row(nn, t)];
-}
-__global__ void lp_from_blk(int nn, const double* __restrict__ b, double* __restrict__ g) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 6 * nn) g[grand_row(nn, t)] = b[t];
-}
-
-__global__ void lp_scale(int n, const double* __restrict__ d, const double* __restrict__ v, double* __restrict__ y) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) y[t] = d[t] * d[t] * v[t];
-}
-
-// dot products (one block): out[q] = x_q . y_q for q < nq
-__global__ void lp_dots(int n, int nq, const double* __restrict__ x0, const double* __restrict__ y0,
-                        const double* __restrict__ x1, const double* __restrict__ y1, double* __restrict__ out) {
-  __shared__ double r0[256], r1[256];
-  double a = 0.0, b = 0.0;
-  for (int i = threadIdx.x; i < n; i += 256) {
-    a += x0[i] * y0[i];
-    if (nq > 1) b += x1[i] * y1[i];
-  }
-  r0[threadIdx.x] = a;
-  r1[threadIdx.x] = b;
+// Waits until every CTA has arrived `turn` times; false when the wait ran out
+// (bounded, ~2 s) here or elsewhere, which ends the kernel.
+__device__ __forceinline__ bool pcg_barrier(const PcgArgs& g, int turn) {
+  __shared__ int ok;
   __syncthreads();
-  for (int d = 128; d > 0; d >>= 1) {
-    if (threadIdx.x < d) {
-      r0[threadIdx.x] += r0[threadIdx.x + d];
-      r1[threadIdx.x] += r1[threadIdx.x + d];
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    out[0] = r0[0];
-    if (nq > 1) out[1] = r1[0];
+    ok = 1;
+    __threadfence();
+    atomicAdd(g.bar, 1);
+    const int target = turn * (int)gridDim.x;
+    long long polls = 0;
+    while (*((volatile int*)g.bar) < target) {
+      if (*((volatile int*)(g.bar + 1)) || ++polls > (1LL << 25)) {
+        atomicExch(g.bar + 1, 1);
+        ok = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    __threadfence();
   }
+  __syncthreads();
+  return ok != 0;
 }
 
-// CG updates with the scalars on the device: alpha = rz / pq;
-// x += alpha p; r -= alpha q
-__global__ void lp_cg_xr(int n, const double* __restrict__ sc, const double* __restrict__ p,
-                         const double* __restrict__ q, double* __restrict__ x, double* __restrict__ r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double alpha = sc[0] / sc[1];
-  x[i] += alpha * p[i];
-  r[i] -= alpha * q[i];
+__device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
-// beta = rz_new / rz; p = z + beta p; rz = rz_new
-__global__ void lp_cg_p(int n, double* __restrict__ sc, const double* __restrict__ z, double* __restrict__ p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = z[i] + (sc[2] / sc[0]) * p[i];
+
+// the CTA's sum of v, on thread 0, into *dst
+__device__ __forceinline__ void pcg_part(double v, double* red, double* dst) {
+  v = warp_sum_d(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = warp_sum_d(threadIdx.x < PCG_THREADS / 32 ? red[threadIdx.x] : 0.0);
+    if (threadIdx.x == 0) *dst = v;
+  }
+  __syncthreads();
 }
-__global__ void lp_cg_roll(double* sc) { sc[0] = sc[2]; }
+
+// the sum of the CTAs' partials, the same on every thread of the grid
+__device__ __forceinline__ double pcg_total(const double* part, double* red) {
+  if (threadIdx.x < 32) {
+    double v = 0.0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += 32) v += __ldcg(part + k);
+    v = warp_sum_d(v);
+    if (threadIdx.x == 0) red[0] = v;
+  }
+  __syncthreads();
+  const double v = red[0];
+  __syncthreads();
+  return v;
+}
+
+__global__ void __launch_bounds__(PCG_THREADS, 1) lp_pcg_kernel(PcgArgs g) {
+  extern __shared__ double ps[];
+  __shared__ double red[32];
+  const int P = 6 * g.nn, t = threadIdx.x, lane = t & 31, nthr = gridDim.x * PCG_THREADS;
+  const int gt = blockIdx.x * PCG_THREADS + t, gw = gt >> 5, nw = nthr >> 5;
+  const bool z_mode = g.mode != RSD_PC_NONE && g.mode != RSD_PC_JACOBI;
+  double *pr = g.part, *pz = pr + gridDim.x, *pq = pz + gridDim.x;
+  // grand index of component c of particle a; particle-block index of grand index i
+  auto gi = [&](int a, int c) { return c < 3 ? 3 * a + c : 3 * g.nn + 3 * a + c - 3; };
+  auto bi = [&](int i) { return i < 3 * g.nn ? 6 * (i / 3) + i % 3 : 6 * ((i - 3 * g.nn) / 3) + 3 + (i - 3 * g.nn) % 3; };
+  double alpha = 0.0, rz = 0.0, bn = 1.0, rn = 0.0;
+  int it = 0, turn = 0;
+  for (;; it++) {
+    const double *r0 = it ? g.r[(it - 1) & 1] : g.b, *p0 = g.p[it & 1];  // p of the last iteration
+    double *r1 = g.r[it & 1], *p1 = g.p[(it + 1) & 1];
+    // ---- residual
+    double s = 0.0;
+    for (int i = gt; i < P; i += nthr) {
+      double v = __ldcg(r0 + i);
+      if (it) {
+        v -= alpha * __ldcg(g.q + i);
+        g.x[i] += alpha * __ldcg(p0 + i);
+      }
+      r1[i] = v;
+      s += v * v;
+    }
+    if (z_mode)  // 8 lanes per row of Z, which share its edges
+      for (int w = gt >> 3; w - ((t & 31) >> 3) < P; w += nthr >> 3) {
+        double v = 0.0;
+        if (w < P) {
+          const int a = w / 6, r = w % 6, e0 = g.off[a], e1 = g.off[a + 1];
+          for (int e = e0 - 1 + (t & 7); e < e1; e += 8) {
+            const int o = e < e0 ? a : g.src[e];
+            if (e >= e0 && o >= a) continue;
+            const float* Z = (e < e0 ? g.zd + (size_t)a * 36 : g.ze + (size_t)e * 36) + r * 6;
+#pragma unroll
+            for (int c = 0; c < 6; c++) {
+              const int j = gi(o, c);
+              double x = __ldcg(r0 + j);
+              if (it) x -= alpha * __ldcg(g.q + j);
+              v = fma((double)Z[c], g.dinv[6 * o + c] * x, v);
+            }
+          }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (w < P && (t & 7) == 0) g.tmp[w] = v;
+      }
+    pcg_part(s, red, pr + blockIdx.x);
+    if (!pcg_barrier(g, ++turn)) return;
+    rn = sqrt(pcg_total(pr, red));
+    if (it == 0) bn = rn > 0.0 ? rn : 1.0;
+    if (!(rn > g.tol * bn) || it >= g.maxit || !isfinite(rn)) break;
+    // ---- z
+    s = 0.0;
+    if (z_mode) {
+      for (int w = gt >> 3; w - ((t & 31) >> 3) < P; w += nthr >> 3) {
+        double v = 0.0;
+        const int b = w / 6, c = w % 6;
+        if (w < P) {
+          const int e0 = g.off[b], e1 = g.off[b + 1];
+          for (int e = e0 - 1 + (t & 7); e < e1; e += 8) {
+            const int a = e < e0 ? b : g.src[e];
+            if (e >= e0 && a <= b) continue;
+            const int f = e < e0 ? 0 : g.rev[e];  // (a <- b)
+            if (f < 0) continue;
+            const float* Z = (e < e0 ? g.zd + (size_t)b * 36 : g.ze + (size_t)f * 36) + c;
+#pragma unroll
+            for (int r = 0; r < 6; r++) v = fma((double)Z[6 * r], __ldcg(g.tmp + 6 * a + r), v);
+          }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (w < P && (t & 7) == 0) {
+          const int i = gi(b, c);
+          v *= g.dinv[w];
+          g.z[i] = v;
+          s += v * __ldcg(r1 + i);
+        }
+      }
+    } else {
+      for (int i = gt; i < P; i += nthr) {
+        const double r = __ldcg(r1 + i), d = g.mode == RSD_PC_JACOBI ? g.dinv[bi(i)] : 1.0;
+        const double v = d * d * r;
+        g.z[i] = v;
+        s += v * r;
+      }
+    }
+    pcg_part(s, red, pz + blockIdx.x);
+    if (!pcg_barrier(g, ++turn)) return;
+    // ---- product
+    const double rz1 = pcg_total(pz, red), beta = it ? rz1 / rz : 0.0;
+    rz = rz1;
+    if (g.staged)
+      for (int i = t; i < P; i += PCG_THREADS) ps[i] = it ? fma(beta, __ldcg(p0 + i), __ldcg(g.z + i)) : __ldcg(g.z + i);
+    for (int i = gt; i < P; i += nthr) p1[i] = it ? fma(beta, __ldcg(p0 + i), __ldcg(g.z + i)) : __ldcg(g.z + i);
+    __syncthreads();
+    if (!g.staged && !pcg_barrier(g, ++turn)) return;
+    s = 0.0;
+    for (int i = gw; i < P; i += nw) {
+      const double* a = g.A + (int64_t)i * g.ld;
+      double v = 0.0;
+      if (g.staged) {
+#pragma unroll 8
+        for (int k = lane; k < P; k += 32) v = fma(a[k], ps[k], v);
+      } else {
+#pragma unroll 8
+        for (int k = lane; k < P; k += 32) v = fma(a[k], __ldcg(p1 + k), v);
+      }
+      v = warp_sum_d(v);
+      if (lane == 0) {
+        g.q[i] = v;
+        s += v * (g.staged ? ps[i] : __ldcg(p1 + i));
+      }
+    }
+    pcg_part(s, red, pq + blockIdx.x);
+    if (!pcg_barrier(g, ++turn)) return;
+    alpha = rz / pcg_total(pq, red);
+  }
+  if (gt == 0) {
+    g.out[0] = (double)it;
+    g.out[1] = rn;
+    g.out[2] = bn;
+  }
+}
 
 inline unsigned nb256(int64_t n) { return (unsigned)((n + 255) / 256); }
 
@@ -861,7 +1049,8 @@ static int lp_build_graph(rsd_ctx* ctx, int nn, const double* d_pos, const doubl
   rsd_lat_dev L = rsd_lat_pack(lat);
   int* cnt = (int*)rsd_scratch(ctx, "lp_cnt", sizeof(int) * (nn + 1));
   if (!cnt) return RSD_ENOMEM;
-  lp_count<<<nn, 256, 0, s>>>(nn, L, d_pos, d_radii, cnt); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  const unsigned ng = (unsigned)((nn + GR_WARPS - 1) / GR_WARPS);
+  lp_near<false><<<ng, 32 * GR_WARPS, 0, s>>>(nn, L, d_pos, d_radii, cnt, nullptr, nullptr, nullptr, nullptr); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
   std::vector<int> h(nn + 1);
   RSD_CUDA(ctx, cudaMemcpyAsync(h.data(), cnt, sizeof(int) * nn, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
@@ -879,7 +1068,7 @@ static int lp_build_graph(rsd_ctx* ctx, int nn, const double* d_pos, const doubl
   if (!g->off || !g->src || !g->dst || !g->rev || !g->lower || !g->gap) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemcpyAsync(g->off, off.data(), sizeof(int) * (nn + 1), cudaMemcpyHostToDevice, s));
   if (ne > 0) {
-    lp_fill<<<(nn + 7) / 8, 256, 0, s>>>(nn, L, d_pos, d_radii, g->off, g->src, g->dst, g->gap); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    lp_near<true><<<ng, 32 * GR_WARPS, 0, s>>>(nn, L, d_pos, d_radii, nullptr, g->off, g->src, g->dst, g->gap); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
     lp_rev<<<nb256(ne), 256, 0, s>>>(ne, g->off, g->src, g->dst, g->rev); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
     lp_lower_flags<<<nb256(ne), 256, 0, s>>>(ne, g->src, g->dst, g->lower); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
   }
@@ -943,13 +1132,13 @@ struct lp_acts {
 
 static int lp_layer(rsd_ctx* ctx, const LayerArgs& a) {
   if (a.rows <= 0) return RSD_OK;
-  const size_t smem = sizeof(float) * ((size_t)a.kin * a.kout + (size_t)LW * a.kin);
+  const size_t smem = sizeof(float) * ((size_t)a.kin * a.kout + (size_t)LW * LR4 * a.kin);
   static bool attr = false;
   if (!attr) {
     RSD_CUDA(ctx, cudaFuncSetAttribute(lp_layer_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     attr = true;
   }
-  const int grid = (int)std::min<int64_t>((a.rows + LW - 1) / LW, 8LL * (ctx->sm_count > 0 ? ctx->sm_count : 148));
+  const int grid = (int)std::min<int64_t>((a.rows + LW * LR4 - 1) / (LW * LR4), 2LL * (ctx->sm_count > 0 ? ctx->sm_count : 148));
   lp_layer_fwd<<<grid, 32 * LW, smem, ctx->stream>>>(a); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
   return RSD_OK;
 }
@@ -1125,66 +1314,57 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
                   int* iters, double* resid) {
   cudaStream_t s = ctx->stream;
   const int nn = g.nn, P = 6 * nn;
-  double* V = (double*)rsd_scratch(ctx, "lp_pcg", sizeof(double) * (6 * (size_t)P + 16));
+  const int grid = ctx->sm_count;  // one CTA per SM: all are resident (cooperative launch)
+  double* V = (double*)rsd_scratch(ctx, "lp_pcg", sizeof(double) * (7 * (size_t)P + 3 * (size_t)grid + 8));
   if (!V) return RSD_ENOMEM;
-  double *r = V, *z = r + P, *p = z + P, *q = p + P, *tmp = q + P, *rb = tmp + P, *sc = rb + P;
+  PcgArgs a{};
+  a.nn = nn;
+  a.mode = mode;
+  a.off = g.off;
+  a.src = g.src;
+  a.rev = g.rev;
+  a.zd = zd;
+  a.ze = ze;
+  a.dinv = dinv;
+  a.A = A;
+  a.ld = ld;
+  a.r[0] = V;
+  a.r[1] = V + P;
+  a.p[0] = V + 2 * (size_t)P;
+  a.p[1] = V + 3 * (size_t)P;
+  a.z = V + 4 * (size_t)P;
+  a.q = V + 5 * (size_t)P;
+  a.tmp = V + 6 * (size_t)P;
+  a.part = V + 7 * (size_t)P;
+  a.out = a.part + 3 * (size_t)grid;
+  a.bar = reinterpret_cast<int*>(a.out + 4);
+  a.tol = tol;
+  a.maxit = maxit;
+  a.staged = sizeof(double) * (size_t)P <= PCG_STAGE;
+  const size_t smem = a.staged ? sizeof(double) * (size_t)P : 0;
+  RSD_CUDA(ctx, cudaFuncSetAttribute(lp_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PCG_STAGE));
   int worst_it = 0;
   double worst_res = 0.0;
-  auto precond = [&](const double* in, double* out) -> int {
-    if (mode == RSD_PC_NONE) {
-      RSD_CUDA(ctx, cudaMemcpyAsync(out, in, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
-    } else if (mode == RSD_PC_JACOBI) {
-      lp_scale<<<nb256(P), 256, 0, s>>>(P, dinv, in, out); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    } else {
-      lp_apply_z<<<nb256(P), 256, 0, s>>>(nn, g.off, g.src, zd, ze, dinv, in, tmp); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-      lp_apply_zt<<<nb256(P), 256, 0, s>>>(nn, g.off, g.src, g.rev, zd, ze, dinv, tmp, out); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    }
-    return RSD_OK;
-  };
-  // the operator in the particle-block layout: q = P A P^T p
-  auto matvec = [&](const double* in, double* out) -> int {
-    lp_from_blk<<<nb256(P), 256, 0, s>>>(nn, in, tmp); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    RSD_TRY(rsd_gemv<double>(ctx, 0, P, P, 1.0, A, ld, tmp, P, 1, 0.0, rb, P));
-    lp_to_blk<<<nb256(P), 256, 0, s>>>(nn, rb, out); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    return RSD_OK;
-  };
-  double h[4];
   for (int c = 0; c < nrhs; c++) {
-    double* xc = x + (size_t)c * P;
-    // r = b (block layout), x = 0
-    lp_to_blk<<<nb256(P), 256, 0, s>>>(nn, b + (size_t)c * P, r); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    RSD_CUDA(ctx, cudaMemsetAsync(xc, 0, sizeof(double) * P, s));
-    RSD_TRY(precond(r, z));
-    RSD_CUDA(ctx, cudaMemcpyAsync(p, z, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
-    lp_dots<<<1, 256, 0, s>>>(P, 2, r, z, r, r, sc); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();  // sc[0] = rz, sc[1] = rr
-    RSD_CUDA(ctx, cudaMemcpyAsync(h, sc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    a.b = b + (size_t)c * P;
+    a.x = x + (size_t)c * P;
+    RSD_CUDA(ctx, cudaMemsetAsync(a.x, 0, sizeof(double) * P, s));
+    RSD_CUDA(ctx, cudaMemsetAsync(a.bar, 0, 2 * sizeof(int), s));
+    void* args[] = {&a};
+    RSD_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)lp_pcg_kernel, dim3(grid), dim3(PCG_THREADS), args, smem, s)); RSD_LAUNCH_NOTE();
+    double h[5];
+    RSD_CUDA(ctx, cudaMemcpyAsync(h, a.out, 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
     RSD_CUDA(ctx, cudaStreamSynchronize(s));
-    const double bn = sqrt(h[1]) > 0 ? sqrt(h[1]) : 1.0;
-    double rn = sqrt(h[1]);
-    int it = 0;
-    while (rn > tol * bn && it < maxit) {
-      RSD_TRY(matvec(p, q));
-      lp_dots<<<1, 256, 0, s>>>(P, 1, p, q, p, q, sc + 1); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();  // sc[1] = pq
-      lp_cg_xr<<<nb256(P), 256, 0, s>>>(P, sc, p, q, xc, r); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-      RSD_TRY(precond(r, z));
-      lp_dots<<<1, 256, 0, s>>>(P, 2, r, z, r, r, sc + 2); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();  // sc[2] = rz', sc[3] = rr
-      lp_cg_p<<<nb256(P), 256, 0, s>>>(P, sc, z, p); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-      lp_cg_roll<<<1, 1, 0, s>>>(sc); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-      RSD_CUDA(ctx, cudaMemcpyAsync(h, sc + 3, sizeof(double), cudaMemcpyDeviceToHost, s));
-      RSD_CUDA(ctx, cudaStreamSynchronize(s));
-      rn = sqrt(h[0]);
-      it++;
-      if (!std::isfinite(rn)) return rsd_fail(ctx, RSD_ENAN, "PCG residual is not finite");
-    }
-    // x back to the grand layout, in place through tmp
-    lp_from_blk<<<nb256(P), 256, 0, s>>>(nn, xc, tmp); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    RSD_CUDA(ctx, cudaMemcpyAsync(xc, tmp, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
+    int bar[2];
+    memcpy(bar, h + 4, sizeof bar);
+    if (bar[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "PCG: a wait for the other thread blocks timed out");
+    const int it = (int)h[0];
+    if (it > 0 && !std::isfinite(h[1])) return rsd_fail(ctx, RSD_ENAN, "PCG residual is not finite");
     worst_it = std::max(worst_it, it);
-    worst_res = std::max(worst_res, rn / bn);
+    worst_res = std::max(worst_res, h[1] / h[2]);
   }
   if (iters) *iters = worst_it;
   if (resid) *resid = worst_res;
-  RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
 
