@@ -738,6 +738,212 @@ __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int6
   }
 }
 
+// Two FP32 operations in one instruction: the same rate per lane as two, half
+// the issue slots and instruction fetch.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// The same block (jb <= 128, padded with the identity) by Gauss-Jordan on [S |
+// I], the form of the factorisations inside a step.  One 128 x 128 array in
+// registers, 8 x 8 per thread, holds S above the diagonal and the growing
+// inverse Z of the unit lower factor below it: step k subtracts l_ik = S_ki /
+// d_k times row k from every row i > k, and in column k, where S is done, Z
+// starts as -l_ik (what the entry held until then is dropped).  The owners of
+// row k + 1 update and publish it first, then one barrier, and the other rows'
+// updates of step k run beside the loads and the reciprocal of step k + 1.
+// The square roots come last, all at once.  A thread holds rows 32 v + 2 ty +
+// {0, 1} and columns 32 c + 2 tx + {0, 1}, so that 32 steps run through one
+// small loop (rows of earlier v are done and left out): unrolled over 32-wide
+// sub-blocks it took 54 us and with 8 contiguous rows per thread 39 us, most
+// of it instruction fetch; potf2_inv_f32 takes 42 us.
+struct gj_regs {
+  uint64_t T[8][4];  // row 2 v + p of this thread, column pairs
+  uint64_t s[4];     // row k at this thread's columns
+  float l[8];        // its rows' multipliers, negated
+};
+
+__device__ __forceinline__ void gj_row(uint64_t (&T)[4], const uint64_t (&s)[4], float l) {
+  const uint64_t ll = f2_pack(l, l);
+#pragma unroll
+  for (int c = 0; c < 4; c++) T[c] = f2_fma(ll, s[c], T[c]);
+}
+
+__device__ __forceinline__ void gj_publish(const uint64_t (&T)[4], float* row, int tx) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) *reinterpret_cast<uint64_t*>(row + 32 * c + 2 * tx) = T[c];
+}
+
+// operands of step k = 32 V + 2 kk + P from its published row
+template <int V, int P>
+__device__ __forceinline__ void gj_load(gj_regs& g, const float* row, int kk, int tx, int ty) {
+  const float inv = -__fdividef(1.f, row[32 * V + 2 * kk + P]);
+#pragma unroll
+  for (int c = 0; c < 4; c++) g.s[c] = *reinterpret_cast<const uint64_t*>(row + 32 * c + 2 * tx);
+#pragma unroll
+  for (int v = V; v < 4; v++) {
+    const float2 e = *reinterpret_cast<const float2*>(row + 32 * v + 2 * ty);
+    g.l[2 * v] = e.x * inv;
+    g.l[2 * v + 1] = e.y * inv;
+  }
+  // rows up to k stay: of this V, those of ty < kk and, for ty = kk, up to P
+  const bool r0 = ty > kk, r1 = ty > kk || (P == 0 && ty == kk);
+  g.l[2 * V] = r0 ? g.l[2 * V] : 0.f;
+  g.l[2 * V + 1] = r1 ? g.l[2 * V + 1] : 0.f;
+  // column k: the identity enters
+  const bool own = tx == kk;
+  float x, y;
+  f2_unpack(g.s[V], x, y);
+  g.s[V] = P ? f2_pack(x, own ? 1.f : y) : f2_pack(own ? 1.f : x, y);
+#pragma unroll
+  for (int u = 2 * V; u < 8; u++) {
+    const bool z = own && (u == 2 * V ? r0 : (u == 2 * V + 1 ? r1 : true));
+    f2_unpack(g.T[u][V], x, y);
+    g.T[u][V] = P ? f2_pack(x, z ? 0.f : y) : f2_pack(z ? 0.f : x, y);
+  }
+}
+
+// step k: the next row first (register U of the threads ty = owner), then the rest
+template <int V, int U>
+__device__ __forceinline__ void gj_next(gj_regs& g, float* row, int owner, int tx, int ty) {
+  if (ty == owner) {
+    gj_row(g.T[U], g.s, g.l[U]);
+    g.l[U] = 0.f;  // done
+    gj_publish(g.T[U], row, tx);
+  }
+}
+
+template <int V>
+__device__ __forceinline__ void gj_block(gj_regs& g, float (&row)[2][NB], float* dd, int tx, int ty, int t) {
+#pragma unroll 1
+  for (int kk = 0; kk < 16; kk++) {
+    // step 32 V + 2 kk (row in row[0]), next row in row[1]
+    gj_next<V, 2 * V + 1>(g, row[1], kk, tx, ty);
+    __syncthreads();
+#pragma unroll
+    for (int u = 2 * V; u < 8; u++) gj_row(g.T[u], g.s, g.l[u]);
+    if (t == 0) dd[32 * V + 2 * kk + 1] = row[1][32 * V + 2 * kk + 1];
+    gj_load<V, 1>(g, row[1], kk, tx, ty);
+    // step 32 V + 2 kk + 1
+    if (kk < 15) {
+      gj_next<V, 2 * V>(g, row[0], kk + 1, tx, ty);
+    } else if (V < 3) {
+      gj_next<V, (2 * V + 2) & 7>(g, row[0], 0, tx, ty);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 2 * V; u < 8; u++) gj_row(g.T[u], g.s, g.l[u]);
+    if (kk < 15) {
+      if (t == 0) dd[32 * V + 2 * kk + 2] = row[0][32 * V + 2 * kk + 2];
+      gj_load<V, 0>(g, row[0], kk + 1, tx, ty);
+    } else if (V < 3) {
+      if (t == 0) dd[32 * V + 32] = row[0][(32 * V + 32) & (NB - 1)];
+      gj_load<(V + 1) & 3, 0>(g, row[0], 0, tx, ty);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64_t lda, int jb, int* __restrict__ info,
+                                                    int j0, float* __restrict__ Wout) {
+  __shared__ __align__(16) float row[2][NB];
+  __shared__ float dd[NB];
+  __shared__ int failed;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  const bool vec = ((lda & 1) == 0) && (((uintptr_t)A & 7) == 0) && jb == NB;
+  gj_regs g;
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int i = 32 * v + 2 * ty, j = 32 * c + 2 * tx;
+      float e[2][2];
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        if (vec && i + 1 <= j + q) {
+          const float2 a = *reinterpret_cast<const float2*>(A + i + (int64_t)(j + q) * lda);
+          e[0][q] = a.x;
+          e[1][q] = a.y;
+        } else {
+#pragma unroll
+          for (int p = 0; p < 2; p++)
+            e[p][q] = i + p <= j + q && j + q < jb ? A[i + p + (int64_t)(j + q) * lda] : (i + p == j + q ? 1.f : 0.f);
+        }
+      }
+      g.T[2 * v][c] = f2_pack(e[0][0], e[0][1]);
+      g.T[2 * v + 1][c] = f2_pack(e[1][0], e[1][1]);
+    }
+  if (t == 0) failed = 0;
+  if (ty == 0) gj_publish(g.T[0], row[0], tx);
+  __syncthreads();
+  if (t == 0) dd[0] = row[0][0];
+  gj_load<0, 0>(g, row[0], 0, tx, ty);
+  gj_block<0>(g, row, dd, tx, ty, t);
+  gj_block<1>(g, row, dd, tx, ty, t);
+  gj_block<2>(g, row, dd, tx, ty, t);
+  gj_block<3>(g, row, dd, tx, ty, t);
+  __syncthreads();
+  if (t < NB) {  // the first pivot that is not positive and finite
+    const float d = dd[t];
+    const unsigned m = __ballot_sync(0xffffffffu, !(d > 0.f && d <= 3.402823466e38f));
+    if (m && (t & 31) == 0) atomicMin(&failed, t + __ffs(m) - NB - 1);  // k - NB < 0, k the 0-based index
+  }
+  __syncthreads();
+  if (failed) {
+    if (t == 0) atomicCAS(info, 0, j0 + failed + NB + 1);
+    return;
+  }
+  // U_ij = S_ij / sqrt(d_i) above the diagonal; below it W_ji = Z_ij / sqrt(d_i)
+#pragma unroll
+  for (int v = 0; v < 4; v++) {
+    const int i = 32 * v + 2 * ty;
+    const float d0 = dd[i], d1 = dd[i + 1], s0 = 1.f / sqrtf(d0), s1 = 1.f / sqrtf(d1);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int j = 32 * c + 2 * tx;
+      float x[2][2];
+      f2_unpack(g.T[2 * v][c], x[0][0], x[0][1]);
+      f2_unpack(g.T[2 * v + 1][c], x[1][0], x[1][1]);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        x[0][q] *= s0;
+        x[1][q] *= s1;
+      }
+      if (i == j) {
+        x[0][0] = d0 * s0;
+        x[1][1] = d1 * s1;
+      }
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        float w[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+          w[q] = i + p < jb && j + q < jb ? (i + p > j + q ? x[p][q] : (i + p == j + q ? (p ? s1 : s0) : 0.f)) : 0.f;
+        *reinterpret_cast<float2*>(Wout + j + (i + p) * NB) = make_float2(w[0], w[1]);
+      }
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        if (vec && i + 1 <= j + q) {
+          *reinterpret_cast<float2*>(A + i + (int64_t)(j + q) * lda) = make_float2(x[0][q], x[1][q]);
+        } else {
+#pragma unroll
+          for (int p = 0; p < 2; p++)
+            if (i + p <= j + q && j + q < jb) A[i + p + (int64_t)(j + q) * lda] = x[p][q];
+        }
+      }
+    }
+  }
+}
+
 // Inverses of all diagonal blocks of an upper triangular U (one CTA each).
 template <typename T>
 __global__ void __launch_bounds__(256) trtri_diag(int n, const T* __restrict__ U, int64_t ldu, T* __restrict__ W) {
@@ -889,6 +1095,17 @@ int smem_trsv() {
   return (NB * NB + NB * 4) * (int)sizeof(T);
 }
 
+// exported: the factor ends in a matrix that is handed out (the FP32 RPP of
+// rsd_resistance_pp_dev), whose TF32 rounding goes with the last bits of every
+// block; potf2_inv_f32 keeps them what they were.
+void launch_potf2(cudaStream_t s, bool exported, float* A, int64_t lda, int jb, int* info, int j0, float* W) {
+  if (exported)
+    potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s>>>(A, lda, jb, info, j0, W);
+  else
+    potf2_gj_f32<<<1, 256, 0, s>>>(A, lda, jb, info, j0, W);
+  RSD_LAUNCH_NOTE();
+}
+
 template <typename T>
 const char* tname();
 template <>
@@ -1025,7 +1242,7 @@ int trailing_update(rsd_ctx* ctx, int tc, const T* P, int64_t ldp, int kb, int m
 // Events: A (a's near work done), B (the work the next near step reads),
 // M (the previous remainder, which the next diagonal tile reads).
 constexpr int NBO = 512;
-static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
+static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
   cudaStream_t s = ctx->stream, s2 = ctx->side;
   RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
   for (int J0 = 0; J0 < n; J0 += NBO) {
@@ -1037,7 +1254,7 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
+      launch_potf2(s2, exported, Ajj, lda, jb, st, j0, Wb);
       if (rest <= 0) continue;
       // row panel U_jj^-T B = W_jj^T B in place on tensor cores (each output
       // tile reads only its own columns of B)
@@ -1065,7 +1282,7 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
   return RSD_OK;
 }
 
-static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
+static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
   cudaStream_t s = ctx->stream, sa = ctx->side, sb = ctx->side2;
   cudaEvent_t evA = ctx->ev_la[0], evB = ctx->ev_la[1], evM = ctx->ev_la[2], evS = ctx->ev_la[3];
   int* err = st + 1;
@@ -1083,7 +1300,7 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, sa>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
+      launch_potf2(sa, exported, Ajj, lda, jb, st, j0, Wb);
       if (rest <= 0) continue;
       RSD_CUDA(ctx, cudaStreamWaitEvent(sa, evB, 0));
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel below block k
@@ -1143,9 +1360,9 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
   return RSD_OK;
 }
 
-int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st) {
-  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W, st)
-                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W, st);
+int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
+  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W, st, exported)
+                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W, st, exported);
 }
 
 // Blocked right-looking upper Cholesky with one step of look-ahead: the
@@ -1153,7 +1370,8 @@ int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, fl
 // higher-priority stream as soon as the first tile row of step j's trailing
 // update has landed, while the rest of that update runs on the main stream.
 template <typename T>
-int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc, int* d_status) {
+int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc, int* d_status,
+                      bool exported) {
   if (n < 1 || lda < n) return rsd_fail(ctx, RSD_EARG, "potrf: n=%d lda=%lld", n, (long long)lda);
   RSD_TRY(ensure_attrs<T>(ctx));
   RSD_TRY(rsd_side_stream(ctx));
@@ -1172,7 +1390,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
   bool two_level = false;
   if constexpr (F32) two_level = tc && ctx->use_tc && rsd_tc_syrk_ok(d_A, lda, d_A, lda, NB);
   if constexpr (F32) {
-    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W, st));
+    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W, st, exported));
   }
   if (!two_level) {
     RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
@@ -1186,7 +1404,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
       {
         // factor + inverse of the diagonal block, then the panel as W_jj^T B
         T* Wb = W + (size_t)b * NB * NB;
-        potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s2>>>(Ajj, lda, jb, st, j0, Wb); RSD_LAUNCH_NOTE();
+        launch_potf2(s2, exported, Ajj, lda, jb, st, j0, Wb);
         if (rest > 0) {
           launch_gemm<T>(s2, gp(jb, rest, jb, 1.0, Wb, NB, 1, Apan, lda, 0, 0.0, T1, NB));
           RSD_CUDA(ctx, cudaMemcpy2DAsync(Apan, lda * sizeof(T), T1, NB * sizeof(T), jb * sizeof(T), rest,
@@ -1862,7 +2080,7 @@ template int rsd_gemv<float>(rsd_ctx*, int, int, int, float, const float*, int64
                              float*, int64_t);
 template int rsd_gemv<double>(rsd_ctx*, int, int, int, double, const double*, int64_t, const double*, int64_t, int,
                               double, double*, int64_t);
-template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*);
+template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*, bool);
 template int rsd_potri_upper_t<float>(rsd_ctx*, int, float*, int64_t, const char*, int, const float*, int*);
 template int rsd_potrs_upper_t<float>(rsd_ctx*, int, const float*, int64_t, float*, int64_t, int, const char*,
                                       const float*);
@@ -1912,7 +2130,7 @@ extern "C" int rsd_potrf_f32_dev(rsd_ctx* ctx, int32_t n, float* d_A, int64_t ld
   RSD_TRY(check_prec(ctx, prec));
   RSD_TRY(rsd_set_device(ctx));
   int inf = 0;
-  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec, nullptr));
+  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec, nullptr, false));
   *info = inf;
   return RSD_OK;
 }
