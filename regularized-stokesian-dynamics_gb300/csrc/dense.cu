@@ -22,6 +22,7 @@
 
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
@@ -736,22 +737,6 @@ __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int6
         if (i + q <= j && i + q < jb) A[i + q + (int64_t)j * lda] = uv[q];
     }
   }
-}
-
-// Two FP32 operations in one instruction: the same rate per lane as two, half
-// the issue slots and instruction fetch.
-__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
 }
 
 // The same block (jb <= 128, padded with the identity) by Gauss-Jordan on [S |
@@ -1564,68 +1549,98 @@ int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag,
 // wide-block solves: each block copied out (lower part zero) and inverted in
 // place by the blocked triangular inverse.  W2: nblk2 blocks of NB2 x NB2.
 constexpr int NB2 = 512;
-// The NB2 diagonal blocks of U (n x n, blockIdx.z = block) into D (one NB2 x
-// NB2 block each, lower part and what lies past n zero).
-__global__ void copy_upper_blocks(int64_t n, const float* __restrict__ U, int64_t ldu, float* __restrict__ D) {
+// D_b, one NB2 x NB2 block per diagonal block b = blockIdx.z of U (n x n): the
+// inverses W of its NB-wide diagonal blocks, U's entries right of them, zero
+// below and past n.
+__global__ void wide_init(int64_t n, const float* __restrict__ U, int64_t ldu, const float* __restrict__ W,
+                          float* __restrict__ D) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.z;
-  if (t >= NB2 * NB2) return;
   const int i = t % NB2, j = t / NB2;
   const int64_t o = (int64_t)b * NB2;
-  D[(size_t)b * NB2 * NB2 + t] = i <= j && o + j < n ? U[(o + i) + (o + j) * ldu] : 0.0f;
-}
-
-// D_b(j0:j0+NB, j0:j0+NB) = W_{b NB2/NB + j0/NB} for every block b = blockIdx.z
-// (nb128 blocks W exist; a block past them stays zero)
-__global__ void put_diag_blocks(int j0, int nb128, const float* __restrict__ W, float* __restrict__ D) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.z;
-  if (t >= NB * NB || b * (NB2 / NB) + j0 / NB >= nb128) return;
-  const int i = t % NB, j = t / NB;
-  D[(size_t)b * NB2 * NB2 + (j0 + i) + (int64_t)(j0 + j) * NB2] = W[((size_t)b * (NB2 / NB) + j0 / NB) * NB * NB + t];
-}
-
-// In-place inverses of nblk upper triangular NB2 x NB2 blocks D_b (ld NB2,
-// stride NB2^2) from their NB diagonal-block inverses: trtri_inplace_t on
-// all blocks at once, one batched GEMM pair per NB column block.
-int trtri_wide_batched_s(rsd_ctx* ctx, int nblk, int nb128, float* D, const float* W, float* T1) {
-  cudaStream_t s = ctx->stream;
-  for (int j0 = 0; j0 < NB2; j0 += NB) {
-    if (j0 > 0) {
-      GemmP g = gp(j0, NB, j0, 1.0, D, NB2, 0, D + (int64_t)j0 * NB2, NB2, 0, 0.0, T1, NB2);
-      g.kA_row = 1;
-      g.offA = 0;
-      g.batch = nblk;
-      g.sA = g.sB = (int64_t)NB2 * NB2;
-      g.sC = (int64_t)NB2 * NB;
-      launch_gemm<float>(s, g);
-      GemmP g2 = gp(j0, NB, NB, -1.0, T1, NB2, 0, W + (size_t)(j0 / NB) * NB * NB, NB, 0, 0.0,
-                    D + (int64_t)j0 * NB2, NB2);
-      g2.batch = nblk;
-      g2.sA = (int64_t)NB2 * NB;
-      g2.sB = (int64_t)(NB2 / NB) * NB * NB;
-      g2.sC = (int64_t)NB2 * NB2;
-      launch_gemm<float>(s, g2);
-    }
-    put_diag_blocks<<<dim3(NB * NB / 256, 1, nblk), 256, 0, s>>>(j0, nb128, W, D); RSD_LAUNCH_NOTE();
+  float v = 0.f;
+  if (i / NB == j / NB) {
+    const int64_t blk = (o + j) / NB;
+    if (blk * NB < n) v = W[blk * NB * NB + i % NB + (j % NB) * NB];
+  } else if (i < j && o + j < n) {
+    v = U[(o + i) + (o + j) * ldu];
   }
-  return RSD_OK;
+  D[(size_t)b * NB2 * NB2 + t] = v;
 }
 
-// W128: the NB x NB diagonal-block inverses that the FP32 potrf of U left
-// (NB-block b at W128 + b NB^2); the NB2 blocks start from them, all blocks in
-// one batched pass.
+// One product of the recursive inverse [V11, -V11 U12 V22; 0, V22] of every
+// pair of h-wide blocks of every D_b (ld NB2): STEP 0 forms T = U12 V22, STEP
+// 1 V12 = -V11 T in U12's place.  32 x 32 outputs per CTA, four per thread, k
+// in chunks of 32 of the triangle; FP32 multiply-adds.
+template <int STEP>
+__global__ void __launch_bounds__(256) wide_combine(int h, float* __restrict__ D, float* __restrict__ Tb) {
+  __shared__ float As[32][33];
+  __shared__ __align__(16) float Bs[32][36];
+  const int pairs = NB2 / (2 * h), b = blockIdx.z / pairs, p = blockIdx.z % pairs;
+  float* Db = D + (size_t)b * NB2 * NB2 + (size_t)(2 * p * h) * (NB2 + 1);  // the pair's corner
+  float* T = Tb + (size_t)blockIdx.z * h * h;
+  const float* A = STEP ? Db : Db + (size_t)h * NB2;            // V11 or U12
+  const float* B = STEP ? T : Db + (size_t)h * (NB2 + 1);        // T or V22
+  const int ldb = STEP ? h : NB2, r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  const int kbeg = STEP ? r0 : 0, kend = STEP ? h : c0 + 32;     // V11 and V22 are upper triangular
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  float ra[4], rb[4];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      ra[q] = A[r0 + lane + (size_t)(k0 + w + 8 * q) * NB2];
+      rb[q] = B[k0 + lane + (size_t)(c0 + w + 8 * q) * ldb];
+    }
+  };
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  load(kbeg);
+  for (int k0 = kbeg; k0 < kend; k0 += 32) {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      As[w + 8 * q][lane] = ra[q];
+      Bs[lane][w + 8 * q] = rb[q];
+    }
+    __syncthreads();
+    if (k0 + 32 < kend) load(k0 + 32);
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+      const float a = As[k][lane];
+      const float4 x = *reinterpret_cast<const float4*>(&Bs[k][4 * w]);
+      acc[0] = fmaf(a, x.x, acc[0]);
+      acc[1] = fmaf(a, x.y, acc[1]);
+      acc[2] = fmaf(a, x.z, acc[2]);
+      acc[3] = fmaf(a, x.w, acc[3]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int c = c0 + 4 * w + q;
+    if (STEP)
+      Db[r0 + lane + (size_t)(h + c) * NB2] = -acc[q];
+    else
+      T[r0 + lane + (size_t)c * h] = acc[q];
+  }
+}
+
+// The inverses of U's NB2-wide diagonal blocks, from the NB-wide ones that the
+// FP32 potrf of U left (NB-block b at W128 + b NB^2), two levels of pairs.
+// (By block columns with 128 x 128 tiles a factor's six products took 134 us:
+// one or two CTAs, K up to 384; these take 44 us at n = 1038, 104 at 3072.)
 int rsd_wide_inverses_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const char* tag, const float* W128,
                         float** W2out) {
-  const int nblk2 = (n + NB2 - 1) / NB2, nb128 = (n + NB - 1) / NB;
+  const int nblk2 = (n + NB2 - 1) / NB2;
   std::string name = std::string("wide_W_") + tag;
   float* W2 = (float*)rsd_scratch(ctx, name.c_str(), sizeof(float) * (size_t)nblk2 * NB2 * NB2);
-  float* Tb = (float*)rsd_scratch(ctx, "wide_T1b", sizeof(float) * (size_t)nblk2 * NB * NB2);
-  // a whole block of inverses per NB2 block is addressed in the batch
-  float* Wp = (float*)rsd_scratch(ctx, "wide_Wpad", sizeof(float) * (size_t)nblk2 * (NB2 / NB) * NB * NB);
-  if (!W2 || !Tb || !Wp) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemsetAsync(Wp, 0, sizeof(float) * (size_t)nblk2 * (NB2 / NB) * NB * NB, ctx->stream));
-  RSD_CUDA(ctx, cudaMemcpyAsync(Wp, W128, sizeof(float) * (size_t)nb128 * NB * NB, cudaMemcpyDeviceToDevice, ctx->stream));
-  copy_upper_blocks<<<dim3(NB2 * NB2 / 256, 1, nblk2), 256, 0, ctx->stream>>>(n, U, ldu, W2); RSD_LAUNCH_NOTE();
-  RSD_TRY(trtri_wide_batched_s(ctx, nblk2, nb128, W2, Wp, Tb));
+  float* Tb = (float*)rsd_scratch(ctx, "wide_T", sizeof(float) * (size_t)nblk2 * (NB2 / 2) * (NB2 / 2));
+  if (!W2 || !Tb) return RSD_ENOMEM;
+  cudaStream_t s = ctx->stream;
+  wide_init<<<dim3(NB2 * NB2 / 256, 1, nblk2), 256, 0, s>>>(n, U, ldu, W128, W2); RSD_LAUNCH_NOTE();
+  for (int h = NB; h < NB2; h *= 2) {
+    if (n <= h) break;  // one block: no second half anywhere
+    const dim3 grid(h / 32, h / 32, nblk2 * (NB2 / (2 * h)));
+    wide_combine<0><<<grid, 256, 0, s>>>(h, W2, Tb); RSD_LAUNCH_NOTE();
+    wide_combine<1><<<grid, 256, 0, s>>>(h, W2, Tb); RSD_LAUNCH_NOTE();
+  }
   RSD_CUDA(ctx, cudaGetLastError());
   *W2out = W2;
   return RSD_OK;

@@ -27,6 +27,7 @@
 #include "ewald_gen.cuh"
 #include "overlap.cuh"
 #include "dsf.cuh"
+#include "f32x2.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
@@ -553,16 +554,15 @@ __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, in
 // between moments.
 constexpr int KBW = 64;  // weights per vector (60 used, padded for 16-byte rows)
 
-template <typename T>
-__device__ __forceinline__ void put_weight(T* p, double v) { *p = (T)v; }
-template <>
-__device__ __forceinline__ void put_weight<dsf>(dsf* p, double v) { *p = dsf_from(v); }
-
-template <typename T>
-__global__ void ewald_kblock_list(rsd_lat_dev L, int count, const int* __restrict__ hlist, double a,
-                                  double inv_pimu, T* __restrict__ W) {
+// Block weights of the listed vectors: the first K64 as a row of hi parts and
+// a row of lo parts (2 KBW floats a vector), the K32 others in FP32 (KBW
+// floats).  blockIdx.y = 0 forms the cos outputs, 1 the sin ones: a warp
+// issues an FP64 instruction every 64 cycles, so the kernel's time is one
+// thread's instruction count.
+__global__ void ewald_kblock_lists(rsd_lat_dev L, int K64, int K32, const int* __restrict__ hlist, double a,
+                                   double inv_pimu, float* __restrict__ W64, float* __restrict__ W32) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= count) return;
+  if (q >= K64 + K32) return;
   int nx, ny, nz;
   half_space_index(hlist[q], L.NI, &nx, &ny, &nz);
   double k[3];
@@ -570,117 +570,164 @@ __global__ void ewald_kblock_list(rsd_lat_dev L, int count, const int* __restric
     k[j] = 2.0 * RSD_PI * (nx * L.LI[0 + 3 * j] + ny * L.LI[1 + 3 * j] + nz * L.LI[2 + 3 * j]);
   const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
   const double S = kernel_S<double>(k2, L.lam);
-  double wc[RSD_NMOM_KCOS], ws[RSD_NMOM_KSIN], v[60], w[60];
-  rsd_kcos_weights<double>(k[0], k[1], k[2], S, L.lam, wc);
-  rsd_ksin_weights<double>(k[0], k[1], k[2], S, L.lam, ws);
-  rsd_kcos_epilogue<double>(wc, a, a, L.phix, v);
-  rsd_ksin_epilogue<double>(ws, a, a, L.phix, w);
   // half space counted twice, and the non-dimensionalisation of scale_block
   const double f = 2.0 / L.LV, na = f * inv_pimu / (6.0 * a), na3 = na / (a * a);
-  T* e = W + (size_t)q * KBW;
-  for (int i = 0; i < 60; i++) {
-    const bool a3 = (i >= 6 && i < 12) || (i >= 15 && i < 30) || i >= 45;
-    put_weight<T>(e + i, (kblock_is_sin(i) ? w[i] : v[i]) * (a3 ? na3 : na));
+  auto put = [&](int i, double v) {
+    if (q < K64) {
+      const dsf d = dsf_from(v);
+      W64[(size_t)q * 2 * KBW + i] = d.hi;
+      W64[(size_t)q * 2 * KBW + KBW + i] = d.lo;
+    } else {
+      W32[(size_t)(q - K64) * KBW + i] = (float)v;
+    }
+  };
+  double w[RSD_NMOM_KCOS], v[60];
+  if (blockIdx.y == 0) {
+    rsd_kcos_weights<double>(k[0], k[1], k[2], S, L.lam, w);
+    rsd_kcos_epilogue<double>(w, a, a, L.phix, v);
+#pragma unroll
+    for (int i = 0; i < 60; i++) {
+      const bool a3 = (i >= 6 && i < 12) || (i >= 15 && i < 30) || i >= 45;
+      if (!kblock_is_sin(i)) put(i, v[i] * (a3 ? na3 : na));
+    }
+    for (int i = 60; i < KBW; i++) put(i, 0.0);
+  } else {
+    rsd_ksin_weights<double>(k[0], k[1], k[2], S, L.lam, w);
+    rsd_ksin_epilogue<double>(w, a, a, L.phix, v);
+#pragma unroll
+    for (int i = 0; i < 60; i++)
+      if (kblock_is_sin(i)) put(i, v[i] * na);  // TR and G
   }
-  for (int i = 60; i < KBW; i++) put_weight<T>(e + i, 0.0);
 }
 
-__device__ __forceinline__ void acc_norm(dsacc& a) { dsacc_norm(a); }
-
-// FP32 sum of the vectors of one chunk (f), folded at the end of every chunk
-// into a double-single total (hi + lo, Knuth's two-sum).  A plain FP32 sum
-// over all K32 vectors has a rounding error ~ sqrt(K32) times that of its
-// terms, which grows with the number of FP32 vectors (with lambda^3).
-struct fchunk {
-  float f, hi, lo;
-};
-__device__ __forceinline__ fchunk fma(float e, float c, fchunk a) {
-  a.f = __fmaf_rn(e, c, a.f);
-  return a;
-}
-__device__ __forceinline__ void acc_norm(fchunk& a) {
-  const float s = __fadd_rn(a.hi, a.f);
-  const float bb = __fsub_rn(s, a.hi);
-  a.lo = __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(a.f, bb)));
-  a.hi = s;
-  a.f = 0.f;
-}
-
-__device__ __forceinline__ float trig_c(float2 v) { return v.x; }
-__device__ __forceinline__ float trig_s(float2 v) { return v.y; }
-__device__ __forceinline__ dsf trig_c(float4 v) { return dsf(v.x, v.y); }
-__device__ __forceinline__ dsf trig_s(float4 v) { return dsf(v.z, v.w); }
-
-// Accumulates sum_k W_q(k) {cos, sin}(k.(x_a - x_b)) over Kh vectors into
-// acc, for the pair (a, b) of the calling thread (block 32 x 4).  The
-// weights of 16 vectors and the trig values of the CTA's 32 + 4 particles
-// are staged in shared memory (sw: 16 x KBW, sca: 16 x 32, scb: 16 x 4).
-template <typename T, typename TT, typename A>
-__device__ __forceinline__ void kblock_accumulate(int nn, int Kh, const T* __restrict__ W, const TT* __restrict__ cs,
-                                                  T* sw, TT* sca, TT* scb, bool valid, A (&acc)[60]) {
-  constexpr int KC = 16;
+// Stages 16 vectors' weights (floats per vector: NW) and the trig values of
+// the CTA's 32 + 4 particles in shared memory.
+template <int NW, typename TT>
+__device__ __forceinline__ void kblock_stage(int nn, int h0, int kc, const float* __restrict__ W,
+                                             const TT* __restrict__ cs, float* sw, TT* sca, TT* scb) {
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
   const int a0 = blockIdx.x * blockDim.x, b0 = blockIdx.y * blockDim.y;
-  for (int h0 = 0; h0 < Kh; h0 += KC) {
-    const int kc = min(KC, Kh - h0);
-    __syncthreads();
-    for (int e = tid; e < kc * KBW; e += nthr) sw[e] = W[(size_t)h0 * KBW + e];
-    for (int e = tid; e < kc * 36; e += nthr) {
-      const int hh = e / 36, q = e % 36, part = q < 32 ? a0 + q : b0 + q - 32;
-      if (part < nn) {
-        const TT v = cs[(size_t)(h0 + hh) * nn + part];
-        if (q < 32)
-          sca[hh * 32 + q] = v;
-        else
-          scb[hh * 4 + q - 32] = v;
-      }
+  const float4* src = reinterpret_cast<const float4*>(W + (size_t)h0 * NW);
+  for (int e = tid; e < kc * NW / 4; e += nthr) reinterpret_cast<float4*>(sw)[e] = src[e];
+  for (int e = tid; e < kc * 36; e += nthr) {
+    const int hh = e / 36, q = e % 36, part = q < 32 ? a0 + q : b0 + q - 32;
+    if (part < nn) {
+      const TT v = cs[(size_t)(h0 + hh) * nn + part];
+      if (q < 32)
+        sca[hh * 32 + q] = v;
+      else
+        scb[hh * 4 + q - 32] = v;
     }
-    __syncthreads();
-    if (!valid) continue;
-    for (int hh = 0; hh < kc; hh++) {
-      const TT ua = sca[hh * 32 + threadIdx.x], ub = scb[hh * 4 + threadIdx.y];
-      const T ca = trig_c(ua), sa = trig_s(ua), cb = trig_c(ub), sb = trig_s(ub);
-      const T c = ca * cb + sa * sb;   // cos(k.(x_a - x_b))
-      const T sn = sa * cb - ca * sb;  // sin(k.(x_a - x_b))
-      const T* e = sw + hh * KBW;
-#pragma unroll
-      for (int q = 0; q < 60; q++) acc[q] = fma(e[q], kblock_is_sin(q) ? sn : c, acc[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 60; q++) acc_norm(acc[q]);  // at most 16 steps between renormalisations
   }
 }
 
-// Reciprocal-space pair blocks with per-vector block weights (equal radii):
-// the K32 FP32 vectors first, then the K64 double-single ones on top of the
-// FP32 sums; the blocks are written (add = 0) or added (add = 1) once.
+// Reciprocal-space pair blocks with per-vector block weights (equal radii),
+// the sums sum_k W_q(k) {cos, sin}(k.(x_a - x_b)) in packed pairs of outputs
+// (30 pairs; a pair takes cos, sin or, at two seams, one of each):
+//   - the K32 FP32 vectors first, a chunk of 16 summed in FP32 and folded into
+//     a double-single total (hi + lo, Knuth's two-sum): a plain FP32 sum over
+//     all K32 vectors has a rounding error ~ sqrt(K32) times that of its
+//     terms, which grows with lambda^3;
+//   - then the K64 double-single ones on top, as dsacc's multiply-add (dsf.cuh)
+//     with the products taken against -cos, -sin, so that no sign is flipped.
+// The blocks are written (add = 0) or added (add = 1) once.  Bound by FP32
+// issue at 8 warps per SM (accumulators in registers); the packed form halves
+// the instructions: N = 2048 10.4 -> 8.1 ms, N = 512 0.74 -> 0.56 ms.
 __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const float* __restrict__ W32,
                                                          const float2* __restrict__ c32, int K64,
-                                                         const dsf* __restrict__ W64, const float4* __restrict__ c64,
+                                                         const float* __restrict__ W64, const float4* __restrict__ c64,
                                                          PlaneSink sk, int add) {
   constexpr int KC = 16;
-  __shared__ __align__(16) dsf sw[KC * KBW];  // the FP32 phase uses the first half as floats
+  __shared__ __align__(16) float sw[KC * 2 * KBW];  // the FP32 phase uses the first half
   __shared__ __align__(16) float4 sca[KC * 32], scb[KC * 4];
   if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
   int a, b;
   const bool valid = pair_of(nn, &a, &b);
-  dsacc acc[60];
+  uint64_t hi[30], lo[30];
+#pragma unroll
+  for (int p = 0; p < 30; p++) hi[p] = lo[p] = 0;
   {
-    fchunk f[60];
+    uint64_t f[30];
 #pragma unroll
-    for (int q = 0; q < 60; q++) f[q] = fchunk{0.f, 0.f, 0.f};
-    kblock_accumulate<float, float2>(nn, K32, W32, c32, reinterpret_cast<float*>(sw),
-                                     reinterpret_cast<float2*>(sca), reinterpret_cast<float2*>(scb), valid, f);
+    for (int p = 0; p < 30; p++) f[p] = 0;
+    float2 *ta = reinterpret_cast<float2*>(sca), *tb = reinterpret_cast<float2*>(scb);
+    for (int h0 = 0; h0 < K32; h0 += KC) {
+      const int kc = min(KC, K32 - h0);
+      __syncthreads();
+      kblock_stage<KBW>(nn, h0, kc, W32, c32, sw, ta, tb);
+      __syncthreads();
+      if (!valid) continue;
+      for (int hh = 0; hh < kc; hh++) {
+        const float2 ua = ta[hh * 32 + threadIdx.x], ub = tb[hh * 4 + threadIdx.y];
+        const float c = ua.x * ub.x + ua.y * ub.y;   // cos(k.(x_a - x_b))
+        const float sn = ua.y * ub.x - ua.x * ub.y;  // sin(k.(x_a - x_b))
+        const uint64_t cc = f2_pack(c, c), ss = f2_pack(sn, sn), sc = f2_pack(sn, c);
+        const ulonglong2* e = reinterpret_cast<const ulonglong2*>(sw + hh * KBW);
 #pragma unroll
-    for (int q = 0; q < 60; q++) acc[q] = dsacc(f[q].hi, f[q].lo);
+        for (int g = 0; g < 15; g++) {
+          const ulonglong2 w = e[g];
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const int q = 4 * g + 2 * u;
+            f[2 * g + u] = f2_fma(u ? w.y : w.x, !kblock_is_sin(q) ? cc : (kblock_is_sin(q + 1) ? ss : sc), f[2 * g + u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 30; p++) {
+        const uint64_t s = f2_add(hi[p], f[p]), bb = f2_sub(s, hi[p]);
+        lo[p] = f2_add(lo[p], f2_add(f2_sub(hi[p], f2_sub(s, bb)), f2_sub(f[p], bb)));
+        hi[p] = s;
+        f[p] = 0;
+      }
+    }
   }
-  kblock_accumulate<dsf, float4>(nn, K64, W64, c64, sw, sca, scb, valid, acc);
+  for (int h0 = 0; h0 < K64; h0 += KC) {
+    const int kc = min(KC, K64 - h0);
+    __syncthreads();
+    kblock_stage<2 * KBW>(nn, h0, kc, W64, c64, sw, sca, scb);
+    __syncthreads();
+    if (!valid) continue;
+    for (int hh = 0; hh < kc; hh++) {
+      const float4 ua = sca[hh * 32 + threadIdx.x], ub = scb[hh * 4 + threadIdx.y];
+      const dsf ca(ua.x, ua.y), sa(ua.z, ua.w), cb(ub.x, ub.y), sb(ub.z, ub.w);
+      const dsf c = ca * cb + sa * sb, sn = sa * cb - ca * sb;
+      const uint64_t ch[3] = {f2_pack(c.hi, c.hi), f2_pack(sn.hi, sn.hi), f2_pack(sn.hi, c.hi)};
+      const uint64_t nh[3] = {f2_pack(-c.hi, -c.hi), f2_pack(-sn.hi, -sn.hi), f2_pack(-sn.hi, -c.hi)};
+      const uint64_t nl[3] = {f2_pack(-c.lo, -c.lo), f2_pack(-sn.lo, -sn.lo), f2_pack(-sn.lo, -c.lo)};
+      const ulonglong2* eh = reinterpret_cast<const ulonglong2*>(sw + hh * 2 * KBW);
+      const ulonglong2* el = reinterpret_cast<const ulonglong2*>(sw + hh * 2 * KBW + KBW);
+#pragma unroll
+      for (int g = 0; g < 15; g++) {
+        const ulonglong2 wh = eh[g], wl = el[g];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int q = 4 * g + 2 * u, p = 2 * g + u;
+          const int k = !kblock_is_sin(q) ? 0 : (kblock_is_sin(q + 1) ? 1 : 2);
+          const uint64_t xh = u ? wh.y : wh.x, xl = u ? wl.y : wl.x;
+          const uint64_t pr = f2_mul(xh, ch[k]);
+          const uint64_t ne = f2_fma(xh, nl[k], f2_fma(xl, nh[k], f2_fma(xh, nh[k], pr)));  // minus the product's error
+          const uint64_t s = f2_add(hi[p], pr), bb = f2_sub(s, hi[p]);
+          const uint64_t e = f2_add(f2_sub(hi[p], f2_sub(s, bb)), f2_sub(pr, bb));
+          lo[p] = f2_add(lo[p], f2_sub(e, ne));
+          hi[p] = s;
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < 30; p++) {  // at most 16 steps between renormalisations
+      const uint64_t s = f2_add(hi[p], lo[p]);
+      lo[p] = f2_sub(lo[p], f2_sub(s, hi[p]));
+      hi[p] = s;
+    }
+  }
   if (!valid) return;
   dsf o[60];
 #pragma unroll
-  for (int q = 0; q < 60; q++) {
-    dsacc_norm(acc[q]);
-    o[q] = dsf(acc[q].hi, acc[q].lo);
+  for (int p = 0; p < 30; p++) {
+    const uint64_t s = f2_add(hi[p], lo[p]), l = f2_sub(lo[p], f2_sub(s, hi[p]));
+    f2_unpack(s, o[2 * p].hi, o[2 * p + 1].hi);
+    f2_unpack(l, o[2 * p].lo, o[2 * p + 1].lo);
   }
   store_pair_rows_a(sk, nn, a, b, o, add);
 }
@@ -838,19 +885,6 @@ struct RealEqShared {
   float ol[60][REAL_THREADS];  // lo of the sum
 };
 constexpr int SMEM_REAL_EQ = (int)sizeof(RealEqShared);
-
-// The coefficient tables for radius a (double-single and FP32).
-__global__ void ewald_real_epi_table(double a, double phix, double inv_pimu, dsf* __restrict__ cr,
-                                     float* __restrict__ cf) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double c[RSD_REAL_EPI_NC];
-  const double s1 = inv_pimu / (6.0 * a), s3 = s1 / (a * a);
-  rsd_real_epi_coef_scaled<double>(a, a, phix, s1, s3, c);
-  for (int k = 0; k < RSD_REAL_EPI_NC; k++) {
-    cr[k] = dsf_from(c[k]);
-    cf[k] = (float)c[k];
-  }
-}
 
 __device__ __forceinline__ int pack_image(int nx, int ny, int nz, int NR) {
   return (nx + NR) | ((ny + NR) << 8) | ((nz + NR) << 16);
@@ -1693,22 +1727,48 @@ int upload_lists(rsd_ctx* ctx, const ewald_lists& H, bool equal, double a, const
   return RSD_OK;
 }
 
-// The weights of D's vectors and the diagonal blocks.
+// The weights of D's vectors on the context's stream, then the diagonal
+// blocks beside what follows there, on the side stream: latency-bound kernels
+// of one CTA (~65 us).  A self_join makes the stream wait for them, on every
+// way out of its scope.
+struct self_join {
+  rsd_ctx* ctx;
+  bool open = true;
+  int close() {
+    open = false;
+    RSD_CUDA(ctx, cudaEventRecord(ctx->ev_la[1], ctx->side));
+    RSD_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_la[1], 0));
+    return RSD_OK;
+  }
+  ~self_join() {
+    if (open) close();
+  }
+};
+
 template <typename S>
 int assemble_self(rsd_ctx* ctx, int nn, const double* d_radii, double a0, bool equal, const rsd_lat_dev& L,
-                  double inv_pimu, const ewald_dev_lists& D, const S& sk) {
-  cudaStream_t s = ctx->stream;
+                  double inv_pimu, const ewald_dev_lists& D, bool weights_beside, const S& sk) {
+  RSD_TRY(rsd_side_stream(ctx));
+  cudaStream_t s = ctx->side, ws = weights_beside ? s : ctx->stream;
+  auto fork = [&]() -> int {
+    RSD_CUDA(ctx, cudaEventRecord(ctx->ev_la[0], ctx->stream));
+    RSD_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_la[0], 0));
+    return RSD_OK;
+  };
+  if (weights_beside) RSD_TRY(fork());
   double* W = (double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
   double* self = (double*)rsd_scratch(ctx, "ewald_self_sums", sizeof(double) * SELF_NMOM);
   if (!W || !self) return RSD_ENOMEM;
   const dim3 wg((unsigned)((D.Kh + 31) / 32), 2);
   if (equal) {
-    ewald_weights<true><<<wg, 32, 0, s>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    ewald_weights<true><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    if (!weights_beside) RSD_TRY(fork());
     ewald_self_sums<true><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
                                                      D.etab, self); RSD_LAUNCH_NOTE();
     ewald_self_eq<<<(121 * nn + 255) / 256, 256, 0, s>>>(nn, self, sk); RSD_LAUNCH_NOTE();
   } else {
-    ewald_weights<false><<<wg, 32, 0, s>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    ewald_weights<false><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    if (!weights_beside) RSD_TRY(fork());
     ewald_self_sums<false><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
                                                       D.etab, self); RSD_LAUNCH_NOTE();
     ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, self, d_radii, inv_pimu, sk); RSD_LAUNCH_NOTE();
@@ -1730,8 +1790,9 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
   ewald_dev_lists D;
   RSD_TRY(upload_lists(ctx, cube ? ewald_cube_lists(L) : ewald_sphere_lists(L, L.lam, false), equal, a0, L, inv_pimu,
                        &D));
-  RSD_TRY(assemble_self(ctx, nn, d_radii, a0, equal, L, inv_pimu, D, sk));
-  if (nn < 2) return RSD_OK;
+  RSD_TRY(assemble_self(ctx, nn, d_radii, a0, equal, L, inv_pimu, D, false, sk));
+  self_join join{ctx};
+  if (nn < 2) return join.close();
   double2* cs = (double2*)rsd_scratch(ctx, "ewald_trig", sizeof(double2) * (size_t)D.Kh * nn);
   const double* W = (const double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
   if (!cs || !W) return RSD_ENOMEM;
@@ -1752,7 +1813,7 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
     equal ? go(narrow{}, std::true_type{}) : go(narrow{}, std::false_type{});
   }
   RSD_CUDA(ctx, cudaGetLastError());
-  return RSD_OK;
+  return join.close();
 }
 }  // namespace
 
@@ -1773,7 +1834,8 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
   const ewald_lists SL = ewald_sphere_lists(L, L.lam, /*self_only=*/true);
   ewald_dev_lists D;
   RSD_TRY(upload_lists(ctx, SL, equal, h_radii[0], L, inv_pimu, &D));
-  RSD_TRY(assemble_self(ctx, nn, d_radii, h_radii[0], equal, L, inv_pimu, D, psk));
+  RSD_TRY(assemble_self(ctx, nn, d_radii, h_radii[0], equal, L, inv_pimu, D, true, psk));
+  self_join join{ctx};
   if (nn > 1) {
     dim3 blk(32, 4), grd((nn + 31) / 32, (nn + 3) / 4);
     {
@@ -1810,15 +1872,33 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
           h32.push_back(h);
       }
       const int K64 = (int)h64.size(), K32 = (int)h32.size();
-      int* dh = (int*)rsd_scratch(ctx, "ewald_hlist", sizeof(int) * (size_t)Kh);
-      double* t64 = (double*)rsd_scratch(ctx, "ewald_ktab64", sizeof(double) * (size_t)(K64 > 0 ? K64 : 1) * KW);
-      float* t32 = (float*)rsd_scratch(ctx, "ewald_ktab32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KW);
+      // one copy: the vector indices and, for equal radii, the coefficients of
+      // the real-space epilogue (double-single, FP32)
+      const size_t nidx = (h64.size() + h32.size() + 3) / 4 * 4;
+      std::vector<int> up(nidx + 3 * RSD_REAL_EPI_NC, 0);
+      std::copy(h64.begin(), h64.end(), up.begin());
+      std::copy(h32.begin(), h32.end(), up.begin() + h64.size());
+      if (equal) {
+        double c[RSD_REAL_EPI_NC];
+        const double s1 = inv_pimu / (6.0 * h_radii[0]);
+        rsd_real_epi_coef_scaled<double>(h_radii[0], h_radii[0], L.phix, s1, s1 / (h_radii[0] * h_radii[0]), c);
+        dsf* hr = reinterpret_cast<dsf*>(up.data() + nidx);
+        float* hf = reinterpret_cast<float*>(hr + RSD_REAL_EPI_NC);
+        for (int k = 0; k < RSD_REAL_EPI_NC; k++) {
+          const float h = (float)c[k];
+          hr[k].hi = hf[k] = h;
+          hr[k].lo = (float)(c[k] - (double)h);
+        }
+      }
+      int* dh = (int*)rsd_scratch(ctx, "ewald_hlist", sizeof(int) * up.size());
+      double* t64 = equal ? nullptr : (double*)rsd_scratch(ctx, "ewald_ktab64", sizeof(double) * (size_t)(K64 > 0 ? K64 : 1) * KW);
+      float* t32 = equal ? nullptr : (float*)rsd_scratch(ctx, "ewald_ktab32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KW);
       float4* c64 = (float4*)rsd_scratch(ctx, "ewald_trig64", sizeof(float4) * (size_t)(K64 > 0 ? K64 : 1) * nn);
       float2* c32 = (float2*)rsd_scratch(ctx, "ewald_trig32", sizeof(float2) * (size_t)(K32 > 0 ? K32 : 1) * nn);
-      if (!dh || !t64 || !t32 || !c64 || !c32) return RSD_ENOMEM;
-      std::vector<int> all(h64);
-      all.insert(all.end(), h32.begin(), h32.end());
-      RSD_CUDA(ctx, cudaMemcpyAsync(dh, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice, s));
+      if (!dh || (!equal && (!t64 || !t32)) || !c64 || !c32) return RSD_ENOMEM;
+      RSD_CUDA(ctx, cudaMemcpyAsync(dh, up.data(), sizeof(int) * up.size(), cudaMemcpyHostToDevice, s));
+      const dsf* cr = reinterpret_cast<const dsf*>(dh + nidx);
+      const float* cf = reinterpret_cast<const float*>(cr + RSD_REAL_EPI_NC);
       if (K64) {
         ewald_trig_list<float4><<<dim3((nn + 127) / 128, K64), 128, 0, s>>>(nn, L, dh, d_pos, c64); RSD_LAUNCH_NOTE();
       }
@@ -1826,14 +1906,11 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         ewald_trig_list<float2><<<dim3((nn + 127) / 128, K32), 128, 0, s>>>(nn, L, dh + K64, d_pos, c32); RSD_LAUNCH_NOTE();
       }
       if (equal) {
-        dsf* w64 = (dsf*)rsd_scratch(ctx, "ewald_kblock64", sizeof(dsf) * (size_t)(K64 > 0 ? K64 : 1) * KBW);
+        float* w64 = (float*)rsd_scratch(ctx, "ewald_kblock64", sizeof(float) * (size_t)(K64 > 0 ? K64 : 1) * 2 * KBW);
         float* w32 = (float*)rsd_scratch(ctx, "ewald_kblock32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KBW);
         if (!w64 || !w32) return RSD_ENOMEM;
-        if (K64) {
-          ewald_kblock_list<dsf><<<(K64 + 127) / 128, 128, 0, s>>>(L, K64, dh, h_radii[0], inv_pimu, w64); RSD_LAUNCH_NOTE();
-        }
-        if (K32) {
-          ewald_kblock_list<float><<<(K32 + 127) / 128, 128, 0, s>>>(L, K32, dh + K64, h_radii[0], inv_pimu, w32); RSD_LAUNCH_NOTE();
+        if (K64 + K32) {
+          ewald_kblock_lists<<<dim3((K64 + K32 + 31) / 32, 2), 32, 0, s>>>(L, K64, K32, dh, h_radii[0], inv_pimu, w64, w32); RSD_LAUNCH_NOTE();
         }
         ewald_pair_kblock<<<grd, blk, 0, s>>>(nn, K32, w32, c32, K64, w64, c64, psk, 0); RSD_LAUNCH_NOTE();
       } else {
@@ -1847,10 +1924,6 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         ewald_pair_k<float, float2><<<grd, blk, 0, s>>>(nn, L, K32, t32, c32, d_radii, inv_pimu, psk, 1); RSD_LAUNCH_NOTE();
       }
       if (equal) {
-        dsf* cr = (dsf*)rsd_scratch(ctx, "ewald_real_cr", sizeof(dsf) * RSD_REAL_EPI_NC);
-        float* cf = (float*)rsd_scratch(ctx, "ewald_real_cf", sizeof(float) * RSD_REAL_EPI_NC);
-        if (!cr || !cf) return RSD_ENOMEM;
-        ewald_real_epi_table<<<1, 32, 0, s>>>(h_radii[0], L.phix, inv_pimu, cr, cf); RSD_LAUNCH_NOTE();
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
         ewald_pair_real_near_ds<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, rc2, psk); RSD_LAUNCH_NOTE();
@@ -1859,5 +1932,5 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
     }
   }
   RSD_CUDA(ctx, cudaGetLastError());
-  return RSD_OK;
+  return join.close();
 }
