@@ -56,6 +56,21 @@ void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes) {
   return b.p;
 }
 
+void* rsd_pinned(rsd_ctx* ctx, size_t bytes) {
+  if (ctx->h_io_bytes >= bytes) return ctx->h_io;
+  if (ctx->h_io) cudaFreeHost(ctx->h_io);
+  ctx->h_io = nullptr;
+  ctx->h_io_bytes = 0;
+  if (cudaMallocHost(&ctx->h_io, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->h_io = nullptr;
+    rsd_fail(ctx, RSD_ENOMEM, "cannot allocate %zu pinned bytes", bytes);
+    return nullptr;
+  }
+  ctx->h_io_bytes = bytes;
+  return ctx->h_io;
+}
+
 int rsd_set_device(rsd_ctx* ctx) {
   RSD_CUDA(ctx, cudaSetDevice(ctx->device));
   return RSD_OK;
@@ -83,8 +98,8 @@ extern "C" int rsd_ctx_create(rsd_ctx** out, int device) {
   c->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_info, 64 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMallocHost(&c->h_info, 64 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&c->d_info, RSD_INFO_BYTES);
+  if (e == cudaSuccess) e = cudaMallocHost(&c->h_info, RSD_INFO_BYTES);
   for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) {
@@ -130,6 +145,7 @@ extern "C" int rsd_ctx_destroy(rsd_ctx* c) {
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->d_info) cudaFree(c->d_info);
   if (c->h_info) cudaFreeHost(c->h_info);
+  if (c->h_io) cudaFreeHost(c->h_io);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return RSD_OK;

@@ -1961,16 +1961,16 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
   const int gsm = ctx->sm_count > 0 ? ctx->sm_count : 148;
   if (nblk2 > TRI_MAX_BLOCKS) return rsd_fail(ctx, RSD_EUNSUP, "uhat solve: order %d above %d", n, TRI_MAX_BLOCKS * NB2);
   // [0] error (cumulative), [1], [2] tickets, then the ready counts of the two sweeps
-  int* sync = rsd_uhat_error_flag(ctx);
+  int* sync = (int*)rsd_scratch(ctx, "tri_sync", sizeof(int) * (size_t)(2 * TRI_MAX_BLOCKS + 2));
   if (!sync) return RSD_ENOMEM;
   // leading zero blocks of the right-hand side: the forward sweep starts at
   // the first block that can be nonzero (z is zero before it)
   const int b0 = zero_lead > 0 ? min(zero_lead / NB2, nblk2 - 1) : 0;
-  TriArgs A{h->Uh, h->ld, n, nblk2, X, ldx, sync + 3, sync + 1, sync, b0,
+  TriArgs A{h->Uh, h->ld, n, nblk2, X, ldx, sync + 2, sync, rsd_uhat_error_flag(ctx), b0,
             ctx->tri_spin_polls > 0 ? ctx->tri_spin_polls : TRI_SPIN_LIMIT};
   const int tasks = TRI_Q * (nblk2 - 1);
   const int ftasks = TRI_Q * (nblk2 - 1 - b0);
-  if (tasks > 0) RSD_CUDA(ctx, cudaMemsetAsync(sync + 1, 0, sizeof(int) * (size_t)(2 + 2 * nblk2), s));
+  if (tasks > 0) RSD_CUDA(ctx, cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)(2 + 2 * nblk2), s));
   if (ftasks > 0) {  // forward, in place on X
     const int fgrid = max(1, min(ftasks, 4 * gsm));
     if (nrhs == 1)
@@ -1987,8 +1987,8 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
   if (tasks > 0) {  // backward, in place on Y
     A.V = Y;
     A.b0 = 0;
-    A.ticket = sync + 2;
-    A.ready = sync + 3 + nblk2;
+    A.ticket = sync + 1;
+    A.ready = sync + 2 + nblk2;
     const int grid = max(1, min(tasks, 4 * gsm));
     if (nrhs == 1)
       tri_backward<1><<<grid, TRI_THREADS, 0, s>>>(A);
@@ -2000,12 +2000,10 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
   return RSD_OK;
 }
 
-// The dataflow sweeps' synchronisation words; element 0 is a cumulative
-// error flag, nonzero once a sweep's wait timed out (the caller zeroes it
-// and reads it after synchronising the stream).
-int* rsd_uhat_error_flag(rsd_ctx* ctx) {
-  return (int*)rsd_scratch(ctx, "tri_sync", sizeof(int) * (size_t)(2 * TRI_MAX_BLOCKS + 3));
-}
+// The dataflow sweeps' cumulative error flag (status word 24), nonzero once a
+// sweep's wait timed out (the caller zeroes it and reads it after
+// synchronising the stream).
+int* rsd_uhat_error_flag(rsd_ctx* ctx) { return ctx->d_info + 24; }
 
 // The same by blocks on the factor itself (FP32 SIMT form): X is overwritten,
 // the solution is in Y.

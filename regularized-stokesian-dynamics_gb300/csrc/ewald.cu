@@ -1695,7 +1695,7 @@ struct ewald_dev_lists {
 
 // One copy brings the lists and, for equal radii, the coefficients of the
 // real-space epilogue to the device.
-int upload_lists(rsd_ctx* ctx, const ewald_lists& H, bool equal, double a, const rsd_lat_dev& L, double inv_pimu,
+int upload_lists(rsd_ctx* ctx, cudaStream_t s, const ewald_lists& H, bool equal, double a, const rsd_lat_dev& L, double inv_pimu,
                  ewald_dev_lists* D) {
   const size_t ni = H.img.size() / 3, nk = H.kv.size() / 3;
   const size_t nt = 5 * ni + 3 * nk + RSD_REAL_EPI_NC;  // float4 = two doubles
@@ -1715,7 +1715,7 @@ int upload_lists(rsd_ctx* ctx, const ewald_lists& H, bool equal, double a, const
   }
   double* d = (double*)rsd_scratch(ctx, "ewald_lists", sizeof(double) * nd);
   if (!d) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemcpyAsync(d, h.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, ctx->stream));
+  RSD_CUDA(ctx, cudaMemcpyAsync(d, h.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, s));
   D->nimg = (int)ni;
   D->Kh = (int)nk;
   D->rc2 = (float)H.rc2;
@@ -1727,48 +1727,26 @@ int upload_lists(rsd_ctx* ctx, const ewald_lists& H, bool equal, double a, const
   return RSD_OK;
 }
 
-// The weights of D's vectors on the context's stream, then the diagonal
-// blocks beside what follows there, on the side stream: latency-bound kernels
-// of one CTA (~65 us).  A self_join makes the stream wait for them, on every
-// way out of its scope.
-struct self_join {
-  rsd_ctx* ctx;
-  bool open = true;
-  int close() {
-    open = false;
-    RSD_CUDA(ctx, cudaEventRecord(ctx->ev_la[1], ctx->side));
-    RSD_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_la[1], 0));
-    return RSD_OK;
-  }
-  ~self_join() {
-    if (open) close();
-  }
-};
-
+// The weights of D's vectors on stream ws, then the diagonal blocks on the
+// side stream, beside the pair kernels: latency-bound kernels of one CTA (~65
+// us).  Forked by the caller when ws is the side stream, else here.
 template <typename S>
 int assemble_self(rsd_ctx* ctx, int nn, const double* d_radii, double a0, bool equal, const rsd_lat_dev& L,
-                  double inv_pimu, const ewald_dev_lists& D, bool weights_beside, const S& sk) {
-  RSD_TRY(rsd_side_stream(ctx));
-  cudaStream_t s = ctx->side, ws = weights_beside ? s : ctx->stream;
-  auto fork = [&]() -> int {
-    RSD_CUDA(ctx, cudaEventRecord(ctx->ev_la[0], ctx->stream));
-    RSD_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_la[0], 0));
-    return RSD_OK;
-  };
-  if (weights_beside) RSD_TRY(fork());
+                  double inv_pimu, const ewald_dev_lists& D, cudaStream_t ws, rsd_fork& beside, const S& sk) {
+  cudaStream_t s = beside.side;
   double* W = (double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
   double* self = (double*)rsd_scratch(ctx, "ewald_self_sums", sizeof(double) * SELF_NMOM);
   if (!W || !self) return RSD_ENOMEM;
   const dim3 wg((unsigned)((D.Kh + 31) / 32), 2);
   if (equal) {
     ewald_weights<true><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
-    if (!weights_beside) RSD_TRY(fork());
+    if (ws != s) RSD_TRY(beside.fork());
     ewald_self_sums<true><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
                                                      D.etab, self); RSD_LAUNCH_NOTE();
     ewald_self_eq<<<(121 * nn + 255) / 256, 256, 0, s>>>(nn, self, sk); RSD_LAUNCH_NOTE();
   } else {
     ewald_weights<false><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
-    if (!weights_beside) RSD_TRY(fork());
+    if (ws != s) RSD_TRY(beside.fork());
     ewald_self_sums<false><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
                                                       D.etab, self); RSD_LAUNCH_NOTE();
     ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, self, d_radii, inv_pimu, sk); RSD_LAUNCH_NOTE();
@@ -1788,11 +1766,12 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
   const bool cube = !cubes_converged(L);
   if (!cube) L.lam *= EWALD64_SCALE;
   ewald_dev_lists D;
-  RSD_TRY(upload_lists(ctx, cube ? ewald_cube_lists(L) : ewald_sphere_lists(L, L.lam, false), equal, a0, L, inv_pimu,
-                       &D));
-  RSD_TRY(assemble_self(ctx, nn, d_radii, a0, equal, L, inv_pimu, D, false, sk));
-  self_join join{ctx};
-  if (nn < 2) return join.close();
+  RSD_TRY(upload_lists(ctx, s, cube ? ewald_cube_lists(L) : ewald_sphere_lists(L, L.lam, false), equal, a0, L,
+                       inv_pimu, &D));
+  RSD_TRY(rsd_side_stream(ctx));
+  rsd_fork beside{ctx, ctx->side, ctx->ev_la[0], ctx->ev_la[1]};
+  RSD_TRY(assemble_self(ctx, nn, d_radii, a0, equal, L, inv_pimu, D, s, beside, sk));
+  if (nn < 2) return beside.join();
   double2* cs = (double2*)rsd_scratch(ctx, "ewald_trig", sizeof(double2) * (size_t)D.Kh * nn);
   const double* W = (const double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
   if (!cs || !W) return RSD_ENOMEM;
@@ -1813,7 +1792,7 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
     equal ? go(narrow{}, std::true_type{}) : go(narrow{}, std::false_type{});
   }
   RSD_CUDA(ctx, cudaGetLastError());
-  return join.close();
+  return beside.join();
 }
 }  // namespace
 
@@ -1831,11 +1810,9 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
     return assemble_fp64(ctx, nn, d_pos, d_radii, h_radii[0], equal, L, inv_pimu, DenseSink{d_M, ldm});
   // M as FP32 planes hi + lo (PlaneSink), in the buffer of the FP64 matrix
   const PlaneSink psk{reinterpret_cast<float*>(d_M), reinterpret_cast<float*>(d_M) + (size_t)ldm * (11LL * nn), ldm};
-  const ewald_lists SL = ewald_sphere_lists(L, L.lam, /*self_only=*/true);
-  ewald_dev_lists D;
-  RSD_TRY(upload_lists(ctx, SL, equal, h_radii[0], L, inv_pimu, &D));
-  RSD_TRY(assemble_self(ctx, nn, d_radii, h_radii[0], equal, L, inv_pimu, D, true, psk));
-  self_join join{ctx};
+  RSD_TRY(rsd_side_stream(ctx));
+  rsd_fork beside{ctx, ctx->side, ctx->ev_la[0], ctx->ev_la[1]};
+  RSD_TRY(beside.fork());
   if (nn > 1) {
     dim3 blk(32, 4), grd((nn + 31) / 32, (nn + 3) / 4);
     {
@@ -1931,6 +1908,11 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       }
     }
   }
+  // last: the host makes their lists while the pair kernels run
+  ewald_dev_lists D;
+  RSD_TRY(upload_lists(ctx, beside.side, ewald_sphere_lists(L, L.lam, /*self_only=*/true), equal, h_radii[0], L,
+                       inv_pimu, &D));
+  RSD_TRY(assemble_self(ctx, nn, d_radii, h_radii[0], equal, L, inv_pimu, D, beside.side, beside, psk));
   RSD_CUDA(ctx, cudaGetLastError());
-  return join.close();
+  return beside.join();
 }

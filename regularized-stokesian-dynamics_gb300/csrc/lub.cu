@@ -480,24 +480,36 @@ static double* lubtab_device(rsd_ctx* ctx, const rsd_lubtab* tab) {
   return d;
 }
 
+constexpr int LUB_NPAIR = 26;  // the mirror word that takes the pair count
+
 // The pair stage shared by the dense and the sparse assembly: near-pair
 // list, pair blocks (unscaled), second-particle lists and contact count.
-static int lub_pair_stage(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is_period, const double* d_pos,
-                          const double* d_radii, const rsd_lattice* lat, rsd_lub_sparse* sp, int* dcon) {
+// The host waits for the pair count in between, so that a caller with other
+// work to launch calls rsd_lub_begin first.
+int rsd_lub_begin(rsd_ctx* ctx, cudaStream_t s, int nn, int nb, int is_period, const double* d_pos,
+                  const double* d_radii, const rsd_lattice* lat) {
+  int* cnt = (int*)rsd_scratch(ctx, "lub_count", sizeof(int) * (nn + 1));
+  int* off = (int*)rsd_scratch(ctx, "lub_off", sizeof(int) * (nn + 1));
+  if (!cnt || !off) return RSD_ENOMEM;
+  lub_near<false><<<(nn + LUB_WARPS - 1) / LUB_WARPS, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, rsd_lat_pack(lat),
+                                                                              d_pos, d_radii, cnt, nullptr, nullptr); RSD_LAUNCH_NOTE();
+  lub_scan<<<1, 1024, 0, s>>>(nn, cnt, off); RSD_LAUNCH_NOTE();
+  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + LUB_NPAIR, off + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
+  return RSD_OK;
+}
+
+static int lub_pair_stage(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, int nn, int nb, int is_period,
+                          const double* d_pos, const double* d_radii, const rsd_lattice* lat, rsd_lub_sparse* sp) {
   double* dt = lubtab_device(ctx, tab);
   if (!dt) return rsd_fail(ctx, RSD_ENOMEM, "lub table upload failed");
   lub_dev_tab T{dt, dt + 64 * 11, dt + 64 * 18, tab->nabc, tab->ngh, tab->nm};
   rsd_lat_dev Ld = rsd_lat_pack(lat);
-  cudaStream_t s = ctx->stream;
-  int* cnt = (int*)rsd_scratch(ctx, "lub_count", sizeof(int) * (nn + 1));
-  int* off = (int*)rsd_scratch(ctx, "lub_off", sizeof(int) * (nn + 1));
-  if (!cnt || !off) return RSD_ENOMEM;
+  const int* off = (const int*)rsd_scratch(ctx, "lub_off", sizeof(int) * (nn + 1));
+  if (!off) return RSD_ENOMEM;
   const unsigned ng = (unsigned)((nn + LUB_WARPS - 1) / LUB_WARPS);
-  lub_near<false><<<ng, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, cnt, nullptr, nullptr); RSD_LAUNCH_NOTE();
-  lub_scan<<<1, 1024, 0, s>>>(nn, cnt, off); RSD_LAUNCH_NOTE();
-  int npair = 0;
-  RSD_CUDA(ctx, cudaMemcpyAsync(&npair, off + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
+  const int npair = ctx->h_info[LUB_NPAIR];
+  int* dcon = ctx->d_info + RSD_INFO_CONTACTS;
   int2* pairs = (int2*)rsd_scratch(ctx, "lub_pairs", sizeof(int2) * (size_t)(npair > 0 ? npair : 1));
   double* blk = (double*)rsd_scratch(ctx, "lub_blocks", sizeof(double) * PB * (size_t)(npair > 0 ? npair : 1));
   int* cnt2 = (int*)rsd_scratch(ctx, "lub_count2", sizeof(int) * (nn + 1));
@@ -519,6 +531,7 @@ static int lub_pair_stage(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, i
   } else {
     RSD_CUDA(ctx, cudaMemsetAsync(off2, 0, sizeof(int) * (nn + 1), s));
   }
+  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + RSD_INFO_CONTACTS, dcon, sizeof(int), cudaMemcpyDeviceToHost, s));
   sp->nn = nn;
   sp->npair = npair;
   sp->pairs = pairs;
@@ -534,15 +547,14 @@ int rsd_lub_assemble(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is
                      int accumulate, int* n_contact) {
   if (!tab) return rsd_fail(ctx, RSD_EARG, "no lubrication tables");
   if (nn < 1 || ldl < 11LL * nn) return rsd_fail(ctx, RSD_EARG, "bad size nn=%d ldl=%lld", nn, (long long)ldl);
-  int* dcon = (int*)rsd_scratch(ctx, "lub_contacts", sizeof(int) * 2);
-  if (!dcon) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;
   if (!accumulate) {
     const int64_t tot = 121LL * nn * nn;
     zero_matrix<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(11LL * nn, 11LL * nn, d_L, ldl); RSD_LAUNCH_NOTE();
   }
   rsd_lub_sparse sp;
-  RSD_TRY(lub_pair_stage(ctx, tab, nn, nb, is_period, d_pos, d_radii, lat, &sp, dcon));
+  RSD_TRY(rsd_lub_begin(ctx, s, nn, nb, is_period, d_pos, d_radii, lat));
+  RSD_TRY(lub_pair_stage(ctx, s, tab, nn, nb, is_period, d_pos, d_radii, lat, &sp));
   const double scale = 6.0 * (RSD_PI * mu_f);
   if (sp.npair > 0) {
     const int64_t tc = 121LL * sp.npair;
@@ -553,35 +565,28 @@ int rsd_lub_assemble(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is
   }
   RSD_CUDA(ctx, cudaGetLastError());
   if (n_contact) {
-    RSD_CUDA(ctx, cudaMemcpyAsync(n_contact, dcon, sizeof(int), cudaMemcpyDeviceToHost, s));
     RSD_CUDA(ctx, cudaStreamSynchronize(s));
+    *n_contact = ctx->h_info[RSD_INFO_CONTACTS];
   }
   return RSD_OK;
 }
 
 // Sparse form for the mixed-precision refinement: the same pair blocks and
 // the per-particle self blocks (scaled), no dense 11N x 11N matrix.
-int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is_period, const double* d_pos,
-                         const double* d_radii, const rsd_lattice* lat, double mu_f, rsd_lub_sparse* sp,
-                         int* n_contact) {
+int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, int nn, int nb, int is_period,
+                         const double* d_pos, const double* d_radii, const rsd_lattice* lat, double mu_f,
+                         rsd_lub_sparse* sp) {
   if (!tab) return rsd_fail(ctx, RSD_EARG, "no lubrication tables");
   if (nn < 1) return rsd_fail(ctx, RSD_EARG, "bad size nn=%d", nn);
-  int* dcon = (int*)rsd_scratch(ctx, "lub_contacts", sizeof(int) * 2);
   double* self = (double*)rsd_scratch(ctx, "lub_self_blocks", sizeof(double) * 121 * (size_t)nn);
-  if (!dcon || !self) return RSD_ENOMEM;
-  cudaStream_t s = ctx->stream;
-  RSD_TRY(lub_pair_stage(ctx, tab, nn, nb, is_period, d_pos, d_radii, lat, sp, dcon));
+  if (!self) return RSD_ENOMEM;
+  RSD_TRY(lub_pair_stage(ctx, s, tab, nn, nb, is_period, d_pos, d_radii, lat, sp));
   sp->scale = 6.0 * (RSD_PI * mu_f);
-  sp->contacts = dcon;
   sp->self = self;
   const int64_t ts = 121LL * nn;
   lub_self<<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(nn, sp->off, sp->off2, sp->list2, sp->blk, sp->scale,
                                                           nullptr, 0, 0, self); RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
-  if (n_contact) {
-    RSD_CUDA(ctx, cudaMemcpyAsync(n_contact, dcon, sizeof(int), cudaMemcpyDeviceToHost, s));
-    RSD_CUDA(ctx, cudaStreamSynchronize(s));
-  }
   return RSD_OK;
 }
 

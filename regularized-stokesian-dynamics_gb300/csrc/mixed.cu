@@ -502,11 +502,12 @@ __global__ void gm_nrm2(int64_t len, const double* __restrict__ v, double* __res
 
 }  // namespace
 
+// The mixed step's solve on M's planes; lub: the sparse FP64 lubrication
+// operator (R_lub - R_2B in the grand layout) or null.
 // rpp_out (optional): stop once RPP32 = A^-1 + rfu is formed and copy it
 // there (6nn x 6nn, ld rpp_ld, full symmetric storage, FP32).
-int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d_pos, const double* d_radii,
-                    const rsd_lattice* lat, const rsd_lubtab* tab, const rsd_step_params* p, const double* ein,
-                    const double* Fe, double* U_par, double* S_hyd, rsd_step_info* info, float* rpp_out,
+int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_sparse* lub, const rsd_step_params* p,
+                    const double* ein, const double* Fe, double* U_par, double* S_hyd, rsd_step_info* info, float* rpp_out,
                     int64_t rpp_ld) {
   cudaStream_t s = ctx->stream;
   const int64_t N = nn, n = 11 * N, P = 6 * N, Q = 5 * N;
@@ -535,27 +536,21 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   if (!fs || !gpart) return RSD_ENOMEM;
   float* M32 = (float*)rsd_scratch(ctx, "mixed_M32", sizeof(float) * d.np * d.np);
   float* A32 = (float*)rsd_scratch(ctx, "mixed_A32", sizeof(float) * d.Pp * d.Pp);
-  const size_t nvec = (size_t)nr * (5 * n + 2 * P) + 2 * 2 * IT_BLOCKS;
+  const size_t nvec = (size_t)nr * (5 * n + 2 * P);
   double* V = (double*)rsd_scratch(ctx, "mixed_vec", sizeof(double) * nvec);
   float* V32 = (float*)rsd_scratch(ctx, "mixed_vec32", sizeof(float) * (size_t)nr * (2 * d.np + 2 * d.Pp));
   if (!M32 || !A32 || !V || !V32) return RSD_ENOMEM;
   double *f = V, *U = f + nr * n, *w = U + nr * P, *r1 = w + nr * n, *Lw = r1 + nr * n, *r2 = Lw + nr * n,
-         *y = r2 + nr * P, *nrm = y + nr * n;
+         *y = r2 + nr * P, *nrm = rsd_sums(ctx->d_info);
   float *t32 = V32, *x32 = t32 + nr * d.np, *u32 = x32 + nr * d.np, *du32 = u32 + nr * d.Pp;
   // Status words of the factorisations, read once with the first residual (a
   // failed factor leaves values that nothing branches on): info and timeout
   // of the factor of M', timeout of the inverse, info and timeout of the
-  // factor of RPP, timeouts of the block-scaled factors, contacts.
+  // factor of RPP, timeouts of the block-scaled factors; word 8 is the
+  // sweeps' (rsd_uhat_error_flag).
   int* st = ctx->d_info + 16;
-  RSD_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(int) * 8, s));
-  // sparse FP64 lubrication operator (R_lub - R_2B in the grand layout)
-  rsd_lub_sparse lub;
+  RSD_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(int) * 9, s));
   info->n_contact = 0;
-  if (p->use_lub) {
-    RSD_TRY(rsd_lub_build_sparse(ctx, tab, nn, p->nb, 1, d_pos, d_radii, lat, p->mu_f, &lub, nullptr));
-    RSD_CUDA(ctx, cudaMemcpyAsync(st + 7, lub.contacts, sizeof(int), cudaMemcpyDeviceToDevice, s));
-  }
-  cudaEventRecord(ctx->ev[6], s);
   // FP32 factor of M' (stresslets first)
   {
     const unsigned nt = (unsigned)((d.np + 31) / 32);
@@ -583,7 +578,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   RSD_TRY(rsd_potri_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp, "a32", ctx->use_tc == 3 ? 3 : 1,
                                    rpp_out ? nullptr : W128 + (size_t)(d.Qp / 128) * 128 * 128, st + 2));
   RSD_TRY(rsd_mirror_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp));
-  if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f32(ctx, &lub, A32, d.Pp));
+  if (lub) RSD_TRY(rsd_lub_add_pp_f32(ctx, lub, A32, d.Pp));
   if (!rpp_out) RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp, &inf, "rpp32", 3, st + 3));
   float* W_r = nullptr;
   if (!rpp_out)
@@ -592,7 +587,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
   // the status words, once the stream has been waited for
   auto status = [&]() -> int {
     const int* h = ctx->h_info + 16;
-    info->n_contact = h[7];
+    info->n_contact = lub ? ctx->h_info[RSD_INFO_CONTACTS] : 0;
     if (h[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "potrf: tensor-core update timed out (code %d)", h[1]);
     if (h[0]) {  // in [Q, P] order without the padding
       info->info = h[0] > d.Qp ? h[0] - (int)(d.Qp - d.Q) : h[0];
@@ -607,16 +602,19 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     if (h[5] || h[6]) return rsd_fail(ctx, RSD_ETIMEOUT, "uhat: tensor-core GEMM timed out");
     return RSD_OK;
   };
+  // and, in the same copy, the sweeps' error flag and the residual's sums
+  const size_t nsum = 2 * (size_t)nr * IT_BLOCKS;
+  double* hn = rsd_sums(ctx->h_info);
   auto read_status = [&]() -> int {
-    RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 16, st, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
-    return RSD_OK;
+    RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 16, st, sizeof(int) * (RSD_INFO_WORDS - 16) + sizeof(double) * nsum,
+                                  cudaMemcpyDeviceToHost, s));
+    RSD_CUDA(ctx, cudaStreamSynchronize(s));
+    return status();
   };
   if (rpp_out) {
     RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(float) * rpp_ld, A32, sizeof(float) * d.Pp, sizeof(float) * P, P,
                                     cudaMemcpyDeviceToDevice, s));
-    RSD_TRY(read_status());
-    RSD_CUDA(ctx, cudaStreamSynchronize(s));
-    return status();
+    return read_status();
   }
   // the solves with the two factors: X (overwritten) -> Y
   auto solve_m = [&](float* X, int cols, float* Y, int zero_lead) -> int {
@@ -628,9 +626,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     return rsd_potrs_wide_s(ctx, (int)d.Pp, A32, d.Pp, W_r, X, d.Pp, cols, Y);
   };
   // refinement
-  int* tri_err = rsd_uhat_error_flag(ctx);
-  if (!tri_err) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemsetAsync(tri_err, 0, sizeof(int), s));
+  const int* tri_err = rsd_uhat_error_flag(ctx);
   // Right-preconditioned flexible GMRES(m) per right-hand side, FP64
   // residuals; the preconditioner is the stationary iteration's correction.
   // Starts from zero; gm_maxit bounds the iterations over all right-hand
@@ -665,8 +661,8 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
       gm_neg<<<nblk(n), 256, 0, s>>>(n, wc, out); RSD_LAUNCH_NOTE();
       RSD_TRY(symv_add(fc, out));  // out = M f - w
       gm_neg<<<nblk(n), 256, 0, s>>>(n, out, out); RSD_LAUNCH_NOTE();  // r1 = w - M f
-      if (p->use_lub) {
-        RSD_TRY(rsd_lub_spmv(ctx, &lub, 1, wc, n, Lc, n));
+      if (lub) {
+        RSD_TRY(rsd_lub_spmv(ctx, lub, 1, wc, n, Lc, n));
       } else {
         RSD_CUDA(ctx, cudaMemsetAsync(Lc, 0, sizeof(double) * n, s));
       }
@@ -690,8 +686,8 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
       gm_u0<<<nblk(n), 256, 0, s>>>(P, n, z + n, dv); RSD_LAUNCH_NOTE();  // [zU; 0]
       gm_neg<<<nblk(n), 256, 0, s>>>(n, dv, a); RSD_LAUNCH_NOTE();
       RSD_TRY(symv_add(z, a));  // M zf - [zU; 0]
-      if (p->use_lub) {
-        RSD_TRY(rsd_lub_spmv(ctx, &lub, 1, dv, n, Lz, n));
+      if (lub) {
+        RSD_TRY(rsd_lub_spmv(ctx, lub, 1, dv, n, Lz, n));
         gm_a2<<<nblk(P), 256, 0, s>>>(P, z, Lz, a + n); RSD_LAUNCH_NOTE();
       } else {
         RSD_CUDA(ctx, cudaMemcpyAsync(a + n, z, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
@@ -702,14 +698,10 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
     std::vector<double> bnorm(nr);
     {
       it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();  // b part only is used
-      std::vector<double> hb(2 * nr * IT_BLOCKS);
-      RSD_CUDA(ctx, cudaMemcpyAsync(hb.data(), nrm, sizeof(double) * hb.size(), cudaMemcpyDeviceToHost, s));
       RSD_TRY(read_status());
-      RSD_CUDA(ctx, cudaStreamSynchronize(s));
-      RSD_TRY(status());
       for (int c = 0; c < nr; c++) {
         double b2 = 0.0;
-        for (int k = 0; k < IT_BLOCKS; k++) b2 += hb[2 * (c * IT_BLOCKS + k) + 1];
+        for (int k = 0; k < IT_BLOCKS; k++) b2 += hn[2 * (c * IT_BLOCKS + k) + 1];
         bnorm[c] = b2 > 0 ? sqrt(b2) : 1.0;
       }
     }
@@ -809,12 +801,11 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
       return rsd_fail(ctx, RSD_ENOCONV, "refinement did not converge: residual %.3e after %d iterations", res, its);
     return RSD_OK;
   }
-  int h_tri_err = 0;
   RSD_CUDA(ctx, cudaMemsetAsync(f, 0, sizeof(double) * nr * n, s));
   RSD_CUDA(ctx, cudaMemsetAsync(U, 0, sizeof(double) * nr * P, s));
   double worst = 0.0, best_res = INFINITY;
   int it = 0;
-  std::vector<double> hn(2 * nr * IT_BLOCKS), hist;
+  std::vector<double> hist;
   for (;; it++) {
     it_begin<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, U, ein, f, w, r1, fs); RSD_LAUNCH_NOTE();
     // r1 -= M f, double-single products of the two planes, both right-hand
@@ -826,18 +817,14 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d
       symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
     }
     symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, nr, nbt, gpart, pcol, -1.0, r1, n); RSD_LAUNCH_NOTE();
-    if (p->use_lub) {
-      RSD_TRY(rsd_lub_spmv(ctx, &lub, nr, w, n, Lw, n));
+    if (lub) {
+      RSD_TRY(rsd_lub_spmv(ctx, lub, nr, w, n, Lw, n));
     } else {
       RSD_CUDA(ctx, cudaMemsetAsync(Lw, 0, sizeof(double) * nr * n, s));
     }
     it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();
-    RSD_CUDA(ctx, cudaMemcpyAsync(hn.data(), nrm, sizeof(double) * hn.size(), cudaMemcpyDeviceToHost, s));
-    RSD_CUDA(ctx, cudaMemcpyAsync(&h_tri_err, tri_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (it == 0) RSD_TRY(read_status());
-    RSD_CUDA(ctx, cudaStreamSynchronize(s));
-    if (it == 0) RSD_TRY(status());
-    if (h_tri_err) return rsd_fail(ctx, RSD_ETIMEOUT, "refinement: a triangular sweep's wait timed out");
+    RSD_TRY(read_status());
+    if (ctx->h_info[24]) return rsd_fail(ctx, RSD_ETIMEOUT, "refinement: a triangular sweep's wait timed out");
     worst = 0.0;
     for (int c = 0; c < nr; c++) {
       double a2 = 0.0, b2 = 0.0;

@@ -53,9 +53,17 @@ struct rsd_ctx {
   cudaStream_t side2 = nullptr;  // second high-priority stream: the wide panel work beside the diagonal chain
   cudaEvent_t ev_panel = nullptr, ev_next = nullptr;
   cudaEvent_t ev_la[4] = {};     // look-ahead events of the two-level Cholesky
-  int* d_info = nullptr;  // device-side status words
+  int* d_info = nullptr;  // device-side status words, then the sums that the host reads (rsd_sums)
   int* h_info = nullptr;  // pinned mirror
+  void* h_io = nullptr;   // pinned staging of the host entry points (rsd_pinned)
+  size_t h_io_bytes = 0;
 };
+// The 64 status words are followed by sums that the host reads with them, in
+// one copy: [0, 128) the refinement's residual, [128, 384) and [384, 387) the
+// step's averages.
+constexpr int RSD_INFO_WORDS = 64, RSD_INFO_SUMS = 387;
+constexpr size_t RSD_INFO_BYTES = sizeof(int) * RSD_INFO_WORDS + sizeof(double) * RSD_INFO_SUMS;
+inline double* rsd_sums(int* info) { return reinterpret_cast<double*>(info + RSD_INFO_WORDS); }
 
 struct rsd_lubtab {
   int nabc = 0, ngh = 0, nm = 0;
@@ -84,6 +92,8 @@ int rsd_cuda_check(rsd_ctx* ctx, cudaError_t e, const char* what);
 // allocation failure.
 void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes);
 int rsd_set_device(rsd_ctx* ctx);
+// Grow-only pinned host buffer; nothing may be in flight on it.
+void* rsd_pinned(rsd_ctx* ctx, size_t bytes);
 // Scoped NVTX range around a phase of the step (a no-op unless a profiler
 // is attached), so that a profiler can select one phase's launches.
 struct rsd_range {
@@ -95,6 +105,31 @@ struct rsd_range {
 
 // creates ctx->side, side2, ev_panel, ev_next and ev_la on first use
 int rsd_side_stream(rsd_ctx* ctx);
+
+// Work on a side stream beside the context's stream: fork() makes `side` wait
+// for what the stream holds so far, join() the stream for what `side` holds;
+// a scope left without join() joins too.
+struct rsd_fork {
+  rsd_ctx* ctx;
+  cudaStream_t side;
+  cudaEvent_t out, in;
+  bool open = false;
+  int fork() {
+    RSD_CUDA(ctx, cudaEventRecord(out, ctx->stream));
+    RSD_CUDA(ctx, cudaStreamWaitEvent(side, out, 0));
+    open = true;
+    return RSD_OK;
+  }
+  int join() {
+    open = false;
+    RSD_CUDA(ctx, cudaEventRecord(in, side));
+    RSD_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, in, 0));
+    return RSD_OK;
+  }
+  ~rsd_fork() {
+    if (open) join();
+  }
+};
 
 // ------------------------------------------------------------ lattice
 struct rsd_lat_dev {
@@ -194,12 +229,18 @@ struct rsd_lub_sparse {
   const double* blk = nullptr;
   const int *off = nullptr, *off2 = nullptr, *list2 = nullptr;
   const double* self = nullptr;
-  const int* contacts = nullptr;  // device word: pairs found at s <= 2
   double scale = 0.0;
 };
-int rsd_lub_build_sparse(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is_period, const double* d_pos,
-                         const double* d_radii, const rsd_lattice* lat, double mu_f, rsd_lub_sparse* sp,
-                         int* n_contact);
+// In two parts on stream s, for a caller that launches other work between
+// them: the count of the near pairs, and the rest, which waits for the count
+// on the host.  Contacts (pairs at s <= 2) are counted in status word
+// RSD_INFO_CONTACTS, and copied to its mirror.
+constexpr int RSD_INFO_CONTACTS = 25;
+int rsd_lub_begin(rsd_ctx* ctx, cudaStream_t s, int nn, int nb, int is_period, const double* d_pos,
+                  const double* d_radii, const rsd_lattice* lat);
+int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, int nn, int nb, int is_period,
+                         const double* d_pos, const double* d_radii, const rsd_lattice* lat, double mu_f,
+                         rsd_lub_sparse* sp);
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy);
 int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t lda);

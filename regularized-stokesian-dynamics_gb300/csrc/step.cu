@@ -21,9 +21,15 @@ __global__ void axpy_block_k(int64_t rows, int64_t cols, double alpha, const dou
   A[i + j * lda] += alpha * B[i + j * ldb];
 }
 
-__global__ void fill_ein(int nn, const double* __restrict__ ei5, double* __restrict__ ein) {
+struct ein5 {
+  double v[5];
+};
+// EIN of every particle, and Fe (zero without d_Fe)
+__global__ void fill_inputs(int nn, ein5 e, const double* __restrict__ d_Fe, double* __restrict__ ein,
+                            double* __restrict__ Fe) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 5 * nn) ein[t] = ei5[t % 5];
+  if (t < 5 * nn) ein[t] = e.v[t % 5];
+  if (t < 6 * nn) Fe[t] = d_Fe ? d_Fe[t] : 0.0;
 }
 
 // averageU (src/matrices.f90:230-253): U_ave = sum_i (APP F)(3i) / N with
@@ -181,19 +187,28 @@ static void ei5_of(const double E[9], double out[5]) {
   }
 }
 
-int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const double* d_pos, const double* d_radii,
-                    const rsd_lattice* lat, const rsd_lubtab* tab, const rsd_step_params* p, const double* ein,
-                    const double* Fe, double* U_par, double* S_hyd, rsd_step_info* info, float* rpp_out = nullptr,
+int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_sparse* lub, const rsd_step_params* p,
+                    const double* ein, const double* Fe, double* U_par, double* S_hyd, rsd_step_info* info, float* rpp_out = nullptr,
                     int64_t rpp_ld = 0);
 int rsd_lp_pcg_internal(rsd_ctx* ctx, rsd_lp* net, int mode, int nn, const double* d_pos, const double* d_radii,
                         const rsd_lattice* lat, const double* d_rpp, int64_t ld, int nrhs, const double* d_b,
                         double* d_x, double tol, int maxit, int* iters, double* resid);
 
+// What the host entry point adds to the step: its radii, and its results'
+// copy into pinned memory before the step's last wait.
+struct step_host {
+  const double* radii;
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+
 // The step; with rpp_out it stops once RPP = (M^-1)_PP + rfu is formed and
 // copies it there (FP64 for the FP64 form, FP32 for the mixed form).
 static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params* p, double* d_conf,
                      const double* d_radii, const double* d_Fe, double* d_U_pos, double* d_SijN, double yeta_mu[5],
-                     rsd_step_info* info, void* rpp_out, int64_t rpp_ld, rsd_lattice* lat_out) {
+                     rsd_step_info* info, void* rpp_out, int64_t rpp_ld, rsd_lattice* lat_out,
+                     const step_host* host = nullptr) {
   if (!ctx || !p || !d_conf || !d_radii || (!rpp_out && (!d_U_pos || !d_SijN)) || p->nn < 1 || p->nb < 0 ||
       p->nb > p->nn || !(p->mu_f > 0) || !(p->ews_err > 0) || (p->use_lub && !tab))
     return rsd_fail(ctx, RSD_EARG, "rsd_stepper_stokesian_dev: bad arguments");
@@ -207,10 +222,13 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   // lattice at the start of the step (STEPPER_Stokesian 54-56)
   rsd_lattice lat{};
   RSD_TRY(rsd_set_lattice_skew(p->T, p->LB, p->gamma, 0, 0.0, 0.0, &lat));
-  std::vector<double> radii(nn);
-  RSD_CUDA(ctx, cudaMemcpyAsync(radii.data(), d_radii, nn * sizeof(double), cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaStreamSynchronize(s));
-  RSD_TRY(rsd_calc_lattice_inverse(&lat, p->ews_err, nn, radii.data()));
+  std::vector<double> radii(host ? 0 : nn);
+  const double* h_radii = host ? host->radii : radii.data();
+  if (!host) {
+    RSD_CUDA(ctx, cudaMemcpyAsync(radii.data(), d_radii, nn * sizeof(double), cudaMemcpyDeviceToHost, s));
+    RSD_CUDA(ctx, cudaStreamSynchronize(s));
+  }
+  RSD_TRY(rsd_calc_lattice_inverse(&lat, p->ews_err, nn, h_radii));
   loc.NR = lat.NR;
   loc.NI = lat.NI;
   loc.phi = lat.phi;
@@ -219,29 +237,37 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   // the mixed form's planes have 16-byte aligned columns
   const int64_t ldm = p->precision == RSD_PREC_MIXED ? (n + 3) / 4 * 4 : n;
   double* M = (double*)rsd_scratch(ctx, "step_M", sizeof(double) * ldm * n);
-  double* V = (double*)rsd_scratch(ctx, "step_vec", sizeof(double) * (4 * P + 4 * Q + 1024));
+  double* V = (double*)rsd_scratch(ctx, "step_vec", sizeof(double) * (3 * P + 2 * Q));
   if (!M || !V) return RSD_ENOMEM;
   double* X = V;               // P x 2
   double* Upar = V;            // = X(:,0)
   double* ein = V + 2 * P;     // Q
   double* S = ein + Q;         // Q
-  double* red = S + Q;         // 1024 scratch
-  double* Fe = red + 1024;     // P
-  double Eij[9], omega[3], UOE[9], ei5[5];
+  double* Fe = S + Q;          // P
+  double Eij[9], omega[3], UOE[9];
+  ein5 ei5;
   background(p->gamma, Eij, omega, UOE);
-  ei5_of(Eij, ei5);
-  double* d_ei5 = red + 512;
-  RSD_CUDA(ctx, cudaMemcpyAsync(d_ei5, ei5, sizeof ei5, cudaMemcpyHostToDevice, s));
-  fill_ein<<<(unsigned)((Q + 255) / 256), 256, 0, s>>>(nn, d_ei5, ein); RSD_LAUNCH_NOTE();
-  if (d_Fe)
-    RSD_CUDA(ctx, cudaMemcpyAsync(Fe, d_Fe, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
-  else
-    RSD_CUDA(ctx, cudaMemsetAsync(Fe, 0, sizeof(double) * P, s));
+  ei5_of(Eij, ei5.v);
+  double* sums = rsd_sums(ctx->d_info);
+  double* red = sums + 128;    // 256 partial sums, then yeta's three
+  fill_inputs<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(nn, ei5, d_Fe, ein, Fe); RSD_LAUNCH_NOTE();
   cudaEventRecord(ctx->ev[0], s);
+  // The lubrication operator needs positions and radii only: it is built on a
+  // side stream beside the mobility's pair sums (~190 us of small kernels and
+  // one wait of the host at N = 32, ~310 at 512).
+  RSD_TRY(rsd_side_stream(ctx));
+  rsd_lub_sparse lub;
+  rsd_fork beside{ctx, ctx->side2, ctx->ev_la[2], ctx->ev_la[3]};
+  if (p->use_lub) {
+    RSD_TRY(beside.fork());
+    RSD_TRY(rsd_lub_begin(ctx, beside.side, nn, p->nb, 1, d_conf, d_radii, &lat));
+  }
   {
     // grand mobility
     rsd_range r("rsd_assembly");
-    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, radii.data(), M, ldm));
+    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, h_radii, M, ldm));
+    if (p->use_lub)
+      RSD_TRY(rsd_lub_build_sparse(ctx, beside.side, tab, nn, p->nb, 1, d_conf, d_radii, &lat, p->mu_f, &lub));
     if (ctx->correction_method) {  // overlap corrections (per_GRPY_YZD.f90:98-116)
       int nov = 0;
       RSD_TRY(rsd_count_overlaps(ctx, nn, d_conf, d_radii, &lat, &nov));
@@ -250,12 +276,12 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     }
   }
   cudaEventRecord(ctx->ev[1], s);
+  if (p->use_lub) RSD_TRY(beside.join());
+  cudaEventRecord(ctx->ev[2], s);
   // averageU on APP before it is overwritten
   const bool planes = p->precision == RSD_PREC_MIXED;
   const float* Mh = planes ? reinterpret_cast<const float*>(M) : nullptr;
   sum_app_xx<<<256, 256, 0, s>>>(nn, M, Mh, planes ? Mh + (size_t)ldm * n : nullptr, ldm, red); RSD_LAUNCH_NOTE();
-  std::vector<double> hred(256);
-  RSD_CUDA(ctx, cudaMemcpyAsync(hred.data(), red, 256 * sizeof(double), cudaMemcpyDeviceToHost, s));
   int info_m = 0;
   if (p->precision == RSD_PREC_FP64) {
     // MobToResist_FTS: R_inf = M^-1 through the Schur complement (resist64.cu)
@@ -266,13 +292,9 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
       if (info) *info = loc;
       return info_m;
     }
-    cudaEventRecord(ctx->ev[2], s);
     // arrangResist: RPP = (R_inf)_PP + rfu; the products with rfe and rse
-    // come from the sparse lubrication operator
-    int nc = 0;
-    rsd_lub_sparse lub;
-    if (p->use_lub) RSD_TRY(rsd_lub_build_sparse(ctx, tab, nn, p->nb, 1, d_conf, d_radii, &lat, p->mu_f, &lub, &nc));
-    loc.n_contact = nc;
+    // come from the sparse lubrication operator (the factor has waited for it)
+    if (p->use_lub) loc.n_contact = ctx->h_info[RSD_INFO_CONTACTS];
     double* RPP = (double*)rsd_scratch(ctx, "step_RPP", sizeof(double) * P * P);
     double* f0 = (double*)rsd_scratch(ctx, "step_f0", sizeof(double) * (P + 3 * n));
     if (!RPP || !f0) return RSD_ENOMEM;
@@ -285,7 +307,6 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
       if (info) *info = loc;
       return RSD_OK;
     }
-    cudaEventRecord(ctx->ev[3], s);
     // RHS [Fe + RPQ EIN, RPQ EIN], RPQ EIN = f0 + rfe EIN
     double *w = f0 + P, *Lw = w + n;  // w = [0; EIN], then [X2; -EIN]; Lw = L w
     RSD_TRY(rsd_r64_pq(ctx, &h, ein, f0));
@@ -339,10 +360,9 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     }
     RSD_CUDA(ctx, cudaGetLastError());
   } else {
-    cudaEventRecord(ctx->ev[2], s);
     {
       rsd_range r("rsd_solve");
-      RSD_TRY(rsd_mixed_solve(ctx, nn, M, ldm, d_conf, d_radii, &lat, tab, p, ein, d_Fe ? Fe : nullptr, Upar, S, &loc,
+      RSD_TRY(rsd_mixed_solve(ctx, nn, M, ldm, p->use_lub ? &lub : nullptr, p, ein, d_Fe ? Fe : nullptr, Upar, S, &loc,
                               (float*)rpp_out, rpp_ld));
     }
     if (rpp_out) {
@@ -352,7 +372,6 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     }
     cudaEventRecord(ctx->ev[3], s);
   }
-  cudaEventRecord(ctx->ev[4], s);
   // velocities, Euler step, LE wrap
   bg_flow f{};
   memcpy(f.UOE, UOE, sizeof UOE);
@@ -368,31 +387,22 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   RSD_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int), s));
   nan_check<<<(unsigned)((6 * nn + 255) / 256), 256, 0, s>>>(6LL * nn, d_U_pos, flag); RSD_LAUNCH_NOTE();
   cudaEventRecord(ctx->ev[5], s);
-  double ys[3];
-  RSD_CUDA(ctx, cudaMemcpyAsync(ys, red + 256, sizeof ys, cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 8, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+  // one copy for the status words and the sums, one for a host caller's results
+  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, RSD_INFO_BYTES, cudaMemcpyDeviceToHost, s));
+  if (host)
+    RSD_CUDA(ctx, cudaMemcpyAsync(host->dst, host->src, host->bytes, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
-  float t01, t12, t23, t45;
+  const double* hred = rsd_sums(ctx->h_info) + 128;
+  const double* ys = hred + 256;
+  float t01, t12, t25, t73 = 0.f;  // event 7: factors done, 3: refinement done
   cudaEventElapsedTime(&t01, ctx->ev[0], ctx->ev[1]);
   cudaEventElapsedTime(&t12, ctx->ev[1], ctx->ev[2]);
-  cudaEventElapsedTime(&t23, ctx->ev[2], ctx->ev[3]);
-  cudaEventElapsedTime(&t45, ctx->ev[3], ctx->ev[5]);
+  cudaEventElapsedTime(&t25, ctx->ev[2], ctx->ev[5]);
+  if (p->precision == RSD_PREC_MIXED) cudaEventElapsedTime(&t73, ctx->ev[7], ctx->ev[3]);
   ctx->phase_ms[0] = t01;
-  if (p->precision == RSD_PREC_MIXED) {
-    // the lubrication assembly sits inside the mixed solve (event 6)
-    float t26, t63;
-    cudaEventElapsedTime(&t26, ctx->ev[2], ctx->ev[6]);
-    cudaEventElapsedTime(&t63, ctx->ev[6], ctx->ev[3]);
-    ctx->phase_ms[1] = t26;
-    ctx->phase_ms[2] = t12 + t63 + t45;
-    float t73;  // refinement part of the solve (event 7 = factors done)
-    cudaEventElapsedTime(&t73, ctx->ev[7], ctx->ev[3]);
-    ctx->phase_ms[3] = t73;
-  } else {
-    ctx->phase_ms[1] = t23;
-    ctx->phase_ms[2] = t12 + t45;
-  }
-  if (p->precision != RSD_PREC_MIXED) ctx->phase_ms[3] = 0;
+  ctx->phase_ms[1] = t12;
+  ctx->phase_ms[2] = t25;
+  ctx->phase_ms[3] = t73;
   double sxx = 0.0;
   for (int b = 0; b < 256; b++) sxx += hred[b];
   const double f6 = 6.0 * RSD_PI * p->mu_f * 1.0;  // radii_test = 1 after non-dimensionalisation
@@ -433,22 +443,24 @@ extern "C" int rsd_stepper_stokesian(rsd_ctx* ctx, const rsd_lubtab* tab, const 
   const int nn = p->nn;
   for (int i = 0; i < 3 * nn; i++)
     if (!std::isfinite(conf[i])) return rsd_fail(ctx, RSD_ENAN, "non-finite position");
+  // device [U 6nn | S 5nn | conf 3nn | radii nn | Fe 6nn]: one copy in, one out
   cudaStream_t s = ctx->stream;
-  double* dc = (double*)rsd_scratch(ctx, "io_conf", sizeof(double) * 3 * nn);
-  double* dr = (double*)rsd_scratch(ctx, "io_radii", sizeof(double) * nn);
-  double* du = (double*)rsd_scratch(ctx, "io_upos", sizeof(double) * 6 * nn);
-  double* ds = (double*)rsd_scratch(ctx, "io_sijn", sizeof(double) * 5 * nn);
-  double* df = Fe ? (double*)rsd_scratch(ctx, "io_fe", sizeof(double) * 6 * nn) : nullptr;
-  if (!dc || !dr || !du || !ds || (Fe && !df)) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemcpyAsync(dc, conf, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, s));
-  RSD_CUDA(ctx, cudaMemcpyAsync(dr, radii, sizeof(double) * nn, cudaMemcpyHostToDevice, s));
-  if (Fe) RSD_CUDA(ctx, cudaMemcpyAsync(df, Fe, sizeof(double) * 6 * nn, cudaMemcpyHostToDevice, s));
-  int rc = rsd_stepper_stokesian_dev(ctx, tab, p, dc, dr, df, du, ds, yeta_mu, info);
+  const size_t n1 = (size_t)nn, in = (Fe ? 10 : 4) * n1, out = 14 * n1;
+  double* d = (double*)rsd_scratch(ctx, "io_step", sizeof(double) * 21 * n1);
+  if (!d) return RSD_ENOMEM;
+  RSD_CUDA(ctx, cudaStreamSynchronize(s));  // an earlier call that failed may still use the staging
+  double* h = (double*)rsd_pinned(ctx, sizeof(double) * 21 * n1);
+  if (!h) return RSD_ENOMEM;
+  double *dc = d + 11 * n1, *dr = dc + 3 * n1, *df = Fe ? dr + n1 : nullptr, *hc = h + 11 * n1;
+  memcpy(hc, conf, sizeof(double) * 3 * n1);
+  memcpy(hc + 3 * n1, radii, sizeof(double) * n1);
+  if (Fe) memcpy(hc + 4 * n1, Fe, sizeof(double) * 6 * n1);
+  RSD_CUDA(ctx, cudaMemcpyAsync(dc, hc, sizeof(double) * in, cudaMemcpyHostToDevice, s));
+  const step_host host{radii, h, d, sizeof(double) * out};
+  const int rc = step_impl(ctx, tab, p, dc, dr, df, d, d + 6 * n1, yeta_mu, info, nullptr, 0, nullptr, &host);
   if (rc != RSD_OK) return rc;
-  RSD_CUDA(ctx, cudaMemcpyAsync(conf, dc, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaMemcpyAsync(U_pos, du, sizeof(double) * 6 * nn, cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaMemcpyAsync(SijN, ds, sizeof(double) * 5 * nn, cudaMemcpyDeviceToHost, s));
-  RSD_CUDA(ctx, cudaStreamSynchronize(s));
+  memcpy(U_pos, h, sizeof(double) * 6 * n1);
+  memcpy(SijN, h + 6 * n1, sizeof(double) * 5 * n1);
+  memcpy(conf, hc, sizeof(double) * 3 * n1);
   return RSD_OK;
 }
-
