@@ -744,134 +744,178 @@ __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int6
 // registers, 8 x 8 per thread, holds S above the diagonal and the growing
 // inverse Z of the unit lower factor below it: step k subtracts l_ik = S_ki /
 // d_k times row k from every row i > k, and in column k, where S is done, Z
-// starts as -l_ik (what the entry held until then is dropped).  The owners of
-// row k + 1 update and publish it first, then one barrier, and the other rows'
-// updates of step k run beside the loads and the reciprocal of step k + 1.
-// The square roots come last, all at once.  A thread holds rows 32 v + 2 ty +
-// {0, 1} and columns 32 c + 2 tx + {0, 1}, so that 32 steps run through one
-// small loop (rows of earlier v are done and left out): unrolled over 32-wide
-// sub-blocks it took 54 us and with 8 contiguous rows per thread 39 us, most
-// of it instruction fetch; potf2_inv_f32 takes 42 us.
+// starts as -l_ik (what the entry held until then is dropped).  Two steps go
+// together, for one barrier and one round of loads: their rows lie with the
+// same threads, which publish both as they are, and every thread takes row k
+// from its part of row k + 1 itself.  The owners of the next two rows update
+// and publish them first, then the barrier, and the other rows' updates run
+// beside the loads and the reciprocals of the next two steps.  The square
+// roots come last, all at once.  A thread holds rows 32 v + 2 ty + {0, 1} and
+// columns 32 c + 2 tx + {0, 1}, so that 32 steps run through one small loop
+// (rows of earlier v are done and left out): unrolled over 32-wide sub-blocks
+// it took 54 us and with 8 contiguous rows per thread 39 us, most of it
+// instruction fetch.  The tile comes and goes through shared memory: read as
+// the threads hold it, a branch per entry and 16 lines per request cost 5 us.
+// 25 us where potf2_inv_f32 takes 42 (28 with a barrier per step and unstaged;
+// 33 with the rows published twice over, to save the packing of multipliers).
+// What is left is issue (180 instructions a thread for two steps, 40 of them
+// multiply-adds) and the two reciprocals' chain.
 struct gj_regs {
-  uint64_t T[8][4];  // row 2 v + p of this thread, column pairs
-  uint64_t s[4];     // row k at this thread's columns
-  float l[8];        // its rows' multipliers, negated
+  uint64_t T[8][4];         // row 2 v + p of this thread, column pairs
+  uint64_t s0[4], s1[4];    // rows k and k + 1 (after step k) at this thread's columns
+  float l0[8], l1[8];       // its rows' multipliers, negated
 };
 
-__device__ __forceinline__ void gj_row(uint64_t (&T)[4], const uint64_t (&s)[4], float l) {
-  const uint64_t ll = f2_pack(l, l);
+template <int U>
+__device__ __forceinline__ void gj_row(gj_regs& g) {
+  const uint64_t a = f2_pack(g.l0[U], g.l0[U]), b = f2_pack(g.l1[U], g.l1[U]);
 #pragma unroll
-  for (int c = 0; c < 4; c++) T[c] = f2_fma(ll, s[c], T[c]);
+  for (int c = 0; c < 4; c++) g.T[U][c] = f2_fma(b, g.s1[c], f2_fma(a, g.s0[c], g.T[U][c]));
 }
 
-__device__ __forceinline__ void gj_publish(const uint64_t (&T)[4], float* row, int tx) {
+template <int U>
+__device__ __forceinline__ void gj_publish(const gj_regs& g, float (*row)[NB], int tx) {
 #pragma unroll
-  for (int c = 0; c < 4; c++) *reinterpret_cast<uint64_t*>(row + 32 * c + 2 * tx) = T[c];
+  for (int q = 0; q < 2; q++)
+#pragma unroll
+    for (int c = 0; c < 4; c++) *reinterpret_cast<uint64_t*>(row[q] + 32 * c + 2 * tx) = g.T[U + q][c];
 }
 
-// operands of step k = 32 V + 2 kk + P from its published row
-template <int V, int P>
-__device__ __forceinline__ void gj_load(gj_regs& g, const float* row, int kk, int tx, int ty) {
-  const float inv = -__fdividef(1.f, row[32 * V + 2 * kk + P]);
+template <int V, int U = 2 * V>
+__device__ __forceinline__ void gj_rows(gj_regs& g) {
+  if constexpr (U < 8) {
+    gj_row<U>(g);
+    gj_rows<V, U + 1>(g);
+  }
+}
+
+__device__ __forceinline__ uint64_t gj_sel(bool c, uint64_t a, uint64_t b) { return c ? a : b; }
+
+// The operands of steps k = 32 V + 2 kk and k + 1 from their published rows;
+// between the loads and their use, the updates by the steps before (the rows
+// of VP on).
+template <int V, int VP>
+__device__ __forceinline__ void gj_load(gj_regs& g, const float (*row)[NB], float* dd, int kk, int tx, int ty, int t) {
+  const int k = 32 * V + 2 * kk;
+  const float2 p = *reinterpret_cast<const float2*>(row[0] + k);
+  const float q = row[1][k + 1];
+  uint64_t r0[4], r1[4];
+  float2 a[4], b[4];
 #pragma unroll
-  for (int c = 0; c < 4; c++) g.s[c] = *reinterpret_cast<const uint64_t*>(row + 32 * c + 2 * tx);
+  for (int c = 0; c < 4; c++) {
+    r0[c] = *reinterpret_cast<const uint64_t*>(row[0] + 32 * c + 2 * tx);
+    r1[c] = *reinterpret_cast<const uint64_t*>(row[1] + 32 * c + 2 * tx);
+    if (c >= V) {
+      a[c] = *reinterpret_cast<const float2*>(row[0] + 32 * c + 2 * ty);
+      b[c] = *reinterpret_cast<const float2*>(row[1] + 32 * c + 2 * ty);
+    }
+  }
+  const float i0 = -__fdividef(1.f, p.x), m = p.y * i0, d1 = fmaf(m, p.y, q);
+  const float i1 = -__fdividef(1.f, d1);
+  const uint64_t mm = f2_pack(m, m);
+  const bool own = tx == kk, rest = ty > kk;
+  gj_rows<VP>(g);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    g.s0[c] = r0[c];
+    g.s1[c] = f2_fma(mm, r0[c], r1[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++)  // row k + 1 is done
+    g.T[2 * V + 1][c] = gj_sel(ty == kk, c == V ? gj_sel(own, f2_pack(m, d1), g.s1[c]) : g.s1[c], g.T[2 * V + 1][c]);
+  // columns k and k + 1: the identity enters
+  g.s0[V] = gj_sel(own, f2_pack(1.f, 0.f), g.s0[V]);
+  g.s1[V] = gj_sel(own, f2_pack(m, 1.f), g.s1[V]);
 #pragma unroll
   for (int v = V; v < 4; v++) {
-    const float2 e = *reinterpret_cast<const float2*>(row + 32 * v + 2 * ty);
-    g.l[2 * v] = e.x * inv;
-    g.l[2 * v + 1] = e.y * inv;
+    const bool go = v > V || rest;  // rows up to k + 1 stay
+    g.l0[2 * v] = go ? a[v].x * i0 : 0.f;
+    g.l0[2 * v + 1] = go ? a[v].y * i0 : 0.f;
+    g.l1[2 * v] = go ? fmaf(m, a[v].x, b[v].x) * i1 : 0.f;
+    g.l1[2 * v + 1] = go ? fmaf(m, a[v].y, b[v].y) * i1 : 0.f;
+    g.T[2 * v][V] = gj_sel(own && go, 0, g.T[2 * v][V]);
+    g.T[2 * v + 1][V] = gj_sel(own && go, 0, g.T[2 * v + 1][V]);
   }
-  // rows up to k stay: of this V, those of ty < kk and, for ty = kk, up to P
-  const bool r0 = ty > kk, r1 = ty > kk || (P == 0 && ty == kk);
-  g.l[2 * V] = r0 ? g.l[2 * V] : 0.f;
-  g.l[2 * V + 1] = r1 ? g.l[2 * V + 1] : 0.f;
-  // column k: the identity enters
-  const bool own = tx == kk;
-  float x, y;
-  f2_unpack(g.s[V], x, y);
-  g.s[V] = P ? f2_pack(x, own ? 1.f : y) : f2_pack(own ? 1.f : x, y);
-#pragma unroll
-  for (int u = 2 * V; u < 8; u++) {
-    const bool z = own && (u == 2 * V ? r0 : (u == 2 * V + 1 ? r1 : true));
-    f2_unpack(g.T[u][V], x, y);
-    g.T[u][V] = P ? f2_pack(x, z ? 0.f : y) : f2_pack(z ? 0.f : x, y);
+  if (t == 0) {
+    dd[k] = p.x;
+    dd[k + 1] = d1;
   }
 }
 
-// step k: the next row first (register U of the threads ty = owner), then the rest
-template <int V, int U>
-__device__ __forceinline__ void gj_next(gj_regs& g, float* row, int owner, int tx, int ty) {
+// the next two rows first (registers U, U + 1 of the threads ty = owner)
+template <int U>
+__device__ __forceinline__ void gj_next(gj_regs& g, float (*row)[NB], int owner, int tx, int ty) {
   if (ty == owner) {
-    gj_row(g.T[U], g.s, g.l[U]);
-    g.l[U] = 0.f;  // done
-    gj_publish(g.T[U], row, tx);
+    gj_row<U>(g);
+    gj_row<U + 1>(g);
+    g.l0[U] = g.l0[U + 1] = g.l1[U] = g.l1[U + 1] = 0.f;  // done
+    gj_publish<U>(g, row, tx);
   }
 }
 
 template <int V>
-__device__ __forceinline__ void gj_block(gj_regs& g, float (&row)[2][NB], float* dd, int tx, int ty, int t) {
+__device__ __forceinline__ void gj_block(gj_regs& g, float (*row)[2][NB], float* dd, int tx, int ty, int t) {
 #pragma unroll 1
-  for (int kk = 0; kk < 16; kk++) {
-    // step 32 V + 2 kk (row in row[0]), next row in row[1]
-    gj_next<V, 2 * V + 1>(g, row[1], kk, tx, ty);
+  for (int kk = 0; kk < 15; kk++) {
+    float(*next)[NB] = row[(kk + 1) & 1];
+    gj_next<2 * V>(g, next, kk + 1, tx, ty);
     __syncthreads();
-#pragma unroll
-    for (int u = 2 * V; u < 8; u++) gj_row(g.T[u], g.s, g.l[u]);
-    if (t == 0) dd[32 * V + 2 * kk + 1] = row[1][32 * V + 2 * kk + 1];
-    gj_load<V, 1>(g, row[1], kk, tx, ty);
-    // step 32 V + 2 kk + 1
-    if (kk < 15) {
-      gj_next<V, 2 * V>(g, row[0], kk + 1, tx, ty);
-    } else if (V < 3) {
-      gj_next<V, (2 * V + 2) & 7>(g, row[0], 0, tx, ty);
-    }
+    gj_load<V, V>(g, next, dd, kk + 1, tx, ty, t);
+  }
+  if constexpr (V < 3) {
+    gj_next<2 * V + 2>(g, row[0], 0, tx, ty);
     __syncthreads();
-#pragma unroll
-    for (int u = 2 * V; u < 8; u++) gj_row(g.T[u], g.s, g.l[u]);
-    if (kk < 15) {
-      if (t == 0) dd[32 * V + 2 * kk + 2] = row[0][32 * V + 2 * kk + 2];
-      gj_load<V, 0>(g, row[0], kk + 1, tx, ty);
-    } else if (V < 3) {
-      if (t == 0) dd[32 * V + 32] = row[0][(32 * V + 32) & (NB - 1)];
-      gj_load<(V + 1) & 3, 0>(g, row[0], 0, tx, ty);
-    }
+    gj_load<V + 1, V>(g, row[0], dd, 0, tx, ty, t);
   }
 }
 
+constexpr int GJ_LD = NB + 2;  // of the staged tile: even, and 2 GJ_LD = 4 mod 32
+constexpr int GJ_SMEM = sizeof(float) * NB * GJ_LD;
+
 __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64_t lda, int jb, int* __restrict__ info,
                                                     int j0, float* __restrict__ Wout) {
-  __shared__ __align__(16) float row[2][NB];
+  extern __shared__ __align__(16) float gj_tile[];  // column j at GJ_LD j, through which A comes and goes
+  __shared__ __align__(16) float row[2][2][NB];
   __shared__ float dd[NB];
   __shared__ int failed;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  const bool vec = ((lda & 1) == 0) && (((uintptr_t)A & 7) == 0) && jb == NB;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4, lane = t & 31, warp = t >> 5;
+  const bool vec = ((lda & 3) == 0) && (((uintptr_t)A & 15) == 0) && jb == NB;
+  if (vec) {  // a warp reads a column down to its diagonal, all of them in flight
+    float4 in[16];
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int j = 8 * e + warp;
+      in[e] = 4 * lane <= j ? *reinterpret_cast<const float4*>(A + 4 * lane + (int64_t)j * lda)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      float* c = gj_tile + (8 * e + warp) * GJ_LD + 4 * lane;
+      *reinterpret_cast<float2*>(c) = make_float2(in[e].x, in[e].y);
+      *reinterpret_cast<float2*>(c + 2) = make_float2(in[e].z, in[e].w);
+    }
+  } else {
+    for (int e = t; e < NB * NB; e += 256) {
+      const int i = e % NB, j = e / NB;
+      gj_tile[i + j * GJ_LD] = i <= j && j < jb ? A[i + (int64_t)j * lda] : (i == j ? 1.f : 0.f);
+    }
+  }
+  if (t == 0) failed = 0;
+  __syncthreads();
   gj_regs g;
 #pragma unroll
   for (int v = 0; v < 4; v++)
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int i = 32 * v + 2 * ty, j = 32 * c + 2 * tx;
-      float e[2][2];
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        if (vec && i + 1 <= j + q) {
-          const float2 a = *reinterpret_cast<const float2*>(A + i + (int64_t)(j + q) * lda);
-          e[0][q] = a.x;
-          e[1][q] = a.y;
-        } else {
-#pragma unroll
-          for (int p = 0; p < 2; p++)
-            e[p][q] = i + p <= j + q && j + q < jb ? A[i + p + (int64_t)(j + q) * lda] : (i + p == j + q ? 1.f : 0.f);
-        }
-      }
-      g.T[2 * v][c] = f2_pack(e[0][0], e[0][1]);
-      g.T[2 * v + 1][c] = f2_pack(e[1][0], e[1][1]);
+      const float2 a = *reinterpret_cast<const float2*>(gj_tile + i + j * GJ_LD);
+      const float2 b = *reinterpret_cast<const float2*>(gj_tile + i + (j + 1) * GJ_LD);
+      g.T[2 * v][c] = f2_pack(i <= j ? a.x : 0.f, i <= j + 1 ? b.x : 0.f);
+      g.T[2 * v + 1][c] = f2_pack(i + 1 <= j ? a.y : 0.f, i <= j ? b.y : 0.f);
     }
-  if (t == 0) failed = 0;
-  if (ty == 0) gj_publish(g.T[0], row[0], tx);
+  if (ty == 0) gj_publish<0>(g, row[0], tx);
   __syncthreads();
-  if (t == 0) dd[0] = row[0][0];
-  gj_load<0, 0>(g, row[0], 0, tx, ty);
+  gj_load<0, 4>(g, row[0], dd, 0, tx, ty, t);
   gj_block<0>(g, row, dd, tx, ty, t);
   gj_block<1>(g, row, dd, tx, ty, t);
   gj_block<2>(g, row, dd, tx, ty, t);
@@ -896,17 +940,15 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
     for (int c = 0; c < 4; c++) {
       const int j = 32 * c + 2 * tx;
       float x[2][2];
-      f2_unpack(g.T[2 * v][c], x[0][0], x[0][1]);
-      f2_unpack(g.T[2 * v + 1][c], x[1][0], x[1][1]);
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        x[0][q] *= s0;
-        x[1][q] *= s1;
-      }
+      f2_unpack(f2_mul(g.T[2 * v][c], f2_pack(s0, s0)), x[0][0], x[0][1]);
+      f2_unpack(f2_mul(g.T[2 * v + 1][c], f2_pack(s1, s1)), x[1][0], x[1][1]);
       if (i == j) {
         x[0][0] = d0 * s0;
         x[1][1] = d1 * s1;
       }
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+        *reinterpret_cast<float2*>(gj_tile + i + (j + q) * GJ_LD) = make_float2(x[0][q], x[1][q]);
 #pragma unroll
       for (int p = 0; p < 2; p++) {
         float w[2];
@@ -915,16 +957,28 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
           w[q] = i + p < jb && j + q < jb ? (i + p > j + q ? x[p][q] : (i + p == j + q ? (p ? s1 : s0) : 0.f)) : 0.f;
         *reinterpret_cast<float2*>(Wout + j + (i + p) * NB) = make_float2(w[0], w[1]);
       }
+    }
+  }
+  __syncthreads();
+  if (vec) {
 #pragma unroll
-      for (int q = 0; q < 2; q++) {
-        if (vec && i + 1 <= j + q) {
-          *reinterpret_cast<float2*>(A + i + (int64_t)(j + q) * lda) = make_float2(x[0][q], x[1][q]);
-        } else {
+    for (int e = 0; e < 16; e++) {
+      const int j = 8 * e + warp, i = 4 * lane;
+      const float* c = gj_tile + j * GJ_LD + i;
+      float* o = A + i + (int64_t)j * lda;
+      if (i + 3 <= j) {
+        const float2 u = *reinterpret_cast<const float2*>(c), w = *reinterpret_cast<const float2*>(c + 2);
+        *reinterpret_cast<float4*>(o) = make_float4(u.x, u.y, w.x, w.y);
+      } else {
 #pragma unroll
-          for (int p = 0; p < 2; p++)
-            if (i + p <= j + q && j + q < jb) A[i + p + (int64_t)(j + q) * lda] = x[p][q];
-        }
+        for (int q = 0; q < 3; q++)
+          if (i + q <= j) o[q] = c[q];
       }
+    }
+  } else {
+    for (int e = t; e < NB * NB; e += 256) {
+      const int i = e % NB, j = e / NB;
+      if (i <= j && j < jb) A[i + (int64_t)j * lda] = gj_tile[i + j * GJ_LD];
     }
   }
 }
@@ -1087,7 +1141,7 @@ void launch_potf2(cudaStream_t s, bool exported, float* A, int64_t lda, int jb, 
   if (exported)
     potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s>>>(A, lda, jb, info, j0, W);
   else
-    potf2_gj_f32<<<1, 256, 0, s>>>(A, lda, jb, info, j0, W);
+    potf2_gj_f32<<<1, 256, GJ_SMEM, s>>>(A, lda, jb, info, j0, W);
   RSD_LAUNCH_NOTE();
 }
 
@@ -1116,6 +1170,7 @@ int ensure_attrs(rsd_ctx* ctx) {
   RSD_CUDA(ctx, cudaFuncSetAttribute(trsv_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_trsv<T>()));
   RSD_CUDA(ctx, cudaFuncSetAttribute(trtri_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_potf2<T>(NB)));
   RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_inv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_POTF2_INV));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_gj_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
   done = true;
   return RSD_OK;
 }
