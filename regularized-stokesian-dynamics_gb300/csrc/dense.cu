@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "f32x2.cuh"
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
@@ -52,6 +53,7 @@ struct GemmP {
 // memory with the next tile prefetched into registers during the FMAs.
 template <typename T, int BM, int BN, int BK>
 __global__ void __launch_bounds__(256) gemm_kernel(GemmP g) {
+  pdl_enter();
   constexpr int TM = BM / 16, TN = BN / 16;
   constexpr int LA = BM * BK / 256, LB = BN * BK / 256;
   const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(256) gemm_kernel(GemmP g) {
 // epilogue are float4 accesses; k in steps of 8, double-buffered with the
 // next tile prefetched into registers.
 __global__ void __launch_bounds__(256) sgemm_vec(GemmP g) {
+  pdl_enter();
   constexpr int BM = 128, BN = 128, BK = 8;
   const int row0 = blockIdx.x * BM, col0 = blockIdx.y * BN;
   if (g.uplo && row0 >= col0 + BN) return;
@@ -340,12 +343,12 @@ void launch_gemm(cudaStream_t s, const GemmP& g) {
   const bool strides16 = (g.sA % 4 == 0) && (g.sB % 4 == 0) && (g.sC % 4 == 0);
   if (sizeof(T) == 4 && strides16 && aligned16(g.A, g.lda) && aligned16(g.B, g.ldb) && aligned16(g.C, g.ldc)) {
     dim3 grd((g.m + 127) / 128, (g.n + 127) / 128, nb);
-    sgemm_vec<<<grd, 256, 0, s>>>(g); RSD_LAUNCH_NOTE();
+    pdl_launch(sgemm_vec, grd, 256, 0, s, g);
     return;
   }
   constexpr int BM = Tile<T>::BM, BN = Tile<T>::BN, BK = Tile<T>::BK;
   dim3 grd((g.m + BM - 1) / BM, (g.n + BN - 1) / BN, nb);
-  gemm_kernel<T, BM, BN, BK><<<grd, 256, 0, s>>>(g); RSD_LAUNCH_NOTE();
+  pdl_launch(gemm_kernel<T, BM, BN, BK>, grd, 256, 0, s, g);
 }
 
 GemmP gp(int m, int n, int k, double alpha, const void* A, int64_t lda, int ta, const void* B, int64_t ldb, int tb,
@@ -622,6 +625,7 @@ __device__ __forceinline__ void w_column_block(const float* __restrict__ S, floa
 constexpr int SMEM_POTF2_INV = (2 * NB * PV + NB * DV + 4 * 32 * DV + 32 * TV) * (int)sizeof(float);
 __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int64_t lda, int jb,
                                                      int* __restrict__ info, int j0, float* __restrict__ Wout) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   float* S = (float*)smraw;      // U, NB x NB, ld PV
   float* Wm = S + NB * PV;       // W, NB x NB, ld PV
@@ -874,6 +878,7 @@ constexpr int GJ_SMEM = sizeof(float) * NB * GJ_LD;
 
 __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64_t lda, int jb, int* __restrict__ info,
                                                     int j0, float* __restrict__ Wout) {
+  pdl_enter();
   extern __shared__ __align__(16) float gj_tile[];  // column j at GJ_LD j, through which A comes and goes
   __shared__ __align__(16) float row[2][2][NB];
   __shared__ float dd[NB];
@@ -986,6 +991,7 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
 // Inverses of all diagonal blocks of an upper triangular U (one CTA each).
 template <typename T>
 __global__ void __launch_bounds__(256) trtri_diag(int n, const T* __restrict__ U, int64_t ldu, T* __restrict__ W) {
+  pdl_enter();
   extern __shared__ unsigned char smraw[];
   T* S = (T*)smraw;
   T* col = S + NB * NB;
@@ -1017,6 +1023,7 @@ __global__ void __launch_bounds__(256) trtri_diag(int n, const T* __restrict__ U
 
 template <typename T>
 __global__ void zero_lower_k(int n, T* __restrict__ A, int64_t lda) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)n * n) return;
   const int i = (int)(t % n), j = (int)(t / n);
@@ -1025,6 +1032,7 @@ __global__ void zero_lower_k(int n, T* __restrict__ A, int64_t lda) {
 
 template <typename T>
 __global__ void mirror_upper_k(int n, T* __restrict__ A, int64_t lda) {
+  pdl_enter();
   __shared__ T tile[32][33];
   const int bi = blockIdx.x, bj = blockIdx.y;
   if (bi < bj) return;
@@ -1107,6 +1115,7 @@ __global__ void gemv_t_k(int m, int k, const T* __restrict__ A, int64_t lda, con
 template <typename T>
 __global__ void __launch_bounds__(256) trsv_diag(int jb, const T* __restrict__ W, int ldw, int trans,
                                                  T* __restrict__ X, int64_t ldx, int nrhs) {
+  pdl_enter();
   extern __shared__ unsigned char smraw[];
   T* Ws = (T*)smraw;           // jb x jb
   T* b = Ws + NB * NB;         // jb x nrhs
@@ -1139,10 +1148,9 @@ int smem_trsv() {
 // block; potf2_inv_f32 keeps them what they were.
 void launch_potf2(cudaStream_t s, bool exported, float* A, int64_t lda, int jb, int* info, int j0, float* W) {
   if (exported)
-    potf2_inv_f32<<<1, 256, SMEM_POTF2_INV, s>>>(A, lda, jb, info, j0, W);
+    pdl_launch(potf2_inv_f32, 1, 256, SMEM_POTF2_INV, s, A, lda, jb, info, j0, W);
   else
-    potf2_gj_f32<<<1, 256, GJ_SMEM, s>>>(A, lda, jb, info, j0, W);
-  RSD_LAUNCH_NOTE();
+    pdl_launch(potf2_gj_f32, 1, 256, GJ_SMEM, s, A, lda, jb, info, j0, W);
 }
 
 template <typename T>
@@ -1232,7 +1240,7 @@ int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t
 template <typename T>
 int rsd_zero_lower_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda) {
   const int64_t tot = (int64_t)n * n;
-  zero_lower_k<T><<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(n, d_A, lda); RSD_LAUNCH_NOTE();
+  pdl_launch(zero_lower_k<T>, (unsigned)((tot + 255) / 256), 256, 0, ctx->stream, n, d_A, lda);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -1240,7 +1248,7 @@ int rsd_zero_lower_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda) {
 template <typename T>
 int rsd_mirror_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda) {
   const int nt = (n + 31) / 32;
-  mirror_upper_k<T><<<dim3(nt, nt), dim3(32, 8), 0, ctx->stream>>>(n, d_A, lda); RSD_LAUNCH_NOTE();
+  pdl_launch(mirror_upper_k<T>, dim3(nt, nt), dim3(32, 8), 0, ctx->stream, n, d_A, lda);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -1487,7 +1495,7 @@ int rsd_diag_inverses_t(rsd_ctx* ctx, int n, const T* U, int64_t ldu, const char
   T* W = diag_inverses<T>(ctx, n, tag);
   if (!W) return RSD_ENOMEM;
   const int nblk = (n + NB - 1) / NB;
-  trtri_diag<T><<<nblk, 256, smem_potf2<T>(NB), ctx->stream>>>(n, U, ldu, W); RSD_LAUNCH_NOTE();
+  pdl_launch(trtri_diag<T>, nblk, 256, smem_potf2<T>(NB), ctx->stream, n, U, ldu, W);
   RSD_CUDA(ctx, cudaGetLastError());
   *Wout = W;
   return RSD_OK;
@@ -1516,6 +1524,7 @@ int trtri_inplace_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const T* W, T* T1,
 
 // WT(j0:j0+jb, j0:j0+jb) = W_jj^T for the diagonal blocks
 __global__ void put_diag_transposed(int jb, const float* __restrict__ Wb, float* __restrict__ WT, int64_t ldw) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= jb * jb) return;
   const int i = t % jb, j = t / jb;  // WT(i, j) = W(j, i)
@@ -1545,7 +1554,7 @@ int potri_tc_s(rsd_ctx* ctx, int prec, int n, float* d_A, int64_t lda, const cha
   for (int j0 = 0, b = 0; j0 < n; j0 += NB, b++) {
     const int jb = n - j0 < NB ? n - j0 : NB;
     const float* Wb = W + (size_t)b * NB * NB;
-    put_diag_transposed<<<(jb * jb + 255) / 256, 256, 0, s>>>(jb, Wb, WT + j0 + (int64_t)j0 * ldw, ldw); RSD_LAUNCH_NOTE();
+    pdl_launch(put_diag_transposed, (jb * jb + 255) / 256, 256, 0, s, jb, Wb, WT + j0 + (int64_t)j0 * ldw, ldw);
     if (j0 == 0) continue;
     // long K ranges are split across CTAs (their partial products added
     // into the zeroed T1), so that a step does not wait on its longest tile
@@ -1609,6 +1618,7 @@ constexpr int NB2 = 512;
 // below and past n.
 __global__ void wide_init(int64_t n, const float* __restrict__ U, int64_t ldu, const float* __restrict__ W,
                           float* __restrict__ D) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.z;
   const int i = t % NB2, j = t / NB2;
   const int64_t o = (int64_t)b * NB2;
@@ -1628,6 +1638,7 @@ __global__ void wide_init(int64_t n, const float* __restrict__ U, int64_t ldu, c
 // in chunks of 32 of the triangle; FP32 multiply-adds.
 template <int STEP>
 __global__ void __launch_bounds__(256) wide_combine(int h, float* __restrict__ D, float* __restrict__ Tb) {
+  pdl_enter();
   __shared__ float As[32][33];
   __shared__ __align__(16) float Bs[32][36];
   const int pairs = NB2 / (2 * h), b = blockIdx.z / pairs, p = blockIdx.z % pairs;
@@ -1689,12 +1700,12 @@ int rsd_wide_inverses_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const 
   float* Tb = (float*)rsd_scratch(ctx, "wide_T", sizeof(float) * (size_t)nblk2 * (NB2 / 2) * (NB2 / 2));
   if (!W2 || !Tb) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;
-  wide_init<<<dim3(NB2 * NB2 / 256, 1, nblk2), 256, 0, s>>>(n, U, ldu, W128, W2); RSD_LAUNCH_NOTE();
+  pdl_launch(wide_init, dim3(NB2 * NB2 / 256, 1, nblk2), 256, 0, s, n, U, ldu, W128, W2);
   for (int h = NB; h < NB2; h *= 2) {
     if (n <= h) break;  // one block: no second half anywhere
     const dim3 grid(h / 32, h / 32, nblk2 * (NB2 / (2 * h)));
-    wide_combine<0><<<grid, 256, 0, s>>>(h, W2, Tb); RSD_LAUNCH_NOTE();
-    wide_combine<1><<<grid, 256, 0, s>>>(h, W2, Tb); RSD_LAUNCH_NOTE();
+    pdl_launch(wide_combine<0>, grid, 256, 0, s, h, W2, Tb);
+    pdl_launch(wide_combine<1>, grid, 256, 0, s, h, W2, Tb);
   }
   RSD_CUDA(ctx, cudaGetLastError());
   *W2out = W2;
@@ -1716,6 +1727,7 @@ int rsd_wide_inverses_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const 
 namespace {
 
 __global__ void transpose_block(int nb2, const float* __restrict__ W, float* __restrict__ WT) {
+  pdl_enter();
   __shared__ float t[32][33];
   const int b = blockIdx.z;
   const float* Wb = W + (size_t)b * nb2 * nb2;
@@ -1743,6 +1755,8 @@ constexpr int TRI_Q = 16, TRI_QS = NB2 / TRI_Q;  // parts per block, columns/row
 constexpr int TRI_THREADS = 256;
 constexpr long long TRI_SPIN_LIMIT = 1LL << 21;  // polls of >= 64 ns: a fraction of a second
 constexpr int TRI_MAX_BLOCKS = 256;              // order up to 131072
+// two tickets, then the ready counts of the two sweeps
+constexpr size_t TRI_SYNC_BYTES = sizeof(int) * (2 + 2 * TRI_MAX_BLOCKS);
 
 struct TriArgs {
   const float* Uh;  // strict upper block strips, ld
@@ -1778,6 +1792,7 @@ __device__ __forceinline__ void tri_wait(const TriArgs& A, int blk, volatile int
 // forward: z_j = V_j - sum_{c<j} Uh_cj^T z_c, in place on V (z_0 = V_0)
 template <int NR>
 __global__ void __launch_bounds__(TRI_THREADS) tri_forward(TriArgs A) {
+  pdl_enter();
   __shared__ __align__(16) float zs[NR][NB2];
   __shared__ int task_s;
   __shared__ volatile int abort_s;
@@ -1851,6 +1866,7 @@ __global__ void __launch_bounds__(TRI_THREADS) tri_forward(TriArgs A) {
 // backward: x_b = V_b - sum_{c>b} Uh_bc x_c, in place on V (x_{nb-1} = V_{nb-1})
 template <int NR>
 __global__ void __launch_bounds__(TRI_THREADS) tri_backward(TriArgs A) {
+  pdl_enter();
   __shared__ __align__(16) float xs[NR][NB2];
   __shared__ float red[32][NR][TRI_QS];
   __shared__ int task_s;
@@ -1929,7 +1945,13 @@ __global__ void __launch_bounds__(TRI_THREADS) tri_backward(TriArgs A) {
 // warps, reduced in shared memory
 template <int NR>
 __global__ void __launch_bounds__(256) blockdiag_gemv(int n, const float* __restrict__ G, const float* __restrict__ z,
-                                                      float* __restrict__ w, int64_t ldx) {
+                                                      float* __restrict__ w, int64_t ldx, int* __restrict__ sync,
+                                                      int nblk) {
+  pdl_enter();
+  if (sync && blockIdx.x == 0) {  // clears the words of the forward sweep that is done and the backward one to come
+    if (threadIdx.x < 2) sync[threadIdx.x] = 0;
+    for (int e = threadIdx.x; e < nblk; e += 256) sync[2 + e] = sync[2 + TRI_MAX_BLOCKS + e] = 0;
+  }
   __shared__ __align__(16) float zsh[NR][NB2];
   __shared__ float red[8][NR][128];
   const int b = blockIdx.x / (NB2 / 128), rq = blockIdx.x % (NB2 / 128);
@@ -1985,9 +2007,11 @@ int rsd_uhat_build(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const float
   float* Uh = (float*)rsd_scratch(ctx, nu.c_str(), sizeof(float) * (size_t)ldu * n);
   float* G = (float*)rsd_scratch(ctx, ng.c_str(), sizeof(float) * (size_t)nblk2 * NB2 * NB2);
   float* WT = (float*)rsd_scratch(ctx, "uhat_WT", sizeof(float) * (size_t)nblk2 * NB2 * NB2);
-  if (!Uh || !G || !WT) return RSD_ENOMEM;
+  int* sync = (int*)rsd_scratch(ctx, "tri_sync", TRI_SYNC_BYTES);
+  if (!Uh || !G || !WT || !sync) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;
-  transpose_block<<<dim3(NB2 / 32, NB2 / 32, nblk2), dim3(32, 8), 0, s>>>(NB2, W2, WT); RSD_LAUNCH_NOTE();
+  RSD_CUDA(ctx, cudaMemsetAsync(sync, 0, TRI_SYNC_BYTES, s));
+  pdl_launch(transpose_block, dim3(NB2 / 32, NB2 / 32, nblk2), dim3(32, 8), 0, s, NB2, W2, WT);
   // all blocks in two batched launches: G_b = W_b W_b^T, and the strips
   // Uh_b = W_b^T U(block b rows, columns after block b), whose width drops
   // by NB2 from one block to the next
@@ -2015,8 +2039,9 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
   cudaStream_t s = ctx->stream;
   const int gsm = ctx->sm_count > 0 ? ctx->sm_count : 148;
   if (nblk2 > TRI_MAX_BLOCKS) return rsd_fail(ctx, RSD_EUNSUP, "uhat solve: order %d above %d", n, TRI_MAX_BLOCKS * NB2);
-  // [0] error (cumulative), [1], [2] tickets, then the ready counts of the two sweeps
-  int* sync = (int*)rsd_scratch(ctx, "tri_sync", sizeof(int) * (size_t)(2 * TRI_MAX_BLOCKS + 2));
+  // the sweeps' tickets and ready counts, zero on entry (a solve leaves its
+  // forward words zero, and zeroes the backward ones before their use)
+  int* sync = (int*)rsd_scratch(ctx, "tri_sync", TRI_SYNC_BYTES);
   if (!sync) return RSD_ENOMEM;
   // leading zero blocks of the right-hand side: the forward sweep starts at
   // the first block that can be nonzero (z is zero before it)
@@ -2025,31 +2050,27 @@ int rsd_uhat_solve(rsd_ctx* ctx, const rsd_uhat* h, float* X, int64_t ldx, int n
             ctx->tri_spin_polls > 0 ? ctx->tri_spin_polls : TRI_SPIN_LIMIT};
   const int tasks = TRI_Q * (nblk2 - 1);
   const int ftasks = TRI_Q * (nblk2 - 1 - b0);
-  if (tasks > 0) RSD_CUDA(ctx, cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)(2 + 2 * nblk2), s));
   if (ftasks > 0) {  // forward, in place on X
     const int fgrid = max(1, min(ftasks, 4 * gsm));
     if (nrhs == 1)
-      tri_forward<1><<<fgrid, TRI_THREADS, 0, s>>>(A);
+      pdl_launch(tri_forward<1>, fgrid, TRI_THREADS, 0, s, A);
     else
-      tri_forward<2><<<fgrid, TRI_THREADS, 0, s>>>(A);
-    RSD_LAUNCH_NOTE();
+      pdl_launch(tri_forward<2>, fgrid, TRI_THREADS, 0, s, A);
   }
   if (nrhs == 1)
-    blockdiag_gemv<1><<<nblk2 * (NB2 / 128), 256, 0, s>>>(n, h->G, X, Y, ldx);
+    pdl_launch(blockdiag_gemv<1>, nblk2 * (NB2 / 128), 256, 0, s, n, h->G, X, Y, ldx, tasks > 0 ? sync : nullptr, nblk2);
   else
-    blockdiag_gemv<2><<<nblk2 * (NB2 / 128), 256, 0, s>>>(n, h->G, X, Y, ldx);
-  RSD_LAUNCH_NOTE();
+    pdl_launch(blockdiag_gemv<2>, nblk2 * (NB2 / 128), 256, 0, s, n, h->G, X, Y, ldx, tasks > 0 ? sync : nullptr, nblk2);
   if (tasks > 0) {  // backward, in place on Y
     A.V = Y;
     A.b0 = 0;
     A.ticket = sync + 1;
-    A.ready = sync + 2 + nblk2;
+    A.ready = sync + 2 + TRI_MAX_BLOCKS;
     const int grid = max(1, min(tasks, 4 * gsm));
     if (nrhs == 1)
-      tri_backward<1><<<grid, TRI_THREADS, 0, s>>>(A);
+      pdl_launch(tri_backward<1>, grid, TRI_THREADS, 0, s, A);
     else
-      tri_backward<2><<<grid, TRI_THREADS, 0, s>>>(A);
-    RSD_LAUNCH_NOTE();
+      pdl_launch(tri_backward<2>, grid, TRI_THREADS, 0, s, A);
   }
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
@@ -2126,7 +2147,7 @@ int rsd_potrs_upper_t(rsd_ctx* ctx, int n, const T* d_U, int64_t ldu, T* d_X, in
   // forward: U^T y = b
   for (int b = 0; b < nblk; b++) {
     const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB, rest = n - j0 - jb;
-    trsv_diag<T><<<1, 256, smem_trsv<T>(), s>>>(jb, W + (size_t)b * NB * NB, NB, 1, d_X + j0, ldx, nrhs); RSD_LAUNCH_NOTE();
+    pdl_launch(trsv_diag<T>, 1, 256, smem_trsv<T>(), s, jb, W + (size_t)b * NB * NB, NB, 1, d_X + j0, ldx, nrhs);
     if (rest > 0)
       RSD_TRY(rsd_gemv<T>(ctx, 1, rest, jb, T(-1), d_U + j0 + (int64_t)(j0 + jb) * ldu, ldu, d_X + j0, ldx, nrhs,
                           T(1), d_X + j0 + jb, ldx));
@@ -2134,7 +2155,7 @@ int rsd_potrs_upper_t(rsd_ctx* ctx, int n, const T* d_U, int64_t ldu, T* d_X, in
   // backward: U x = y
   for (int b = nblk - 1; b >= 0; b--) {
     const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB;
-    trsv_diag<T><<<1, 256, smem_trsv<T>(), s>>>(jb, W + (size_t)b * NB * NB, NB, 0, d_X + j0, ldx, nrhs); RSD_LAUNCH_NOTE();
+    pdl_launch(trsv_diag<T>, 1, 256, smem_trsv<T>(), s, jb, W + (size_t)b * NB * NB, NB, 0, d_X + j0, ldx, nrhs);
     if (j0 > 0)
       RSD_TRY(rsd_gemv<T>(ctx, 0, j0, jb, T(-1), d_U + (int64_t)j0 * ldu, ldu, d_X + j0, ldx, nrhs, T(1), d_X, ldx));
   }

@@ -41,6 +41,7 @@
 #include <string>
 #include <type_traits>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -142,6 +143,7 @@ constexpr int SPLIT_THREADS = 256, SPLIT_COLS = 8, SPLIT_TCOLS = 32;
 // memory, so that reads and writes stay coalesced.  Integer arithmetic on the
 // bits throughout: the FP64 pipe would bound it.
 __global__ void __launch_bounds__(SPLIT_THREADS) oz_split(oz_split_job J0, oz_split_job J1) {
+  pdl_enter();
   const oz_split_job& J = blockIdx.y ? J1 : J0;
   const int z = blockIdx.z, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (z >= J.nb) return;
@@ -282,6 +284,7 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, un
 // 65 ms.
 __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__ CUtensorMap tmS,
                                                          const __grid_constant__ CUtensorMap tmR, const oz_args a) {
+  pdl_enter();
   const int row0 = blockIdx.x * OZ_TR, col0 = blockIdx.y * OZ_TC, z = blockIdx.z;
   const int nz = min(a.n, a.ncap - z * a.nstep);
   if (col0 >= nz || (a.tri && row0 > col0 + OZ_TC - 1)) return;
@@ -477,12 +480,14 @@ __device__ __forceinline__ int half_exponent(double d) {
   return E == 0 || E == 0x7ff ? 0 : (E - 1023) >> 1;
 }
 __global__ void diag_exponents(int n, const double* __restrict__ A, int64_t lda, int* __restrict__ e) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) e[i] = half_exponent(A[i + (int64_t)i * lda]);
 }
 __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int64_t lda, int jb,
                                                      int* __restrict__ info, int j0, double* __restrict__ Wout,
                                                      int* __restrict__ ks) {
+  pdl_enter();
   __shared__ double S[NB64 * PF_LD];  // S(i, j) at [i * PF_LD + j]
   __shared__ double l[2][NB64], rd[NB64];
   __shared__ int failed;
@@ -567,6 +572,7 @@ template <int NR>
 __global__ void __launch_bounds__(256) trsv64_fwd(int n, int b, const double* __restrict__ U, int64_t ldu,
                                                   const double* __restrict__ W, double* __restrict__ X,
                                                   double* __restrict__ Y, int64_t ldx) {
+  pdl_enter();
   __shared__ double x[NR][NB64], y[NR][NB64];
   const int j0 = b * NB64, jb = min(NB64, n - j0), t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int e = t; e < NB64 * NR; e += 256) x[e / NB64][e % NB64] = e % NB64 < jb ? X[j0 + e % NB64 + (e / NB64) * ldx] : 0.0;
@@ -604,6 +610,7 @@ template <int NR>
 __global__ void __launch_bounds__(128) trsv64_bwd(int n, int b, const double* __restrict__ U, int64_t ldu,
                                                   const double* __restrict__ W, double* __restrict__ Y,
                                                   double* __restrict__ X, int64_t ldx) {
+  pdl_enter();
   __shared__ double x[NR][NB64], y[NR][NB64];
   const int j0 = b * NB64, jb = min(NB64, n - j0), t = threadIdx.x;
   for (int e = t; e < NB64 * NR; e += 128) y[e / NB64][e % NB64] = e % NB64 < jb ? Y[j0 + e % NB64 + (e / NB64) * ldx] : 0.0;
@@ -655,6 +662,7 @@ __global__ void __launch_bounds__(128) trsv64_bwd(int n, int b, const double* __
 
 // the NB64 diagonal inverses into the diagonal of V (ld)
 __global__ void put_diag64(int n, const double* __restrict__ W, double* __restrict__ V, int64_t ld) {
+  pdl_enter();
   const int b = blockIdx.x, j0 = b * NB64, jb = min(NB64, n - j0);
   for (int e = threadIdx.x; e < NB64 * NB64; e += blockDim.x) {
     const int i = e % NB64, j = e / NB64;
@@ -711,7 +719,7 @@ int oz_split_blocks(const oz_split_job& J) {
 void oz_split_launch(cudaStream_t s, const oz_split_job& J0, const oz_split_job* J1 = nullptr) {
   const int nx = std::max(oz_split_blocks(J0), J1 ? oz_split_blocks(*J1) : 0);
   const int nz = std::max(J0.nb, J1 ? J1->nb : 0);
-  oz_split<<<dim3(nx, J1 ? 2 : 1, nz), SPLIT_THREADS, 0, s>>>(J0, J1 ? *J1 : J0); RSD_LAUNCH_NOTE();
+  pdl_launch(oz_split, dim3(nx, J1 ? 2 : 1, nz), SPLIT_THREADS, 0, s, J0, J1 ? *J1 : J0);
 }
 
 int oz_map(rsd_ctx* ctx, CUtensorMap* tm, const oz_op& o, int box_rows) {
@@ -746,7 +754,7 @@ int oz_gemm_launch(rsd_ctx* ctx, const oz_op& R, const oz_op& S, int m, int n, d
   a.err = ctx->d_info + 1;
   a.wait_ns = ctx->tc_wait_ns > 0 ? (unsigned long long)ctx->tc_wait_ns : OZ_WAIT_NS;
   const dim3 grid((m + OZ_TR - 1) / OZ_TR, (n + OZ_TC - 1) / OZ_TC, S.nb);
-  oz_gemm<<<grid, OZ_THREADS, OZ_SMEM, ctx->stream>>>(tmS, tmR, a); RSD_LAUNCH_NOTE();
+  pdl_launch(oz_gemm, grid, OZ_THREADS, OZ_SMEM, ctx->stream, tmS, tmR, a);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -787,13 +795,13 @@ int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info
   RSD_TRY(oz_alloc(ctx, "oz_a", NB64, n, 1, &b));
   RSD_TRY(oz_alloc(ctx, "oz_b", NBO64, n, 1, &o));
   RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
-  diag_exponents<<<(n + 255) / 256, 256, 0, s>>>(n, d_A, lda, f.dexp); RSD_LAUNCH_NOTE();
+  pdl_launch(diag_exponents, (n + 255) / 256, 256, 0, s, n, d_A, lda, f.dexp);
   for (int J0 = 0; J0 < n; J0 += NBO64) {
     const int JB = n - J0 < NBO64 ? n - J0 : NBO64;
     for (int j0 = J0; j0 < J0 + JB; j0 += NB64) {
       const int jb = n - j0 < NB64 ? n - j0 : NB64, rest = n - j0 - jb;
       double* Wb = f.W + (size_t)(j0 / NB64) * NB64 * NB64;
-      potf2_inv_f64<<<1, 256, 0, s>>>(d_A + j0 + (int64_t)j0 * lda, lda, jb, ctx->d_info, j0, Wb, ks); RSD_LAUNCH_NOTE();
+      pdl_launch(potf2_inv_f64, 1, 256, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, jb, ctx->d_info, j0, Wb, ks);
       if (rest <= 0) break;
       double* P = d_A + j0 + (int64_t)(j0 + jb) * lda;
       b.cols = rest;
@@ -833,7 +841,7 @@ int rsd_potri64(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const rsd_factor6
   double* V = (double*)rsd_scratch(ctx, "potri64_V", sizeof(double) * (size_t)n * n);
   if (!V) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
-  put_diag64<<<(n + NB64 - 1) / NB64, 256, 0, s>>>(n, f.W, V, n); RSD_LAUNCH_NOTE();
+  pdl_launch(put_diag64, (n + NB64 - 1) / NB64, 256, 0, s, n, f.W, V, n);
   for (int h = NB64; h < n; h *= 2) {
     // pair z: blocks [2 z h, 2 z h + h) and [2 z h + h, min(2 z h + 2 h, n))
     const int np = (n - h + 2 * h - 1) / (2 * h);
@@ -904,12 +912,11 @@ int rsd_trsv64_fwd(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const doub
     const int rest = std::max(0, n - (b + 1) * NB64);
     const int grid = std::max(1, std::min(2 * ctx->sm_count, (rest + 7) / 8));
     switch (nrhs) {
-      case 1: trsv64_fwd<1><<<grid, 256, 0, s>>>(n, b, U, ldu, W, X, Y, ldx); break;
-      case 2: trsv64_fwd<2><<<grid, 256, 0, s>>>(n, b, U, ldu, W, X, Y, ldx); break;
-      case 3: trsv64_fwd<3><<<grid, 256, 0, s>>>(n, b, U, ldu, W, X, Y, ldx); break;
-      default: trsv64_fwd<4><<<grid, 256, 0, s>>>(n, b, U, ldu, W, X, Y, ldx); break;
+      case 1: pdl_launch(trsv64_fwd<1>, grid, 256, 0, s, n, b, U, ldu, W, X, Y, ldx); break;
+      case 2: pdl_launch(trsv64_fwd<2>, grid, 256, 0, s, n, b, U, ldu, W, X, Y, ldx); break;
+      case 3: pdl_launch(trsv64_fwd<3>, grid, 256, 0, s, n, b, U, ldu, W, X, Y, ldx); break;
+      default: pdl_launch(trsv64_fwd<4>, grid, 256, 0, s, n, b, U, ldu, W, X, Y, ldx); break;
     }
-    RSD_LAUNCH_NOTE();
   }
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
@@ -923,12 +930,11 @@ int rsd_trsv64_bwd(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const doub
   for (int b = (n + NB64 - 1) / NB64 - 1; b >= 0; b--) {
     const int grid = std::max(1, std::min(2 * ctx->sm_count, (b * NB64 + 31) / 32));
     switch (nrhs) {
-      case 1: trsv64_bwd<1><<<grid, 128, 0, s>>>(n, b, U, ldu, W, Y, X, ldx); break;
-      case 2: trsv64_bwd<2><<<grid, 128, 0, s>>>(n, b, U, ldu, W, Y, X, ldx); break;
-      case 3: trsv64_bwd<3><<<grid, 128, 0, s>>>(n, b, U, ldu, W, Y, X, ldx); break;
-      default: trsv64_bwd<4><<<grid, 128, 0, s>>>(n, b, U, ldu, W, Y, X, ldx); break;
+      case 1: pdl_launch(trsv64_bwd<1>, grid, 128, 0, s, n, b, U, ldu, W, Y, X, ldx); break;
+      case 2: pdl_launch(trsv64_bwd<2>, grid, 128, 0, s, n, b, U, ldu, W, Y, X, ldx); break;
+      case 3: pdl_launch(trsv64_bwd<3>, grid, 128, 0, s, n, b, U, ldu, W, Y, X, ldx); break;
+      default: pdl_launch(trsv64_bwd<4>, grid, 128, 0, s, n, b, U, ldu, W, Y, X, ldx); break;
     }
-    RSD_LAUNCH_NOTE();
   }
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;

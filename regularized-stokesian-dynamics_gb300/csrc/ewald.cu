@@ -28,6 +28,7 @@
 #include "overlap.cuh"
 #include "dsf.cuh"
 #include "f32x2.cuh"
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
@@ -61,6 +62,7 @@ __device__ inline T kernel_S(T k2, T lam) {
 template <bool EQ>
 __global__ void ewald_weights(rsd_lat_dev L, int Kh, const double* __restrict__ kv, double a, double inv_pimu,
                               double* __restrict__ W) {
+  pdl_enter();
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= Kh) return;
   const double k0 = kv[3 * h], k1 = kv[3 * h + 1], k2v = kv[3 * h + 2];
@@ -97,6 +99,7 @@ __global__ void ewald_weights(rsd_lat_dev L, int Kh, const double* __restrict__ 
 // cs[a * Kh + h] = (cos, sin)(k_h . x_a)
 __global__ void ewald_trig(int nn, int Kh, const double* __restrict__ kv, const double* __restrict__ pos,
                            double2* __restrict__ cs) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)nn * Kh) return;
   const int a = (int)(t / Kh), h = (int)(t % Kh);
@@ -109,6 +112,7 @@ __global__ void ewald_trig(int nn, int Kh, const double* __restrict__ kv, const 
 // precision T (the mixed form splits the reciprocal sum by shell).
 template <typename T>
 __global__ void ewald_ktable_list(rsd_lat_dev L, int count, const int* __restrict__ hlist, T* __restrict__ tab) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= count) return;
   int nx, ny, nz;
@@ -138,6 +142,7 @@ __device__ __forceinline__ void put_trig(float4* p, double c, double sn) {
 template <typename T2>
 __global__ void ewald_trig_list(int nn, rsd_lat_dev L, const int* __restrict__ hlist, const double* __restrict__ pos,
                                 T2* __restrict__ cs) {
+  pdl_enter();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = blockIdx.y;
   if (a >= nn) return;
@@ -407,6 +412,7 @@ template <typename T, typename T2, typename S>
 __global__ void __launch_bounds__(128) ewald_pair_k(int nn, rsd_lat_dev L, int Kh, const T* __restrict__ tab,
                                                     const T2* __restrict__ cs, const double* __restrict__ radii,
                                                     double inv_pimu, S sk, int add) {
+  pdl_enter();
   constexpr int KWT = 3 + RSD_NMOM_KCOS + RSD_NMOM_KSIN;
   constexpr int NW = RSD_NMOM_KCOS + RSD_NMOM_KSIN;  // 80
   constexpr int KC = 16;
@@ -483,6 +489,7 @@ template <typename S>
 __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, int Kh, const double* __restrict__ tab,
                                                        const float4* __restrict__ cs, const double* __restrict__ radii,
                                                        double inv_pimu, S sk, int add) {
+  pdl_enter();
   constexpr int KWT = 3 + RSD_NMOM_KCOS + RSD_NMOM_KSIN;
   constexpr int NW = RSD_NMOM_KCOS + RSD_NMOM_KSIN;
   constexpr int KC = 16;
@@ -561,6 +568,7 @@ constexpr int KBW = 64;  // weights per vector (60 used, padded for 16-byte rows
 // thread's instruction count.
 __global__ void ewald_kblock_lists(rsd_lat_dev L, int K64, int K32, const int* __restrict__ hlist, double a,
                                    double inv_pimu, float* __restrict__ W64, float* __restrict__ W32) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= K64 + K32) return;
   int nx, ny, nz;
@@ -637,6 +645,7 @@ __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const 
                                                          const float2* __restrict__ c32, int K64,
                                                          const float* __restrict__ W64, const float4* __restrict__ c64,
                                                          PlaneSink sk, int add) {
+  pdl_enter();
   constexpr int KC = 16;
   __shared__ __align__(16) float sw[KC * 2 * KBW];  // the FP32 phase uses the first half
   __shared__ __align__(16) float4 sca[KC * 32], scb[KC * 4];
@@ -764,6 +773,7 @@ template <typename S>
 __global__ void __launch_bounds__(128) ewald_pair_real_far(int nn, rsd_lat_dev L, const double* __restrict__ pos,
                                                            const double* __restrict__ radii, double inv_pimu,
                                                            double rc2, double rmax2, S sk) {
+  pdl_enter();
   int a, b;
   if (!pair_of(nn, &a, &b)) return;
   double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
@@ -808,6 +818,7 @@ template <typename S>
 __global__ void __launch_bounds__(128) ewald_pair_real_near_ds(int nn, rsd_lat_dev L, const double* __restrict__ pos,
                                                                const double* __restrict__ radii, double inv_pimu,
                                                                double rc2, S sk) {
+  pdl_enter();
   __shared__ dsf_tables T;
   // blocks entirely on or below the diagonal (a >= b everywhere) have no work
   if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
@@ -986,6 +997,7 @@ __global__ void __launch_bounds__(REAL_THREADS, MINB) ewald_pair_real_eq(int nn,
                                                                         const dsf* __restrict__ cr_g,
                                                                         const float* __restrict__ cf_g, float rc2,
                                                                         float rmax2, PlaneSink sk) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw_real[];
   RealEqShared& sh = *reinterpret_cast<RealEqShared*>(smraw_real);
   // blocks entirely on or below the diagonal (a >= b everywhere) have no work
@@ -1152,6 +1164,7 @@ __global__ void __launch_bounds__(P64_THREADS) ewald_pair64(int nn, int64_t npai
                                                             const double* __restrict__ radii, double inv_pimu,
                                                             const double* __restrict__ coef,
                                                             const unsigned short* __restrict__ etab, DenseSink sk) {
+  pdl_enter();
   constexpr int PP = P64_THREADS / G, NK = EQ ? 60 : RSD_NMOM_KCOS + RSD_NMOM_KSIN, NR = RSD_NMOM_REAL;
   __shared__ double mom[PP][NR + NK];
   __shared__ int list[PP][P64_CAP];
@@ -1314,6 +1327,7 @@ __global__ void __launch_bounds__(SELF_THREADS) ewald_self_sums(rsd_lat_dev L, i
                                                                 double inv_pimu, const double* __restrict__ coef,
                                                                 const unsigned short* __restrict__ etab,
                                                                 double* __restrict__ out) {
+  pdl_enter();
   constexpr int NW = SELF_THREADS / 32, NR = RSD_NMOM_REAL, NQ = EQ ? 60 : RSD_NMOM_KCOS;
   __shared__ double part[NW][NR], mom[NR], ks[NQ];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -1373,6 +1387,7 @@ __device__ __forceinline__ void sink_put(const PlaneSink& sk, int64_t o, double 
 template <typename S>
 __global__ void __launch_bounds__(64) ewald_self(int nn, rsd_lat_dev L, const double* __restrict__ mom,
                                                  const double* __restrict__ radii, double inv_pimu, S sk) {
+  pdl_enter();
   const int64_t ldm = sk.ld;
   auto M = [&](int64_t o, double x) { sink_put(sk, o, x); };
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1434,6 +1449,7 @@ __global__ void __launch_bounds__(64) ewald_self(int nn, rsd_lat_dev L, const do
 // per_GRPY_YZD.f90:63-66), a thread per entry.
 template <typename S>
 __global__ void ewald_self_eq(int nn, const double* __restrict__ v, S sk) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 121 * nn) return;
   const int a = t % nn, r = t / nn % 11, c = t / nn / 11;
@@ -1443,6 +1459,7 @@ __global__ void ewald_self_eq(int nn, const double* __restrict__ v, S sk) {
 
 __global__ void overlap_count(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
                               int* __restrict__ count) {
+  pdl_enter();
   int a, b;
   if (!pair_of(nn, &a, &b)) return;
   double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
@@ -1456,6 +1473,7 @@ __global__ void overlap_count(int nn, rsd_lat_dev L, const double* __restrict__ 
 // number found.
 __global__ void overlap_list(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
                              int cap, int2* __restrict__ list, int* __restrict__ count) {
+  pdl_enter();
   int a, b;
   if (!pair_of(nn, &a, &b)) return;
   double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
@@ -1475,6 +1493,7 @@ template <typename S>
 __global__ void __launch_bounds__(64) overlap_correct(int method, int npair, const int2* __restrict__ list, int nn,
                                                        rsd_lat_dev L, const double* __restrict__ pos,
                                                        const double* __restrict__ radii, double inv_pimu, S sk) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= npair) return;
   const int a = list[q].x, b = list[q].y;
@@ -1498,18 +1517,18 @@ int rsd_overlap_correct(rsd_ctx* ctx, int method, int precision, int nn, const d
   if (!cnt || !list) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int), ctx->stream));
   dim3 blk(32, 4), grd((nn + 31) / 32, (nn + 3) / 4);
-  overlap_list<<<grd, blk, 0, ctx->stream>>>(nn, L, d_pos, d_radii, npair, list, cnt); RSD_LAUNCH_NOTE();
+  pdl_launch(overlap_list, grd, blk, 0, ctx->stream, nn, L, d_pos, d_radii, npair, list, cnt);
   const double inv_pimu = 1.0 / (RSD_PI * mu_f);
   const unsigned nblk = (unsigned)((npair + 63) / 64);
   if (precision == RSD_PREC_MIXED) {
     float* hi = reinterpret_cast<float*>(d_M);
     const PlaneSink psk{hi, hi + (size_t)ldm * (11LL * nn), ldm};
-    overlap_correct<PlaneSink><<<nblk, 64, 0, ctx->stream>>>(method, npair, list, nn, L, d_pos, d_radii, inv_pimu,
-                                                             psk); RSD_LAUNCH_NOTE();
+    pdl_launch(overlap_correct<PlaneSink>, nblk, 64, 0, ctx->stream, method, npair, list, nn, L, d_pos, d_radii, inv_pimu,
+                                                             psk);
   } else {
     const DenseSink dsk{d_M, ldm};
-    overlap_correct<DenseSink><<<nblk, 64, 0, ctx->stream>>>(method, npair, list, nn, L, d_pos, d_radii, inv_pimu,
-                                                             dsk); RSD_LAUNCH_NOTE();
+    pdl_launch(overlap_correct<DenseSink>, nblk, 64, 0, ctx->stream, method, npair, list, nn, L, d_pos, d_radii, inv_pimu,
+                                                             dsk);
   }
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
@@ -1522,7 +1541,7 @@ int rsd_count_overlaps(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
   if (!d) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemsetAsync(d, 0, sizeof(int), ctx->stream));
   dim3 blk(32, 4), grd((nn + 31) / 32, (nn + 3) / 4);
-  overlap_count<<<grd, blk, 0, ctx->stream>>>(nn, L, d_pos, d_radii, d); RSD_LAUNCH_NOTE();
+  pdl_launch(overlap_count, grd, blk, 0, ctx->stream, nn, L, d_pos, d_radii, d);
   RSD_CUDA(ctx, cudaGetLastError());
   RSD_CUDA(ctx, cudaMemcpyAsync(count, d, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   RSD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1569,7 +1588,7 @@ int launch_real_eq_t(rsd_ctx* ctx, dim3 grd, dim3 blk, int nn, const rsd_lat_dev
                                        SMEM_REAL_EQ));
     attr = true;
   }
-  ewald_pair_real_eq<NP, MINB><<<grd, blk, SMEM_REAL_EQ, ctx->stream>>>(nn, L, d_pos, cr, cf, rc2, rmax2, psk); RSD_LAUNCH_NOTE();
+  pdl_launch(ewald_pair_real_eq<NP, MINB>, grd, blk, SMEM_REAL_EQ, ctx->stream, nn, L, d_pos, cr, cf, rc2, rmax2, psk);
   return RSD_OK;
 }
 
@@ -1739,17 +1758,17 @@ int assemble_self(rsd_ctx* ctx, int nn, const double* d_radii, double a0, bool e
   if (!W || !self) return RSD_ENOMEM;
   const dim3 wg((unsigned)((D.Kh + 31) / 32), 2);
   if (equal) {
-    ewald_weights<true><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    pdl_launch(ewald_weights<true>, wg, 32, 0, ws, L, D.Kh, D.kv, a0, inv_pimu, W);
     if (ws != s) RSD_TRY(beside.fork());
-    ewald_self_sums<true><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
-                                                     D.etab, self); RSD_LAUNCH_NOTE();
-    ewald_self_eq<<<(121 * nn + 255) / 256, 256, 0, s>>>(nn, self, sk); RSD_LAUNCH_NOTE();
+    pdl_launch(ewald_self_sums<true>, 1, SELF_THREADS, 0, s, L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
+                                                     D.etab, self);
+    pdl_launch(ewald_self_eq<S>, (121 * nn + 255) / 256, 256, 0, s, nn, self, sk);
   } else {
-    ewald_weights<false><<<wg, 32, 0, ws>>>(L, D.Kh, D.kv, a0, inv_pimu, W); RSD_LAUNCH_NOTE();
+    pdl_launch(ewald_weights<false>, wg, 32, 0, ws, L, D.Kh, D.kv, a0, inv_pimu, W);
     if (ws != s) RSD_TRY(beside.fork());
-    ewald_self_sums<false><<<1, SELF_THREADS, 0, s>>>(L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
-                                                      D.etab, self); RSD_LAUNCH_NOTE();
-    ewald_self<<<(nn + 63) / 64, 64, 0, s>>>(nn, L, self, d_radii, inv_pimu, sk); RSD_LAUNCH_NOTE();
+    pdl_launch(ewald_self_sums<false>, 1, SELF_THREADS, 0, s, L, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, a0, inv_pimu, D.coef,
+                                                      D.etab, self);
+    pdl_launch(ewald_self<S>, (nn + 63) / 64, 64, 0, s, nn, L, self, d_radii, inv_pimu, sk);
   }
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
@@ -1775,14 +1794,13 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
   double2* cs = (double2*)rsd_scratch(ctx, "ewald_trig", sizeof(double2) * (size_t)D.Kh * nn);
   const double* W = (const double*)rsd_scratch(ctx, "ewald_weights", sizeof(double) * (size_t)D.Kh * 80);
   if (!cs || !W) return RSD_ENOMEM;
-  ewald_trig<<<(unsigned)(((int64_t)nn * D.Kh + 127) / 128), 128, 0, s>>>(nn, D.Kh, D.kv, d_pos, cs); RSD_LAUNCH_NOTE();
+  pdl_launch(ewald_trig, (unsigned)(((int64_t)nn * D.Kh + 127) / 128), 128, 0, s, nn, D.Kh, D.kv, d_pos, cs);
   const int64_t npair = (int64_t)nn * (nn - 1) / 2;
   auto go = [&](auto lanes, auto eq) {
     constexpr int G = decltype(lanes)::value;
     constexpr int PP = P64_THREADS / G;
-    ewald_pair64<G, decltype(eq)::value><<<(unsigned)((npair + PP - 1) / PP), P64_THREADS, 0, s>>>(
+    pdl_launch(ewald_pair64<G, decltype(eq)::value>, (unsigned)((npair + PP - 1) / PP), P64_THREADS, 0, s, 
         nn, npair, L, cube, D.nimg, D.img, D.imgf, D.rc2, D.Kh, W, cs, d_pos, d_radii, inv_pimu, D.coef, D.etab, sk);
-    RSD_LAUNCH_NOTE();
   };
   using wide = std::integral_constant<int, 32>;
   using narrow = std::integral_constant<int, 8>;
@@ -1877,34 +1895,34 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       const dsf* cr = reinterpret_cast<const dsf*>(dh + nidx);
       const float* cf = reinterpret_cast<const float*>(cr + RSD_REAL_EPI_NC);
       if (K64) {
-        ewald_trig_list<float4><<<dim3((nn + 127) / 128, K64), 128, 0, s>>>(nn, L, dh, d_pos, c64); RSD_LAUNCH_NOTE();
+        pdl_launch(ewald_trig_list<float4>, dim3((nn + 127) / 128, K64), 128, 0, s, nn, L, dh, d_pos, c64);
       }
       if (K32) {
-        ewald_trig_list<float2><<<dim3((nn + 127) / 128, K32), 128, 0, s>>>(nn, L, dh + K64, d_pos, c32); RSD_LAUNCH_NOTE();
+        pdl_launch(ewald_trig_list<float2>, dim3((nn + 127) / 128, K32), 128, 0, s, nn, L, dh + K64, d_pos, c32);
       }
       if (equal) {
         float* w64 = (float*)rsd_scratch(ctx, "ewald_kblock64", sizeof(float) * (size_t)(K64 > 0 ? K64 : 1) * 2 * KBW);
         float* w32 = (float*)rsd_scratch(ctx, "ewald_kblock32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KBW);
         if (!w64 || !w32) return RSD_ENOMEM;
         if (K64 + K32) {
-          ewald_kblock_lists<<<dim3((K64 + K32 + 31) / 32, 2), 32, 0, s>>>(L, K64, K32, dh, h_radii[0], inv_pimu, w64, w32); RSD_LAUNCH_NOTE();
+          pdl_launch(ewald_kblock_lists, dim3((K64 + K32 + 31) / 32, 2), 32, 0, s, L, K64, K32, dh, h_radii[0], inv_pimu, w64, w32);
         }
-        ewald_pair_kblock<<<grd, blk, 0, s>>>(nn, K32, w32, c32, K64, w64, c64, psk, 0); RSD_LAUNCH_NOTE();
+        pdl_launch(ewald_pair_kblock, grd, blk, 0, s, nn, K32, w32, c32, K64, w64, c64, psk, 0);
       } else {
         if (K64) {
-          ewald_ktable_list<double><<<(K64 + 127) / 128, 128, 0, s>>>(L, K64, dh, t64); RSD_LAUNCH_NOTE();
+          pdl_launch(ewald_ktable_list<double>, (K64 + 127) / 128, 128, 0, s, L, K64, dh, t64);
         }
         if (K32) {
-          ewald_ktable_list<float><<<(K32 + 127) / 128, 128, 0, s>>>(L, K32, dh + K64, t32); RSD_LAUNCH_NOTE();
+          pdl_launch(ewald_ktable_list<float>, (K32 + 127) / 128, 128, 0, s, L, K32, dh + K64, t32);
         }
-        ewald_pair_k_ds<<<grd, blk, 0, s>>>(nn, L, K64, t64, c64, d_radii, inv_pimu, psk, 0); RSD_LAUNCH_NOTE();
-        ewald_pair_k<float, float2><<<grd, blk, 0, s>>>(nn, L, K32, t32, c32, d_radii, inv_pimu, psk, 1); RSD_LAUNCH_NOTE();
+        pdl_launch(ewald_pair_k_ds<PlaneSink>, grd, blk, 0, s, nn, L, K64, t64, c64, d_radii, inv_pimu, psk, 0);
+        pdl_launch(ewald_pair_k<float, float2, PlaneSink>, grd, blk, 0, s, nn, L, K32, t32, c32, d_radii, inv_pimu, psk, 1);
       }
       if (equal) {
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
-        ewald_pair_real_near_ds<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, rc2, psk); RSD_LAUNCH_NOTE();
-        ewald_pair_real_far<<<grd, blk, 0, s>>>(nn, L, d_pos, d_radii, inv_pimu, rc2, rmax2, psk); RSD_LAUNCH_NOTE();
+        pdl_launch(ewald_pair_real_near_ds<PlaneSink>, grd, blk, 0, s, nn, L, d_pos, d_radii, inv_pimu, rc2, psk);
+        pdl_launch(ewald_pair_real_far<PlaneSink>, grd, blk, 0, s, nn, L, d_pos, d_radii, inv_pimu, rc2, rmax2, psk);
       }
     }
   }

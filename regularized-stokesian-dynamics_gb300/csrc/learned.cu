@@ -32,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 template <typename T>
@@ -124,6 +125,7 @@ template <bool FILL>
 __global__ void lp_near(int nn, rsd_lat_dev L, const double* __restrict__ pos, const double* __restrict__ radii,
                         int* __restrict__ cnt, const int* __restrict__ off, int* __restrict__ src,
                         int* __restrict__ dst, float* __restrict__ gap) {
+  pdl_enter();
   __shared__ int cand[GR_WARPS][GR_CAND];
   const int warp = threadIdx.x / 32, a = blockIdx.x * GR_WARPS + warp, lane = threadIdx.x & 31;
   if (a >= nn) return;
@@ -183,6 +185,7 @@ __global__ void lp_near(int nn, rsd_lat_dev L, const double* __restrict__ pos, c
 // rev[e]: the edge (src <- dst) in src's list (binary search, lists sorted)
 __global__ void lp_rev(int ne, const int* __restrict__ off, const int* __restrict__ src, const int* __restrict__ dst,
                        int* __restrict__ rev) {
+  pdl_enter();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const int b = src[e], a = dst[e];
@@ -217,6 +220,7 @@ __device__ __forceinline__ double rpp_at(const T* A, int64_t ld, int nn, int i, 
 // dinv[i] = 1 / sqrt(RPP(i, i)) in the particle-block layout
 template <typename T>
 __global__ void lp_dinv(int nn, const T* __restrict__ A, int64_t ld, double* __restrict__ dinv, int* __restrict__ bad) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 6 * nn) return;
   const double d = rpp_at(A, ld, nn, i, i);
@@ -236,6 +240,7 @@ template <typename T>
 __global__ void lp_features(int nn, int ne, const T* __restrict__ A, int64_t ld, const double* __restrict__ dinv,
                             const int* __restrict__ src, const int* __restrict__ dst, const float* __restrict__ gap,
                             __nv_bfloat16* __restrict__ xn, __nv_bfloat16* __restrict__ xe) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nn * 36) {
     const int a = t / 36, q = t % 36, r = q / 6, c = q % 6;
@@ -305,6 +310,7 @@ __global__ void __launch_bounds__(FS_THREADS) lp_fsai(int nn, int lower_only_sel
                                                       const int* __restrict__ src, const float* __restrict__ gap,
                                                       float* __restrict__ zd, float* __restrict__ ze,
                                                       float* __restrict__ wt, int* __restrict__ bad) {
+  pdl_enter();
   extern __shared__ double fs_smem[];
   __shared__ int nb_s[LP_KMAX + 1];
   __shared__ int eidx_s[LP_KMAX];
@@ -450,6 +456,7 @@ __global__ void __launch_bounds__(FS_THREADS) lp_normalize(int nn, const T* __re
                                                            const float* __restrict__ gap,
                                                            const float* __restrict__ w, float* __restrict__ zd,
                                                            float* __restrict__ ze) {
+  pdl_enter();
   extern __shared__ double fs_smem[];
   __shared__ int nb_s[LP_KMAX + 1];
   __shared__ int eidx_s[LP_KMAX];
@@ -553,6 +560,7 @@ constexpr int LW = 8;  // warps per CTA
 constexpr int LR4 = 4;  // rows per warp at a time: a weight read from shared memory serves four rows
 
 __global__ void __launch_bounds__(32 * LW) lp_layer_fwd(LayerArgs A) {
+  pdl_enter();
   extern __shared__ __align__(16) float ls[];
   float* Wt = ls;                       // [kin][kout]
   float* xs = ls + A.kin * A.kout;      // [LW][kin][LR4]
@@ -607,6 +615,7 @@ __global__ void __launch_bounds__(32 * LW) lp_layer_fwd(LayerArgs A) {
 // agg[a] = sum of msg over the edges into a (CSR, fixed order)
 __global__ void lp_aggregate(int nn, const int* __restrict__ off, const __nv_bfloat16* __restrict__ msg,
                              __nv_bfloat16* __restrict__ agg) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nn * H) return;
   const int a = t / H, c = t % H;
@@ -634,6 +643,7 @@ struct LayerBwdArgs {
 };
 
 __global__ void __launch_bounds__(256) lp_layer_bwd(LayerBwdArgs A) {
+  pdl_enter();
   extern __shared__ float bs[];
   float* Ws = bs;                          // [kout][kin]
   float* xs = Ws + A.kout * A.kin;         // [LB_ROWS][kin]
@@ -718,6 +728,7 @@ __global__ void __launch_bounds__(256) lp_layer_bwd(LayerBwdArgs A) {
 // grad[w_off + q] += sum over CTAs of part (fixed order); bias after weights
 __global__ void lp_reduce_parts(int nparts, int nw, int nb, const float* __restrict__ part, float* __restrict__ gw,
                                 float* __restrict__ gb) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nw + nb) return;
   float s = 0.f;
@@ -731,6 +742,7 @@ __global__ void lp_reduce_parts(int nparts, int nw, int nb, const float* __restr
 // dmsg[e] += dagg[dst[e]] (the aggregation's backward)
 __global__ void lp_agg_bwd(int ne, const int* __restrict__ dst, const float* __restrict__ dagg,
                            float* __restrict__ dmsg) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ne * H) return;
   dmsg[t] += dagg[(size_t)dst[t / H] * H + t % H];
@@ -743,6 +755,7 @@ __global__ void lp_agg_bwd(int ne, const int* __restrict__ dst, const float* __r
 __global__ void lp_loss(int ne, const float* __restrict__ ze, const float* __restrict__ te,
                         const int* __restrict__ lower, float inv_cnt, float* __restrict__ dze,
                         double* __restrict__ loss) {
+  pdl_enter();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   double l = 0.0;
   if (u < ne * 36) {
@@ -762,6 +775,7 @@ __global__ void lp_loss(int ne, const float* __restrict__ ze, const float* __res
 // entries of the targets that enter the loss
 __global__ void lp_count_targets(int ne, const float* __restrict__ te, const int* __restrict__ lower,
                                  int* __restrict__ cnt) {
+  pdl_enter();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   int c = 0;
   if (u < ne * 36) {
@@ -773,6 +787,7 @@ __global__ void lp_count_targets(int ne, const float* __restrict__ te, const int
 }
 
 __global__ void lp_lower_flags(int ne, const int* __restrict__ src, const int* __restrict__ dst, int* __restrict__ f) {
+  pdl_enter();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < ne) f[e] = src[e] < dst[e];
 }
@@ -1050,7 +1065,7 @@ static int lp_build_graph(rsd_ctx* ctx, int nn, const double* d_pos, const doubl
   int* cnt = (int*)rsd_scratch(ctx, "lp_cnt", sizeof(int) * (nn + 1));
   if (!cnt) return RSD_ENOMEM;
   const unsigned ng = (unsigned)((nn + GR_WARPS - 1) / GR_WARPS);
-  lp_near<false><<<ng, 32 * GR_WARPS, 0, s>>>(nn, L, d_pos, d_radii, cnt, nullptr, nullptr, nullptr, nullptr); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_near<false>, ng, 32 * GR_WARPS, 0, s, nn, L, d_pos, d_radii, cnt, nullptr, nullptr, nullptr, nullptr); RSD_LP_CHECK();
   std::vector<int> h(nn + 1);
   RSD_CUDA(ctx, cudaMemcpyAsync(h.data(), cnt, sizeof(int) * nn, cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
@@ -1068,9 +1083,9 @@ static int lp_build_graph(rsd_ctx* ctx, int nn, const double* d_pos, const doubl
   if (!g->off || !g->src || !g->dst || !g->rev || !g->lower || !g->gap) return RSD_ENOMEM;
   RSD_CUDA(ctx, cudaMemcpyAsync(g->off, off.data(), sizeof(int) * (nn + 1), cudaMemcpyHostToDevice, s));
   if (ne > 0) {
-    lp_near<true><<<ng, 32 * GR_WARPS, 0, s>>>(nn, L, d_pos, d_radii, nullptr, g->off, g->src, g->dst, g->gap); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    lp_rev<<<nb256(ne), 256, 0, s>>>(ne, g->off, g->src, g->dst, g->rev); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-    lp_lower_flags<<<nb256(ne), 256, 0, s>>>(ne, g->src, g->dst, g->lower); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    pdl_launch(lp_near<true>, ng, 32 * GR_WARPS, 0, s, nn, L, d_pos, d_radii, nullptr, g->off, g->src, g->dst, g->gap); RSD_LP_CHECK();
+    pdl_launch(lp_rev, nb256(ne), 256, 0, s, ne, g->off, g->src, g->dst, g->rev); RSD_LP_CHECK();
+    pdl_launch(lp_lower_flags, nb256(ne), 256, 0, s, ne, g->src, g->dst, g->lower); RSD_LP_CHECK();
   }
   RSD_CUDA(ctx, cudaStreamSynchronize(s));  // off must outlive the host vector's copy
   RSD_CUDA(ctx, cudaGetLastError());
@@ -1087,13 +1102,13 @@ static int lp_scale_features(rsd_ctx* ctx, const lp_graph& g, const T* A, int64_
   if (!*dinv) return RSD_ENOMEM;
   int* bad = ctx->d_info + 9;
   RSD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), s));
-  lp_dinv<T><<<nb256(6 * nn), 256, 0, s>>>(nn, A, ld, *dinv, bad); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_dinv<T>, nb256(6 * nn), 256, 0, s, nn, A, ld, *dinv, bad); RSD_LP_CHECK();
   if (xn) {
     *xn = (__nv_bfloat16*)rsd_scratch(ctx, "lp_xn", sizeof(__nv_bfloat16) * (size_t)nn * NF_NODE);
     *xe = (__nv_bfloat16*)rsd_scratch(ctx, "lp_xe", sizeof(__nv_bfloat16) * ((size_t)ne * NF_EDGE + 1));
     if (!*xn || !*xe) return RSD_ENOMEM;
-    lp_features<T><<<nb256((int64_t)nn * 36 + (int64_t)ne * NF_EDGE), 256, 0, s>>>(nn, ne, A, ld, *dinv, g.src, g.dst,
-                                                                                   g.gap, *xn, *xe); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    pdl_launch(lp_features<T>, nb256((int64_t)nn * 36 + (int64_t)ne * NF_EDGE), 256, 0, s, nn, ne, A, ld, *dinv, g.src, g.dst,
+                                                                                   g.gap, *xn, *xe); RSD_LP_CHECK();
   }
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 9, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
@@ -1118,7 +1133,7 @@ static int lp_exact_fsai(rsd_ctx* ctx, const lp_graph& g, const T* A, int64_t ld
   }
   int* bad = ctx->d_info + 10;
   RSD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), s));
-  lp_fsai<T><<<g.nn, FS_THREADS, LP_LOCAL_SMEM, s>>>(g.nn, self_only, A, ld, dinv, g.off, g.src, g.gap, zd, ze, wt, bad); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_fsai<T>, g.nn, FS_THREADS, LP_LOCAL_SMEM, s, g.nn, self_only, A, ld, dinv, g.off, g.src, g.gap, zd, ze, wt, bad); RSD_LP_CHECK();
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + 10, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
   if (ctx->h_info[10]) return rsd_fail(ctx, RSD_ENAN, "FSAI: a local block of RPP is not positive definite");
@@ -1139,7 +1154,7 @@ static int lp_layer(rsd_ctx* ctx, const LayerArgs& a) {
     attr = true;
   }
   const int grid = (int)std::min<int64_t>((a.rows + LW * LR4 - 1) / (LW * LR4), 2LL * (ctx->sm_count > 0 ? ctx->sm_count : 148));
-  lp_layer_fwd<<<grid, 32 * LW, smem, ctx->stream>>>(a); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_layer_fwd, grid, 32 * LW, smem, ctx->stream, a); RSD_LP_CHECK();
   return RSD_OK;
 }
 
@@ -1178,7 +1193,7 @@ static int lp_forward(rsd_ctx* ctx, rsd_lp* net, const lp_graph& g, const __nv_b
     a.res = A->m[l];
     a.sum = A->m[l + 1];
     RSD_TRY(lp_layer(ctx, a));
-    lp_aggregate<<<nb256((int64_t)nn * H), 256, 0, ctx->stream>>>(nn, g.off, A->msg[l], A->agg[l]); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    pdl_launch(lp_aggregate, nb256((int64_t)nn * H), 256, 0, ctx->stream, nn, g.off, A->msg[l], A->agg[l]); RSD_LP_CHECK();
     a = LayerArgs{nn, 2 * H, H, 1, {seg(A->h[l], nullptr, H), seg(A->agg[l], nullptr, H)}, 2, W + LAY.upd_w[l],
                   B + LAY.upd_b[l], A->u[l]};
     a.res = A->h[l];
@@ -1211,9 +1226,9 @@ static int lp_layer_back(rsd_ctx* ctx, rsd_lp* net, LayerBwdArgs b, int64_t w_of
     RSD_CUDA(ctx, cudaFuncSetAttribute(lp_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     attr = true;
   }
-  lp_layer_bwd<<<nparts, 256, smem, ctx->stream>>>(b); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
-  lp_reduce_parts<<<nb256(nw + b.kout), 256, 0, ctx->stream>>>(nparts, nw, b.kout, part, net->g + w_off,
-                                                                net->g + b_off); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_layer_bwd, nparts, 256, smem, ctx->stream, b); RSD_LP_CHECK();
+  pdl_launch(lp_reduce_parts, nb256(nw + b.kout), 256, 0, ctx->stream, nparts, nw, b.kout, part, net->g + w_off,
+                                                                net->g + b_off); RSD_LP_CHECK();
   return RSD_OK;
 }
 
@@ -1252,7 +1267,7 @@ static int lp_backward(rsd_ctx* ctx, rsd_lp* net, const lp_graph& g, const __nv_
     // m[l+1] = m[l] + msg[l]: dmsg = dm + dagg[dst]; dm flows to m[l]
     RSD_CUDA(ctx, cudaMemcpyAsync(dmsg, dm, sizeof(float) * (size_t)ne * H, cudaMemcpyDeviceToDevice, s));
     if (ne > 0) {
-      lp_agg_bwd<<<nb256((int64_t)ne * H), 256, 0, s>>>(ne, g.dst, dagg, dmsg); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+      pdl_launch(lp_agg_bwd, nb256((int64_t)ne * H), 256, 0, s, ne, g.dst, dagg, dmsg); RSD_LP_CHECK();
     }
     RSD_CUDA(ctx, cudaMemcpyAsync(dm2, dm, sizeof(float) * (size_t)ne * H, cudaMemcpyDeviceToDevice, s));
     b = LayerBwdArgs{ne, 3 * H, H, 1, {seg(A.h[l], g.dst, H), seg(A.h[l], g.src, H), seg(A.m[l], nullptr, H)}, 3,
@@ -1296,8 +1311,8 @@ static int lp_make_z(rsd_ctx* ctx, rsd_lp* net, int mode, const lp_graph& g, con
                                          (int)LP_LOCAL_SMEM));
       attr[which] = true;
     }
-    lp_normalize<T><<<g.nn, FS_THREADS, LP_LOCAL_SMEM, ctx->stream>>>(g.nn, A, ld, *dinv, g.off, g.src, g.gap, wp,
-                                                                      *zd, *ze); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    pdl_launch(lp_normalize<T>, g.nn, FS_THREADS, LP_LOCAL_SMEM, ctx->stream, g.nn, A, ld, *dinv, g.off, g.src, g.gap, wp,
+                                                                      *zd, *ze); RSD_LP_CHECK();
     return RSD_OK;
   }
   RSD_TRY(lp_scale_features<T>(ctx, g, A, ld, dinv, nullptr, nullptr));
@@ -1508,7 +1523,7 @@ extern "C" int rsd_lp_forward_dev(rsd_ctx* ctx, rsd_lp* net, int32_t nn, int32_t
   __nv_bfloat16* xe = (__nv_bfloat16*)rsd_scratch(ctx, "lp_xe_t", sizeof(__nv_bfloat16) * ((size_t)ne * NF_EDGE + 1));
   if (!g.lower || !xn || !xe) return RSD_ENOMEM;
   if (ne) {
-    lp_lower_flags<<<nb256(ne), 256, 0, s>>>(ne, g.src, g.dst, g.lower); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+    pdl_launch(lp_lower_flags, nb256(ne), 256, 0, s, ne, g.src, g.dst, g.lower); RSD_LP_CHECK();
   }
   lp_to_bf16<<<nb256((int64_t)nn * NF_NODE), 256, 0, s>>>((int64_t)nn * NF_NODE, d_xn, xn); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
   if (ne) {
@@ -1576,12 +1591,12 @@ static int lp_train_t(rsd_ctx* ctx, rsd_lp* net, int nn, const double* d_pos, co
   RSD_TRY(lp_forward(ctx, net, g, xn, xe, &acts, zd, ze));
   int hcnt = 0;
   RSD_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int), s));
-  lp_count_targets<<<nb256((int64_t)g.ne * 36), 256, 0, s>>>(g.ne, te, g.lower, cnt); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_count_targets, nb256((int64_t)g.ne * 36), 256, 0, s, g.ne, te, g.lower, cnt); RSD_LP_CHECK();
   RSD_CUDA(ctx, cudaMemcpyAsync(&hcnt, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));
   RSD_CUDA(ctx, cudaMemsetAsync(dl, 0, sizeof(double), s));
   RSD_CUDA(ctx, cudaMemsetAsync(dzd, 0, sizeof(float) * (size_t)nn * 36, s));  // the node head is not trained
-  lp_loss<<<nb256((int64_t)g.ne * 36), 256, 0, s>>>(g.ne, ze, te, g.lower, hcnt ? 1.f / hcnt : 0.f, dze, dl); RSD_LAUNCH_NOTE(); RSD_LP_CHECK();
+  pdl_launch(lp_loss, nb256((int64_t)g.ne * 36), 256, 0, s, g.ne, ze, te, g.lower, hcnt ? 1.f / hcnt : 0.f, dze, dl); RSD_LP_CHECK();
   RSD_TRY(lp_backward(ctx, net, g, xn, xe, acts, dzd, dze));
   RSD_CUDA(ctx, cudaMemcpyAsync(loss, dl, sizeof(double), cudaMemcpyDeviceToHost, s));
   RSD_CUDA(ctx, cudaStreamSynchronize(s));

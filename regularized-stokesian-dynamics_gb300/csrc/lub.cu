@@ -16,6 +16,7 @@
 // zeroed matrix or added into one (arrangResist, src/matrices.f90:218-228).
 #include <cuda_runtime.h>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
@@ -125,6 +126,7 @@ template <bool LIST>
 __global__ void lub_near(int nn, int nb, int is_period, rsd_lat_dev L, const double* __restrict__ pos,
                          const double* __restrict__ radii, int* __restrict__ count, const int* __restrict__ off,
                          int2* __restrict__ pairs) {
+  pdl_enter();
   __shared__ int cand[LUB_WARPS][LUB_CAND];
   const int warp = threadIdx.x / 32, a = blockIdx.x * LUB_WARPS + warp, lane = threadIdx.x & 31;
   if (a >= nn) return;
@@ -170,6 +172,7 @@ __global__ void lub_near(int nn, int nb, int is_period, rsd_lat_dev L, const dou
 
 // exclusive scan of count[0..n) into off[0..n], one block of 1024 threads
 __global__ void lub_scan(int n, const int* __restrict__ count, int* __restrict__ off) {
+  pdl_enter();
   __shared__ int part[1024];
   const int t = threadIdx.x;
   const int per = (n + 1023) / 1024;
@@ -254,6 +257,7 @@ __global__ void __launch_bounds__(32) lub_pairs(int npair, lub_dev_tab tab, int 
                                                 const double* __restrict__ pos, const double* __restrict__ radii,
                                                 const int2* __restrict__ pairs, double* __restrict__ blk,
                                                 int* __restrict__ contacts) {
+  pdl_enter();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npair) return;
   const int a = pairs[p].x, b = pairs[p].y;
@@ -313,6 +317,7 @@ __device__ inline double self_entry(const double* B, int r, int c, double sgn) {
 // 121 entries of the (a,b) block and 121 of the (b,a) block per pair
 __global__ void lub_cross(int npair, int N, const int2* __restrict__ pairs, const double* __restrict__ blk,
                           double scale, double* __restrict__ L, int64_t ld, int acc) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)npair * 121) return;
   const int p = (int)(t / 121), e = (int)(t % 121);
@@ -326,12 +331,14 @@ __global__ void lub_cross(int npair, int N, const int2* __restrict__ pairs, cons
 // Second-particle lists: for each particle u, the pairs (a,u) with a < u,
 // in pair order (which is a-ascending, the order lubmxcalc adds them in).
 __global__ void lub_second_count(int npair, const int2* __restrict__ pairs, int* __restrict__ cnt2) {
+  pdl_enter();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < npair) atomicAdd(&cnt2[pairs[p].y], 1);
 }
 
 __global__ void lub_second_fill(int npair, const int2* __restrict__ pairs, const int* __restrict__ off2,
                                 int* __restrict__ cur, int* __restrict__ list2) {
+  pdl_enter();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npair) return;
   const int b = pairs[p].y;
@@ -342,6 +349,7 @@ __global__ void lub_second_fill(int npair, const int2* __restrict__ pairs, const
 // particle's list, a thread per entry
 __global__ void lub_second_rank(int npair, const int2* __restrict__ pairs, const int* __restrict__ off2,
                                 const int* __restrict__ raw, int* __restrict__ list2) {
+  pdl_enter();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npair) return;
   const int u = pairs[p].y, lo = off2[u], hi = off2[u + 1];
@@ -356,6 +364,7 @@ __global__ void lub_second_rank(int npair, const int2* __restrict__ pairs, const
 __global__ void lub_self(int N, const int* __restrict__ off, const int* __restrict__ off2,
                          const int* __restrict__ list2, const double* __restrict__ blk, double scale,
                          double* __restrict__ L, int64_t ld, int acc, double* __restrict__ self) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)N * 121) return;
   const int u = (int)(t / 121), e = (int)(t % 121);
@@ -400,6 +409,7 @@ __global__ void __launch_bounds__(128) lub_spmv_w(int N, const int* __restrict__
                                                   const double* __restrict__ blk, const double* __restrict__ self,
                                                   double scale, const double* __restrict__ w, int64_t ldw,
                                                   double* __restrict__ y, int64_t ldy) {
+  pdl_enter();
   __shared__ double sv[121], pv[121];
   const int u = blockIdx.x, t = threadIdx.x, r = t % 11, c = t / 11;
   const double* wc = w + blockIdx.y * ldw;
@@ -439,6 +449,7 @@ __global__ void __launch_bounds__(128) lub_spmv_w(int N, const int* __restrict__
 template <typename T>
 __global__ void lub_pp_pairs(int npair, int N, const int2* __restrict__ pairs, const double* __restrict__ blk,
                              double scale, T* __restrict__ A, int64_t lda) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)npair * 36) return;
   const int p = (int)(t / 36), e = (int)(t % 36);
@@ -451,6 +462,7 @@ __global__ void lub_pp_pairs(int npair, int N, const int2* __restrict__ pairs, c
 
 template <typename T>
 __global__ void lub_pp_self(int N, const double* __restrict__ self, T* __restrict__ A, int64_t lda) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)N * 36) return;
   const int u = (int)(t / 36), e = (int)(t % 36);
@@ -459,6 +471,7 @@ __global__ void lub_pp_self(int N, const double* __restrict__ self, T* __restric
 }
 
 __global__ void zero_matrix(int64_t rows, int64_t cols, double* __restrict__ A, int64_t ld) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= rows * cols) return;
   A[(t % rows) + (t / rows) * ld] = 0.0;
@@ -491,9 +504,9 @@ int rsd_lub_begin(rsd_ctx* ctx, cudaStream_t s, int nn, int nb, int is_period, c
   int* cnt = (int*)rsd_scratch(ctx, "lub_count", sizeof(int) * (nn + 1));
   int* off = (int*)rsd_scratch(ctx, "lub_off", sizeof(int) * (nn + 1));
   if (!cnt || !off) return RSD_ENOMEM;
-  lub_near<false><<<(nn + LUB_WARPS - 1) / LUB_WARPS, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, rsd_lat_pack(lat),
-                                                                              d_pos, d_radii, cnt, nullptr, nullptr); RSD_LAUNCH_NOTE();
-  lub_scan<<<1, 1024, 0, s>>>(nn, cnt, off); RSD_LAUNCH_NOTE();
+  pdl_launch(lub_near<false>, (nn + LUB_WARPS - 1) / LUB_WARPS, 32 * LUB_WARPS, 0, s, nn, nb, is_period, rsd_lat_pack(lat),
+                                                                              d_pos, d_radii, cnt, nullptr, nullptr);
+  pdl_launch(lub_scan, 1, 1024, 0, s, nn, cnt, off);
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info + LUB_NPAIR, off + nn, sizeof(int), cudaMemcpyDeviceToHost, s));
   return RSD_OK;
 }
@@ -522,12 +535,12 @@ static int lub_pair_stage(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, i
   RSD_CUDA(ctx, cudaMemsetAsync(cnt2, 0, sizeof(int) * (nn + 1), s));
   RSD_CUDA(ctx, cudaMemsetAsync(cur, 0, sizeof(int) * (nn + 1), s));
   if (npair > 0) {
-    lub_near<true><<<ng, 32 * LUB_WARPS, 0, s>>>(nn, nb, is_period, Ld, d_pos, d_radii, nullptr, off, pairs); RSD_LAUNCH_NOTE();
-    lub_pairs<<<(npair + 31) / 32, 32, 0, s>>>(npair, T, is_period, Ld, d_pos, d_radii, pairs, blk, dcon); RSD_LAUNCH_NOTE();
-    lub_second_count<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, cnt2); RSD_LAUNCH_NOTE();
-    lub_scan<<<1, 1024, 0, s>>>(nn, cnt2, off2); RSD_LAUNCH_NOTE();
-    lub_second_fill<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, off2, cur, raw2); RSD_LAUNCH_NOTE();
-    lub_second_rank<<<(npair + 255) / 256, 256, 0, s>>>(npair, pairs, off2, raw2, list2); RSD_LAUNCH_NOTE();
+    pdl_launch(lub_near<true>, ng, 32 * LUB_WARPS, 0, s, nn, nb, is_period, Ld, d_pos, d_radii, nullptr, off, pairs);
+    pdl_launch(lub_pairs, (npair + 31) / 32, 32, 0, s, npair, T, is_period, Ld, d_pos, d_radii, pairs, blk, dcon);
+    pdl_launch(lub_second_count, (npair + 255) / 256, 256, 0, s, npair, pairs, cnt2);
+    pdl_launch(lub_scan, 1, 1024, 0, s, nn, cnt2, off2);
+    pdl_launch(lub_second_fill, (npair + 255) / 256, 256, 0, s, npair, pairs, off2, cur, raw2);
+    pdl_launch(lub_second_rank, (npair + 255) / 256, 256, 0, s, npair, pairs, off2, raw2, list2);
   } else {
     RSD_CUDA(ctx, cudaMemsetAsync(off2, 0, sizeof(int) * (nn + 1), s));
   }
@@ -550,7 +563,7 @@ int rsd_lub_assemble(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is
   cudaStream_t s = ctx->stream;
   if (!accumulate) {
     const int64_t tot = 121LL * nn * nn;
-    zero_matrix<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(11LL * nn, 11LL * nn, d_L, ldl); RSD_LAUNCH_NOTE();
+    pdl_launch(zero_matrix, (unsigned)((tot + 255) / 256), 256, 0, s, 11LL * nn, 11LL * nn, d_L, ldl);
   }
   rsd_lub_sparse sp;
   RSD_TRY(rsd_lub_begin(ctx, s, nn, nb, is_period, d_pos, d_radii, lat));
@@ -558,10 +571,10 @@ int rsd_lub_assemble(rsd_ctx* ctx, const rsd_lubtab* tab, int nn, int nb, int is
   const double scale = 6.0 * (RSD_PI * mu_f);
   if (sp.npair > 0) {
     const int64_t tc = 121LL * sp.npair;
-    lub_cross<<<(unsigned)((tc + 255) / 256), 256, 0, s>>>(sp.npair, nn, sp.pairs, sp.blk, scale, d_L, ldl, 1); RSD_LAUNCH_NOTE();
+    pdl_launch(lub_cross, (unsigned)((tc + 255) / 256), 256, 0, s, sp.npair, nn, sp.pairs, sp.blk, scale, d_L, ldl, 1);
     const int64_t ts = 121LL * nn;
-    lub_self<<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(nn, sp.off, sp.off2, sp.list2, sp.blk, scale, d_L, ldl, 1,
-                                                            nullptr); RSD_LAUNCH_NOTE();
+    pdl_launch(lub_self, (unsigned)((ts + 255) / 256), 256, 0, s, nn, sp.off, sp.off2, sp.list2, sp.blk, scale, d_L, ldl, 1,
+                                                            nullptr);
   }
   RSD_CUDA(ctx, cudaGetLastError());
   if (n_contact) {
@@ -584,8 +597,8 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, in
   sp->scale = 6.0 * (RSD_PI * mu_f);
   sp->self = self;
   const int64_t ts = 121LL * nn;
-  lub_self<<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(nn, sp->off, sp->off2, sp->list2, sp->blk, sp->scale,
-                                                          nullptr, 0, 0, self); RSD_LAUNCH_NOTE();
+  pdl_launch(lub_self, (unsigned)((ts + 255) / 256), 256, 0, s, nn, sp->off, sp->off2, sp->list2, sp->blk, sp->scale,
+                                                          nullptr, 0, 0, self);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -593,8 +606,8 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, in
 // y (11N x nr, grand layout, ld ldy) = L w
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy) {
-  lub_spmv_w<<<dim3(sp->nn, nr), 128, 0, ctx->stream>>>(sp->nn, sp->off, sp->off2, sp->list2, sp->pairs, sp->blk,
-                                                        sp->self, sp->scale, w, ldw, y, ldy); RSD_LAUNCH_NOTE();
+  pdl_launch(lub_spmv_w, dim3(sp->nn, nr), 128, 0, ctx->stream, sp->nn, sp->off, sp->off2, sp->list2, sp->pairs, sp->blk,
+                                                        sp->self, sp->scale, w, ldw, y, ldy);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -605,11 +618,11 @@ static int lub_add_pp(rsd_ctx* ctx, const rsd_lub_sparse* sp, T* A, int64_t lda)
   cudaStream_t s = ctx->stream;
   if (sp->npair > 0) {
     const int64_t tp = 36LL * sp->npair;
-    lub_pp_pairs<T><<<(unsigned)((tp + 255) / 256), 256, 0, s>>>(sp->npair, sp->nn, sp->pairs, sp->blk, sp->scale, A,
-                                                                 lda); RSD_LAUNCH_NOTE();
+    pdl_launch(lub_pp_pairs<T>, (unsigned)((tp + 255) / 256), 256, 0, s, sp->npair, sp->nn, sp->pairs, sp->blk, sp->scale, A,
+                                                                 lda);
   }
   const int64_t ts = 36LL * sp->nn;
-  lub_pp_self<T><<<(unsigned)((ts + 255) / 256), 256, 0, s>>>(sp->nn, sp->self, A, lda); RSD_LAUNCH_NOTE();
+  pdl_launch(lub_pp_self<T>, (unsigned)((ts + 255) / 256), 256, 0, s, sp->nn, sp->self, A, lda);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }

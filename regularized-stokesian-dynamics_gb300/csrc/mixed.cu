@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "dsf.cuh"
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 template <typename T>
@@ -75,6 +76,7 @@ __device__ __forceinline__ int64_t perm_src(const mixed_dims& d, int64_t i) {  /
 
 __global__ void convert_perm_half(int N, mixed_dims d, const float* __restrict__ Mh, int64_t ld,
                                   float* __restrict__ M32) {
+  pdl_enter();
   __shared__ float D[32][33], T[32][33];
   __shared__ int64_t si[32], sj[32];
   __shared__ int pi[32], pj[32], need;
@@ -123,6 +125,7 @@ __global__ void convert_perm_half(int N, mixed_dims d, const float* __restrict__
 
 // x (FP64) as float pairs
 __global__ void to_dsf_vec(int64_t n, const double* __restrict__ x, float2* __restrict__ xs) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const dsf d = dsf_from(x[t]);
@@ -145,6 +148,7 @@ __global__ void __launch_bounds__(256) symv_planes_part(int N, int n, const floa
                                                         const float* __restrict__ Ml, int64_t ld,
                                                         const float2* __restrict__ xs, int nbt,
                                                         double* __restrict__ prow, double* __restrict__ pcol) {
+  pdl_enter();
   // dynamic shared memory (symv_smem(NR) bytes): the row partials of the 8
   // warps, then the per-lane column partials, reduced after the tile
   extern __shared__ __align__(16) unsigned char symv_raw[];
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(256) symv_planes_part(int N, int n, const floa
 __global__ void symv_planes_reduce(int n, int nr, int nbt, const double* __restrict__ prow,
                                    const double* __restrict__ pcol, double alpha, double* __restrict__ y,
                                    int64_t ldy) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int K = i / SYMV_T, e = i % SYMV_T;
@@ -261,6 +266,7 @@ __global__ void symv_planes_reduce(int n, int nr, int nbt, const double* __restr
 
 __global__ void copy_block_f(int64_t rows, int64_t cols, const float* __restrict__ S, int64_t lds,
                              float* __restrict__ D, int64_t ldd) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= rows * cols) return;
   const int64_t i = t % rows, j = t / rows;
@@ -270,6 +276,7 @@ __global__ void copy_block_f(int64_t rows, int64_t cols, const float* __restrict
 // w = [U; -EIN] per column
 __global__ void build_w(int64_t P, int64_t Q, int nr, const double* __restrict__ U, const double* __restrict__ ein,
                         double* __restrict__ w) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n = P + Q;
   if (t >= n * nr) return;
@@ -280,6 +287,7 @@ __global__ void build_w(int64_t P, int64_t Q, int nr, const double* __restrict__
 // r2 = Fe_c - f_P - (Lw)_P  (Fe only in column 0 when have_fe)
 __global__ void build_r2(int64_t P, int64_t n, int nr, const double* __restrict__ Fe, int have_fe,
                          const double* __restrict__ f, const double* __restrict__ Lw, double* __restrict__ r2) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P * nr) return;
   const int64_t i = t % P, c = t / P;
@@ -295,6 +303,7 @@ __global__ void build_r2(int64_t P, int64_t n, int nr, const double* __restrict_
 __global__ void it_begin(int64_t P, int64_t Q, int nr, const double* __restrict__ U, const double* __restrict__ ein,
                          const double* __restrict__ f, double* __restrict__ w, double* __restrict__ r1,
                          float2* __restrict__ fs) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n = P + Q;
   if (t >= n * nr) return;
   const int64_t i = t % n, c = t / n;
@@ -312,6 +321,7 @@ __global__ void __launch_bounds__(256) it_residual(mixed_dims d, const double* _
                                                    int have_fe, const double* __restrict__ f,
                                                    const double* __restrict__ Lw, double* __restrict__ r2,
                                                    float* __restrict__ t32, double* __restrict__ part) {
+  pdl_enter();
   __shared__ double sr[256], sb[256];
   const int c = blockIdx.y;
   const double *r1c = r1 + c * d.n, *fc = f + c * d.n, *lc = Lw + c * d.n;
@@ -355,6 +365,7 @@ __global__ void __launch_bounds__(256) it_residual(mixed_dims d, const double* _
 // y = unperm(x32) (y = M^-1 r1); u32 = r2 - y_P, zero past P
 __global__ void it_velocity(mixed_dims d, int nr, const float* __restrict__ x32, const double* __restrict__ r2,
                             double* __restrict__ y, float* __restrict__ u32) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.np * nr) return;
   const int64_t i = t % d.np, c = t / d.np, q = perm_src(d, i);
@@ -368,6 +379,7 @@ __global__ void it_velocity(mixed_dims d, int nr, const float* __restrict__ x32,
 
 // t32 = [0; dU]
 __global__ void it_force(mixed_dims d, int nr, const float* __restrict__ du, float* __restrict__ t32) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.np * nr) return;
   const int64_t i = t % d.np, c = t / d.np;
@@ -377,6 +389,7 @@ __global__ void it_force(mixed_dims d, int nr, const float* __restrict__ du, flo
 // f += y + unperm(x32), U += dU
 __global__ void it_update(mixed_dims d, int nr, const float* __restrict__ x32, const double* __restrict__ y,
                           const float* __restrict__ du, double* __restrict__ f, double* __restrict__ U) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.np * nr) return;
   const int64_t i = t % d.np, c = t / d.np, q = perm_src(d, i);
@@ -389,6 +402,7 @@ __global__ void it_update(mixed_dims d, int nr, const float* __restrict__ x32, c
 
 // y32 = x in the padded [Q, P] order
 __global__ void to32_perm(mixed_dims d, const double* __restrict__ x, float* __restrict__ y) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.np) return;
   const int64_t q = perm_src(d, t);
@@ -397,6 +411,7 @@ __global__ void to32_perm(mixed_dims d, const double* __restrict__ x, float* __r
 
 // y (FP64, [P, Q] order) += unperm(x32)
 __global__ void from32_add(mixed_dims d, const float* __restrict__ x, double* __restrict__ y) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.np) return;
   const int64_t q = perm_src(d, t);
@@ -406,6 +421,7 @@ __global__ void from32_add(mixed_dims d, const float* __restrict__ x, double* __
 // S = f_Q + (Lw)_Q of column c; U_par = U column 0
 __global__ void outputs(int64_t P, int64_t Q, int c, const double* __restrict__ f, const double* __restrict__ Lw,
                         const double* __restrict__ U, double* __restrict__ Upar, double* __restrict__ S) {
+  pdl_enter();
   const int64_t n = P + Q;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < Q) S[t] = f[P + t + c * n] + Lw[P + t + c * n];
@@ -422,6 +438,7 @@ inline unsigned nblk(int64_t n) { return (unsigned)((n + 255) / 256); }
 // out[k] = V_k . w for k < nk (one block per k)
 __global__ void gm_dots(int64_t len, int nk, const double* __restrict__ V, int64_t ldv, const double* __restrict__ w,
                         double* __restrict__ out) {
+  pdl_enter();
   __shared__ double red[256];
   const int k = blockIdx.x;
   double a = 0.0;
@@ -438,6 +455,7 @@ __global__ void gm_dots(int64_t len, int nk, const double* __restrict__ V, int64
 // w -= sum_k h[k] V_k; hacc[k] += h[k] (thread 0 of block 0)
 __global__ void gm_orth(int64_t len, int nk, const double* __restrict__ V, int64_t ldv, const double* __restrict__ h,
                         double* __restrict__ w, double* __restrict__ hacc) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0)
     for (int k = 0; k < nk; k++) hacc[k] += h[k];
@@ -450,6 +468,7 @@ __global__ void gm_orth(int64_t len, int nk, const double* __restrict__ V, int64
 // v = w / sqrt(nrm2[0])
 __global__ void gm_scale(int64_t len, const double* __restrict__ w, const double* __restrict__ nrm2,
                          double* __restrict__ v) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < len) v[i] = w[i] / sqrt(nrm2[0]);
 }
@@ -457,6 +476,7 @@ __global__ void gm_scale(int64_t len, const double* __restrict__ w, const double
 // x += sum_k y[k] Z_k
 __global__ void gm_update(int64_t len, int nk, const double* __restrict__ Z, int64_t ldz, const double* __restrict__ y,
                           double* __restrict__ x) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= len) return;
   double s = 0.0;
@@ -466,28 +486,33 @@ __global__ void gm_update(int64_t len, int nk, const double* __restrict__ Z, int
 
 // w = [u; 0] (length n) from u (length P)
 __global__ void gm_u0(int64_t P, int64_t n, const double* __restrict__ u, double* __restrict__ w) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) w[i] = i < P ? u[i] : 0.0;
 }
 
 // a1 = -w (then + M f by the symmetric product); a2 = f_P + Lw_P
 __global__ void gm_neg(int64_t n, const double* __restrict__ w, double* __restrict__ a) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = -w[i];
 }
 __global__ void gm_a2(int64_t P, const double* __restrict__ f, const double* __restrict__ Lw, double* __restrict__ a2) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < P) a2[i] = f[i] + Lw[i];
 }
 
 // FP32 vector to FP64
 __global__ void gm_f2d(int64_t n, const float* __restrict__ x, double* __restrict__ y) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = (double)x[i];
 }
 
 // sum of squares of v[0:len] into out[0] (one block)
 __global__ void gm_nrm2(int64_t len, const double* __restrict__ v, double* __restrict__ out) {
+  pdl_enter();
   __shared__ double red[256];
   double a = 0.0;
   for (int64_t i = threadIdx.x; i < len; i += 256) a += v[i] * v[i];
@@ -554,7 +579,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   // FP32 factor of M' (stresslets first)
   {
     const unsigned nt = (unsigned)((d.np + 31) / 32);
-    convert_perm_half<<<dim3(nt, nt), dim3(32, 8), 0, s>>>(nn, d, Mh, ld, M32); RSD_LAUNCH_NOTE();
+    pdl_launch(convert_perm_half, dim3(nt, nt), dim3(32, 8), 0, s, nn, d, Mh, ld, M32);
   }
   // Tensor-core precision per factor.  The refinement contracts by about the
   // preconditioner's relative error times the condition number it meets:
@@ -574,7 +599,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   const bool use_uh = ctx->use_tc && !rpp_out;
   if (use_uh) RSD_TRY(rsd_uhat_build(ctx, (int)d.np, M32, d.np, W_m, "m32", &uh_m, st + 5));
   // A^-1 from the trailing factor block, then RPP32 = A^-1 + rfu and its factor
-  copy_block_f<<<nblk(d.Pp * d.Pp), 256, 0, s>>>(d.Pp, d.Pp, M32 + d.Qp * (d.np + 1), d.np, A32, d.Pp); RSD_LAUNCH_NOTE();
+  pdl_launch(copy_block_f, nblk(d.Pp * d.Pp), 256, 0, s, d.Pp, d.Pp, M32 + d.Qp * (d.np + 1), d.np, A32, d.Pp);
   RSD_TRY(rsd_potri_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp, "a32", ctx->use_tc == 3 ? 3 : 1,
                                    rpp_out ? nullptr : W128 + (size_t)(d.Qp / 128) * 128 * 128, st + 2));
   RSD_TRY(rsd_mirror_upper_t<float>(ctx, (int)d.Pp, A32, d.Pp));
@@ -647,48 +672,48 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     if (!dv) return RSD_ENOMEM;
     // the product M v (FP64 v of length n, planes in double-single) into out (added)
     auto symv_add = [&](const double* v, double* out) -> int {
-      to_dsf_vec<<<nblk(n), 256, 0, s>>>(n, v, fs); RSD_LAUNCH_NOTE();
+      pdl_launch(to_dsf_vec, nblk(n), 256, 0, s, n, v, fs);
       double* pcol = gpart + (size_t)nbt * nbt * SYMV_T;
-      symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
-      symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, 1, nbt, gpart, pcol, 1.0, out, n); RSD_LAUNCH_NOTE();
+      pdl_launch(symv_planes_part<1>, dim3(nbt, nbt), 256, symv_smem(1), s, nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol);
+      pdl_launch(symv_planes_reduce, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, 1, nbt, gpart, pcol, 1.0, out, n);
       return RSD_OK;
     };
     // residual of column c: (r1, r2) = b - A x into out (length n + P);
     // Lw (column c) keeps L [U; -EIN] for the stresslet output
     auto residual = [&](int c, double* out) -> int {
       double *fc = f + (size_t)c * n, *Uc = U + (size_t)c * P, *wc = w + (size_t)c * n, *Lc = Lw + (size_t)c * n;
-      build_w<<<nblk(n), 256, 0, s>>>(P, Q, 1, Uc, ein, wc); RSD_LAUNCH_NOTE();
-      gm_neg<<<nblk(n), 256, 0, s>>>(n, wc, out); RSD_LAUNCH_NOTE();
+      pdl_launch(build_w, nblk(n), 256, 0, s, P, Q, 1, Uc, ein, wc);
+      pdl_launch(gm_neg, nblk(n), 256, 0, s, n, wc, out);
       RSD_TRY(symv_add(fc, out));  // out = M f - w
-      gm_neg<<<nblk(n), 256, 0, s>>>(n, out, out); RSD_LAUNCH_NOTE();  // r1 = w - M f
+      pdl_launch(gm_neg, nblk(n), 256, 0, s, n, out, out);  // r1 = w - M f
       if (lub) {
         RSD_TRY(rsd_lub_spmv(ctx, lub, 1, wc, n, Lc, n));
       } else {
         RSD_CUDA(ctx, cudaMemsetAsync(Lc, 0, sizeof(double) * n, s));
       }
-      build_r2<<<nblk(P), 256, 0, s>>>(P, n, 1, Fe, have_fe && c == 0, fc, Lc, out + n); RSD_LAUNCH_NOTE();
+      pdl_launch(build_r2, nblk(P), 256, 0, s, P, n, 1, Fe, have_fe && c == 0, fc, Lc, out + n);
       return RSD_OK;
     };
     // z = P v (v, z of length n + P)
     auto precond = [&](const double* v, double* z) -> int {
-      to32_perm<<<nblk(d.np), 256, 0, s>>>(d, v, t32); RSD_LAUNCH_NOTE();
+      pdl_launch(to32_perm, nblk(d.np), 256, 0, s, d, v, t32);
       RSD_TRY(solve_m(t32, 1, x32, 0));
-      it_velocity<<<nblk(d.np), 256, 0, s>>>(d, 1, x32, v + n, z, u32); RSD_LAUNCH_NOTE();  // y = M^-1 v1
+      pdl_launch(it_velocity, nblk(d.np), 256, 0, s, d, 1, x32, v + n, z, u32);  // y = M^-1 v1
       RSD_TRY(solve_r(u32, 1, du32));
-      it_force<<<nblk(d.np), 256, 0, s>>>(d, 1, du32, t32); RSD_LAUNCH_NOTE();
+      pdl_launch(it_force, nblk(d.np), 256, 0, s, d, 1, du32, t32);
       RSD_TRY(solve_m(t32, 1, x32, (int)d.Qp));
-      from32_add<<<nblk(d.np), 256, 0, s>>>(d, x32, z); RSD_LAUNCH_NOTE();          // df
-      gm_f2d<<<nblk(P), 256, 0, s>>>(P, du32, z + n); RSD_LAUNCH_NOTE();             // dU
+      pdl_launch(from32_add, nblk(d.np), 256, 0, s, d, x32, z);          // df
+      pdl_launch(gm_f2d, nblk(P), 256, 0, s, P, du32, z + n);             // dU
       return RSD_OK;
     };
     // a = A z
     auto apply_a = [&](const double* z, double* a) -> int {
-      gm_u0<<<nblk(n), 256, 0, s>>>(P, n, z + n, dv); RSD_LAUNCH_NOTE();  // [zU; 0]
-      gm_neg<<<nblk(n), 256, 0, s>>>(n, dv, a); RSD_LAUNCH_NOTE();
+      pdl_launch(gm_u0, nblk(n), 256, 0, s, P, n, z + n, dv);  // [zU; 0]
+      pdl_launch(gm_neg, nblk(n), 256, 0, s, n, dv, a);
       RSD_TRY(symv_add(z, a));  // M zf - [zU; 0]
       if (lub) {
         RSD_TRY(rsd_lub_spmv(ctx, lub, 1, dv, n, Lz, n));
-        gm_a2<<<nblk(P), 256, 0, s>>>(P, z, Lz, a + n); RSD_LAUNCH_NOTE();
+        pdl_launch(gm_a2, nblk(P), 256, 0, s, P, z, Lz, a + n);
       } else {
         RSD_CUDA(ctx, cudaMemcpyAsync(a + n, z, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
       }
@@ -697,7 +722,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     // |b_c|: b = ([0; -EIN], Fe_c)
     std::vector<double> bnorm(nr);
     {
-      it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();  // b part only is used
+      pdl_launch(it_residual, dim3(IT_BLOCKS, nr), 256, 0, s, d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm);  // b part only is used
       RSD_TRY(read_status());
       for (int c = 0; c < nr; c++) {
         double b2 = 0.0;
@@ -712,7 +737,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
       double rel = 0.0;
       for (int cycle = 0;; cycle++) {
         RSD_TRY(residual(c, Vb));
-        gm_nrm2<<<1, 256, 0, s>>>(len, Vb, dn); RSD_LAUNCH_NOTE();
+        pdl_launch(gm_nrm2, 1, 256, 0, s, len, Vb, dn);
         double beta2 = 0.0;
         int herr = 0;
         RSD_CUDA(ctx, cudaMemcpyAsync(&beta2, dn, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -723,7 +748,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
         rel = beta / bnorm[c];
         if (!std::isfinite(rel)) return rsd_fail(ctx, RSD_ENAN, "refinement residual is not finite");
         if (rel <= tol || total_it >= gm_maxit) break;
-        gm_scale<<<nblk(len), 256, 0, s>>>(len, Vb, dn, Vb); RSD_LAUNCH_NOTE();
+        pdl_launch(gm_scale, nblk(len), 256, 0, s, len, Vb, dn, Vb);
         std::fill(g.begin(), g.end(), 0.0);
         g[0] = beta;
         int j = 0;
@@ -737,16 +762,16 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
           // classical Gram-Schmidt, twice
           RSD_CUDA(ctx, cudaMemsetAsync(hacc, 0, sizeof(double) * (j + 1), s));
           for (int pass = 0; pass < 2; pass++) {
-            gm_dots<<<j + 1, 256, 0, s>>>(len, j + 1, Vb, len, vn, hbuf); RSD_LAUNCH_NOTE();
-            gm_orth<<<nblk(len), 256, 0, s>>>(len, j + 1, Vb, len, hbuf, vn, hacc); RSD_LAUNCH_NOTE();
+            pdl_launch(gm_dots, j + 1, 256, 0, s, len, j + 1, Vb, len, vn, hbuf);
+            pdl_launch(gm_orth, nblk(len), 256, 0, s, len, j + 1, Vb, len, hbuf, vn, hacc);
           }
-          gm_nrm2<<<1, 256, 0, s>>>(len, vn, dn); RSD_LAUNCH_NOTE();
+          pdl_launch(gm_nrm2, 1, 256, 0, s, len, vn, dn);
           RSD_CUDA(ctx, cudaMemcpyAsync(hh.data(), hacc, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, s));
           RSD_CUDA(ctx, cudaMemcpyAsync(hh.data() + j + 1, dn, sizeof(double), cudaMemcpyDeviceToHost, s));
           RSD_CUDA(ctx, cudaStreamSynchronize(s));
           const double hn = sqrt(hh[j + 1]);
           if (hn > 0.0) {
-            gm_scale<<<nblk(len), 256, 0, s>>>(len, vn, dn, vn); RSD_LAUNCH_NOTE();
+            pdl_launch(gm_scale, nblk(len), 256, 0, s, len, vn, dn, vn);
           }
           // Givens rotations on column j of H
           double* Hj = H.data() + (size_t)j * (m + 1);
@@ -777,8 +802,8 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
         }
         RSD_CUDA(ctx, cudaMemcpyAsync(hbuf, yv.data(), sizeof(double) * j, cudaMemcpyHostToDevice, s));
         // x = (f_c, U_c) is not contiguous: update the two parts
-        gm_update<<<nblk(n), 256, 0, s>>>(n, j, Zb, len, hbuf, f + (size_t)c * n); RSD_LAUNCH_NOTE();
-        gm_update<<<nblk(P), 256, 0, s>>>(P, j, Zb + n, len, hbuf, U + (size_t)c * P); RSD_LAUNCH_NOTE();
+        pdl_launch(gm_update, nblk(n), 256, 0, s, n, j, Zb, len, hbuf, f + (size_t)c * n);
+        pdl_launch(gm_update, nblk(P), 256, 0, s, P, j, Zb + n, len, hbuf, U + (size_t)c * P);
       }
       worst = fmax(worst, rel);
     }
@@ -793,7 +818,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     int its = 0;
     double res = 0.0;
     RSD_TRY(run_gmres(maxit, &its, &res));
-    outputs<<<nblk(P), 256, 0, s>>>(P, Q, nr - 1, f, Lw, U, U_par, S_hyd); RSD_LAUNCH_NOTE();
+    pdl_launch(outputs, nblk(P), 256, 0, s, P, Q, nr - 1, f, Lw, U, U_par, S_hyd);
     RSD_CUDA(ctx, cudaGetLastError());
     info->iterations = its;
     info->residual = res;
@@ -801,28 +826,27 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
       return rsd_fail(ctx, RSD_ENOCONV, "refinement did not converge: residual %.3e after %d iterations", res, its);
     return RSD_OK;
   }
-  RSD_CUDA(ctx, cudaMemsetAsync(f, 0, sizeof(double) * nr * n, s));
-  RSD_CUDA(ctx, cudaMemsetAsync(U, 0, sizeof(double) * nr * P, s));
+  RSD_CUDA(ctx, cudaMemsetAsync(f, 0, sizeof(double) * nr * (n + P), s));  // and U, behind it
   double worst = 0.0, best_res = INFINITY;
   int it = 0;
   std::vector<double> hist;
   for (;; it++) {
-    it_begin<<<nblk(n * nr), 256, 0, s>>>(P, Q, nr, U, ein, f, w, r1, fs); RSD_LAUNCH_NOTE();
+    pdl_launch(it_begin, nblk(n * nr), 256, 0, s, P, Q, nr, U, ein, f, w, r1, fs);
     // r1 -= M f, double-single products of the two planes, both right-hand
     // sides in one pass over the stored half of M
     double* pcol = gpart + (size_t)nbt * nbt * SYMV_T * nr;
     if (nr == 2) {
-      symv_planes_part<2><<<dim3(nbt, nbt), 256, symv_smem(2), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
+      pdl_launch(symv_planes_part<2>, dim3(nbt, nbt), 256, symv_smem(2), s, nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol);
     } else {
-      symv_planes_part<1><<<dim3(nbt, nbt), 256, symv_smem(1), s>>>(nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol); RSD_LAUNCH_NOTE();
+      pdl_launch(symv_planes_part<1>, dim3(nbt, nbt), 256, symv_smem(1), s, nn, (int)n, Mh, Ml, ld, fs, nbt, gpart, pcol);
     }
-    symv_planes_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((int)n, nr, nbt, gpart, pcol, -1.0, r1, n); RSD_LAUNCH_NOTE();
+    pdl_launch(symv_planes_reduce, (unsigned)((n + 255) / 256), 256, 0, s, (int)n, nr, nbt, gpart, pcol, -1.0, r1, n);
     if (lub) {
       RSD_TRY(rsd_lub_spmv(ctx, lub, nr, w, n, Lw, n));
     } else {
       RSD_CUDA(ctx, cudaMemsetAsync(Lw, 0, sizeof(double) * nr * n, s));
     }
-    it_residual<<<dim3(IT_BLOCKS, nr), 256, 0, s>>>(d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm); RSD_LAUNCH_NOTE();
+    pdl_launch(it_residual, dim3(IT_BLOCKS, nr), 256, 0, s, d, r1, ein, Fe, have_fe, f, Lw, r2, t32, nrm);
     RSD_TRY(read_status());
     if (ctx->h_info[24]) return rsd_fail(ctx, RSD_ETIMEOUT, "refinement: a triangular sweep's wait timed out");
     worst = 0.0;
@@ -850,11 +874,11 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     hist.push_back(worst);
     if (it >= 2 && worst <= 100.0 * tol && worst > 0.5 * fmin(hist[it - 1], hist[it - 2])) break;
     RSD_TRY(solve_m(t32, nr, x32, 0));  // y = M^-1 r1
-    it_velocity<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, x32, r2, y, u32); RSD_LAUNCH_NOTE();
+    pdl_launch(it_velocity, nblk(d.np * nr), 256, 0, s, d, nr, x32, r2, y, u32);
     RSD_TRY(solve_r(u32, nr, du32));    // dU = RPP^-1 (r2 - y_P)
-    it_force<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, du32, t32); RSD_LAUNCH_NOTE();
+    pdl_launch(it_force, nblk(d.np * nr), 256, 0, s, d, nr, du32, t32);
     RSD_TRY(solve_m(t32, nr, x32, (int)d.Qp));
-    it_update<<<nblk(d.np * nr), 256, 0, s>>>(d, nr, x32, y, du32, f, U); RSD_LAUNCH_NOTE();  // df = y + M^-1 [dU; 0]
+    pdl_launch(it_update, nblk(d.np * nr), 256, 0, s, d, nr, x32, y, du32, f, U);  // df = y + M^-1 [dU; 0]
   }
   if (!(worst <= accept)) {
     // diverged or stalled above the band: flexible GMRES from zero over the
@@ -867,7 +891,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     worst = res;
     info->fallback = 1;
   }
-  outputs<<<nblk(P), 256, 0, s>>>(P, Q, nr - 1, f, Lw, U, U_par, S_hyd); RSD_LAUNCH_NOTE();
+  pdl_launch(outputs, nblk(P), 256, 0, s, P, Q, nr - 1, f, Lw, U, U_par, S_hyd);
   RSD_CUDA(ctx, cudaGetLastError());
   info->iterations = it;
   info->residual = worst;

@@ -13,6 +13,7 @@
 // blocks of U'.
 #include <cuda_runtime.h>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 template <typename T>
@@ -34,6 +35,7 @@ constexpr int R64_BLOCK = 64;
 // PQ block transposed through shared memory.
 __global__ void permute_qp(int N, int64_t Qp, int64_t np, const double* __restrict__ M, int64_t ld,
                            double* __restrict__ Mp) {
+  pdl_enter();
   __shared__ double T[32][33];
   const int64_t I0 = (int64_t)blockIdx.x * 32, J0 = (int64_t)blockIdx.y * 32, P = 6LL * N, Q = 5LL * N;
   if (I0 > J0) return;
@@ -62,6 +64,7 @@ __global__ void permute_qp(int N, int64_t Qp, int64_t np, const double* __restri
 }
 
 __global__ void copy_upper64(int64_t n, const double* __restrict__ S, int64_t lds, double* __restrict__ D) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n * n) return;
   const int64_t i = t % n, j = t / n;
@@ -70,17 +73,20 @@ __global__ void copy_upper64(int64_t n, const double* __restrict__ S, int64_t ld
 
 // x = [e; 0] of length Qp
 __global__ void pad_q(int64_t Q, int64_t Qp, const double* __restrict__ e, double* __restrict__ x) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < Qp) x[i] = i < Q ? e[i] : 0.0;
 }
 
 __global__ void axpy64(int64_t n, double a, const double* __restrict__ x, double* __restrict__ y) {
+  pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
 }
 
 // S(i, r) = -X(i, r), i < Q
 __global__ void negate_q(int64_t Q, int64_t Qp, int nr, const double* __restrict__ X, double* __restrict__ S) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < Q * nr) S[t] = -X[t % Q + (t / Q) * Qp];
 }
@@ -103,7 +109,7 @@ int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int*
   if (!h->Mp || !h->Ai) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;
   const unsigned nt = (unsigned)((h->np + 31) / 32);
-  permute_qp<<<dim3(nt, nt), dim3(32, 8), 0, s>>>(nn, h->Qp, h->np, M, ld, h->Mp); RSD_LAUNCH_NOTE();
+  pdl_launch(permute_qp, dim3(nt, nt), dim3(32, 8), 0, s, nn, h->Qp, h->np, M, ld, h->Mp);
   int inf = 0;
   RSD_TRY(rsd_potrf_upper_tag(ctx, (int)h->np, h->Mp, h->np, &inf, "mob"));
   if (inf) {
@@ -114,7 +120,7 @@ int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int*
   }
   *info = 0;
   RSD_TRY(rsd_potrf64_factor(ctx, (int)h->np, "mob", &h->f));
-  copy_upper64<<<blocks(P * P), 256, 0, s>>>(P, h->Mp + h->Qp * (h->np + 1), h->np, h->Ai); RSD_LAUNCH_NOTE();
+  pdl_launch(copy_upper64, blocks(P * P), 256, 0, s, P, h->Mp + h->Qp * (h->np + 1), h->np, h->Ai);
   const rsd_factor64 fp{h->f.W + (size_t)(h->Qp / R64_BLOCK) * R64_BLOCK * R64_BLOCK, h->f.dexp + h->Qp};
   RSD_TRY(rsd_potri64(ctx, (int)P, h->Ai, P, fp));
   return rsd_mirror_upper(ctx, (int)P, h->Ai, P);
@@ -126,7 +132,7 @@ int rsd_r64_pq(rsd_ctx* ctx, rsd_r64* h, const double* ein, double* f0) {
   if (!w) return RSD_ENOMEM;
   h->z = w;
   double *x = w + h->Qp, *v = x + h->Qp;
-  pad_q<<<blocks(h->Qp), 256, 0, ctx->stream>>>(h->Q, h->Qp, ein, x); RSD_LAUNCH_NOTE();
+  pdl_launch(pad_q, blocks(h->Qp), 256, 0, ctx->stream, h->Q, h->Qp, ein, x);
   RSD_TRY(rsd_trsv64_fwd(ctx, (int)h->Qp, h->Mp, h->np, h->f.W, x, h->z, h->Qp, 1));
   RSD_TRY(rsd_gemv<double>(ctx, 1, (int)h->P, (int)h->Qp, 1.0, h->Mp + h->Qp * h->np, h->np, h->z, h->Qp, 1, 0.0, v,
                            h->P));
@@ -141,12 +147,12 @@ int rsd_r64_stresslet(rsd_ctx* ctx, rsd_r64* h, const double* Y, int nr, const d
   cudaStream_t s = ctx->stream;
   double *u = w + nr * h->P, *x = u + nr * h->Qp;
   RSD_TRY(rsd_gemv<double>(ctx, 1, (int)h->P, (int)h->P, 1.0, h->Ai, h->P, Y, h->P, nr, 0.0, w, h->P));
-  axpy64<<<blocks(h->P), 256, 0, s>>>(h->P, -1.0, f0, w); RSD_LAUNCH_NOTE();
+  pdl_launch(axpy64, blocks(h->P), 256, 0, s, h->P, -1.0, f0, w);
   RSD_TRY(rsd_gemv<double>(ctx, 0, (int)h->Qp, (int)h->P, 1.0, h->Mp + h->Qp * h->np, h->np, w, h->P, nr, 0.0, u,
                            h->Qp));
-  axpy64<<<blocks(h->Qp), 256, 0, s>>>(h->Qp, 1.0, h->z, u); RSD_LAUNCH_NOTE();
+  pdl_launch(axpy64, blocks(h->Qp), 256, 0, s, h->Qp, 1.0, h->z, u);
   RSD_TRY(rsd_trsv64_bwd(ctx, (int)h->Qp, h->Mp, h->np, h->f.W, u, x, h->Qp, nr));
-  negate_q<<<blocks(h->Q * nr), 256, 0, s>>>(h->Q, h->Qp, nr, x, S); RSD_LAUNCH_NOTE();
+  pdl_launch(negate_q, blocks(h->Q * nr), 256, 0, s, h->Q, h->Qp, nr, x, S);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }

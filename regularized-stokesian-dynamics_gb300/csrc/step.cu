@@ -9,12 +9,14 @@
 #include <cstring>
 #include <vector>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 
 namespace {
 
 __global__ void axpy_block_k(int64_t rows, int64_t cols, double alpha, const double* __restrict__ B, int64_t ldb,
                              double* __restrict__ A, int64_t lda) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= rows * cols) return;
   const int64_t i = t % rows, j = t / rows;
@@ -27,6 +29,7 @@ struct ein5 {
 // EIN of every particle, and Fe (zero without d_Fe)
 __global__ void fill_inputs(int nn, ein5 e, const double* __restrict__ d_Fe, double* __restrict__ ein,
                             double* __restrict__ Fe) {
+  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 5 * nn) ein[t] = e.v[t % 5];
   if (t < 6 * nn) Fe[t] = d_Fe ? d_Fe[t] : 0.0;
@@ -38,6 +41,7 @@ __global__ void fill_inputs(int nn, ein5 e, const double* __restrict__ d_Fe, dou
 // particle <= column particle stored); null for FP64 M
 __global__ void sum_app_xx(int nn, const double* __restrict__ M, const float* __restrict__ Mh,
                            const float* __restrict__ Ml, int64_t ld, double* __restrict__ out) {
+  pdl_enter();
   __shared__ double red[256];
   double s = 0.0;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)nn * nn;
@@ -89,6 +93,7 @@ __device__ inline void period_correction(double R[3], const bg_flow& f) {
 // with the wrapped positions.
 __global__ void euler_update(int nn, int nb, bg_flow f, const double* __restrict__ U_par, double* __restrict__ conf,
                              double* __restrict__ U_pos) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nn) return;
   double x[3] = {conf[3 * i], conf[3 * i + 1], conf[3 * i + 2]};
@@ -109,6 +114,7 @@ __global__ void euler_update(int nn, int nb, bg_flow f, const double* __restrict
 // S(5i+3) / (-2 EIN(5i+3))
 __global__ void yeta_sums(int nn, const double* __restrict__ Sh, const double* __restrict__ Sfp,
                           const double* __restrict__ Sb, const double* __restrict__ ein, double* __restrict__ out) {
+  pdl_enter();
   __shared__ double r0[256], r1[256], r2[256];
   double a = 0, b = 0, c = 0;
   for (int i = threadIdx.x; i < nn; i += blockDim.x) {
@@ -138,6 +144,7 @@ __global__ void yeta_sums(int nn, const double* __restrict__ Sh, const double* _
 }
 
 __global__ void nan_check(int64_t n, const double* __restrict__ v, int* __restrict__ flag) {
+  pdl_enter();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n && !isfinite(v[t])) atomicExch(flag, 1);
 }
@@ -148,7 +155,7 @@ int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, in
                    double alpha) {
   const int64_t tot = rows * cols;
   if (tot <= 0) return RSD_OK;
-  axpy_block_k<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(rows, cols, alpha, B, ldb, A, lda); RSD_LAUNCH_NOTE();
+  pdl_launch(axpy_block_k, (unsigned)((tot + 255) / 256), 256, 0, ctx->stream, rows, cols, alpha, B, ldb, A, lda);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -250,7 +257,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   ei5_of(Eij, ei5.v);
   double* sums = rsd_sums(ctx->d_info);
   double* red = sums + 128;    // 256 partial sums, then yeta's three
-  fill_inputs<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(nn, ei5, d_Fe, ein, Fe); RSD_LAUNCH_NOTE();
+  pdl_launch(fill_inputs, (unsigned)((P + 255) / 256), 256, 0, s, nn, ei5, d_Fe, ein, Fe);
   cudaEventRecord(ctx->ev[0], s);
   // The lubrication operator needs positions and radii only: it is built on a
   // side stream beside the mobility's pair sums (~190 us of small kernels and
@@ -281,7 +288,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   // averageU on APP before it is overwritten
   const bool planes = p->precision == RSD_PREC_MIXED;
   const float* Mh = planes ? reinterpret_cast<const float*>(M) : nullptr;
-  sum_app_xx<<<256, 256, 0, s>>>(nn, M, Mh, planes ? Mh + (size_t)ldm * n : nullptr, ldm, red); RSD_LAUNCH_NOTE();
+  pdl_launch(sum_app_xx, 256, 256, 0, s, nn, M, Mh, planes ? Mh + (size_t)ldm * n : nullptr, ldm, red);
   int info_m = 0;
   if (p->precision == RSD_PREC_FP64) {
     // MobToResist_FTS: R_inf = M^-1 through the Schur complement (resist64.cu)
@@ -380,12 +387,12 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   f.T = p->T;
   f.dt = p->dt;
   f.gamma = p->gamma;
-  euler_update<<<(nn + 127) / 128, 128, 0, s>>>(nn, p->nb, f, Upar, d_conf, d_U_pos); RSD_LAUNCH_NOTE();
+  pdl_launch(euler_update, (nn + 127) / 128, 128, 0, s, nn, p->nb, f, Upar, d_conf, d_U_pos);
   RSD_CUDA(ctx, cudaMemcpyAsync(d_SijN, S, sizeof(double) * Q, cudaMemcpyDeviceToDevice, s));
-  yeta_sums<<<1, 256, 0, s>>>(nn, S, nullptr, nullptr, ein, red + 256); RSD_LAUNCH_NOTE();
+  pdl_launch(yeta_sums, 1, 256, 0, s, nn, S, nullptr, nullptr, ein, red + 256);
   int* flag = ctx->d_info + 8;
   RSD_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int), s));
-  nan_check<<<(unsigned)((6 * nn + 255) / 256), 256, 0, s>>>(6LL * nn, d_U_pos, flag); RSD_LAUNCH_NOTE();
+  pdl_launch(nan_check, (unsigned)((6 * nn + 255) / 256), 256, 0, s, 6LL * nn, d_U_pos, flag);
   cudaEventRecord(ctx->ev[5], s);
   // one copy for the status words and the sums, one for a host caller's results
   RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, RSD_INFO_BYTES, cudaMemcpyDeviceToHost, s));

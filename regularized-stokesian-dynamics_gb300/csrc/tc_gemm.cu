@@ -32,6 +32,7 @@
 
 #include <cstring>
 
+#include "pdl.cuh"
 #include "rsd_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcCfg<PREC>::MIN_CTAS)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
+  pdl_enter();  // the barriers and the tensor memory are set up by now
   const uint32_t taddr = *tslot;
 
   if (warp == 0) {
@@ -374,11 +376,10 @@ int rsd_tc_gemm(rsd_ctx* ctx, int prec, int m, int n, int K, float alpha, const 
   const dim3 grid((m + TC_TILE - 1) / TC_TILE, (n + TC_TILE - 1) / TC_TILE, ksplit > 0 ? (K + ksplit - 1) / ksplit : 1);
   cudaStream_t st = stream ? stream : ctx->stream;
   if (prec == 1) {
-    tc_gemm_kernel<1><<<grid, TC_THREADS, TcCfg<1>::SMEM, st>>>(tmA, tmB, tmC, a);
+    pdl_launch(tc_gemm_kernel<1>, grid, TC_THREADS, TcCfg<1>::SMEM, st, tmA, tmB, tmC, a);
   } else {
-    tc_gemm_kernel<3><<<grid, TC_THREADS, TcCfg<3>::SMEM, st>>>(tmA, tmB, tmC, a);
+    pdl_launch(tc_gemm_kernel<3>, grid, TC_THREADS, TcCfg<3>::SMEM, st, tmA, tmB, tmC, a);
   }
-  RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
@@ -402,11 +403,10 @@ int rsd_tc_gemm_zbatch(rsd_ctx* ctx, int prec, int m, int n, int K, float alpha,
   TcArgs a{K, 0, 0, 0, 0, alpha, d_err, wait_limit(ctx), zak, zam, zbk, zbn, zcm, zcn, n, ndec};
   const dim3 grid((m + TC_TILE - 1) / TC_TILE, (n + TC_TILE - 1) / TC_TILE, nbatch);
   if (prec == 1) {
-    tc_gemm_kernel<1><<<grid, TC_THREADS, TcCfg<1>::SMEM, ctx->stream>>>(tmA, tmB, tmC, a);
+    pdl_launch(tc_gemm_kernel<1>, grid, TC_THREADS, TcCfg<1>::SMEM, ctx->stream, tmA, tmB, tmC, a);
   } else {
-    tc_gemm_kernel<3><<<grid, TC_THREADS, TcCfg<3>::SMEM, ctx->stream>>>(tmA, tmB, tmC, a);
+    pdl_launch(tc_gemm_kernel<3>, grid, TC_THREADS, TcCfg<3>::SMEM, ctx->stream, tmA, tmB, tmC, a);
   }
-  RSD_LAUNCH_NOTE();
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
