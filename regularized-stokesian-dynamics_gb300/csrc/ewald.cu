@@ -641,11 +641,23 @@ __device__ __forceinline__ void kblock_stage(int nn, int h0, int kc, const float
 // The blocks are written (add = 0) or added (add = 1) once.  Bound by FP32
 // issue at 8 warps per SM (accumulators in registers); the packed form halves
 // the instructions: N = 2048 10.4 -> 8.1 ms, N = 512 0.74 -> 0.56 ms.
+// SLICED: slice blockIdx.z of each list is summed, into part (see
+// ewald_join_slices).
+template <bool SLICED>
 __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const float* __restrict__ W32,
                                                          const float2* __restrict__ c32, int K64,
                                                          const float* __restrict__ W64, const float4* __restrict__ c64,
-                                                         PlaneSink sk, int add) {
+                                                         PlaneSink sk, int add, float2* __restrict__ part) {
   pdl_enter();
+  if (SLICED) {
+    const int z = blockIdx.z, S = gridDim.z, f = K32 * z / S, g = K64 * z / S;
+    K32 = K32 * (z + 1) / S - f;
+    W32 += (size_t)f * KBW;
+    c32 += (size_t)f * nn;
+    K64 = K64 * (z + 1) / S - g;
+    W64 += (size_t)g * 2 * KBW;
+    c64 += (size_t)g * nn;
+  }
   constexpr int KC = 16;
   __shared__ __align__(16) float sw[KC * 2 * KBW];  // the FP32 phase uses the first half
   __shared__ __align__(16) float4 sca[KC * 32], scb[KC * 4];
@@ -738,7 +750,14 @@ __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const 
     f2_unpack(s, o[2 * p].hi, o[2 * p + 1].hi);
     f2_unpack(l, o[2 * p].lo, o[2 * p + 1].lo);
   }
-  store_pair_rows_a(sk, nn, a, b, o, add);
+  if (SLICED) {
+    const int64_t np = (int64_t)nn * (nn - 1) / 2;
+    part += (int64_t)blockIdx.z * 60 * np + (int64_t)b * (b - 1) / 2 + a;
+#pragma unroll
+    for (int q = 0; q < 60; q++) part[q * np] = make_float2(o[q].hi, o[q].lo);
+  } else {
+    store_pair_rows_a(sk, nn, a, b, o, add);
+  }
 }
 
 // Near/far split of the real-space images for the mixed form.  Image nz of
@@ -908,10 +927,10 @@ __device__ __forceinline__ void column_base_f(const float* Rf, const float* A, i
 
 // Lists the next images of the set (near: r2 < rc2; far: rc2 <= r2 < rmax2)
 // from the resumable position (col, nz) into list[.][t], at most REAL_CAP;
-// returns the count.
+// takes every step-th column; returns the count.
 template <bool NEAR>
-__device__ __forceinline__ int list_images(RealEqShared& sh, int t, const float* Rf, const float* A, int NR, int& col,
-                                           int& nz, float rc2, float rmax2) {
+__device__ __forceinline__ int list_images(int (*list)[REAL_THREADS], int t, const float* Rf, const float* A, int NR,
+                                           int& col, int& nz, int step, float rc2, float rmax2) {
   const int w = 2 * NR + 1, ncol = w * w;
   int cnt = 0, nx = 0, ny = 0;
   float p[3];
@@ -925,10 +944,10 @@ __device__ __forceinline__ int list_images(RealEqShared& sh, int t, const float*
     }
     float y0, y1, y2;
     const float r2 = image_r2f(p[0], p[1], p[2], A[6], A[7], A[8], nz, &y0, &y1, &y2);
-    if (NEAR ? (r2 < rc2) : (r2 >= rc2 && r2 < rmax2)) sh.list[cnt++][t] = pack_image(nx, ny, nz, NR);
+    if (NEAR ? (r2 < rc2) : (r2 >= rc2 && r2 < rmax2)) list[cnt++][t] = pack_image(nx, ny, nz, NR);
     if (++nz > NR) {
       nz = -NR;
-      col++;
+      col += step;
       base = false;
     }
   }
@@ -936,19 +955,18 @@ __device__ __forceinline__ int list_images(RealEqShared& sh, int t, const float*
 }
 
 // The near images' moments of part P (of NP, rsd_mom_part): one pass over
-// the near set, then that part's share of every output added into the pair
-// block held in shared memory (oh + ol).
+// the near set of the columns col, col + step, ..., into acc (normalised).
 template <int NP, int P>
-__device__ __forceinline__ void near_part(RealEqShared& sh, int t, const float* Rf, const float* A, const dsf* Rs,
-                                          const dsf* As, int NR, float rc2, dsf lam_s, dsf cd_s) {
-  dsacc acc[RSD_NMOM_REAL];
+__device__ __forceinline__ void near_moments(const dsf_tables& T, int (*list)[REAL_THREADS], int t, const float* Rf,
+                                             const float* A, const dsf* Rs, const dsf* As, int NR, float rc2,
+                                             dsf lam_s, dsf cd_s, int col, int step, dsacc* acc) {
 #pragma unroll
   for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = dsacc(0);
-  int col = 0, nz = -NR;
+  int nz = -NR;
   do {
-    const int cnt = list_images<true>(sh, t, Rf, A, NR, col, nz, rc2, 0.f);
+    const int cnt = list_images<true>(list, t, Rf, A, NR, col, nz, step, rc2, 0.f);
     for (int q = 0; q < cnt; q++) {
-      const int e = sh.list[q][t];
+      const int e = list[q][t];
       const int ix = (e & 255) - NR, iy = ((e >> 8) & 255) - NR, iz = (e >> 16) - NR;
       const dsf x0 = Rs[0] + ix * As[0] + iy * As[3] + iz * As[6];
       const dsf x1 = Rs[1] + ix * As[1] + iy * As[4] + iz * As[7];
@@ -956,7 +974,7 @@ __device__ __forceinline__ void near_part(RealEqShared& sh, int t, const float* 
       const dsf r = dsf_sqrt(x0 * x0 + x1 * x1 + x2 * x2);
       const dsf ir = dsf_rcp(r);
       dsf E0, G;
-      dsf_erfc_gauss(lam_s * r, sh.T, &E0, &G);
+      dsf_erfc_gauss(lam_s * r, T, &E0, &G);
       rsd_real_image<dsf, dsacc, NP, P>(x0, x1, x2, r, ir, E0, cd_s * G, lam_s, acc);
       if ((q & 3) == 3) {  // keep the accumulators' lo parts small
 #pragma unroll
@@ -966,6 +984,37 @@ __device__ __forceinline__ void near_part(RealEqShared& sh, int t, const float* 
 #pragma unroll
     for (int m = 0; m < RSD_NMOM_REAL; m++) dsacc_norm(acc[m]);
   } while (col < (2 * NR + 1) * (2 * NR + 1));
+}
+
+// The same for the far images, in FP32.
+__device__ __forceinline__ void far_moments(int (*list)[REAL_THREADS], int t, const float* Rf, const float* A, int NR,
+                                            float rc2, float rmax2, float lamf, float cdf, int col, int step,
+                                            float* acc) {
+  const float lam2f = lamf * lamf;
+#pragma unroll
+  for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.f;
+  int nz = -NR;
+  do {
+    const int cnt = list_images<false>(list, t, Rf, A, NR, col, nz, step, rc2, rmax2);
+    for (int q = 0; q < cnt; q++) {
+      const int e = list[q][t];
+      const int ix = (e & 255) - NR, iy = ((e >> 8) & 255) - NR, iz = (e >> 16) - NR;
+      float p[3], x0, x1, x2;
+      column_base_f(Rf, A, ix, iy, p);
+      const float r2 = image_r2f(p[0], p[1], p[2], A[6], A[7], A[8], iz, &x0, &x1, &x2);
+      const float r = sqrtf(r2), ir = 1.f / r;
+      rsd_real_image<float>(x0, x1, x2, r, ir, erfcf(lamf * r), cdf * expf(-r2 * lam2f), lamf, acc);
+    }
+  } while (col < (2 * NR + 1) * (2 * NR + 1));
+}
+
+// Part P's share of every output, added into the pair block held in shared
+// memory (oh + ol).
+template <int NP, int P>
+__device__ __forceinline__ void near_part(RealEqShared& sh, int t, const float* Rf, const float* A, const dsf* Rs,
+                                          const dsf* As, int NR, float rc2, dsf lam_s, dsf cd_s) {
+  dsacc acc[RSD_NMOM_REAL];
+  near_moments<NP, P>(sh.T, sh.list, t, Rf, A, Rs, As, NR, rc2, lam_s, cd_s, 0, 1, acc);
   dsf accn[RSD_NMOM_REAL];
 #pragma unroll
   for (int m = 0; m < RSD_NMOM_REAL; m++) accn[m] = dsf(acc[m].hi, acc[m].lo);
@@ -985,6 +1034,32 @@ __device__ __forceinline__ void near_parts(RealEqShared& sh, int t, const float*
   if constexpr (P < NP) {
     near_part<NP, P>(sh, t, Rf, A, Rs, As, NR, rc2, lam_s, cd_s);
     near_parts<NP, P + 1>(sh, t, Rf, A, Rs, As, NR, rc2, lam_s, cd_s);
+  }
+}
+
+// The lattice and the minimum image of pair (a, b): the shift found in FP32,
+// applied in double-single.
+struct RealPair {
+  float A[9], Rf[3];
+  dsf As[9], Rs[3];
+};
+__device__ __forceinline__ void real_pair(const rsd_lat_dev& L, const double* __restrict__ pos, int a, int b,
+                                          RealPair& g) {
+  float LIf[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    g.As[k] = dsf_from(L.LR[k]);
+    g.A[k] = g.As[k].hi;
+    LIf[k] = (float)L.LI[k];
+  }
+  const double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
+  const float R0[3] = {(float)R[0], (float)R[1], (float)R[2]};
+  int k[3];
+  rsd_skew_shift_f32(g.A, LIf, R0, k);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    g.Rs[i] = dsf_from(R[i]) - (k[0] * g.As[i] + k[1] * g.As[3 + i] + k[2] * g.As[6 + i]);
+    g.Rf[i] = g.Rs[i].hi;
   }
 }
 
@@ -1011,45 +1086,12 @@ __global__ void __launch_bounds__(REAL_THREADS, MINB) ewald_pair_real_eq(int nn,
   __syncthreads();
   int a, b;
   if (!pair_of(nn, &a, &b)) return;
-  float A[9], LIf[9];
-  dsf As[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    As[k] = dsf_from(L.LR[k]);
-    A[k] = As[k].hi;
-    LIf[k] = (float)L.LI[k];
-  }
-  // minimum image: the lattice shift found in FP32, applied in double-single
-  const double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
-  dsf Rs[3];
-  {
-    const float R0[3] = {(float)R[0], (float)R[1], (float)R[2]};
-    int k[3];
-    rsd_skew_shift_f32(A, LIf, R0, k);
-#pragma unroll
-    for (int i = 0; i < 3; i++) Rs[i] = dsf_from(R[i]) - (k[0] * As[i] + k[1] * As[3 + i] + k[2] * As[6 + i]);
-  }
-  const float Rf[3] = {Rs[0].hi, Rs[1].hi, Rs[2].hi};
+  RealPair g;
+  real_pair(L, pos, a, b, g);
   const int NR = L.NR;
-  const float lamf = (float)L.lam, lam2f = lamf * lamf, cdf = (float)(2.0 * RSD_PIP5 * L.lam);
-  // far images, FP32
   {
     float acc[RSD_NMOM_REAL];
-#pragma unroll
-    for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.f;
-    int col = 0, nz = -NR;
-    do {
-      const int cnt = list_images<false>(sh, t, Rf, A, NR, col, nz, rc2, rmax2);
-      for (int q = 0; q < cnt; q++) {
-        const int e = sh.list[q][t];
-        const int ix = (e & 255) - NR, iy = ((e >> 8) & 255) - NR, iz = (e >> 16) - NR;
-        float p[3], x0, x1, x2;
-        column_base_f(Rf, A, ix, iy, p);
-        const float r2 = image_r2f(p[0], p[1], p[2], A[6], A[7], A[8], iz, &x0, &x1, &x2);
-        const float r = sqrtf(r2), ir = 1.f / r;
-        rsd_real_image<float>(x0, x1, x2, r, ir, erfcf(lamf * r), cdf * expf(-r2 * lam2f), lamf, acc);
-      }
-    } while (col < (2 * NR + 1) * (2 * NR + 1));
+    far_moments(sh.list, t, g.Rf, g.A, NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
 #pragma unroll
     for (int q = 0; q < 60; q++) {
       sh.oh[q][t] = rsd_real_epi_row<float, float, float>(q, acc, sh.cf);
@@ -1057,7 +1099,7 @@ __global__ void __launch_bounds__(REAL_THREADS, MINB) ewald_pair_real_eq(int nn,
     }
   }
   // near images, double-single, in NP passes
-  near_parts<NP, 0>(sh, t, Rf, A, Rs, As, NR, rc2, dsf_from(L.lam), dsf_from(2.0 * RSD_PIP5 * L.lam));
+  near_parts<NP, 0>(sh, t, g.Rf, g.A, g.Rs, g.As, NR, rc2, dsf_from(L.lam), dsf_from(2.0 * RSD_PIP5 * L.lam));
   dsf v[60];
 #pragma unroll
   for (int q = 0; q < 60; q++) v[q] = dsf(sh.oh[q][t], sh.ol[q][t]);
@@ -1125,7 +1167,8 @@ __device__ __forceinline__ void group_sum(double (&v)[N], int gl, double* dst) {
 }
 
 // Entry (r, c) of the 11 x 11 block (a, b), a < b, from the pair's 60 values.
-__device__ __forceinline__ double pair_block_entry(const double* v, int r, int c) {
+template <typename T>
+__device__ __forceinline__ T pair_block_entry(const T* v, int r, int c) {
   const int rs = r < 3 ? 0 : (r < 6 ? 1 : 2), cs = c < 3 ? 0 : (c < 6 ? 1 : 2);
   const int i = rs == 2 ? r - 6 : r - 3 * rs, j = cs == 2 ? c - 6 : c - 3 * cs;
   if (rs == cs && rs < 2) {  // TT, RR: symmetric 3 x 3 as 00 01 02 11 12 22
@@ -1138,18 +1181,117 @@ __device__ __forceinline__ double pair_block_entry(const double* v, int r, int c
   }
   if (rs < 2 && cs < 2) {  // TR: antisymmetric, odd under a <-> b
     const int t = rs == 0 ? i : j, q = rs == 0 ? j : i;
-    if (t == q) return 0.0;
-    const double x = v[12 + min(t, q) + max(t, q) - 1];
+    if (t == q) return T(0);
+    const T x = v[12 + min(t, q) + max(t, q) - 1];
     return (t < q) == (rs == 0) ? x : -x;
   }
   if (rs < 2) return v[(rs ? 45 : 30) + 5 * i + j];   // G, H
-  const double x = v[(cs ? 45 : 30) + 5 * j + i];
+  const T x = v[(cs ? 45 : 30) + 5 * j + i];
   return cs == 0 ? -x : x;                             // G is odd under a <-> b
 }
 
 // grand-matrix index of component k (0..10) of particle p
 __device__ __forceinline__ int64_t grand_row(int N, int p, int k) {
   return k < 3 ? 3 * p + k : (k < 6 ? 3 * N + 3 * p + k - 3 : 6 * N + 5 * p + k - 6);
+}
+
+// ------------------------------------- equal radii, mixed, a small system
+// Fewer pairs than the GPU holds threads leave the two kernels above waiting
+// on one thread's chain (N = 32: 8 CTAs, 116 and 160 us).  The vectors of a
+// pair and its images are then dealt out over S slices (blockIdx.z: a range of
+// the vectors, every S-th column of images), the two kernels run side by side
+// and write partial sums - the block's 60 values, the 97 moments near
+// (double-single) and far (FP32) - at [slice][value][pair], pair (a, b) at
+// b (b - 1) / 2 + a; the last kernel adds them up in double-single and writes
+// the blocks.  N = 32: 285 -> 90 us from the trig tables to the blocks, N = 173
+// 470 -> 250; against the FP64 step both orders of summation differ by the same
+// 2e-11 to 6e-11 in the velocities (the far images' FP32).
+struct RealSliceShared {
+  dsf_tables T;
+  int list[REAL_CAP][REAL_THREADS];
+};
+
+__global__ void __launch_bounds__(REAL_THREADS, 2) ewald_real_slices(int nn, rsd_lat_dev L,
+                                                                    const double* __restrict__ pos, float rc2,
+                                                                    float rmax2, float2* __restrict__ near,
+                                                                    float* __restrict__ far) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char smraw_real[];
+  RealSliceShared& sh = *reinterpret_cast<RealSliceShared*>(smraw_real);
+  if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
+  const int t = threadIdx.y * blockDim.x + threadIdx.x, z = blockIdx.z, S = gridDim.z;
+  dsf_tables_fill(sh.T, t, REAL_THREADS);
+  __syncthreads();
+  int a, b;
+  if (!pair_of(nn, &a, &b)) return;
+  RealPair g;
+  real_pair(L, pos, a, b, g);
+  const int64_t np = (int64_t)nn * (nn - 1) / 2, o = (int64_t)z * RSD_NMOM_REAL * np + (int64_t)b * (b - 1) / 2 + a;
+  {
+    float acc[RSD_NMOM_REAL];
+    far_moments(sh.list, t, g.Rf, g.A, L.NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), z, S, acc);
+#pragma unroll
+    for (int m = 0; m < RSD_NMOM_REAL; m++) far[o + m * np] = acc[m];
+  }
+  dsacc acc[RSD_NMOM_REAL];
+  near_moments<1, 0>(sh.T, sh.list, t, g.Rf, g.A, g.Rs, g.As, L.NR, rc2, dsf_from(L.lam),
+                     dsf_from(2.0 * RSD_PIP5 * L.lam), z, S, acc);
+#pragma unroll
+  for (int m = 0; m < RSD_NMOM_REAL; m++) near[o + m * np] = make_float2(acc[m].hi, acc[m].lo);
+}
+
+constexpr int JOIN_PAIRS = 16;
+__global__ void __launch_bounds__(256) ewald_join_slices(int nn, int S, const float2* __restrict__ kpart,
+                                                         const float2* __restrict__ near,
+                                                         const float* __restrict__ far, const dsf* __restrict__ cr,
+                                                         const unsigned short* __restrict__ etab, PlaneSink sk) {
+  pdl_enter();
+  __shared__ dsf mom[RSD_NMOM_REAL][JOIN_PAIRS], v[JOIN_PAIRS][61], c[RSD_REAL_EPI_NC];
+  __shared__ unsigned short tab[61 + RSD_REAL_EPI_NC];
+  __shared__ int2 ab[JOIN_PAIRS];
+  const int t = threadIdx.x;
+  const int64_t np = (int64_t)nn * (nn - 1) / 2, p0 = (int64_t)blockIdx.x * JOIN_PAIRS;
+  const int cnt = (int)min((int64_t)JOIN_PAIRS, np - p0);
+  for (int k = t; k < RSD_REAL_EPI_NC; k += 256) c[k] = cr[k];
+  for (int k = t; k < 61 + RSD_REAL_EPI_NC; k += 256) tab[k] = etab[k];
+  if (t < cnt) {
+    int b = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)(p0 + t))) * 0.5f);
+    while ((int64_t)b * (b - 1) / 2 > p0 + t) b--;
+    while ((int64_t)b * (b + 1) / 2 <= p0 + t) b++;
+    ab[t] = make_int2((int)(p0 + t - (int64_t)b * (b - 1) / 2), b);
+  }
+  for (int e = t; e < RSD_NMOM_REAL * JOIN_PAIRS; e += 256) {
+    const int m = e / JOIN_PAIRS, i = e % JOIN_PAIRS;
+    dsf s(0);
+    if (i < cnt)
+      for (int z = 0; z < S; z++) {
+        const int64_t o = ((int64_t)z * RSD_NMOM_REAL + m) * np + p0 + i;
+        const float2 x = near[o];
+        s = s + dsf(x.x, x.y) + dsf(far[o], 0.f);
+      }
+    mom[m][i] = s;
+  }
+  __syncthreads();
+  for (int e = t; e < 60 * JOIN_PAIRS; e += 256) {
+    const int q = e / JOIN_PAIRS, i = e % JOIN_PAIRS;
+    dsf s(0);
+    if (i < cnt)
+      for (int z = 0; z < S; z++) {
+        const float2 x = kpart[((int64_t)z * 60 + q) * np + p0 + i];
+        s = s + dsf(x.x, x.y);
+      }
+    for (int k = tab[q]; k < tab[q + 1]; k++) s = fma(c[k], mom[tab[61 + k]][i], s);
+    v[i][q] = s;
+  }
+  __syncthreads();
+  for (int e = t; e < 121 * JOIN_PAIRS; e += 256) {
+    const int i = e % JOIN_PAIRS, rc = e / JOIN_PAIRS, r = rc % 11, col = rc / 11;
+    if (i >= cnt) continue;
+    const dsf x = pair_block_entry(v[i], r, col);
+    const int64_t o = grand_row(nn, ab[i].x, r) + grand_row(nn, ab[i].y, col) * sk.ld;
+    sk.hi[o] = x.hi;
+    sk.lo[o] = x.lo;
+  }
 }
 
 // cube: every listed image counts, around the exact minimum image of
@@ -1592,6 +1734,47 @@ int launch_real_eq_t(rsd_ctx* ctx, dim3 grd, dim3 blk, int nn, const rsd_lat_dev
   return RSD_OK;
 }
 
+constexpr int EWALD_SLICES = 16;
+struct slice_parts {
+  float2 *k, *near;
+  float* far;
+};
+int slice_buffers(rsd_ctx* ctx, int S, int nn, slice_parts* o) {
+  const size_t np = (size_t)nn * (nn - 1) / 2, nm = (size_t)S * RSD_NMOM_REAL * np;
+  o->k = (float2*)rsd_scratch(ctx, "ewald_slices_k", sizeof(float2) * S * 60 * np);
+  o->near = (float2*)rsd_scratch(ctx, "ewald_slices_near", sizeof(float2) * nm);
+  o->far = (float*)rsd_scratch(ctx, "ewald_slices_far", sizeof(float) * nm);
+  return o->k && o->near && o->far ? RSD_OK : RSD_ENOMEM;
+}
+
+// The images' slices on stream s (the side stream), ctx->ev_panel behind them.
+int real_slices(rsd_ctx* ctx, cudaStream_t s, int S, dim3 grd, dim3 blk, int nn, const rsd_lat_dev& L,
+                const double* d_pos, float rc2, float rmax2) {
+  slice_parts p;
+  RSD_TRY(slice_buffers(ctx, S, nn, &p));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(ewald_real_slices, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(RealSliceShared)));
+  grd.z = S;
+  pdl_launch(ewald_real_slices, grd, blk, sizeof(RealSliceShared), s, nn, L, d_pos, rc2, rmax2, p.near, p.far);
+  RSD_CUDA(ctx, cudaEventRecord(ctx->ev_panel, s));
+  return RSD_OK;
+}
+
+// The vectors' slices, then the blocks from all of them.
+int join_slices(rsd_ctx* ctx, int S, dim3 grd, dim3 blk, int nn, int K32, const float* w32, const float2* c32, int K64,
+                const float* w64, const float4* c64, const dsf* cr, const unsigned short* etab, const PlaneSink& psk) {
+  cudaStream_t s = ctx->stream;
+  slice_parts p;
+  RSD_TRY(slice_buffers(ctx, S, nn, &p));
+  grd.z = S;
+  pdl_launch(ewald_pair_kblock<true>, grd, blk, 0, s, nn, K32, w32, c32, K64, w64, c64, psk, 0, p.k);
+  RSD_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_panel, 0));
+  const int64_t np = (int64_t)nn * (nn - 1) / 2;
+  pdl_launch(ewald_join_slices, (unsigned)((np + JOIN_PAIRS - 1) / JOIN_PAIRS), 256, 0, s, nn, S, p.k, p.near, p.far,
+             cr, etab, psk);
+  return RSD_OK;
+}
+
 int launch_real_eq(rsd_ctx* ctx, int passes, dim3 grd, dim3 blk, int nn, const rsd_lat_dev& L, const double* d_pos,
                    const dsf* cr, const float* cf, float rc2, float rmax2, const PlaneSink& psk) {
   switch (passes) {
@@ -1815,7 +1998,7 @@ int assemble_fp64(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_rad
 }  // namespace
 
 int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
-                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm) {
+                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm, bool exported) {
   if (nn < 1 || ldm < 11LL * nn) return rsd_fail(ctx, RSD_EARG, "bad size nn=%d ldm=%lld", nn, (long long)ldm);
   rsd_lat_dev L = rsd_lat_pack(lat);
   if (precision == RSD_PREC_MIXED) L = mixed_lattice(ctx, L);
@@ -1870,7 +2053,7 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       // one copy: the vector indices and, for equal radii, the coefficients of
       // the real-space epilogue (double-single, FP32)
       const size_t nidx = (h64.size() + h32.size() + 3) / 4 * 4;
-      std::vector<int> up(nidx + 3 * RSD_REAL_EPI_NC, 0);
+      std::vector<int> up(nidx + 3 * RSD_REAL_EPI_NC + (61 + RSD_REAL_EPI_NC + 1) / 2, 0);
       std::copy(h64.begin(), h64.end(), up.begin());
       std::copy(h32.begin(), h32.end(), up.begin() + h64.size());
       if (equal) {
@@ -1884,7 +2067,17 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
           hr[k].hi = hf[k] = h;
           hr[k].lo = (float)(c[k] - (double)h);
         }
+        unsigned short* e = reinterpret_cast<unsigned short*>(hf + RSD_REAL_EPI_NC);
+        for (int q = 0; q < 61; q++) e[q] = (unsigned short)rsd_real_epi_off(q);
+        for (int k = 0; k < RSD_REAL_EPI_NC; k++) e[61 + k] = (unsigned short)rsd_real_epi_mom(k);
       }
+      // Slices of a small system: so many that their CTAs (those above the
+      // diagonal) come to two per SM, what the kernels' registers allow.
+      int ctas = 0;
+      for (unsigned y = 0; y < grd.y; y++) ctas += std::min((4 * (int)y + 3 + 31) / 32, (int)grd.x);
+      const int S = std::min(EWALD_SLICES, 2 * ctx->sm_count / ctas);
+      const bool sliced = equal && !exported && S >= 2;
+      if (sliced) RSD_TRY(real_slices(ctx, beside.side, S, grd, blk, nn, L, d_pos, (float)rc2, (float)rmax2));
       int* dh = (int*)rsd_scratch(ctx, "ewald_hlist", sizeof(int) * up.size());
       double* t64 = equal ? nullptr : (double*)rsd_scratch(ctx, "ewald_ktab64", sizeof(double) * (size_t)(K64 > 0 ? K64 : 1) * KW);
       float* t32 = equal ? nullptr : (float*)rsd_scratch(ctx, "ewald_ktab32", sizeof(float) * (size_t)(K32 > 0 ? K32 : 1) * KW);
@@ -1907,7 +2100,12 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         if (K64 + K32) {
           pdl_launch(ewald_kblock_lists, dim3((K64 + K32 + 31) / 32, 2), 32, 0, s, L, K64, K32, dh, h_radii[0], inv_pimu, w64, w32);
         }
-        pdl_launch(ewald_pair_kblock, grd, blk, 0, s, nn, K32, w32, c32, K64, w64, c64, psk, 0);
+        if (sliced) {
+          RSD_TRY(join_slices(ctx, S, grd, blk, nn, K32, w32, c32, K64, w64, c64, cr,
+                              reinterpret_cast<const unsigned short*>(cf + RSD_REAL_EPI_NC), psk));
+        } else {
+          pdl_launch(ewald_pair_kblock<false>, grd, blk, 0, s, nn, K32, w32, c32, K64, w64, c64, psk, 0, nullptr);
+        }
       } else {
         if (K64) {
           pdl_launch(ewald_ktable_list<double>, (K64 + 127) / 128, 128, 0, s, L, K64, dh, t64);
@@ -1918,7 +2116,8 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         pdl_launch(ewald_pair_k_ds<PlaneSink>, grd, blk, 0, s, nn, L, K64, t64, c64, d_radii, inv_pimu, psk, 0);
         pdl_launch(ewald_pair_k<float, float2, PlaneSink>, grd, blk, 0, s, nn, L, K32, t32, c32, d_radii, inv_pimu, psk, 1);
       }
-      if (equal) {
+      if (sliced) {
+      } else if (equal) {
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
         pdl_launch(ewald_pair_real_near_ds<PlaneSink>, grd, blk, 0, s, nn, L, d_pos, d_radii, inv_pimu, rc2, psk);

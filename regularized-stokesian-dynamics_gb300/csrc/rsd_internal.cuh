@@ -206,8 +206,12 @@ __host__ __device__ inline void rsd_skew_shift_f32(const float* LR, const float*
 // only the entries whose row's particle is at most the column's are written
 // (M is symmetric; its readers take the others at the mirrored position).
 // h_radii: the radii on the host.
+// exported (mixed): the matrix ends in an FP32 RPP that is handed out, whose
+// TF32 factors turn its last bits into 1e-4: one order of summation for every
+// size.
 int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
-                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm);
+                       double mu_f, int precision, const double* h_radii, double* d_M, int64_t ldm,
+                       bool exported = false);
 int rsd_count_overlaps(rsd_ctx* ctx, int nn, const double* d_pos, const double* d_radii, const rsd_lattice* lat,
                        int* count);
 // Adds the overlap correction of correction_method 1 or 2 (GRPY_YZD.f90:

@@ -272,7 +272,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   {
     // grand mobility
     rsd_range r("rsd_assembly");
-    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, h_radii, M, ldm));
+    RSD_TRY(rsd_ewald_assemble(ctx, nn, d_conf, d_radii, &lat, p->mu_f, p->precision, h_radii, M, ldm, rpp_out != nullptr));
     if (p->use_lub)
       RSD_TRY(rsd_lub_build_sparse(ctx, beside.side, tab, nn, p->nb, 1, d_conf, d_radii, &lat, p->mu_f, &lub));
     if (ctx->correction_method) {  // overlap corrections (per_GRPY_YZD.f90:98-116)
