@@ -1358,9 +1358,8 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
         continue;
       }
       const int jn = m_in < NB ? m_in : NB;  // width of block k+1
-      // near: row panel k on block k+1's columns, then the diagonal tile (k+1, k+1)
-      RSD_TRY(rsd_tc_gemm(ctx, tc, jb, jn, jb, 1.0f, Wb, NB, Apan, lda, Apan, lda, 0, 0, 0, err, sa));
-      RSD_TRY(rsd_tc_gemm(ctx, tc, jn, jn, jb, -1.0f, Apan, lda, Apan, lda, Apan + jb, lda, 1, 1, 0, err, sa));
+      // near: row panel k on block k+1's columns, and the diagonal tile (k+1, k+1)
+      RSD_TRY(rsd_tc_near(ctx, tc, jn, Wb, Apan, lda, Apan + jb, err, sa));
       RSD_CUDA(ctx, cudaEventRecord(evA, sa));
       // far, beside block k+1's factor
       RSD_CUDA(ctx, cudaStreamWaitEvent(sb, evA, 0));

@@ -282,6 +282,8 @@ int rsd_axpy_block(rsd_ctx* ctx, int64_t rows, int64_t cols, const double* B, in
 // C = alpha A^T B (store) or C += alpha A^T B (reduce) on 128-tiles, prec 1
 // (TF32) or 3 (3xTF32); and the blocked-Cholesky trailing update on top of it.
 int rsd_tc_gemm_ok(const float* A, int64_t lda, const float* B, int64_t ldb, const float* C, int64_t ldc);
+int rsd_tc_near(rsd_ctx* ctx, int prec, int n, const float* W, float* B, int64_t ldb, float* D, int* d_err,
+                cudaStream_t st);
 int rsd_tc_gemm(rsd_ctx* ctx, int prec, int m, int n, int K, float alpha, const float* A, int64_t lda,
                 const float* B, int64_t ldb, float* C, int64_t ldc, int reduce, int tri, int klo_col, int* d_err,
                 cudaStream_t stream = 0, int ksplit = 0);

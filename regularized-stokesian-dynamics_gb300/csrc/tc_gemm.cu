@@ -17,6 +17,7 @@
 //               shared memory; then the epilogue: tcgen05.ld of the
 //               accumulator (TMEM lane = output row), alpha * D staged
 //               column-major in shared memory, one TMA store or reduce-add.
+// (tc_near_kernel at the end chains two such tiles in one CTA.)
 // Options per launch: skip the tiles strictly below the diagonal, and start
 // the K range of a tile at its first column (for triangular operands whose
 // rows below that are zero).
@@ -303,6 +304,240 @@ __global__ void __launch_bounds__(TC_THREADS, TcCfg<PREC>::MIN_CTAS)
   }
 }
 
+// The chain of the blocked Cholesky between two diagonal blocks in one launch
+// of one CTA: P = W^T B (B the 128 x n tile of the row panel in block k+1's
+// columns, W = U_kk^-1; stored over B), then D -= P^T P for block k+1's
+// diagonal tile, with P kept in shared memory as the second product's two
+// operands (same values and order of products as two launches of
+// tc_gemm_kernel; a block of the chain takes 36.5 us where those two make it
+// 39.3).  Roles and bounds of the waits as
+// there.  Shared memory: the stages; once their products are done P (PREC 3:
+// heads, then tails), behind it the column-major staging of P and D.
+template <int PREC>
+struct NearCfg {
+  static constexpr int STAGES = PREC == 1 ? 4 : 3;
+  static constexpr int STAGE_BYTES = TcCfg<PREC>::STAGE_BYTES;
+  static constexpr int P_BYTES = (PREC == 1 ? 4 : 8) * TC_CHUNK;
+  static constexpr int BAR_BYTES = (3 * STAGES + 3) * 8 + 16;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
+  static_assert(STAGES * STAGE_BYTES >= P_BYTES + TC_TILE * TC_TILE * 4, "P and the staging");
+};
+
+template <int PREC>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+    tc_near_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmD, int* err,
+                   unsigned long long wait_ns) {
+  using Cfg = NearCfg<PREC>;
+  constexpr int ST = Cfg::STAGES, SB = Cfg::STAGE_BYTES, NCH = TC_TILE / TC_KC;
+  extern __shared__ unsigned char smraw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
+  uint64_t* bars = (uint64_t*)(base + ST * SB);  // full[ST], conv[ST], empty[ST], done, ready, done2
+  uint32_t* tslot = (uint32_t*)(bars + 3 * ST + 3);
+  __shared__ volatile int abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t sbase = smem_u32(base), bar0 = smem_u32(bars);
+  auto full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
+  auto conv = [&](int s) { return bar0 + 8u * (uint32_t)(ST + s); };
+  auto empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * ST + s); };
+  const uint32_t done = bar0 + 8u * (3 * ST), ready = done + 8, done2 = done + 16;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                 "r"(2 * TC_TILE));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < ST; s++) {
+      mbar_init(full(s), 1);
+      mbar_init(conv(s), 128);
+      mbar_init(empty(s), 1);
+    }
+    mbar_init(done, 1);
+    mbar_init(ready, 128);
+    mbar_init(done2, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    abort_flag = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  pdl_enter();
+  const uint32_t taddr = *tslot;
+
+  if (warp == 0) {
+    if (lane == 0) {  // TMA producer
+      int last[ST];
+      for (int s = 0; s < ST; s++) last[s] = -1;
+      for (int c = 0; c < NCH; c++) {
+        const int s = c % ST;
+        if (c >= ST && !mbar_wait(empty(s), ((c / ST) - 1) & 1, &abort_flag, err, 1, wait_ns)) break;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full(s)), "r"(2 * TC_CHUNK)
+                     : "memory");
+        tma_load(sbase + s * SB, &tmW, c * TC_KC, 0, full(s));
+        tma_load(sbase + s * SB + TC_CHUNK, &tmB, c * TC_KC, 0, full(s));
+        last[s] = c;
+      }
+      // the loads have landed before the CTA may exit, whatever became of the rest
+      for (int s = 0; s < ST; s++)
+        if (last[s] >= 0) {
+          const uint64_t t0 = global_ns();
+          while (!mbar_try_wait(full(s), (last[s] / ST) & 1) && global_ns() - t0 < TC_WAIT_NS) {
+          }
+        }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issuer
+      auto products = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t al, uint32_t bl, bool first) {
+#pragma unroll
+        for (int kk = 0; kk < TC_KC / 8; kk++) {
+          mma_tf32(d, a + kk * 32, b + kk * 32, first && kk == 0 ? 0u : 1u);
+          if (PREC == 3) {
+            mma_tf32(d, a + kk * 32, bl + kk * 32, 1u);
+            mma_tf32(d, al + kk * 32, b + kk * 32, 1u);
+          }
+        }
+      };
+      bool ok = true;
+      int issued = 0;
+      for (int c = 0; c < NCH && ok; c++) {
+        const int s = c % ST;
+        ok = mbar_wait(PREC == 3 ? conv(s) : full(s), (c / ST) & 1, &abort_flag, err, 2, wait_ns);
+        if (!ok) break;
+        issued = c + 1;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t st = sbase + s * SB;
+        products(taddr, st, st + TC_CHUNK, st + 2 * TC_CHUNK, st + 3 * TC_CHUNK, c == 0);
+        mma_commit(empty(s));
+      }
+      if (issued > 0) mma_commit(done);
+      bool second = false;
+      if (ok && mbar_wait(ready, 0, &abort_flag, err, 5, wait_ns)) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        for (int c = 0; c < NCH; c++) {
+          const uint32_t ph = sbase + c * TC_CHUNK, pl = sbase + (NCH + c) * TC_CHUNK;
+          products(taddr + TC_TILE, ph, ph, pl, pl, c == 0);
+        }
+        mma_commit(done2);
+        second = true;
+      }
+      // what was issued has finished before the tensor memory is freed
+      const uint64_t t0 = global_ns();
+      while (((issued > 0 && !mbar_try_wait(done, 0)) || (second && !mbar_try_wait(done2, 0))) &&
+             global_ns() - t0 < TC_WAIT_NS) {
+      }
+    }
+  } else {
+    const int t = threadIdx.x - 64;  // 0..127
+    if (PREC == 3) {  // split each landed stage into TF32 head and tail
+      for (int c = 0; c < NCH; c++) {
+        const int s = c % ST;
+        if (!mbar_wait(full(s), (c / ST) & 1, &abort_flag, err, 3, wait_ns)) break;
+        unsigned char* st = base + s * SB;
+#pragma unroll
+        for (int op = 0; op < 2; op++) {
+          float4* hi = reinterpret_cast<float4*>(st + op * TC_CHUNK);
+          float4* lo = reinterpret_cast<float4*>(st + (2 + op) * TC_CHUNK);
+#pragma unroll
+          for (int q = 0; q < TC_CHUNK / 16 / 128; q++) {
+            const int idx = t + 128 * q;
+            const float4 v = hi[idx];
+            float4 h;
+            h.x = __uint_as_float(__float_as_uint(v.x) & 0xffffe000u);
+            h.y = __uint_as_float(__float_as_uint(v.y) & 0xffffe000u);
+            h.z = __uint_as_float(__float_as_uint(v.z) & 0xffffe000u);
+            h.w = __uint_as_float(__float_as_uint(v.w) & 0xffffe000u);
+            hi[idx] = h;
+            lo[idx] = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(conv(s)) : "memory");
+      }
+    }
+    float* sOut = reinterpret_cast<float*>(base + Cfg::P_BYTES);
+    const int q = warp & 3;  // this warp may read TMEM lanes 32q..32q+31
+    const int row = 32 * q + lane;
+    auto read32 = [&](uint32_t col, uint32_t (&v)[32]) {
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+          "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+            "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+            "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+          : "r"(taddr + ((uint32_t)(32 * q) << 16) + col));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    };
+    // warp-uniform: tcgen05.ld is a warp-collective instruction
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(done, 0, &abort_flag, err, 4, wait_ns) ? 1 : 0) != 0;
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int cc = 0; cc < TC_TILE / 32; cc++) {
+        uint32_t v[32];
+        read32((uint32_t)(cc * 32), v);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          const int c = cc * 32 + j;
+          const float x = __uint_as_float(v[j]);
+          sOut[c * TC_TILE + row] = x;
+          // K-major with the 128-byte swizzle: row c of P^T, k = row
+          unsigned char* p = base + q * TC_CHUNK + c * 128 + (((lane >> 2) ^ (c & 7)) << 4) + (lane & 3) * 4;
+          if (PREC == 3) {
+            const float h = __uint_as_float(v[j] & 0xffffe000u);
+            *reinterpret_cast<float*>(p) = h;
+            *reinterpret_cast<float*>(p + NCH * TC_CHUNK) = x - h;
+          } else {
+            *reinterpret_cast<float*>(p) = x;
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ready) : "memory");
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (t == 0 && ok && !abort_flag) {
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                       reinterpret_cast<uint64_t>(&tmP)),
+                   "r"(0), "r"(0), "r"(sbase + Cfg::P_BYTES)
+                   : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    const bool ok2 =
+        __all_sync(0xffffffffu, ok && mbar_wait(done2, 0, &abort_flag, err, 6, wait_ns) ? 1 : 0) != 0;
+    if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the staging is free again
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (ok2) {
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int cc = 0; cc < TC_TILE / 32; cc++) {
+        uint32_t v[32];
+        read32((uint32_t)(TC_TILE + cc * 32), v);
+#pragma unroll
+        for (int j = 0; j < 32; j++) sOut[(cc * 32 + j) * TC_TILE + row] = -__uint_as_float(v[j]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (t == 0) {
+      if (ok2 && !abort_flag) {
+        asm volatile(
+            "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                reinterpret_cast<uint64_t>(&tmD)),
+            "r"(0), "r"(0), "r"(sbase + Cfg::P_BYTES)
+            : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(2 * TC_TILE));
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
 int tc_init(rsd_ctx* ctx) {
@@ -316,6 +551,8 @@ int tc_init(rsd_ctx* ctx) {
   }
   RSD_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<1>::SMEM));
   RSD_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<3>::SMEM));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_near_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, NearCfg<1>::SMEM));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_near_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, NearCfg<3>::SMEM));
   g_encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
   return RSD_OK;
 }
@@ -380,6 +617,26 @@ int rsd_tc_gemm(rsd_ctx* ctx, int prec, int m, int n, int K, float alpha, const 
   } else {
     pdl_launch(tc_gemm_kernel<3>, grid, TC_THREADS, TcCfg<3>::SMEM, st, tmA, tmB, tmC, a);
   }
+  RSD_CUDA(ctx, cudaGetLastError());
+  return RSD_OK;
+}
+
+// B <- W^T B (W 128 x 128, ld 128; B 128 x n, n <= 128, ld ldb), then D -=
+// B^T B (n x n, ld ldb): the chain between two diagonal blocks.
+int rsd_tc_near(rsd_ctx* ctx, int prec, int n, const float* W, float* B, int64_t ldb, float* D, int* d_err,
+                cudaStream_t st) {
+  if (n < 1 || n > TC_TILE || (prec != 1 && prec != 3) || !rsd_tc_gemm_ok(W, TC_TILE, B, ldb, D, ldb))
+    return rsd_fail(ctx, RSD_EARG, "tc_near: unsupported arguments (n=%d prec=%d)", n, prec);
+  RSD_TRY(tc_init(ctx));
+  CUtensorMap tmW, tmB, tmP, tmD;
+  RSD_TRY(encode_2d(ctx, &tmW, W, TC_TILE, TC_TILE, TC_TILE, TC_KC, TC_TILE, CU_TENSOR_MAP_SWIZZLE_128B));
+  RSD_TRY(encode_2d(ctx, &tmB, B, TC_TILE, n, ldb, TC_KC, TC_TILE, CU_TENSOR_MAP_SWIZZLE_128B));
+  RSD_TRY(encode_2d(ctx, &tmP, B, TC_TILE, n, ldb, TC_TILE, TC_TILE, CU_TENSOR_MAP_SWIZZLE_NONE));
+  RSD_TRY(encode_2d(ctx, &tmD, D, n, n, ldb, TC_TILE, TC_TILE, CU_TENSOR_MAP_SWIZZLE_NONE));
+  if (prec == 1)
+    pdl_launch(tc_near_kernel<1>, 1, TC_THREADS, NearCfg<1>::SMEM, st, tmW, tmB, tmP, tmD, d_err, wait_limit(ctx));
+  else
+    pdl_launch(tc_near_kernel<3>, 1, TC_THREADS, NearCfg<3>::SMEM, st, tmW, tmB, tmP, tmD, d_err, wait_limit(ctx));
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }
