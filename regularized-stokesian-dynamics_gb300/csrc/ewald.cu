@@ -649,16 +649,17 @@ __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const 
                                                          const float* __restrict__ W64, const float4* __restrict__ c64,
                                                          PlaneSink sk, int add, float2* __restrict__ part) {
   pdl_enter();
+  constexpr int KC = 16;
   if (SLICED) {
-    const int z = blockIdx.z, S = gridDim.z, f = K32 * z / S, g = K64 * z / S;
-    K32 = K32 * (z + 1) / S - f;
+    // whole chunks of the FP32 vectors, so that their FP32 sums are those of one slice
+    const int z = blockIdx.z, S = gridDim.z, nc = (K32 + KC - 1) / KC, f = KC * (nc * z / S), g = K64 * z / S;
+    K32 = min(K32, KC * (nc * (z + 1) / S)) - f;
     W32 += (size_t)f * KBW;
     c32 += (size_t)f * nn;
     K64 = K64 * (z + 1) / S - g;
     W64 += (size_t)g * 2 * KBW;
     c64 += (size_t)g * nn;
   }
-  constexpr int KC = 16;
   __shared__ __align__(16) float sw[KC * 2 * KBW];  // the FP32 phase uses the first half
   __shared__ __align__(16) float4 sca[KC * 32], scb[KC * 4];
   if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
@@ -1204,8 +1205,8 @@ __device__ __forceinline__ int64_t grand_row(int N, int p, int k) {
 // (double-single) and far (FP32) - at [slice][value][pair], pair (a, b) at
 // b (b - 1) / 2 + a; the last kernel adds them up in double-single and writes
 // the blocks.  N = 32: 285 -> 90 us from the trig tables to the blocks, N = 173
-// 470 -> 250; against the FP64 step both orders of summation differ by the same
-// 2e-11 to 6e-11 in the velocities (the far images' FP32).
+// 470 -> 250.  The FP32 vectors are cut at whole chunks, so that a step's
+// outputs move by ~1e-13 only (cut anywhere: 5e-10, their FP32 rounding).
 struct RealSliceShared {
   dsf_tables T;
   int list[REAL_CAP][REAL_THREADS];
