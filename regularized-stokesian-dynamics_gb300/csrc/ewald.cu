@@ -481,10 +481,12 @@ __global__ void __launch_bounds__(128) ewald_pair_k(int nn, rsd_lat_dev L, int K
   store_pair_d(sk, nn, a, b, o, add);
 }
 
-// Reciprocal-space pair sums of the FP64 shells of the mixed form in
-// double-single: the trig table holds (cos, sin) as float pairs (float4 per
-// vector and particle), the weights are converted to float pairs as they are
-// staged in shared memory, and the epilogue runs in FP64.
+// Reciprocal-space pair sums of the FP64 shells of the mixed form (unequal
+// radii) in double-single: the trig table holds (cos, sin) as float pairs
+// (float4 per vector and particle), the moment weights are split into float
+// pairs as they are staged in shared memory, two moments go through each
+// packed instruction (dsacc's multiply-add as in ewald_pair_kblock; N = 300
+// 440 -> 365 us), and the epilogue runs in FP64.
 template <typename S>
 __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, int Kh, const double* __restrict__ tab,
                                                        const float4* __restrict__ cs, const double* __restrict__ radii,
@@ -492,23 +494,26 @@ __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, in
   pdl_enter();
   constexpr int KWT = 3 + RSD_NMOM_KCOS + RSD_NMOM_KSIN;
   constexpr int NW = RSD_NMOM_KCOS + RSD_NMOM_KSIN;
+  static_assert(NW % 4 == 0, "16-byte rows");
   constexpr int KC = 16;
-  __shared__ __align__(16) dsf sw[KC * NW];
+  __shared__ __align__(16) float sw[KC][2][NW];  // heads, tails
   __shared__ float4 sca[KC][32], scb[KC][4];  // trig values of the CTA's 32 + 4 particles (block 32 x 4)
   if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
   int a, b;
   const bool valid = pair_of(nn, &a, &b);
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
   const int a0 = blockIdx.x * blockDim.x, b0 = blockIdx.y * blockDim.y;
-  dsf ac[RSD_NMOM_KCOS], as[RSD_NMOM_KSIN];
+  uint64_t hi[NW / 2], lo[NW / 2];
 #pragma unroll
-  for (int m = 0; m < RSD_NMOM_KCOS; m++) ac[m] = dsf(0);
-#pragma unroll
-  for (int m = 0; m < RSD_NMOM_KSIN; m++) as[m] = dsf(0);
+  for (int p = 0; p < NW / 2; p++) hi[p] = lo[p] = 0;
   for (int h0 = 0; h0 < Kh; h0 += KC) {
     const int kc = min(KC, Kh - h0);
     __syncthreads();
-    for (int e = tid; e < kc * NW; e += nthr) sw[e] = dsf_from(tab[(size_t)(h0 + e / NW) * KWT + 3 + e % NW]);
+    for (int e = tid; e < kc * NW; e += nthr) {
+      const dsf w = dsf_from(tab[(size_t)(h0 + e / NW) * KWT + 3 + e % NW]);
+      sw[e / NW][0][e % NW] = w.hi;
+      sw[e / NW][1][e % NW] = w.lo;
+    }
     for (int e = tid; e < kc * 36; e += nthr) {
       const int hh = e / 36, q = e % 36, part = q < 32 ? a0 + q : b0 + q - 32;
       if (part < nn) {
@@ -526,19 +531,52 @@ __global__ void __launch_bounds__(128) ewald_pair_k_ds(int nn, rsd_lat_dev L, in
       const dsf ca(ua.x, ua.y), sa(ua.z, ua.w), cb(ub.x, ub.y), sb(ub.z, ub.w);
       const dsf c = ca * cb + sa * sb;   // cos(k.(x_a - x_b))
       const dsf sn = sa * cb - ca * sb;  // sin(k.(x_a - x_b))
-      const dsf* e = sw + hh * NW;
+      // cos, sin, or one of each where the moments turn from the one to the other
+      const uint64_t ch[3] = {f2_pack(c.hi, c.hi), f2_pack(sn.hi, sn.hi), f2_pack(c.hi, sn.hi)};
+      const uint64_t nh[3] = {f2_pack(-c.hi, -c.hi), f2_pack(-sn.hi, -sn.hi), f2_pack(-c.hi, -sn.hi)};
+      const uint64_t nl[3] = {f2_pack(-c.lo, -c.lo), f2_pack(-sn.lo, -sn.lo), f2_pack(-c.lo, -sn.lo)};
+      const ulonglong2* eh = reinterpret_cast<const ulonglong2*>(sw[hh][0]);
+      const ulonglong2* el = reinterpret_cast<const ulonglong2*>(sw[hh][1]);
 #pragma unroll
-      for (int m = 0; m < RSD_NMOM_KCOS; m++) ac[m] = fma(e[m], c, ac[m]);
+      for (int g = 0; g < NW / 4; g++) {
+        const ulonglong2 wh = eh[g], wl = el[g];
 #pragma unroll
-      for (int m = 0; m < RSD_NMOM_KSIN; m++) as[m] = fma(e[RSD_NMOM_KCOS + m], sn, as[m]);
+        for (int u = 0; u < 2; u++) {
+          const int p = 2 * g + u, k = 2 * p + 1 < RSD_NMOM_KCOS ? 0 : (2 * p >= RSD_NMOM_KCOS ? 1 : 2);
+          const uint64_t xh = u ? wh.y : wh.x, xl = u ? wl.y : wl.x;
+          const uint64_t pr = f2_mul(xh, ch[k]);
+          const uint64_t ne = f2_fma(xh, nl[k], f2_fma(xl, nh[k], f2_fma(xh, nh[k], pr)));  // minus the product's error
+          const uint64_t s = f2_add(hi[p], pr), bb = f2_sub(s, hi[p]);
+          const uint64_t e = f2_add(f2_sub(hi[p], f2_sub(s, bb)), f2_sub(pr, bb));
+          lo[p] = f2_add(lo[p], f2_sub(e, ne));
+          hi[p] = s;
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < NW / 2; p++) {  // at most 16 steps between renormalisations
+      const uint64_t s = f2_add(hi[p], lo[p]);
+      lo[p] = f2_sub(lo[p], f2_sub(s, hi[p]));
+      hi[p] = s;
     }
   }
   if (!valid) return;
   double acd[RSD_NMOM_KCOS], asd[RSD_NMOM_KSIN];
 #pragma unroll
-  for (int m = 0; m < RSD_NMOM_KCOS; m++) acd[m] = dsf_to(ac[m]);
+  for (int p = 0; p < NW / 2; p++) {
+    float h[2], l[2];
+    f2_unpack(hi[p], h[0], h[1]);
+    f2_unpack(lo[p], l[0], l[1]);
 #pragma unroll
-  for (int m = 0; m < RSD_NMOM_KSIN; m++) asd[m] = dsf_to(as[m]);
+    for (int u = 0; u < 2; u++) {
+      const int m = 2 * p + u;
+      const double d = (double)h[u] + (double)l[u];
+      if (m < RSD_NMOM_KCOS)
+        acd[m] = d;
+      else
+        asd[m - RSD_NMOM_KCOS] = d;
+    }
+  }
   double v[60], w[60];
   rsd_kcos_epilogue<double>(acd, radii[a], radii[b], L.phix, v);
   rsd_ksin_epilogue<double>(asd, radii[a], radii[b], L.phix, w);
@@ -761,18 +799,6 @@ __global__ void __launch_bounds__(128) ewald_pair_kblock(int nn, int K32, const 
   }
 }
 
-// Near/far split of the real-space images for the mixed form.  Image nz of
-// lattice column (nx, ny) has FP32 coordinates p + a3 nz, where p = R + nx a1
-// + ny a2 is formed in FP64 and rounded once; it is "near" when its FP32
-// squared distance, computed by exactly the sequence below, is below rc^2.
-// The near (double-single) and far (FP32) kernels evaluate the same sequence
-// on the same inputs, so every image is summed by exactly one of them.  An
-// image within a rounding of the boundary may fall on either side; both
-// sides are accurate there.
-__device__ __forceinline__ void column_base(const double R[3], const double* LR, int nx, int ny, double p[3]) {
-  for (int k = 0; k < 3; k++) p[k] = __fma_rn(LR[3 + k], (double)ny, __fma_rn(LR[k], (double)nx, R[k]));
-}
-
 __device__ __forceinline__ float image_r2f(float p0, float p1, float p2, float a0, float a1, float a2, int nz,
                                            float* x0, float* x1, float* x2) {
   const float z = (float)nz;
@@ -782,115 +808,17 @@ __device__ __forceinline__ float image_r2f(float p0, float p1, float p2, float a
   return __fmaf_rn(*x2, *x2, __fmaf_rn(*x1, *x1, __fmul_rn(*x0, *x0)));
 }
 
-// Far real-space images of the mixed form in FP32: lambda r from the
-// context's mixed_rcut up to mixed_rmax (beyond which the terms change a
-// block by less than ~1e-12 of its largest entry), with FP32 coordinates
-// p + a3 nz from each column's FP64 base point.  The radial functions of
-// erfc(lambda r) feed moments that the epilogue combines with 2-3 orders of
-// cancellation, so FP32 is kept for images whose terms are below ~1e-6 of a
-// block (a few 1e-11 of a block after the epilogue).
-template <typename S>
-__global__ void __launch_bounds__(128) ewald_pair_real_far(int nn, rsd_lat_dev L, const double* __restrict__ pos,
-                                                           const double* __restrict__ radii, double inv_pimu,
-                                                           double rc2, double rmax2, S sk) {
-  pdl_enter();
-  int a, b;
-  if (!pair_of(nn, &a, &b)) return;
-  double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
-  double dmin;
-  rsd_skew_correction(L.LR, L.LI, R, &dmin);
-  float acc[RSD_NMOM_REAL];
-#pragma unroll
-  for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.f;
-  const float lam = (float)L.lam, lam2 = lam * lam, cd = (float)(2.0 * RSD_PIP5) * lam;
-  const float a0 = __double2float_rn(L.LR[6]), a1 = __double2float_rn(L.LR[7]), a2 = __double2float_rn(L.LR[8]);
-  const float rc2f = __double2float_rn(rc2), rmax2f = __double2float_rn(rmax2);
-  const int NR = L.NR;
-  for (int nx = -NR; nx <= NR; nx++)
-    for (int ny = -NR; ny <= NR; ny++) {
-      double p[3];
-      column_base(R, L.LR, nx, ny, p);
-      const float p0 = __double2float_rn(p[0]), p1 = __double2float_rn(p[1]), p2 = __double2float_rn(p[2]);
-      for (int nz = -NR; nz <= NR; nz++) {
-        float x0, x1, x2;
-        const float r2 = image_r2f(p0, p1, p2, a0, a1, a2, nz, &x0, &x1, &x2);
-        if (r2 < rc2f || r2 >= rmax2f) continue;  // near (the other kernel) or truncated
-        const float r = sqrtf(r2), ir = 1.f / r;
-        rsd_real_image<float>(x0, x1, x2, r, ir, erfcf(lam * r), cd * expf(-r2 * lam2), lam, acc);
-      }
-    }
-  float v[60];
-  rsd_real_epilogue<float>(acc, (float)radii[a], (float)radii[b], (float)L.phix, v);
-  double o[60];
-#pragma unroll
-  for (int q = 0; q < 60; q++) o[q] = (double)v[q];
-  scale_block(o, radii[a], inv_pimu);
-  store_pair_d(sk, nn, a, b, o, 1);
-}
-
-// Near images of the mixed form (lambda r below the context's mixed_rcut) in
-// double-single arithmetic on the FP32 pipe: coordinates p + a3 nz, r, 1/r,
-// erfc(lambda r) and the Gaussian (dsf.cuh), the moments and their sums all
-// carry ~48 bits (so even after the epilogue's 2-3 orders of cancellation a
-// block stays within ~1e-12 of FP64); FP64 is left for the per-column set-up
-// and the FP64 epilogue.  Same image set as the FP32 far kernel's complement.
-template <typename S>
-__global__ void __launch_bounds__(128) ewald_pair_real_near_ds(int nn, rsd_lat_dev L, const double* __restrict__ pos,
-                                                               const double* __restrict__ radii, double inv_pimu,
-                                                               double rc2, S sk) {
-  pdl_enter();
-  __shared__ dsf_tables T;
-  // blocks entirely on or below the diagonal (a >= b everywhere) have no work
-  if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
-  dsf_tables_fill(T, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
-  __syncthreads();
-  int a, b;
-  if (!pair_of(nn, &a, &b)) return;
-  double R[3] = {pos[3 * a] - pos[3 * b], pos[3 * a + 1] - pos[3 * b + 1], pos[3 * a + 2] - pos[3 * b + 2]};
-  double dmin;
-  rsd_skew_correction(L.LR, L.LI, R, &dmin);
-  dsacc acc[RSD_NMOM_REAL];
-#pragma unroll
-  for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = dsacc(0);
-  int since_norm = 0;
-  const dsf lam_s = dsf_from(L.lam), cd_s = dsf_from(2.0 * RSD_PIP5 * L.lam);
-  const dsf a30 = dsf_from(L.LR[6]), a31 = dsf_from(L.LR[7]), a32 = dsf_from(L.LR[8]);
-  const float a0 = __double2float_rn(L.LR[6]), a1 = __double2float_rn(L.LR[7]), a2 = __double2float_rn(L.LR[8]);
-  const float rc2f = __double2float_rn(rc2);
-  const int NR = L.NR;
-  for (int nx = -NR; nx <= NR; nx++)
-    for (int ny = -NR; ny <= NR; ny++) {
-      double p[3];
-      column_base(R, L.LR, nx, ny, p);
-      const float f0 = __double2float_rn(p[0]), f1 = __double2float_rn(p[1]), f2 = __double2float_rn(p[2]);
-      const dsf p0 = dsf_from(p[0]), p1 = dsf_from(p[1]), p2 = dsf_from(p[2]);
-      for (int nz = -NR; nz <= NR; nz++) {
-        float y0, y1, y2;
-        if (!(image_r2f(f0, f1, f2, a0, a1, a2, nz, &y0, &y1, &y2) < rc2f)) continue;
-        const dsf x0 = p0 + nz * a30, x1 = p1 + nz * a31, x2 = p2 + nz * a32;
-        const dsf r = dsf_sqrt(x0 * x0 + x1 * x1 + x2 * x2);
-        const dsf ir = dsf_rcp(r);
-        dsf E0, G;
-        dsf_erfc_gauss(lam_s * r, T, &E0, &G);
-        rsd_real_image<dsf, dsacc>(x0, x1, x2, r, ir, E0, cd_s * G, lam_s, acc);
-        if (++since_norm == 4) {  // keep the accumulators' lo parts small
-#pragma unroll
-          for (int m = 0; m < RSD_NMOM_REAL; m++) dsacc_norm(acc[m]);
-          since_norm = 0;
-        }
-      }
-    }
-  double accd[RSD_NMOM_REAL];
-#pragma unroll
-  for (int m = 0; m < RSD_NMOM_REAL; m++) accd[m] = dsacc_to(acc[m]);
-  double v[60];
-  rsd_real_epilogue<double>(accd, radii[a], radii[b], L.phix, v);
-  scale_block(v, radii[a], inv_pimu);
-  store_pair_d(sk, nn, a, b, v, 1);
-}
-
-// ------------------------------------------ equal radii, real space, mixed
-// One kernel for both real-space image sets of a pair, all in FP32 and
+// ------------------------------------------ real space, mixed
+// Far images (lambda r from the context's mixed_rcut up to mixed_rmax, beyond
+// which the terms change a block by less than ~1e-12 of its largest entry) in
+// FP32, near ones in double-single: the radial functions of erfc(lambda r)
+// feed moments that the epilogue combines with 2-3 orders of cancellation, so
+// FP32 is kept for images whose terms are below ~1e-6 of a block (a few 1e-11
+// of a block after the epilogue), and ~48 bits keep a block within ~1e-12 of
+// FP64.  An image within a rounding of the boundary may fall on either side;
+// both are accurate there.
+//
+// Equal radii: one kernel for both real-space image sets of a pair, all in FP32 and
 // double-single arithmetic (the FP64 pipe of GB300 runs at ~1/60 of the
 // FP32 rate, so no FP64 is left in the image loops or the epilogue):
 //   - images are classified in FP32: column base p = R + nx a1 + ny a2 and
@@ -1062,6 +990,52 @@ __device__ __forceinline__ void real_pair(const rsd_lat_dev& L, const double* __
     g.Rs[i] = dsf_from(R[i]) - (k[0] * g.As[i] + k[1] * g.As[3 + i] + k[2] * g.As[6 + i]);
     g.Rf[i] = g.Rs[i].hi;
   }
+}
+
+// Unequal radii: both image sets as above, one FP64 epilogue on their sum (a
+// pair's radii enter only there).  N = 300: ~510 us; in two kernels over the
+// image cube, with FP64 column bases and minimum images and an epilogue each,
+// 958.
+struct RealMixShared {
+  dsf_tables T;
+  int list[REAL_CAP][REAL_THREADS];
+  float far[RSD_NMOM_REAL][REAL_THREADS];
+};
+__global__ void __launch_bounds__(REAL_THREADS, 2) ewald_pair_real_mix(int nn, rsd_lat_dev L,
+                                                                      const double* __restrict__ pos,
+                                                                      const double* __restrict__ radii,
+                                                                      double inv_pimu, float rc2, float rmax2,
+                                                                      PlaneSink sk) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char smraw_real[];
+  RealMixShared& sh = *reinterpret_cast<RealMixShared*>(smraw_real);
+  // blocks entirely on or below the diagonal (a >= b everywhere) have no work
+  if ((int)(blockIdx.x * blockDim.x) >= (int)(blockIdx.y * blockDim.y + blockDim.y - 1)) return;
+  const int t = threadIdx.y * blockDim.x + threadIdx.x;
+  dsf_tables_fill(sh.T, t, REAL_THREADS);
+  __syncthreads();
+  int a, b;
+  if (!pair_of(nn, &a, &b)) return;
+  RealPair g;
+  real_pair(L, pos, a, b, g);
+  {
+    float acc[RSD_NMOM_REAL];
+    far_moments(sh.list, t, g.Rf, g.A, L.NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
+#pragma unroll
+    for (int m = 0; m < RSD_NMOM_REAL; m++) sh.far[m][t] = acc[m];
+  }
+  double accd[RSD_NMOM_REAL];
+  {
+    dsacc acc[RSD_NMOM_REAL];
+    near_moments<1, 0>(sh.T, sh.list, t, g.Rf, g.A, g.Rs, g.As, L.NR, rc2, dsf_from(L.lam),
+                       dsf_from(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
+#pragma unroll
+    for (int m = 0; m < RSD_NMOM_REAL; m++) accd[m] = dsacc_to(acc[m]) + (double)sh.far[m][t];
+  }
+  double v[60];
+  rsd_real_epilogue<double>(accd, radii[a], radii[b], L.phix, v);
+  scale_block(v, radii[a], inv_pimu);
+  store_pair_d(sk, nn, a, b, v, 1);
 }
 
 // NP: passes over the near images, each summing one part of the moments
@@ -2121,8 +2095,10 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       } else if (equal) {
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
-        pdl_launch(ewald_pair_real_near_ds<PlaneSink>, grd, blk, 0, s, nn, L, d_pos, d_radii, inv_pimu, rc2, psk);
-        pdl_launch(ewald_pair_real_far<PlaneSink>, grd, blk, 0, s, nn, L, d_pos, d_radii, inv_pimu, rc2, rmax2, psk);
+        RSD_CUDA(ctx, cudaFuncSetAttribute(ewald_pair_real_mix, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(RealMixShared)));
+        pdl_launch(ewald_pair_real_mix, grd, blk, sizeof(RealMixShared), s, nn, L, d_pos, d_radii, inv_pimu, (float)rc2,
+                   (float)rmax2, psk);
       }
     }
   }
