@@ -1110,37 +1110,9 @@ __global__ void gemv_t_k(int m, int k, const T* __restrict__ A, int64_t lda, con
   }
 }
 
-// x_j <- W_jj x_j (trans = 0) or W_jj^T x_j (trans = 1) in place, one CTA;
-// the block W_jj is staged in shared memory first
-template <typename T>
-__global__ void __launch_bounds__(256) trsv_diag(int jb, const T* __restrict__ W, int ldw, int trans,
-                                                 T* __restrict__ X, int64_t ldx, int nrhs) {
-  pdl_enter();
-  extern __shared__ unsigned char smraw[];
-  T* Ws = (T*)smraw;           // jb x jb
-  T* b = Ws + NB * NB;         // jb x nrhs
-  const int t = threadIdx.x;
-  for (int e = t; e < jb * jb; e += blockDim.x) Ws[e] = W[(e % jb) + (int64_t)(e / jb) * ldw];
-  for (int e = t; e < jb * nrhs; e += blockDim.x) b[e] = X[(e % jb) + (int64_t)(e / jb) * ldx];
-  __syncthreads();
-  for (int e = t; e < jb * nrhs; e += blockDim.x) {
-    const int i = e % jb, r = e / jb;
-    T s = T(0);
-    if (!trans)
-      for (int p = i; p < jb; p++) s += Ws[i + p * jb] * b[p + r * jb];
-    else
-      for (int p = 0; p <= i; p++) s += Ws[p + i * jb] * b[p + r * jb];
-    X[i + (int64_t)r * ldx] = s;
-  }
-}
-
 template <typename T>
 int smem_potf2(int jb) {
   return (jb * jb + jb) * (int)sizeof(T);
-}
-template <typename T>
-int smem_trsv() {
-  return (NB * NB + NB * 4) * (int)sizeof(T);
 }
 
 // exported: the factor ends in a matrix that is handed out (the FP32 RPP of
@@ -1154,20 +1126,9 @@ void launch_potf2(cudaStream_t s, bool exported, float* A, int64_t lda, int jb, 
 }
 
 template <typename T>
-const char* tname();
-template <>
-const char* tname<double>() {
-  return "d";
-}
-template <>
-const char* tname<float>() {
-  return "s";
-}
-
-template <typename T>
 T* diag_inverses(rsd_ctx* ctx, int n, const char* tag) {
   const int nblk = (n + NB - 1) / NB;
-  std::string name = std::string("potrf_W_") + tname<T>() + tag;
+  std::string name = std::string("potrf_W_s") + tag;
   return (T*)rsd_scratch(ctx, name.c_str(), sizeof(T) * (size_t)nblk * NB * NB);
 }
 
@@ -1175,7 +1136,6 @@ template <typename T>
 int ensure_attrs(rsd_ctx* ctx) {
   static bool done = false;
   if (done) return RSD_OK;
-  RSD_CUDA(ctx, cudaFuncSetAttribute(trsv_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_trsv<T>()));
   RSD_CUDA(ctx, cudaFuncSetAttribute(trtri_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_potf2<T>(NB)));
   RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_inv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_POTF2_INV));
   RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_gj_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
@@ -1186,11 +1146,6 @@ int ensure_attrs(rsd_ctx* ctx) {
 }  // namespace
 
 // ------------------------------------------------------------ templates
-template <typename T>
-void rsd_gemm(cudaStream_t s, int m, int n, int k, double alpha, const T* A, int64_t lda, int ta, const T* B,
-              int64_t ldb, int tb, double beta, T* C, int64_t ldc) {
-  launch_gemm<T>(s, gp(m, n, k, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc));
-}
 
 template <typename T>
 int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t lda, const T* X, int64_t ldx,
@@ -2108,70 +2063,12 @@ int rsd_potrs_wide_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const flo
   return RSD_OK;
 }
 
-// Solve (U^T U) X = B in place (X holds B), nrhs <= 4; W from the factor's
-// diagonal blocks (computed here when W == nullptr)
-template <typename T>
-int rsd_potrs_upper_t(rsd_ctx* ctx, int n, const T* d_U, int64_t ldu, T* d_X, int64_t ldx, int nrhs, const char* tag,
-                      const T* W) {
-  cudaStream_t s = ctx->stream;
-  if (!W) {
-    T* Wn = nullptr;
-    RSD_TRY(rsd_diag_inverses_t<T>(ctx, n, d_U, ldu, tag, &Wn));
-    W = Wn;
-  }
-  const int nblk = (n + NB - 1) / NB;
-  if (nrhs > 4) {
-    // many right-hand sides: left-looking block substitution with GEMMs
-    T* Tb = (T*)rsd_scratch(ctx, sizeof(T) == 8 ? "potrs_tmp_d" : "potrs_tmp_s", sizeof(T) * (size_t)NB * nrhs);
-    if (!Tb) return RSD_ENOMEM;
-    for (int b = 0; b < nblk; b++) {
-      const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB;
-      if (j0 > 0) launch_gemm<T>(s, gp(jb, nrhs, j0, -1.0, d_U + (int64_t)j0 * ldu, ldu, 1, d_X, ldx, 0, 1.0, d_X + j0, ldx));
-      launch_gemm<T>(s, gp(jb, nrhs, jb, 1.0, W + (size_t)b * NB * NB, NB, 1, d_X + j0, ldx, 0, 0.0, Tb, NB));
-      RSD_CUDA(ctx, cudaMemcpy2DAsync(d_X + j0, ldx * sizeof(T), Tb, NB * sizeof(T), jb * sizeof(T), nrhs,
-                                      cudaMemcpyDeviceToDevice, s));
-    }
-    for (int b = nblk - 1; b >= 0; b--) {
-      const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB, rest = n - j0 - jb;
-      if (rest > 0)
-        launch_gemm<T>(s, gp(jb, nrhs, rest, -1.0, d_U + j0 + (int64_t)(j0 + jb) * ldu, ldu, 0, d_X + j0 + jb, ldx, 0,
-                             1.0, d_X + j0, ldx));
-      launch_gemm<T>(s, gp(jb, nrhs, jb, 1.0, W + (size_t)b * NB * NB, NB, 0, d_X + j0, ldx, 0, 0.0, Tb, NB));
-      RSD_CUDA(ctx, cudaMemcpy2DAsync(d_X + j0, ldx * sizeof(T), Tb, NB * sizeof(T), jb * sizeof(T), nrhs,
-                                      cudaMemcpyDeviceToDevice, s));
-    }
-    RSD_CUDA(ctx, cudaGetLastError());
-    return RSD_OK;
-  }
-  // forward: U^T y = b
-  for (int b = 0; b < nblk; b++) {
-    const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB, rest = n - j0 - jb;
-    pdl_launch(trsv_diag<T>, 1, 256, smem_trsv<T>(), s, jb, W + (size_t)b * NB * NB, NB, 1, d_X + j0, ldx, nrhs);
-    if (rest > 0)
-      RSD_TRY(rsd_gemv<T>(ctx, 1, rest, jb, T(-1), d_U + j0 + (int64_t)(j0 + jb) * ldu, ldu, d_X + j0, ldx, nrhs,
-                          T(1), d_X + j0 + jb, ldx));
-  }
-  // backward: U x = y
-  for (int b = nblk - 1; b >= 0; b--) {
-    const int j0 = b * NB, jb = n - j0 < NB ? n - j0 : NB;
-    pdl_launch(trsv_diag<T>, 1, 256, smem_trsv<T>(), s, jb, W + (size_t)b * NB * NB, NB, 0, d_X + j0, ldx, nrhs);
-    if (j0 > 0)
-      RSD_TRY(rsd_gemv<T>(ctx, 0, j0, jb, T(-1), d_U + (int64_t)j0 * ldu, ldu, d_X + j0, ldx, nrhs, T(1), d_X, ldx));
-  }
-  RSD_CUDA(ctx, cudaGetLastError());
-  return RSD_OK;
-}
-
-template void rsd_gemm<float>(cudaStream_t, int, int, int, double, const float*, int64_t, int, const float*, int64_t,
-                              int, double, float*, int64_t);
 template int rsd_gemv<float>(rsd_ctx*, int, int, int, float, const float*, int64_t, const float*, int64_t, int, float,
                              float*, int64_t);
 template int rsd_gemv<double>(rsd_ctx*, int, int, int, double, const double*, int64_t, const double*, int64_t, int,
                               double, double*, int64_t);
 template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*, bool);
 template int rsd_potri_upper_t<float>(rsd_ctx*, int, float*, int64_t, const char*, int, const float*, int*);
-template int rsd_potrs_upper_t<float>(rsd_ctx*, int, const float*, int64_t, float*, int64_t, int, const char*,
-                                      const float*);
 template int rsd_mirror_upper_t<float>(rsd_ctx*, int, float*, int64_t);
 template int rsd_diag_inverses_t<float>(rsd_ctx*, int, const float*, int64_t, const char*, float**);
 

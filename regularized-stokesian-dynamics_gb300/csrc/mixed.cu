@@ -37,12 +37,7 @@ template <typename T>
 int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc, const T* W = nullptr,
                       int* d_err = nullptr);
 template <typename T>
-int rsd_potrs_upper_t(rsd_ctx* ctx, int n, const T* d_U, int64_t ldu, T* d_X, int64_t ldx, int nrhs, const char* tag,
-                      const T* W);
-template <typename T>
 int rsd_mirror_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda);
-template <typename T>
-int rsd_diag_inverses_t(rsd_ctx* ctx, int n, const T* U, int64_t ldu, const char* tag, T** Wout);
 int rsd_wide_inverses_s(rsd_ctx* ctx, int n, const float* U, int64_t ldu, const char* tag, const float* W128,
                         float** W2out);
 const float* rsd_potrf_inverses_s(rsd_ctx* ctx, int n, const char* tag);
