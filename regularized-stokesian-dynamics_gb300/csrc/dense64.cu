@@ -470,8 +470,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
 // step is two FP64 warp instructions per row.  Warp 0 takes row k + 1 first,
 // then the next pivot's reciprocal and multipliers beside the other rows, so
 // a step has one barrier.  Bound by the FP64 pipe (64 cycles per warp
-// instruction and SM quarter): 67 us a block, 96 us with one row in flight
-// per warp; a column-by-column factor and inverse of 128 took 263 + 466 us.  info: first failing global index + 1.
+// instruction and SM quarter): 62 us a block, 67 with the roots taken where
+// they are stored and the pivot tested in FP64, 96 with one row in flight per
+// warp; a column-by-column factor and inverse of 128 took 263 + 466 us.
+// info: first failing global index + 1.
 // ks: half the exponents of the diagonal, the scale of row k of the panel
 // against column k of U.
 constexpr int PF_LD = NB64 + 1;
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
                                                      int* __restrict__ ks) {
   pdl_enter();
   __shared__ double S[NB64 * PF_LD];  // S(i, j) at [i * PF_LD + j]
-  __shared__ double l[2][NB64], rd[NB64];
+  __shared__ double l[2][NB64], sq[NB64], rd[NB64];
   __shared__ int failed;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int e = t; e < NB64 * NB64; e += 256) {
@@ -501,7 +503,8 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
   if (t < jb) ks[t] = half_exponent(S[t * PF_LD + t]);
   // multipliers l_ik of pivot k (d its value) into l[k & 1]
   auto pivot = [&](int k, double d) {
-    if (!(d > 0.0) || !isfinite(d)) {
+    const long long bits = __double_as_longlong(d);  // positive and finite, off the FP64 pipe
+    if (bits <= 0 || bits >= 0x7ff0000000000000LL) {
       if (lane == 0) {
         failed = 1;
         atomicCAS(info, 0, j0 + k + 1);
@@ -555,12 +558,15 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
     __syncthreads();
   }
   if (failed) return;
-  if (t < NB64) rd[t] = 1.0 / sqrt(S[t * PF_LD + t]);
+  if (t < NB64) {
+    sq[t] = sqrt(S[t * PF_LD + t]);
+    rd[t] = 1.0 / sq[t];
+  }
   __syncthreads();
   // U_kj = S_kj / sqrt(d_k); W_ij = (L^-1)_ji / sqrt(d_j) with unit diagonal
   for (int e = t; e < NB64 * NB64; e += 256) {
     const int i = e % NB64, j = e / NB64;
-    if (i <= j && j < jb) A[i + (int64_t)j * lda] = i == j ? sqrt(S[i * PF_LD + i]) : S[i * PF_LD + j] * rd[i];
+    if (i <= j && j < jb) A[i + (int64_t)j * lda] = i == j ? sq[i] : S[i * PF_LD + j] * rd[i];
     Wout[e] = i < j ? S[j * PF_LD + i] * rd[j] : (i == j ? rd[j] : 0.0);
   }
 }
