@@ -1374,7 +1374,7 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
     memcpy(bar, h + 4, sizeof bar);
     if (bar[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "PCG: a wait for the other thread blocks timed out");
     const int it = (int)h[0];
-    if (it > 0 && !std::isfinite(h[1])) return rsd_fail(ctx, RSD_ENAN, "PCG residual is not finite");
+    if (!std::isfinite(h[1])) return rsd_fail(ctx, RSD_ENAN, "PCG residual is not finite");
     worst_it = std::max(worst_it, it);
     worst_res = std::max(worst_res, h[1] / h[2]);
   }
