@@ -31,7 +31,8 @@
 //           step, its FP64 additions, costs as much as 128 of K)
 //   potri   U^-1 by recursive doubling of the diagonal inverses (all pairs of
 //           a level in one batched launch), then U^-1 U^-T as one product
-//   trsv    block substitution for a few right-hand sides, one launch a step
+//   trsv    block substitution for a few right-hand sides, one launch a step;
+//   trsm64  for many, as oz_gemm
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -946,9 +947,78 @@ int rsd_trsv64_bwd(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const doub
   return RSD_OK;
 }
 
-// Solve (U^T U) X = B in place with the factor of `tag`.  Up to 4 right-hand
-// sides by substitution; more (arrangement, matrices.f90:432-445, which
-// multiplies by MATREV's inverse) by the inverse and one product.
+namespace {
+
+// X <- U^-T X (trans) or U^-1 X for many right-hand sides, by blocks as potrf
+// goes: 64 unknowns a step, the product that takes them out of the outer
+// panel's other rows after each step and of all rows beyond it once per panel.
+// A block is solved through its explicit inverse W and corrected once by its
+// residual, which is then that of a substitution whatever the block's
+// condition number (through the inverse of the whole matrix, condition 1e10 and
+// right-hand sides A X0 left 8e-8 of arrangement's result; 1e-15 so).
+// Rows of X and of U^-1 and columns of U carry the scale of the matrix's
+// diagonal (ks, as in potri).  T: 64 x nrhs.
+int trsm64(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const rsd_factor64& f, double* X, int64_t ldx, int nrhs,
+           bool trans, double* T) {
+  RSD_TRY(oz_init(ctx));
+  cudaStream_t s = ctx->stream;
+  // C (rows [r0, r1) of the unknowns) += +-(U^T or U)(rows, [k0, k1)) X([k0, k1)); tri: the diagonal block
+  auto product = [&](int K, int k0, int k1, int r0, int r1, double* C, int64_t ldc, int tri) -> int {
+    if (r1 <= r0) return RSD_OK;
+    oz_op R, S;
+    RSD_TRY(oz_alloc(ctx, "oz_a", K, r1 - r0, 1, &R));
+    RSD_TRY(oz_alloc(ctx, "oz_b", K, nrhs, 1, &S));
+    oz_split_job r = oz_job(R, trans ? U + k0 + (int64_t)r0 * ldu : U + r0 + (int64_t)k0 * ldu, ldu, !trans, tri);
+    oz_split_job x = oz_job(S, X + k0, ldx, 0, 0);
+    r.kn = x.kn = k1 - k0;
+    if (!trans) {
+      r.ks = x.ks = f.dexp + k0;
+      r.ksgn = -1;
+    }
+    oz_split_launch(s, r, &x);
+    oz_args a{};
+    a.add = a.neg = 1;
+    return oz_gemm_launch(ctx, R, S, r1 - r0, nrhs, C, ldc, a);
+  };
+  // X([j0, j1)) = or += (W^T or W) B, W the inverse of the diagonal block
+  auto inverse = [&](int j0, int j1, const double* B, int64_t ldb, int add) -> int {
+    oz_op R, S;
+    RSD_TRY(oz_alloc(ctx, "oz_w", NB64, NB64, 1, &R));
+    RSD_TRY(oz_alloc(ctx, "oz_b", NB64, nrhs, 1, &S));
+    oz_split_job w = oz_job(R, f.W + (size_t)(j0 / NB64) * NB64 * NB64, NB64, !trans, 1);
+    oz_split_job x = oz_job(S, B, ldb, 0, 0);
+    w.kn = x.kn = j1 - j0;
+    if (trans) {
+      w.ks = x.ks = f.dexp + j0;
+      x.ksgn = -1;
+    }
+    oz_split_launch(s, x, &w);
+    oz_args a{};
+    a.add = add;
+    return oz_gemm_launch(ctx, R, S, j1 - j0, nrhs, X + j0, ldx, a);
+  };
+  const int last = (n - 1) / NBO64 * NBO64;
+  for (int P = 0; P <= last; P += NBO64) {
+    const int J0 = trans ? P : last - P, J1 = std::min(n, J0 + NBO64), nb = (J1 - J0 + NB64 - 1) / NB64;
+    for (int q = 0; q < nb; q++) {
+      const int j0 = J0 + (trans ? q : nb - 1 - q) * NB64, j1 = std::min(n, j0 + NB64);
+      RSD_CUDA(ctx, cudaMemcpy2DAsync(T, sizeof(double) * NB64, X + j0, sizeof(double) * ldx, sizeof(double) * (j1 - j0),
+                                      nrhs, cudaMemcpyDeviceToDevice, s));
+      RSD_TRY(inverse(j0, j1, T, NB64, 0));
+      RSD_TRY(product(NB64, j0, j1, j0, j1, T, NB64, 1));
+      RSD_TRY(inverse(j0, j1, T, NB64, 1));
+      RSD_TRY(trans ? product(NB64, j0, j1, j1, J1, X + j1, ldx, 0) : product(NB64, j0, j1, J0, j0, X + J0, ldx, 0));
+    }
+    RSD_TRY(trans ? product(NBO64, J0, J1, J1, n, X + J1, ldx, 0) : product(NBO64, J0, J1, 0, J0, X, ldx, 0));
+  }
+  return RSD_OK;
+}
+
+}  // namespace
+
+// Solve (U^T U) X = B in place with the factor of `tag`: substitution, a
+// launch per 64 unknowns for up to 4 right-hand sides, on the tensor cores for
+// more (arrangement, matrices.f90:432-445).
 int rsd_potrs_upper_tag(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, double* d_X, int64_t ldx, int nrhs,
                         const char* tag) {
   cudaStream_t s = ctx->stream;
@@ -965,17 +1035,13 @@ int rsd_potrs_upper_tag(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, dou
     RSD_CUDA(ctx, cudaMemcpy2DAsync(d_X, sizeof(double) * ldx, X, col, col, nrhs, cudaMemcpyDeviceToDevice, s));
     return RSD_OK;
   }
-  double* Ai = (double*)rsd_scratch(ctx, "potrs64_inv", sizeof(double) * (size_t)n * n);
-  if (!Ai) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemcpy2DAsync(Ai, sizeof(double) * n, d_U, sizeof(double) * ldu, sizeof(double) * n, n,
-                                  cudaMemcpyDeviceToDevice, s));
-  RSD_TRY(rsd_potri64(ctx, n, Ai, n, f));
-  RSD_TRY(rsd_mirror_upper(ctx, n, Ai, n));
-  oz_op R, S;
-  RSD_TRY(oz_alloc(ctx, "oz_a", n, n, 1, &R));
-  RSD_TRY(oz_alloc(ctx, "oz_b", n, nrhs, 1, &S));
-  const oz_split_job r = oz_job(R, Ai, n, 0, 0), q = oz_job(S, d_X, ldx, 0, 0);
-  oz_split_launch(s, r, &q);
-  RSD_TRY(oz_gemm_launch(ctx, R, S, n, nrhs, d_X, ldx, oz_args{}));
+  oz_op big;  // the largest operands first: the buffers grow once
+  RSD_TRY(oz_alloc(ctx, "oz_a", NBO64, n, 1, &big));
+  RSD_TRY(oz_alloc(ctx, "oz_b", NBO64, nrhs, 1, &big));
+  double* T = (double*)rsd_scratch(ctx, "potrs64_T", sizeof(double) * NB64 * (size_t)nrhs);
+  if (!T) return RSD_ENOMEM;
+  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
+  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, true, T));
+  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, false, T));
   return read_status(ctx, "potrs");
 }

@@ -1,0 +1,43 @@
+"""Accuracy of the FP64 factorisations on ill-conditioned matrices, against
+what substitution with multiply-adds in FP64 keeps whatever the condition
+number: residuals of some n eps of the operands' norms."""
+import numpy as np
+import pytest
+
+import __graft_entry__ as ge
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+@pytest.fixture(scope="module")
+def rsd():
+    ge._load_build_module().build()
+    return ge.load_package()
+
+
+@pytest.fixture(scope="module")
+def ctx(rsd):
+    return rsd.Context(0)
+
+
+def spd(n, cond, seed):
+    rng = np.random.default_rng(seed)
+    q, _ = np.linalg.qr(rng.normal(size=(n, n)))
+    a = (q * np.exp(rng.uniform(-np.log(cond), 0.0, n))) @ q.T
+    return 0.5 * (a + a.T)
+
+
+@pytest.mark.parametrize("N", [1, 11, 43])  # 6 N = 6, 66, 258: one block, ragged second block, ragged second panel
+def test_many_right_hand_sides(rsd, ctx, N):
+    """arrangement with RPQ = A X0, condition 1e10: RPQ^T A^-1 RPQ = X0^T A X0.
+    With (A + D) X = RPQ exactly, |D| <= n eps |A|, the result moves by X0^T D X0
+    and the roundings of RPQ and of the product, n eps |X0|^T |A| |X0| each."""
+    p, q = 6 * N, 5 * N
+    A = spd(p, 1e10, N)
+    X0 = np.random.default_rng(N).normal(size=(p, q))
+    B = A @ X0
+    mu, info = rsd.arrangement(ctx, A, B, np.zeros((q, q)))
+    ref = (B.T.astype(np.longdouble) @ X0).astype(np.float64)
+    size = np.abs(X0).T @ np.abs(A) @ np.abs(X0)
+    assert info == 0 and np.abs(mu - ref).max() <= 3 * p * EPS * size.max()
