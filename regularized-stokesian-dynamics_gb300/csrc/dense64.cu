@@ -25,10 +25,10 @@
 // slices [digit][batch][column][K] of bf16; C(r, c) = sum_k R(k, r) S(k, c).
 //
 //   potrf   right-looking, 64 columns a step: the diagonal block and its
-//           inverse in one CTA (potf2_inv_f64), the row panel as W^T B and
-//           the updates P^T P as oz_gemm, of the outer panel's 256 rows after
-//           each step and of the rest once per outer panel (a tile's last
-//           step, its FP64 additions, costs as much as 128 of K)
+//           inverse in one CTA (potf2_inv_f64), the row panel by substitution
+//           (subst64) and the updates P^T P as oz_gemm, of the outer panel's
+//           256 rows after each step and of the rest once per outer panel (a
+//           tile's last step, its FP64 additions, costs as much as 128 of K)
 //   potri   U^-1 by recursive doubling of the diagonal inverses (all pairs of
 //           a level in one batched launch), then U^-1 U^-T as one product
 //   trsv    block substitution for a few right-hand sides, one launch a step;
@@ -475,8 +475,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
 // they are stored and the pivot tested in FP64, 96 with one row in flight per
 // warp; a column-by-column factor and inverse of 128 took 263 + 466 us.
 // info: first failing global index + 1.
-// ks: half the exponents of the diagonal, the scale of row k of the panel
-// against column k of U.
 constexpr int PF_LD = NB64 + 1;
 __device__ __forceinline__ int half_exponent(double d) {
   const int E = (int)(abs_bits(d) >> 52);
@@ -488,8 +486,7 @@ __global__ void diag_exponents(int n, const double* __restrict__ A, int64_t lda,
   if (i < n) e[i] = half_exponent(A[i + (int64_t)i * lda]);
 }
 __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int64_t lda, int jb,
-                                                     int* __restrict__ info, int j0, double* __restrict__ Wout,
-                                                     int* __restrict__ ks) {
+                                                     int* __restrict__ info, int j0, double* __restrict__ Wout) {
   pdl_enter();
   __shared__ double S[NB64 * PF_LD];  // S(i, j) at [i * PF_LD + j]
   __shared__ double l[2][NB64], sq[NB64], rd[NB64];
@@ -501,7 +498,6 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
   }
   if (t == 0) failed = 0;
   __syncthreads();
-  if (t < jb) ks[t] = half_exponent(S[t * PF_LD + t]);
   // multipliers l_ik of pivot k (d its value) into l[k & 1]
   auto pivot = [&](int k, double d) {
     const long long bits = __double_as_longlong(d);  // positive and finite, off the FP64 pipe
@@ -570,6 +566,49 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
     if (i <= j && j < jb) A[i + (int64_t)j * lda] = i == j ? sq[i] : S[i * PF_LD + j] * rd[i];
     Wout[e] = i < j ? S[j * PF_LD + i] * rd[j] : (i == j ? rd[j] : 0.0);
   }
+}
+
+// ------------------------------------------------ substitution, many systems
+// Solves against a 64-wide diagonal block U on the FP64 pipe: system q = the
+// blockIdx.x-th eight, its entry i at B[i si + q sq], U^T x = b in place.  Through
+// the block's explicit inverse the residual would grow by the condition number
+// of the block (stiff pairs at 1e8: 4600 eps of the scaled matrix, 8 so).  16
+// lanes per system, four entries each; with the rows of U divided by their
+// diagonal a step is a broadcast and at most four multiply-adds, and the entries
+// are scaled at the end.  Bound by the FP64 pipe (64 cycles per warp instruction and SM
+// quarter): ~7 us for up to 1216 systems.
+// rdiag: the reciprocals of the diagonal, that of entry k at rdiag[k (NB64 + 1)].
+constexpr int SUB_SYS = 8, SUB_THREADS = 16 * SUB_SYS;
+__global__ void __launch_bounds__(SUB_THREADS) subst64(const double* __restrict__ U, int64_t ldu,
+                                                       const double* __restrict__ rdiag, int nsys,
+                                                       double* __restrict__ B, int64_t si, int64_t sq) {
+  pdl_enter();
+  constexpr int R = NB64 / 16;
+  __shared__ double S[NB64 * PF_LD], rd[NB64];  // S(k, i) = U(k, i) / U(k, k), k < i
+  const int t = threadIdx.x, l = t & 15, q = blockIdx.x * SUB_SYS + (t >> 4);
+  if (t < NB64) rd[t] = rdiag[t * (NB64 + 1)];
+  double b[R];
+#pragma unroll
+  for (int j = 0; j < R; j++) b[j] = q < nsys ? B[(l + 16 * j) * si + q * sq] : 0.0;
+  __syncthreads();
+  for (int e = t; e < NB64 * NB64; e += SUB_THREADS) {
+    const int k = e % NB64, i = e / NB64;
+    if (k < i) S[k * PF_LD + i] = U[k + (int64_t)i * ldu] * rd[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int kb = 0; kb < R; kb++)
+#pragma unroll
+    for (int kk = 0; kk < 16; kk++) {
+      const double x = __shfl_sync(0xffffffffu, b[kb], kk, 16);
+      const double* s = S + (16 * kb + kk) * PF_LD + l;
+      if (kk < 15 && l > kk) b[kb] = fma(-s[16 * kb], x, b[kb]);
+#pragma unroll
+      for (int j = kb + 1; j < R; j++) b[j] = fma(-s[16 * j], x, b[j]);
+    }
+  if (q < nsys)
+#pragma unroll
+    for (int j = 0; j < R; j++) B[(l + 16 * j) * si + q * sq] = b[j] * rd[l + 16 * j];
 }
 
 // ------------------------------------------------------- substitution steps
@@ -795,10 +834,7 @@ int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info
   cudaStream_t s = ctx->stream;
   rsd_factor64 f;
   RSD_TRY(factor64(ctx, n, tag, &f));
-  int* ks = (int*)rsd_scratch(ctx, "potrf64_ks", sizeof(int) * NB64);
-  if (!ks) return RSD_ENOMEM;
-  oz_op w, b, o;
-  RSD_TRY(oz_alloc(ctx, "oz_w", NB64, NB64, 1, &w));
+  oz_op b, o;
   RSD_TRY(oz_alloc(ctx, "oz_a", NB64, n, 1, &b));
   RSD_TRY(oz_alloc(ctx, "oz_b", NBO64, n, 1, &o));
   RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
@@ -808,19 +844,15 @@ int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info
     for (int j0 = J0; j0 < J0 + JB; j0 += NB64) {
       const int jb = n - j0 < NB64 ? n - j0 : NB64, rest = n - j0 - jb;
       double* Wb = f.W + (size_t)(j0 / NB64) * NB64 * NB64;
-      pdl_launch(potf2_inv_f64, 1, 256, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, jb, ctx->d_info, j0, Wb, ks);
+      pdl_launch(potf2_inv_f64, 1, 256, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, jb, ctx->d_info, j0, Wb);
       if (rest <= 0) break;
-      double* P = d_A + j0 + (int64_t)(j0 + jb) * lda;
-      b.cols = rest;
-      oz_split_job jw = oz_job(w, Wb, NB64, 0, 1), jp = oz_job(b, P, lda, 0, 0);
-      jw.ks = jp.ks = ks;
-      jp.ksgn = -1;
-      oz_split_launch(s, jp, &jw);
-      RSD_TRY(oz_gemm_launch(ctx, w, b, NB64, rest, P, lda, oz_args{}));  // row panel W^T P
+      double* P = d_A + j0 + (int64_t)(j0 + jb) * lda;  // the row panel, U^-T P
+      pdl_launch(subst64, (rest + SUB_SYS - 1) / SUB_SYS, SUB_THREADS, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, Wb, rest, P,
+                 1, lda);
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel still to update
       if (m_in <= 0) continue;
-      jp.ks = nullptr;
-      oz_split_launch(s, jp);
+      b.cols = rest;
+      oz_split_launch(s, oz_job(b, P, lda, 0, 0));
       oz_args up{};
       up.tri = up.add = up.neg = 1;
       RSD_TRY(oz_gemm_launch(ctx, b, b, m_in, rest, P + jb, lda, up));

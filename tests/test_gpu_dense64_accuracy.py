@@ -41,3 +41,25 @@ def test_many_right_hand_sides(rsd, ctx, N):
     ref = (B.T.astype(np.longdouble) @ X0).astype(np.float64)
     size = np.abs(X0).T @ np.abs(A) @ np.abs(X0)
     assert info == 0 and np.abs(mu - ref).max() <= 3 * p * EPS * size.max()
+
+
+def stiff_pairs(n, gap, seed):
+    """A well-conditioned matrix with a spring 1 / gap along a random axis between
+    neighbouring bodies of six unknowns, as lubrication adds one."""
+    rng = np.random.default_rng(seed)
+    A = spd(n, 10.0, seed)
+    for i in range(0, n - 9, 6):
+        v, e = np.zeros(n), rng.normal(size=3)
+        v[i:i + 3] = e / np.linalg.norm(e)
+        v[i + 6:i + 9] = -v[i:i + 3]
+        A += np.outer(v, v) / gap
+    return A
+
+
+@pytest.mark.parametrize("n", [65, 128, 300, 577])  # ragged and whole last blocks, one to three outer panels
+def test_factor_residual(rsd, ctx, n):
+    """|A - L L^T| <= n eps sqrt(A_ii A_jj), Cholesky's bound, on stiff pairs."""
+    A = stiff_pairs(n, 1e-8, n)
+    L = rsd.CHOLESKY(ctx, A).astype(np.longdouble)
+    d = np.sqrt(np.diag(A))
+    assert np.abs((A - L @ L.T) / np.outer(d, d)).max() <= n * EPS
