@@ -29,10 +29,12 @@
 //           (subst64) and the updates P^T P as oz_gemm, of the outer panel's
 //           256 rows after each step and of the rest once per outer panel (a
 //           tile's last step, its FP64 additions, costs as much as 128 of K)
+//   trsm64  solves for many right-hand sides, 128 unknowns a step by
+//           substitution, the updates as oz_gemm
 //   potri   U^-1 by recursive doubling of the diagonal inverses (all pairs of
-//           a level in one batched launch), then U^-1 U^-T as one product
-//   trsv    block substitution for a few right-hand sides, one launch a step;
-//   trsm64  for many, as oz_gemm
+//           a level in one batched launch) or by trsm64 on the identity, then
+//           U^-1 U^-T as one product
+//   trsv    block substitution for a few right-hand sides, one launch a step
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -62,6 +64,8 @@ constexpr int OZ_ZERO = -(1 << 20);
 constexpr unsigned long long OZ_WAIT_NS = 500ull * 1000 * 1000;
 constexpr int NB64 = 64;                    // panel width of the factorisation
 constexpr int NBO64 = 256;                  // rows between two updates of the whole trailing matrix
+constexpr int NBS64 = 128;                  // unknowns a step of the solves with many right-hand sides
+constexpr int GROWTH64 = 3;                 // largest exponent of a scaled inverse factor for the fast inverse
 
 // ------------------------------------------------------------------ split
 // Batch z: X + z sX, columns beyond cn - z cstep and K beyond kn - z kstep
@@ -204,6 +208,7 @@ struct oz_args {
   int klo_row, klo_col, khi_col;  // K starts at the tile's first row / column, ends with its last column
   int add;          // 1: C += the product, 0: C = the product
   int neg;          // the product is taken times -1
+  const int* gate;  // no product above GROWTH64
   double* C;
   int64_t ld, sC;
   const int *ER, *ES;  // exponents of R's and S's columns
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
   pdl_enter();
   const int row0 = blockIdx.x * OZ_TR, col0 = blockIdx.y * OZ_TC, z = blockIdx.z;
   const int nz = min(a.n, a.ncap - z * a.nstep);
-  if (col0 >= nz || (a.tri && row0 > col0 + OZ_TC - 1)) return;
+  if (col0 >= nz || (a.tri && row0 > col0 + OZ_TC - 1) || (a.gate && *a.gate > GROWTH64)) return;
   int klo = 0, khi = a.K;
   if (a.klo_row) klo = max(klo, row0);
   if (a.klo_col) klo = max(klo, col0);
@@ -569,31 +574,38 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
 }
 
 // ------------------------------------------------ substitution, many systems
-// Solves against a 64-wide diagonal block U on the FP64 pipe: system q = the
-// blockIdx.x-th eight, its entry i at B[i si + q sq], U^T x = b in place.  Through
+// Solves against a w-wide diagonal block U (w <= W) on the FP64 pipe, in place:
+// U^T x = b, or U x = b (BACK), the entries of system q at B[i + q ldb].  Through
 // the block's explicit inverse the residual would grow by the condition number
-// of the block (stiff pairs at 1e8: 4600 eps of the scaled matrix, 8 so).  16
-// lanes per system, four entries each; with the rows of U divided by their
-// diagonal a step is a broadcast and at most four multiply-adds, and the entries
-// are scaled at the end.  Bound by the FP64 pipe (64 cycles per warp instruction and SM
-// quarter): ~7 us for up to 1216 systems.
-// rdiag: the reciprocals of the diagonal, that of entry k at rdiag[k (NB64 + 1)].
+// of the block (factor of stiff pairs at 1e8: 4600 eps of the scaled matrix, 8
+// so).  16 lanes per system; with U's entries divided by the pivot of their step
+// a step is a broadcast and at most W / 16 multiply-adds, and the unknowns are
+// scaled at the end.  Bound by the FP64 pipe (64 cycles per warp instruction and
+// SM quarter): ~7 us for up to 1216 systems of 64, ~22 of 128.
+// The reciprocals of the diagonal come from the 64-wide inverses in Wd.
 constexpr int SUB_SYS = 8, SUB_THREADS = 16 * SUB_SYS;
-__global__ void __launch_bounds__(SUB_THREADS) subst64(const double* __restrict__ U, int64_t ldu,
-                                                       const double* __restrict__ rdiag, int nsys,
-                                                       double* __restrict__ B, int64_t si, int64_t sq) {
+template <int W>
+constexpr int SUB_SMEM = (W * (W + 1) + W) * (int)sizeof(double);
+template <int W, bool BACK>
+__global__ void __launch_bounds__(SUB_THREADS) subst64(int w, const double* __restrict__ U, int64_t ldu,
+                                                       const double* __restrict__ Wd, int nsys, double* __restrict__ B,
+                                                       int64_t ldb) {
   pdl_enter();
-  constexpr int R = NB64 / 16;
-  __shared__ double S[NB64 * PF_LD], rd[NB64];  // S(k, i) = U(k, i) / U(k, k), k < i
+  constexpr int R = W / 16, LD = W + 1;
+  extern __shared__ __align__(16) double sub_smem[];
+  // step k takes unknown at(k); S(k, i): U's entry of step k and unknown at(i) by the pivot of step k, k < i
+  double *S = sub_smem, *rd = S + W * LD;
   const int t = threadIdx.x, l = t & 15, q = blockIdx.x * SUB_SYS + (t >> 4);
-  if (t < NB64) rd[t] = rdiag[t * (NB64 + 1)];
+  auto at = [](int i) { return BACK ? W - 1 - i : i; };
+  double* Bq = B + (int64_t)q * ldb;
+  if (t < W) rd[t] = at(t) < w ? Wd[(at(t) / NB64) * NB64 * NB64 + (at(t) % NB64) * (NB64 + 1)] : 1.0;
   double b[R];
 #pragma unroll
-  for (int j = 0; j < R; j++) b[j] = q < nsys ? B[(l + 16 * j) * si + q * sq] : 0.0;
+  for (int j = 0; j < R; j++) b[j] = q < nsys && at(l + 16 * j) < w ? Bq[at(l + 16 * j)] : 0.0;
   __syncthreads();
-  for (int e = t; e < NB64 * NB64; e += SUB_THREADS) {
-    const int k = e % NB64, i = e / NB64;
-    if (k < i) S[k * PF_LD + i] = U[k + (int64_t)i * ldu] * rd[k];
+  for (int e = t; e < W * W; e += SUB_THREADS) {  // U(r, c), r < c, by columns
+    const int r = e % W, c = e / W, k = BACK ? at(c) : r, i = BACK ? at(r) : c;
+    if (r < c) S[k * LD + i] = c < w ? U[r + (int64_t)c * ldu] * rd[k] : 0.0;
   }
   __syncthreads();
 #pragma unroll
@@ -601,14 +613,14 @@ __global__ void __launch_bounds__(SUB_THREADS) subst64(const double* __restrict_
 #pragma unroll
     for (int kk = 0; kk < 16; kk++) {
       const double x = __shfl_sync(0xffffffffu, b[kb], kk, 16);
-      const double* s = S + (16 * kb + kk) * PF_LD + l;
+      const double* s = S + (16 * kb + kk) * LD + l;
       if (kk < 15 && l > kk) b[kb] = fma(-s[16 * kb], x, b[kb]);
 #pragma unroll
       for (int j = kb + 1; j < R; j++) b[j] = fma(-s[16 * j], x, b[j]);
     }
-  if (q < nsys)
 #pragma unroll
-    for (int j = 0; j < R; j++) B[(l + 16 * j) * si + q * sq] = b[j] * rd[l + 16 * j];
+  for (int j = 0; j < R; j++)
+    if (q < nsys && at(l + 16 * j) < w) Bq[at(l + 16 * j)] = b[j] * rd[l + 16 * j];
 }
 
 // ------------------------------------------------------- substitution steps
@@ -716,6 +728,21 @@ __global__ void put_diag64(int n, const double* __restrict__ W, double* __restri
   }
 }
 
+__global__ void put_ones64(int n, double* __restrict__ V) {
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) V[i + (int64_t)i * n] = 1.0;
+}
+
+// largest exponent of the rows of V (e) scaled by the diagonal (dexp)
+__global__ void growth64(int n, const int* __restrict__ e, const int* __restrict__ dexp, int* __restrict__ out) {
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int g = i < n ? e[i] + dexp[i] : 0;
+  g = __reduce_max_sync(0xffffffffu, g);
+  if ((threadIdx.x & 31) == 0) atomicMax(out, g);
+}
+
 // ------------------------------------------------------------------- host
 PFN_cuTensorMapEncodeTiled_v12000 g_encode64 = nullptr;
 
@@ -729,6 +756,8 @@ int oz_init(rsd_ctx* ctx) {
     return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled is not available");
   }
   RSD_CUDA(ctx, cudaFuncSetAttribute(oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(subst64<NBS64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM<NBS64>));
+  RSD_CUDA(ctx, cudaFuncSetAttribute(subst64<NBS64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM<NBS64>));
   g_encode64 = (PFN_cuTensorMapEncodeTiled_v12000)fn;
   return RSD_OK;
 }
@@ -805,6 +834,11 @@ int oz_gemm_launch(rsd_ctx* ctx, const oz_op& R, const oz_op& S, int m, int n, d
   return RSD_OK;
 }
 
+template <int W, bool BACK>
+void subst_launch(cudaStream_t s, int w, const double* U, int64_t ldu, const double* Wd, int nsys, double* B, int64_t ldb) {
+  pdl_launch(subst64<W, BACK>, (nsys + SUB_SYS - 1) / SUB_SYS, SUB_THREADS, SUB_SMEM<W>, s, w, U, ldu, Wd, nsys, B, ldb);
+}
+
 // What a factorisation leaves for the inverse and the solves: the inverses of
 // the diagonal blocks and half the exponents of the matrix's diagonal.
 int factor64(rsd_ctx* ctx, int n, const char* tag, rsd_factor64* f) {
@@ -818,7 +852,7 @@ int factor64(rsd_ctx* ctx, int n, const char* tag, rsd_factor64* f) {
 }
 
 int read_status(rsd_ctx* ctx, const char* what) {
-  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  RSD_CUDA(ctx, cudaMemcpyAsync(ctx->h_info, ctx->d_info, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   RSD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (ctx->h_info[1]) return rsd_fail(ctx, RSD_ETIMEOUT, "%s: tensor-core product timed out (code %d)", what, ctx->h_info[1]);
   return RSD_OK;
@@ -847,8 +881,7 @@ int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info
       pdl_launch(potf2_inv_f64, 1, 256, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, jb, ctx->d_info, j0, Wb);
       if (rest <= 0) break;
       double* P = d_A + j0 + (int64_t)(j0 + jb) * lda;  // the row panel, U^-T P
-      pdl_launch(subst64, (rest + SUB_SYS - 1) / SUB_SYS, SUB_THREADS, 0, s, d_A + j0 + (int64_t)j0 * lda, lda, Wb, rest, P,
-                 1, lda);
+      subst_launch<NB64, false>(s, NB64, d_A + j0 + (int64_t)j0 * lda, lda, Wb, rest, P, lda);
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel still to update
       if (m_in <= 0) continue;
       b.cols = rest;
@@ -872,14 +905,56 @@ int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info
   return RSD_OK;
 }
 
-// A^-1 (upper triangle) from the factor in A and what potrf left with it: V = U^-1 grows by pairs of blocks, [V11, -V11 U12 V22; 0,
-// V22], all pairs of a size at once; then A^-1 = V V^T.
-int rsd_potri64(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const rsd_factor64& f) {
+namespace {
+
+// X <- U^-T X (trans) or U^-1 X for many right-hand sides, 128 unknowns a step:
+// the block by substitution, then the product that takes it out of the rows
+// left.  Rows of X, of U^-1 and columns of U carry the scale of the factored
+// matrix's diagonal (dexp).  With explicit inverses of blocks in the
+// substitution's place, or of U, the residual would grow by their condition
+// numbers (condition 1e10, right-hand sides A X0: 8e-8 of arrangement's result
+// through A^-1, 1e-15 so).  eye: X starts as the identity, so block
+// b has columns from its own on.
+int trsm64(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const rsd_factor64& f, double* X, int64_t ldx, int nrhs,
+           bool trans, bool eye) {
   RSD_TRY(oz_init(ctx));
   cudaStream_t s = ctx->stream;
-  double* V = (double*)rsd_scratch(ctx, "potri64_V", sizeof(double) * (size_t)n * n);
-  if (!V) return RSD_ENOMEM;
-  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
+  const int last = (n - 1) / NBS64 * NBS64;
+  for (int p = 0; p <= last; p += NBS64) {
+    const int j0 = trans ? p : last - p, j1 = std::min(n, j0 + NBS64), c0 = eye ? j0 : 0, nc = nrhs - c0;
+    const double *Ub = U + j0 + (int64_t)j0 * ldu, *Wb = f.W + (size_t)(j0 / NB64) * NB64 * NB64;
+    double* Xc = X + (int64_t)c0 * ldx;
+    if (trans)
+      subst_launch<NBS64, false>(s, j1 - j0, Ub, ldu, Wb, nc, Xc + j0, ldx);
+    else
+      subst_launch<NBS64, true>(s, j1 - j0, Ub, ldu, Wb, nc, Xc + j0, ldx);
+    const int r0 = trans ? j1 : 0, m = trans ? n - j1 : j0;  // rows left
+    if (m <= 0) continue;
+    oz_op R, S;
+    RSD_TRY(oz_alloc(ctx, "oz_a", NBS64, m, 1, &R));
+    RSD_TRY(oz_alloc(ctx, "oz_b", NBS64, nc, 1, &S));
+    oz_split_job r = oz_job(R, trans ? U + j0 + (int64_t)r0 * ldu : U + r0 + (int64_t)j0 * ldu, ldu, !trans, 0);
+    oz_split_job x = oz_job(S, Xc + j0, ldx, 0, 0);
+    r.kn = x.kn = j1 - j0;
+    if (!trans) {
+      r.ks = x.ks = f.dexp + j0;
+      r.ksgn = -1;
+    }
+    oz_split_launch(s, r, &x);
+    oz_args a{};
+    a.add = a.neg = 1;
+    RSD_TRY(oz_gemm_launch(ctx, R, S, m, nc, Xc + r0, ldx, a));
+  }
+  return RSD_OK;
+}
+
+}  // namespace
+
+// V = U^-1 by pairs of blocks, [V11, -V11 U12 V22; 0, V22], from the 64-wide
+// inverses on, all pairs of a size at once: few and large products, whose
+// residual grows with the condition number of the blocks.
+static int inverse_by_pairs(rsd_ctx* ctx, int n, const double* d_A, int64_t lda, const rsd_factor64& f, double* V) {
+  cudaStream_t s = ctx->stream;
   pdl_launch(put_diag64, (n + NB64 - 1) / NB64, 256, 0, s, n, f.W, V, n);
   for (int h = NB64; h < n; h *= 2) {
     // pair z: blocks [2 z h, 2 z h + h) and [2 z h + h, min(2 z h + 2 h, n))
@@ -924,13 +999,46 @@ int rsd_potri64(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const rsd_factor6
     b.nstep = 2 * h;
     RSD_TRY(oz_gemm_launch(ctx, R, S, h, c2, T, n, b));
   }
-  oz_op R;
+  return RSD_OK;
+}
+
+// A^-1 (upper triangle) from the factor in A and what potrf left with it, as V
+// V^T with V = U^-1.  V comes by pairs of blocks first; with the rows of V scaled
+// by the diagonal of the factored matrix its largest entry bounds what the pairs
+// add to the residual.  Up to 2^GROWTH64 (mobilities: below 4) A^-1 is formed from
+// it, beyond (near contacts: 1e2 at a gap of 1e-4) the product stands aside for
+// trsm64 on the identity.  ||A X - I|| / (||A|| ||X||) of stiff pairs at 1e4 and
+// 1e8: 12 and 900 eps by pairs, 0.8 and 0.8 by substitution.  N = 512, order 3072:
+// the FP64 step takes 3.6 ms longer that way.
+int rsd_potri64(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const rsd_factor64& f) {
+  RSD_TRY(oz_init(ctx));
+  cudaStream_t s = ctx->stream;
+  double* V = (double*)rsd_scratch(ctx, "potri64_V", sizeof(double) * (size_t)n * n);
+  if (!V) return RSD_ENOMEM;
+  oz_op R, S;  // the largest operands first: the buffers grow once
   RSD_TRY(oz_alloc(ctx, "oz_a", n, n, 1, &R));
-  oz_split_launch(s, oz_job(R, V, n, 1, 1));
-  oz_args a{};
-  a.tri = a.klo_row = a.klo_col = 1;
-  RSD_TRY(oz_gemm_launch(ctx, R, R, n, n, d_A, lda, a));
-  RSD_TRY(read_status(ctx, "potri"));
+  RSD_TRY(oz_alloc(ctx, "oz_b", NBS64, n, 1, &S));
+  RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 3 * sizeof(int), s));
+  for (int exact = 0; exact < 2; exact++) {
+    if (exact) {
+      RSD_CUDA(ctx, cudaMemsetAsync(V, 0, sizeof(double) * (size_t)n * n, s));
+      pdl_launch(put_ones64, (n + 255) / 256, 256, 0, s, n, V);
+      RSD_TRY(trsm64(ctx, n, d_A, lda, f, V, n, n, false, true));
+    } else {
+      RSD_TRY(inverse_by_pairs(ctx, n, d_A, lda, f, V));
+    }
+    RSD_TRY(oz_alloc(ctx, "oz_a", n, n, 1, &R));
+    oz_split_launch(s, oz_job(R, V, n, 1, 1));
+    oz_args a{};
+    a.tri = a.klo_row = a.klo_col = 1;
+    if (!exact) {
+      pdl_launch(growth64, (n + 255) / 256, 256, 0, s, n, R.E, f.dexp, ctx->d_info + 2);
+      a.gate = ctx->d_info + 2;
+    }
+    RSD_TRY(oz_gemm_launch(ctx, R, R, n, n, d_A, lda, a));
+    RSD_TRY(read_status(ctx, "potri"));
+    if (ctx->h_info[2] <= GROWTH64) break;
+  }
   return RSD_OK;
 }
 
@@ -979,75 +1087,6 @@ int rsd_trsv64_bwd(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const doub
   return RSD_OK;
 }
 
-namespace {
-
-// X <- U^-T X (trans) or U^-1 X for many right-hand sides, by blocks as potrf
-// goes: 64 unknowns a step, the product that takes them out of the outer
-// panel's other rows after each step and of all rows beyond it once per panel.
-// A block is solved through its explicit inverse W and corrected once by its
-// residual, which is then that of a substitution whatever the block's
-// condition number (through the inverse of the whole matrix, condition 1e10 and
-// right-hand sides A X0 left 8e-8 of arrangement's result; 1e-15 so).
-// Rows of X and of U^-1 and columns of U carry the scale of the matrix's
-// diagonal (ks, as in potri).  T: 64 x nrhs.
-int trsm64(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const rsd_factor64& f, double* X, int64_t ldx, int nrhs,
-           bool trans, double* T) {
-  RSD_TRY(oz_init(ctx));
-  cudaStream_t s = ctx->stream;
-  // C (rows [r0, r1) of the unknowns) += +-(U^T or U)(rows, [k0, k1)) X([k0, k1)); tri: the diagonal block
-  auto product = [&](int K, int k0, int k1, int r0, int r1, double* C, int64_t ldc, int tri) -> int {
-    if (r1 <= r0) return RSD_OK;
-    oz_op R, S;
-    RSD_TRY(oz_alloc(ctx, "oz_a", K, r1 - r0, 1, &R));
-    RSD_TRY(oz_alloc(ctx, "oz_b", K, nrhs, 1, &S));
-    oz_split_job r = oz_job(R, trans ? U + k0 + (int64_t)r0 * ldu : U + r0 + (int64_t)k0 * ldu, ldu, !trans, tri);
-    oz_split_job x = oz_job(S, X + k0, ldx, 0, 0);
-    r.kn = x.kn = k1 - k0;
-    if (!trans) {
-      r.ks = x.ks = f.dexp + k0;
-      r.ksgn = -1;
-    }
-    oz_split_launch(s, r, &x);
-    oz_args a{};
-    a.add = a.neg = 1;
-    return oz_gemm_launch(ctx, R, S, r1 - r0, nrhs, C, ldc, a);
-  };
-  // X([j0, j1)) = or += (W^T or W) B, W the inverse of the diagonal block
-  auto inverse = [&](int j0, int j1, const double* B, int64_t ldb, int add) -> int {
-    oz_op R, S;
-    RSD_TRY(oz_alloc(ctx, "oz_w", NB64, NB64, 1, &R));
-    RSD_TRY(oz_alloc(ctx, "oz_b", NB64, nrhs, 1, &S));
-    oz_split_job w = oz_job(R, f.W + (size_t)(j0 / NB64) * NB64 * NB64, NB64, !trans, 1);
-    oz_split_job x = oz_job(S, B, ldb, 0, 0);
-    w.kn = x.kn = j1 - j0;
-    if (trans) {
-      w.ks = x.ks = f.dexp + j0;
-      x.ksgn = -1;
-    }
-    oz_split_launch(s, x, &w);
-    oz_args a{};
-    a.add = add;
-    return oz_gemm_launch(ctx, R, S, j1 - j0, nrhs, X + j0, ldx, a);
-  };
-  const int last = (n - 1) / NBO64 * NBO64;
-  for (int P = 0; P <= last; P += NBO64) {
-    const int J0 = trans ? P : last - P, J1 = std::min(n, J0 + NBO64), nb = (J1 - J0 + NB64 - 1) / NB64;
-    for (int q = 0; q < nb; q++) {
-      const int j0 = J0 + (trans ? q : nb - 1 - q) * NB64, j1 = std::min(n, j0 + NB64);
-      RSD_CUDA(ctx, cudaMemcpy2DAsync(T, sizeof(double) * NB64, X + j0, sizeof(double) * ldx, sizeof(double) * (j1 - j0),
-                                      nrhs, cudaMemcpyDeviceToDevice, s));
-      RSD_TRY(inverse(j0, j1, T, NB64, 0));
-      RSD_TRY(product(NB64, j0, j1, j0, j1, T, NB64, 1));
-      RSD_TRY(inverse(j0, j1, T, NB64, 1));
-      RSD_TRY(trans ? product(NB64, j0, j1, j1, J1, X + j1, ldx, 0) : product(NB64, j0, j1, J0, j0, X + J0, ldx, 0));
-    }
-    RSD_TRY(trans ? product(NBO64, J0, J1, J1, n, X + J1, ldx, 0) : product(NBO64, J0, J1, 0, J0, X, ldx, 0));
-  }
-  return RSD_OK;
-}
-
-}  // namespace
-
 // Solve (U^T U) X = B in place with the factor of `tag`: substitution, a
 // launch per 64 unknowns for up to 4 right-hand sides, on the tensor cores for
 // more (arrangement, matrices.f90:432-445).
@@ -1068,12 +1107,10 @@ int rsd_potrs_upper_tag(rsd_ctx* ctx, int n, const double* d_U, int64_t ldu, dou
     return RSD_OK;
   }
   oz_op big;  // the largest operands first: the buffers grow once
-  RSD_TRY(oz_alloc(ctx, "oz_a", NBO64, n, 1, &big));
-  RSD_TRY(oz_alloc(ctx, "oz_b", NBO64, nrhs, 1, &big));
-  double* T = (double*)rsd_scratch(ctx, "potrs64_T", sizeof(double) * NB64 * (size_t)nrhs);
-  if (!T) return RSD_ENOMEM;
+  RSD_TRY(oz_alloc(ctx, "oz_a", NBS64, n, 1, &big));
+  RSD_TRY(oz_alloc(ctx, "oz_b", NBS64, nrhs, 1, &big));
   RSD_CUDA(ctx, cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), s));
-  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, true, T));
-  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, false, T));
+  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, true, false));
+  RSD_TRY(trsm64(ctx, n, d_U, ldu, f, d_X, ldx, nrhs, false, false));
   return read_status(ctx, "potrs");
 }

@@ -63,3 +63,13 @@ def test_factor_residual(rsd, ctx, n):
     L = rsd.CHOLESKY(ctx, A).astype(np.longdouble)
     d = np.sqrt(np.diag(A))
     assert np.abs((A - L @ L.T) / np.outer(d, d)).max() <= n * EPS
+
+
+@pytest.mark.parametrize("make,n,x", [(stiff_pairs, 129, 1e-8), (stiff_pairs, 300, 1e-8), (stiff_pairs, 391, 1e-7),
+                                      (spd, 300, 1e12), (spd, 520, 1e12)])
+def test_inverse_residual(rsd, ctx, make, n, x):
+    """||A X - I|| <= n eps ||A|| ||X||: columns of the inverse by substitution."""
+    A = make(n, x, n)
+    X, info = rsd.MATREV(ctx, A)
+    E = (A.astype(np.longdouble) @ X - np.eye(n)).astype(np.float64)
+    assert info == 0 and np.linalg.norm(E) <= n * EPS * np.linalg.norm(A) * np.linalg.norm(X)
