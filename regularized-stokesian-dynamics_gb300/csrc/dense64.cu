@@ -9,17 +9,21 @@
 //   - an operand column is scaled by a power of two to |x| < 1, rounded to
 //     56 bits and cut into 7 signed base-256 digits (-128..128), each exact
 //     in bf16 (oz_split); where the terms of a sum pair a small factor with a
-//     large one (U^-1 against U), k is scaled by a power of two too, so that
-//     a badly scaled matrix is no worse off than in FP64 arithmetic;
+//     large one (U^-1 against U), k is scaled by a power of two too;
 //   - digit products are integers of at most 2^14; those of one weight s = i
 //     + j are summed in one FP32 accumulator of tensor memory, exactly: K =
 //     128 of them in up to 7 pairs stay below 2^24 (oz_gemm);
-//   - every 128 of K the 7 accumulators (s = 0..6; the dropped ones weigh
-//     2^-58 and less of the largest product) are added into two 64-bit
+//   - every 128 of K the 8 accumulators (s = 0..7) are added into two 64-bit
 //     integers per output, which become one FP64 value at the end.
-// A product is therefore off by about 2^-56 of the product of its columns'
-// largest entries per term, with no rounding in the sum: not more than an
-// FP64 multiply-add chain.
+// Of a term x y, |x|, |y| < 1, the weights left out (s = 8..12) come to less
+// than 2^-61, and the entries' roundings to at most 2^-56 (|x| + |y|), none
+// for entries within a factor of 4 of the largest; there is no rounding in the
+// sum.  (With s = 7 left out too it was up to 2^-53.4 a term, 2^-56.3 in the
+// mean, and residuals of well-conditioned inverses three times those of FP64
+// multiply-adds.)  So a product is off by at most about 2^-54 of its columns'
+// largest entries per term: normwise what a chain of FP64 multiply-adds may be off, not
+// entry by entry, which is why the ill-conditioned solves and inverses below do
+// not multiply by inverses.
 //
 // Layout: both operands are K-major (K contiguous), split beforehand into
 // slices [digit][batch][column][K] of bf16; C(r, c) = sum_k R(k, r) S(k, c).
@@ -50,7 +54,7 @@
 
 namespace {
 
-constexpr int OZ_S = 7;                     // digits
+constexpr int OZ_S = 7, OZ_W = 8;           // digits, and weights kept of their products
 constexpr int OZ_TC = 128, OZ_TR = 64;      // columns and rows of a C tile (MMA M and N)
 constexpr int OZ_KC = 32;                   // K of a stage: 64-byte rows, 64-byte swizzle
 constexpr int OZ_GROUP = 4;                 // stages between two drains: K = 128
@@ -58,7 +62,7 @@ constexpr int OZ_A = OZ_TC * OZ_KC * 2, OZ_B = OZ_TR * OZ_KC * 2;
 constexpr int OZ_STAGES = 2, OZ_STAGE = OZ_S * (OZ_A + OZ_B);
 constexpr int OZ_SMEM = OZ_STAGES * OZ_STAGE + 1024 + 128;
 constexpr int OZ_THREADS = 320;             // TMA, MMA, 8 drain warps
-constexpr int OZ_TMEM = 512;                // 7 x 64 columns used
+constexpr int OZ_TMEM = OZ_W * OZ_TR;
 constexpr int OZ_NONFINITE = 1 << 20;       // exponent of a column that holds an infinity or a NaN
 constexpr int OZ_ZERO = -(1 << 20);
 constexpr unsigned long long OZ_WAIT_NS = 500ull * 1000 * 1000;
@@ -233,12 +237,12 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint32_t a, uint32_t b, int
       "l"(desc_sw64(a)), "l"(desc_sw64(b)), "r"(idesc), "r"(acc));
 }
 
-// sgn (hi + lo 2^-24) 2^e, rounded to nearest, with integer operations (two
+// sgn (hi + lo 2^-32) 2^e, rounded to nearest, with integer operations (two
 // 64-bit conversions and a scaling would take the FP64 pipe ~27 cycles per
 // output and SM lane pair; 2 per cycle and SM is all it does)
 __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, unsigned long long sgn) {
-  unsigned long long L = (unsigned long long)hi << 24;
-  long long H = (hi >> 40) + (lo >> 63);
+  unsigned long long L = (unsigned long long)hi << 32;
+  long long H = (hi >> 32) + (lo >> 63);
   L += (unsigned long long)lo;
   H += L < (unsigned long long)lo;
   if (H < 0) {  // magnitude; the sign goes into the result's bits
@@ -249,7 +253,7 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, un
   unsigned long long m;
   int p;
   if (H) {
-    const int lz = __clzll(H);  // 0 < H < 2^40: 23 < lz < 64
+    const int lz = __clzll(H);  // 0 < H < 2^32: 31 < lz < 64
     m = (unsigned long long)H << lz | L >> (64 - lz);
     p = 127 - lz;
   } else {
@@ -257,11 +261,11 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, un
     m = L << lz;
     p = 63 - lz;
   }
-  const int E = p + e - 24 + 1023;
+  const int E = p + e - 32 + 1023;
   unsigned long long r = (m >> 11) + ((m >> 10) & 1);  // 53 bits, the leading one counts into the exponent
   if (m == 0) return __longlong_as_double((long long)sgn);
   if (E < 1 || E > 2046) {  // out of FP64's normal range
-    const double v = ldexp((double)r, p - 52 + e - 24);
+    const double v = ldexp((double)r, p - 52 + e - 32);
     return sgn >> 63 ? -v : v;
   }
   return __longlong_as_double((long long)(((unsigned long long)(E - 1) << 52) + r) ^ (long long)sgn);
@@ -280,7 +284,7 @@ __device__ __forceinline__ double oz_value(long long hi, long long lo, int e, un
 // slices of R lie one after another in shared memory, so one MMA multiplies
 // digit i of S with several digits of R at once: its N columns land in the
 // accumulators s = i, i + 1, ... which are neighbours in tensor memory.
-// Bound: 8 x 896 cycles of MMA per K = 128, then the drain (7 x 8192 values
+// Bound: 8 x 1088 cycles of MMA per K = 128, then the drain (8 x 8192 values
 // into integers) and, once per tile, the conversion (~40 integer
 // instructions) and an FP64 addition per output.  Measured in the FP64 step
 // at N = 512 (factor of order 5632, inverse and factor of 3072): 9.5 ms of
@@ -379,10 +383,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
           const uint32_t first = (c % OZ_GROUP == 0 && kk == 0) ? 0u : 1u;
 #pragma unroll
           for (int i = 0; i < OZ_S; i++) {
-            const int w = OZ_S - i;  // digits 0..w-1 of R
-            const uint32_t sa = st + i * OZ_A + kk * 32, sb = sr + kk * 32;
-            mma_bf16(taddr + i * OZ_TR, sa, sb, OZ_TR * min(w, 4), i == 0 ? first : 1u);
-            if (w > 4) mma_bf16(taddr + (i + 4) * OZ_TR, sa, sb + 4 * OZ_B, OZ_TR * (w - 4), i == 0 ? first : 1u);
+            const int w = min(OZ_S, OZ_W - i);  // digits 0..w-1 of R
+            const uint32_t sa = st + i * OZ_A + kk * 32, sb = sr + kk * 32, acc = i == 0 ? first : 1u;
+            mma_bf16(taddr + i * OZ_TR, sa, sb, OZ_TR * min(w, 4), acc);
+            if (i == 1) {  // the first of weight 7
+              mma_bf16(taddr + 5 * OZ_TR, sa, sb + 4 * OZ_B, OZ_TR * 2, 1u);
+              mma_bf16(taddr + 7 * OZ_TR, sa, sb + 6 * OZ_B, OZ_TR, first);
+            } else if (w > 4) {
+              mma_bf16(taddr + (i + 4) * OZ_TR, sa, sb + 4 * OZ_B, OZ_TR * (w - 4), acc);
+            }
           }
         }
         mma_commit(OZ_EMPTY(s));
@@ -409,7 +418,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-      for (int s = 0; s < OZ_S; s++) {
+      for (int s = 0; s < OZ_W; s++) {
 #pragma unroll
         for (int jh = 0; jh < 32; jh += 16) {
           uint32_t v[16];
@@ -421,7 +430,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm(const __grid_constant__
             if (s < 4)
               hi[jh + j] += (long long)d * (1 << (8 * (3 - s)));
             else
-              lo[jh + j] += (long long)d * (1 << (8 * (6 - s)));
+              lo[jh + j] += (long long)d * (1 << (8 * (7 - s)));
           }
         }
       }

@@ -73,3 +73,23 @@ def test_inverse_residual(rsd, ctx, make, n, x):
     X, info = rsd.MATREV(ctx, A)
     E = (A.astype(np.longdouble) @ X - np.eye(n)).astype(np.float64)
     assert info == 0 and np.linalg.norm(E) <= n * EPS * np.linalg.norm(A) * np.linalg.norm(X)
+
+
+def test_digits_of_one_sign(rsd, ctx):
+    """Columns whose lower digits are all -128, so that the digit products of
+    every weight add up with one sign over all 256 terms, while the products
+    themselves cancel: A = [I B; B^T C], B exact in 56 bits, whose factor holds
+    C - B^T B in its last block.  Off the diagonal B^T B is near -1; the weights
+    left out may come to 256 2^-61, its rounding and those of the last block's
+    factor to 4 eps."""
+    tail = sum(2.0 ** (-8 * i) for i in range(1, 7))
+    B = np.full((256, 2), 0.5 - tail)
+    B[::2, 1] = -(0.5 + tail)
+    B[255] = 0.75
+    A = np.eye(258)
+    A[:256, 256:], A[256:, :256] = B, B.T
+    A[256:, 256:] = B.T @ B + np.eye(2)
+    L = rsd.CHOLESKY(ctx, A)
+    assert np.array_equal(L[256:, :256], B.T)
+    R = A[256:, 256:].astype(np.longdouble) - L[256:].astype(np.longdouble) @ L[256:].T.astype(np.longdouble)
+    assert abs(float(R[0, 1])) <= 256 * 2.0 ** -61 + 4 * EPS
