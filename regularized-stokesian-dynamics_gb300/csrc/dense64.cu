@@ -504,20 +504,20 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
   pdl_enter();
   __shared__ double S[NB64 * PF_LD];  // S(i, j) at [i * PF_LD + j]
   __shared__ double l[2][NB64], sq[NB64], rd[NB64];
-  __shared__ int failed;
+  __shared__ int failed[2];  // pivot k's verdict in [k & 1]: read in step k, while the next one is made
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int e = t; e < NB64 * NB64; e += 256) {
     const int i = e % NB64, j = e / NB64;
     S[i * PF_LD + j] = i <= j && j < jb ? A[i + (int64_t)j * lda] : (i == j ? 1.0 : 0.0);
   }
-  if (t == 0) failed = 0;
+  if (t < 2) failed[t] = 0;
   __syncthreads();
   // multipliers l_ik of pivot k (d its value) into l[k & 1]
   auto pivot = [&](int k, double d) {
     const long long bits = __double_as_longlong(d);  // positive and finite, off the FP64 pipe
     if (bits <= 0 || bits >= 0x7ff0000000000000LL) {
       if (lane == 0) {
-        failed = 1;
+        failed[k & 1] = 1;
         atomicCAS(info, 0, j0 + k + 1);
       }
       return;
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
   if (warp == 0) pivot(0, S[0]);
   __syncthreads();
   for (int k = 0; k < NB64 - 1; k++) {
-    if (failed) return;
+    if (failed[k & 1]) return;
     const double* lk = l[k & 1];
     // row k; in column k the identity enters: 0 - l_ik 1
     const double s0 = lane == k ? 1.0 : S[k * PF_LD + lane], s1 = lane + 32 == k ? 1.0 : S[k * PF_LD + lane + 32];
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
     }
     __syncthreads();
   }
-  if (failed) return;
+  if (failed[(NB64 - 1) & 1]) return;
   if (t < NB64) {
     sq[t] = sqrt(S[t * PF_LD + t]);
     rd[t] = 1.0 / sq[t];
