@@ -96,8 +96,10 @@ inline unsigned blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
 
 // Factors M' of the grand mobility in M (the upper triangle of the
-// reference's order is read) and forms A^-1 in full.  A positive info is
-// DPOTRF's on M in the reference's order; M is then overwritten.
+// reference's order is read) and forms A^-1 in full.  A matrix within rounding of
+// a singular one may have a positive definite factor in the one order only: then
+// M itself is factored and inverted, like MATREV, and h holds M^-1 in M.  A
+// positive info is DPOTRF's on M in the reference's order; M is then overwritten.
 int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int* info) {
   const int64_t P = 6LL * nn, Q = 5LL * nn;
   h->P = P;
@@ -113,9 +115,14 @@ int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int*
   int inf = 0;
   RSD_TRY(rsd_potrf_upper_tag(ctx, (int)h->np, h->Mp, h->np, &inf, "mob"));
   if (inf) {
-    int own = 0;
-    RSD_TRY(rsd_potrf_upper_tag(ctx, (int)(P + Q), M, ld, &own, "mob"));
-    *info = own ? own : inf;
+    RSD_TRY(rsd_potrf_upper_tag(ctx, (int)(P + Q), M, ld, info, "mob"));
+    if (*info) return RSD_OK;
+    RSD_TRY(rsd_potri_upper_tag(ctx, (int)(P + Q), M, ld, "mob"));
+    RSD_TRY(rsd_mirror_upper(ctx, (int)(P + Q), M, ld));
+    h->R = M;
+    h->ldr = ld;
+    RSD_CUDA(ctx, cudaMemcpy2DAsync(h->Ai, sizeof(double) * P, M, sizeof(double) * ld, sizeof(double) * P, P,
+                                    cudaMemcpyDeviceToDevice, s));
     return RSD_OK;
   }
   *info = 0;
@@ -128,6 +135,10 @@ int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int*
 
 // f0 = (M^-1)_PQ ein (length P); z = U_QQ^-T ein (length Qp) is kept in h
 int rsd_r64_pq(rsd_ctx* ctx, rsd_r64* h, const double* ein, double* f0) {
+  if (h->R) {
+    h->ein = ein;
+    return rsd_gemv<double>(ctx, 0, (int)h->P, (int)h->Q, 1.0, h->R + h->P * h->ldr, h->ldr, ein, h->Q, 1, 0.0, f0, h->P);
+  }
   double* w = (double*)rsd_scratch(ctx, "r64_z", sizeof(double) * (size_t)(2 * h->Qp + h->P));
   if (!w) return RSD_ENOMEM;
   h->z = w;
@@ -140,8 +151,13 @@ int rsd_r64_pq(rsd_ctx* ctx, rsd_r64* h, const double* ein, double* f0) {
 }
 
 // S(:, 0) = (M^-1)_QP Y(:, 0) - (M^-1)_QQ ein, S(:, r) = (M^-1)_QP Y(:, r)
-// for r > 0 (ein and f0 of rsd_r64_pq); Y: P x nr, S: Q x nr, nr <= 4
+// for r > 0 (ein and f0 of rsd_r64_pq, unchanged since); Y: P x nr, S: Q x nr, nr <= 4
 int rsd_r64_stresslet(rsd_ctx* ctx, rsd_r64* h, const double* Y, int nr, const double* f0, double* S) {
+  if (h->R) {
+    const int P = (int)h->P, Q = (int)h->Q;
+    RSD_TRY(rsd_gemv<double>(ctx, 1, Q, P, 1.0, h->R + h->P * h->ldr, h->ldr, Y, P, nr, 0.0, S, Q));
+    return rsd_gemv<double>(ctx, 0, Q, Q, -1.0, h->R + h->P * (h->ldr + 1), h->ldr, h->ein, Q, 1, 1.0, S, Q);
+  }
   double* w = (double*)rsd_scratch(ctx, "r64_s", sizeof(double) * (size_t)nr * (h->P + 2 * h->Qp));
   if (!w) return RSD_ENOMEM;
   cudaStream_t s = ctx->stream;

@@ -270,6 +270,9 @@ struct rsd_r64 {
   double* Ai = nullptr;  // (M^-1)_PP, full
   rsd_factor64 f;
   double* z = nullptr;
+  const double* R = nullptr;  // M^-1 in full, in place of the factor of M'
+  int64_t ldr = 0;
+  const double* ein = nullptr;
 };
 int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int* info);
 int rsd_r64_pq(rsd_ctx* ctx, rsd_r64* h, const double* ein, double* f0);
