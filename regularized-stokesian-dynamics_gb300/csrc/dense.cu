@@ -1134,13 +1134,9 @@ T* diag_inverses(rsd_ctx* ctx, int n, const char* tag) {
 
 template <typename T>
 int ensure_attrs(rsd_ctx* ctx) {
-  static bool done = false;
-  if (done) return RSD_OK;
-  RSD_CUDA(ctx, cudaFuncSetAttribute(trtri_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_potf2<T>(NB)));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_inv_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_POTF2_INV));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(potf2_gj_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
-  done = true;
-  return RSD_OK;
+  RSD_TRY(rsd_smem(ctx, trtri_diag<T>, smem_potf2<T>(NB)));
+  RSD_TRY(rsd_smem(ctx, potf2_inv_f32, SMEM_POTF2_INV));
+  return rsd_smem(ctx, potf2_gj_f32, GJ_SMEM);
 }
 
 }  // namespace

@@ -753,22 +753,10 @@ __global__ void growth64(int n, const int* __restrict__ e, const int* __restrict
 }
 
 // ------------------------------------------------------------------- host
-PFN_cuTensorMapEncodeTiled_v12000 g_encode64 = nullptr;
-
 int oz_init(rsd_ctx* ctx) {
-  if (g_encode64) return RSD_OK;
-  cudaDriverEntryPointQueryResult q;
-  void* fn = nullptr;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-      !fn || q != cudaDriverEntryPointSuccess) {
-    cudaGetLastError();
-    return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled is not available");
-  }
-  RSD_CUDA(ctx, cudaFuncSetAttribute(oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(subst64<NBS64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM<NBS64>));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(subst64<NBS64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM<NBS64>));
-  g_encode64 = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-  return RSD_OK;
+  RSD_TRY(rsd_smem(ctx, oz_gemm, OZ_SMEM));
+  RSD_TRY(rsd_smem(ctx, subst64<NBS64, false>, SUB_SMEM<NBS64>));
+  return rsd_smem(ctx, subst64<NBS64, true>, SUB_SMEM<NBS64>);
 }
 
 // A split operand: nb batches of `cols` columns of K entries each.
@@ -812,7 +800,9 @@ int oz_map(rsd_ctx* ctx, CUtensorMap* tm, const oz_op& o, int box_rows) {
   const cuuint64_t strides[1] = {(cuuint64_t)o.Kld * 2};
   const cuuint32_t box[2] = {OZ_KC, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode64(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, o.D, dims, strides, box, estr,
+  PFN_cuTensorMapEncodeTiled_v12000 encode = rsd_tensor_map_encoder();
+  if (!encode) return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled is not available");
+  CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, o.D, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled failed (%d)", (int)r);

@@ -1699,12 +1699,7 @@ namespace {
 template <int NP, int MINB>
 int launch_real_eq_t(rsd_ctx* ctx, dim3 grd, dim3 blk, int nn, const rsd_lat_dev& L, const double* d_pos,
                      const dsf* cr, const float* cf, float rc2, float rmax2, const PlaneSink& psk) {
-  static bool attr = false;
-  if (!attr) {
-    RSD_CUDA(ctx, cudaFuncSetAttribute(ewald_pair_real_eq<NP, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       SMEM_REAL_EQ));
-    attr = true;
-  }
+  RSD_TRY(rsd_smem(ctx, ewald_pair_real_eq<NP, MINB>, SMEM_REAL_EQ));
   pdl_launch(ewald_pair_real_eq<NP, MINB>, grd, blk, SMEM_REAL_EQ, ctx->stream, nn, L, d_pos, cr, cf, rc2, rmax2, psk);
   return RSD_OK;
 }
@@ -1727,8 +1722,7 @@ int real_slices(rsd_ctx* ctx, cudaStream_t s, int S, dim3 grd, dim3 blk, int nn,
                 const double* d_pos, float rc2, float rmax2) {
   slice_parts p;
   RSD_TRY(slice_buffers(ctx, S, nn, &p));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(ewald_real_slices, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(RealSliceShared)));
+  RSD_TRY(rsd_smem(ctx, ewald_real_slices, (int)sizeof(RealSliceShared)));
   grd.z = S;
   pdl_launch(ewald_real_slices, grd, blk, sizeof(RealSliceShared), s, nn, L, d_pos, rc2, rmax2, p.near, p.far);
   RSD_CUDA(ctx, cudaEventRecord(ctx->ev_panel, s));
@@ -2095,8 +2089,7 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
       } else if (equal) {
         RSD_TRY(launch_real_eq(ctx, ctx->mixed_real_passes, grd, blk, nn, L, d_pos, cr, cf, (float)rc2, (float)rmax2, psk));
       } else {
-        RSD_CUDA(ctx, cudaFuncSetAttribute(ewald_pair_real_mix, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(RealMixShared)));
+        RSD_TRY(rsd_smem(ctx, ewald_pair_real_mix, (int)sizeof(RealMixShared)));
         pdl_launch(ewald_pair_real_mix, grd, blk, sizeof(RealMixShared), s, nn, L, d_pos, d_radii, inv_pimu, (float)rc2,
                    (float)rmax2, psk);
       }

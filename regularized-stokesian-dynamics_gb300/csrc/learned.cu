@@ -1125,12 +1125,7 @@ template <typename T>
 static int lp_exact_fsai(rsd_ctx* ctx, const lp_graph& g, const T* A, int64_t ld, const double* dinv, int self_only,
                          float* zd, float* ze, float* wt = nullptr) {
   cudaStream_t s = ctx->stream;
-  static bool attr[2] = {false, false};
-  const int which = sizeof(T) == 8;
-  if (!attr[which]) {
-    RSD_CUDA(ctx, cudaFuncSetAttribute(lp_fsai<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_LOCAL_SMEM));
-    attr[which] = true;
-  }
+  RSD_TRY(rsd_smem(ctx, lp_fsai<T>, (int)LP_LOCAL_SMEM));
   int* bad = ctx->d_info + 10;
   RSD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(int), s));
   pdl_launch(lp_fsai<T>, g.nn, FS_THREADS, LP_LOCAL_SMEM, s, g.nn, self_only, A, ld, dinv, g.off, g.src, g.gap, zd, ze, wt, bad); RSD_LP_CHECK();
@@ -1148,11 +1143,7 @@ struct lp_acts {
 static int lp_layer(rsd_ctx* ctx, const LayerArgs& a) {
   if (a.rows <= 0) return RSD_OK;
   const size_t smem = sizeof(float) * ((size_t)a.kin * a.kout + (size_t)LW * LR4 * a.kin);
-  static bool attr = false;
-  if (!attr) {
-    RSD_CUDA(ctx, cudaFuncSetAttribute(lp_layer_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    attr = true;
-  }
+  RSD_TRY(rsd_smem(ctx, lp_layer_fwd, 96 * 1024));
   const int grid = (int)std::min<int64_t>((a.rows + LW * LR4 - 1) / (LW * LR4), 2LL * (ctx->sm_count > 0 ? ctx->sm_count : 148));
   pdl_launch(lp_layer_fwd, grid, 32 * LW, smem, ctx->stream, a); RSD_LP_CHECK();
   return RSD_OK;
@@ -1221,11 +1212,7 @@ static int lp_layer_back(rsd_ctx* ctx, rsd_lp* net, LayerBwdArgs b, int64_t w_of
   if (!part) return RSD_ENOMEM;
   b.part = part;
   const size_t smem = sizeof(float) * ((size_t)b.kout * b.kin + (size_t)LB_ROWS * b.kin + (size_t)LB_ROWS * b.kout);
-  static bool attr = false;
-  if (!attr) {
-    RSD_CUDA(ctx, cudaFuncSetAttribute(lp_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    attr = true;
-  }
+  RSD_TRY(rsd_smem(ctx, lp_layer_bwd, 160 * 1024));
   pdl_launch(lp_layer_bwd, nparts, 256, smem, ctx->stream, b); RSD_LP_CHECK();
   pdl_launch(lp_reduce_parts, nb256(nw + b.kout), 256, 0, ctx->stream, nparts, nw, b.kout, part, net->g + w_off,
                                                                 net->g + b_off); RSD_LP_CHECK();
@@ -1304,13 +1291,7 @@ static int lp_make_z(rsd_ctx* ctx, rsd_lp* net, int mode, const lp_graph& g, con
     if (!hd || !wp) return RSD_ENOMEM;
     lp_acts acts;
     RSD_TRY(lp_forward(ctx, net, g, xn, xe, &acts, hd, wp));
-    static bool attr[2] = {false, false};
-    const int which = sizeof(T) == 8;
-    if (!attr[which]) {
-      RSD_CUDA(ctx, cudaFuncSetAttribute(lp_normalize<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)LP_LOCAL_SMEM));
-      attr[which] = true;
-    }
+    RSD_TRY(rsd_smem(ctx, lp_normalize<T>, (int)LP_LOCAL_SMEM));
     pdl_launch(lp_normalize<T>, g.nn, FS_THREADS, LP_LOCAL_SMEM, ctx->stream, g.nn, A, ld, *dinv, g.off, g.src, g.gap, wp,
                                                                       *zd, *ze); RSD_LP_CHECK();
     return RSD_OK;
@@ -1357,7 +1338,7 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
   a.maxit = maxit;
   a.staged = sizeof(double) * (size_t)P <= PCG_STAGE;
   const size_t smem = a.staged ? sizeof(double) * (size_t)P : 0;
-  RSD_CUDA(ctx, cudaFuncSetAttribute(lp_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PCG_STAGE));
+  RSD_TRY(rsd_smem(ctx, lp_pcg_kernel, PCG_STAGE));
   int worst_it = 0;
   double worst_res = 0.0;
   for (int c = 0; c < nrhs; c++) {

@@ -550,7 +550,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   const float* Ml = Mh + (size_t)ld * n;
   if (ld % 4) return rsd_fail(ctx, RSD_EARG, "mixed solve: the planes' leading dimension must be a multiple of 4");
   const int nbt = (int)((n + SYMV_T - 1) / SYMV_T);
-  RSD_CUDA(ctx, cudaFuncSetAttribute(symv_planes_part<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, symv_smem(2)));
+  RSD_TRY(rsd_smem(ctx, symv_planes_part<2>, symv_smem(2)));
   float2* fs = (float2*)rsd_scratch(ctx, "mixed_fs", sizeof(float2) * (size_t)nr * n);
   double* gpart = (double*)rsd_scratch(ctx, "mixed_symv_part", sizeof(double) * 2 * 2 * (size_t)nbt * nbt * SYMV_T);
   if (!fs || !gpart) return RSD_ENOMEM;

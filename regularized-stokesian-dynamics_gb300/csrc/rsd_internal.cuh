@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <atomic>
 #include <map>
+#include <set>
 #include <string>
 
 #include "../../include/rsd_capi.h"
@@ -55,6 +56,7 @@ struct rsd_ctx {
   cudaEvent_t ev_la[4] = {};     // look-ahead events of the two-level Cholesky
   int* d_info = nullptr;  // device-side status words, then the sums that the host reads (rsd_sums)
   int* h_info = nullptr;  // pinned mirror
+  std::set<const void*> smem_kernels;  // kernels granted their dynamic shared memory (rsd_smem)
   void* h_io = nullptr;   // pinned staging of the host entry points (rsd_pinned)
   size_t h_io_bytes = 0;
 };
@@ -92,6 +94,16 @@ int rsd_cuda_check(rsd_ctx* ctx, cudaError_t e, const char* what);
 // allocation failure.
 void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes);
 int rsd_set_device(rsd_ctx* ctx);
+// Dynamic shared memory above 48 KB is granted per kernel and device: asked for
+// at the kernel's first launch from each context.
+template <typename... P>
+int rsd_smem(rsd_ctx* ctx, void (*kernel)(P...), int bytes) {
+  const void* k = reinterpret_cast<const void*>(kernel);
+  if (ctx->smem_kernels.count(k)) return RSD_OK;
+  RSD_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ctx->smem_kernels.insert(k);
+  return RSD_OK;
+}
 // Grow-only pinned host buffer; nothing may be in flight on it.
 void* rsd_pinned(rsd_ctx* ctx, size_t bytes);
 // Scoped NVTX range around a phase of the step (a no-op unless a profiler

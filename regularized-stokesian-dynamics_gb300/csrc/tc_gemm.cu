@@ -538,23 +538,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(2 * TC_TILE));
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-
 int tc_init(rsd_ctx* ctx) {
-  if (g_encode) return RSD_OK;
-  cudaDriverEntryPointQueryResult q;
-  void* fn = nullptr;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-      !fn || q != cudaDriverEntryPointSuccess) {
-    cudaGetLastError();
-    return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled is not available");
-  }
-  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<1>::SMEM));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<3>::SMEM));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_near_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, NearCfg<1>::SMEM));
-  RSD_CUDA(ctx, cudaFuncSetAttribute(tc_near_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, NearCfg<3>::SMEM));
-  g_encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-  return RSD_OK;
+  RSD_TRY(rsd_smem(ctx, tc_gemm_kernel<1>, TcCfg<1>::SMEM));
+  RSD_TRY(rsd_smem(ctx, tc_gemm_kernel<3>, TcCfg<3>::SMEM));
+  RSD_TRY(rsd_smem(ctx, tc_near_kernel<1>, NearCfg<1>::SMEM));
+  return rsd_smem(ctx, tc_near_kernel<3>, NearCfg<3>::SMEM);
 }
 
 int encode_2d(rsd_ctx* ctx, CUtensorMap* tm, const float* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
@@ -564,7 +552,9 @@ int encode_2d(rsd_ctx* ctx, CUtensorMap* tm, const float* ptr, uint64_t inner, u
   const cuuint64_t strides[1] = {(cuuint64_t)(ld * sizeof(float))};
   const cuuint32_t box[2] = {box_inner, box_outer};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)ptr, dims, strides, box, estr,
+  PFN_cuTensorMapEncodeTiled_v12000 encode = rsd_tensor_map_encoder();
+  if (!encode) return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled is not available");
+  CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)ptr, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return rsd_fail(ctx, RSD_EUNSUP, "cuTensorMapEncodeTiled failed (%d)", (int)r);

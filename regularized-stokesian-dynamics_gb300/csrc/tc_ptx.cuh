@@ -61,4 +61,19 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// The driver's tensor-map encoder, looked up once (thread-safe); null if absent.
+inline PFN_cuTensorMapEncodeTiled_v12000 rsd_tensor_map_encoder() {
+  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+    cudaDriverEntryPointQueryResult q;
+    void* fn = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return (PFN_cuTensorMapEncodeTiled_v12000)fn;
+  }();
+  return encode;
+}
+
 }  // namespace
