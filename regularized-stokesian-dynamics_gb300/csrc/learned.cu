@@ -965,7 +965,10 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) lp_pcg_kernel(PcgArgs g) {
     pcg_part(s, red, pr + blockIdx.x);
     if (!pcg_barrier(g, ++turn)) return;
     rn = sqrt(pcg_total(pr, red));
-    if (it == 0) bn = rn > 0.0 ? rn : 1.0;
+    if (it == 0) {
+      bn = rn > 0.0 ? rn : 1.0;
+      for (int i = gt; i < P; i += nthr) g.x[i] = 0.0;  // b has been read: x may be b's memory
+    }
     if (!(rn > g.tol * bn) || it >= g.maxit || !isfinite(rn)) break;
     // ---- z
     s = 0.0;
@@ -1344,7 +1347,6 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
   for (int c = 0; c < nrhs; c++) {
     a.b = b + (size_t)c * P;
     a.x = x + (size_t)c * P;
-    RSD_CUDA(ctx, cudaMemsetAsync(a.x, 0, sizeof(double) * P, s));
     RSD_CUDA(ctx, cudaMemsetAsync(a.bar, 0, 2 * sizeof(int), s));
     void* args[] = {&a};
     RSD_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)lp_pcg_kernel, dim3(grid), dim3(PCG_THREADS), args, smem, s)); RSD_LAUNCH_NOTE();

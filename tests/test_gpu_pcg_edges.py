@@ -1,6 +1,9 @@
 """The PCG of the resistance solve at its edges: right-hand sides that hold a
 NaN or an infinity are refused with RSD_ENAN (by the solve and by the FP64 step
-that uses it), as the factorisation path refuses them."""
+that uses it), as the factorisation path refuses them; the solution may overwrite
+the right-hand side."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -56,3 +59,22 @@ def test_step_with_a_nan_force(rsd, system, mode):
     with pytest.raises(rsd.RSDError) as e:
         rsd.STEPPER_Stokesian(ctx, s["tab"], s["pos"], s["radii"], 0.0, 1e-3, [s["L"]] * 3, 1.0, s["mu"], 1e-10, Fe=Fe)
     assert e.value.code == rsd.RSD_ENAN
+
+
+@pytest.mark.parametrize("mode", ["PC_NONE", "PC_JACOBI", "PC_FSAI"])
+def test_solution_in_place_of_the_right_hand_side(rsd, system, mode):
+    import torch
+    s = system
+    m = getattr(rsd, mode)
+    b = torch.tensor(s["b"], device="cuda")
+    ref, it0, _ = rsd.pcg_dev(s["ctx"], None, m, s["pos_t"], s["radii_t"], s["lat"], s["rpp"], b)
+    it, res = ctypes.c_int32(0), ctypes.c_double(0.0)
+    torch.cuda.synchronize()
+    s["ctx"].check(rsd.library().rsd_lp_pcg_dev(s["ctx"].h, None, m, s["N"], s["pos_t"].data_ptr(),
+                                                s["radii_t"].data_ptr(), ctypes.byref(s["lat"]), s["rpp"].data_ptr(),
+                                                s["rpp"].stride(1), 2, b.data_ptr(), b.data_ptr(), 1e-12, 2000,
+                                                ctypes.byref(it), ctypes.byref(res)))
+    assert it.value == it0 and res.value <= 1e-12 and bool((b == ref).all())
+    zero = torch.zeros_like(ref)  # no iteration: x is still written
+    x, it, res = rsd.pcg_dev(s["ctx"], None, m, s["pos_t"], s["radii_t"], s["lat"], s["rpp"], zero)
+    assert it == 0 and res == 0.0 and bool((x == 0).all())
