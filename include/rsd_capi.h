@@ -126,11 +126,12 @@ int rsd_ctx_set_correction_method(rsd_ctx* ctx, int32_t method);
  * iterations (1..30, 0: 30).  A solve that ends above 100 times the
  * tolerance returns RSD_ENOCONV. */
 int rsd_ctx_set_refinement(rsd_ctx* ctx, int32_t mode, int32_t restart);
-/* Bounds of the device-side waits of the mixed form's FP32 kernels (no
- * counterpart in the reference): every mbarrier wait of the tensor-core
- * GEMMs gives up after tc_wait_ns nanoseconds (0: the default, 0.5 s), and
- * every wait of the refinement's dataflow triangular sweeps after
- * tri_spin_polls polls of at least 64 ns (0: the default, 2^21).  A wait
+/* Bounds of the device-side waits (no counterpart in the reference): every
+ * mbarrier wait of the tensor-core products, FP32 and FP64, gives up after
+ * tc_wait_ns nanoseconds (0: the default, 0.5 s); every wait of the mixed
+ * form's dataflow triangular sweeps (0: the default, 2^21 polls) and of the
+ * PCG's grid barriers (0: 2^25) after tri_spin_polls polls, some tens of
+ * nanoseconds each.  A wait
  * that gives up ends its kernel without a fault: the kernel drains the
  * copies and MMAs it issued, frees its tensor memory, skips its stores and
  * raises an error word; the call returns RSD_ETIMEOUT and the context stays

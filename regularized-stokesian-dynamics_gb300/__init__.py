@@ -198,8 +198,9 @@ class Context:
         self.check(_lib.rsd_ctx_set_correction_method(self.h, int(method)))
 
     def set_wait_limits(self, tc_wait_ns=0, tri_spin_polls=0):
-        """Bounds of the mixed form's device-side waits (0: the defaults,
-        0.5 s and 2^21 polls); a wait that gives up makes the call return
+        """Bounds of the device-side waits: nanoseconds of the tensor-core
+        products' (0: 0.5 s), polls of the triangular sweeps' and the PCG's
+        (0: 2^21 and 2^25); a wait that gives up makes the call return
         RSD_ETIMEOUT."""
         self.check(_lib.rsd_ctx_set_wait_limits(self.h, int(tc_wait_ns), int(tri_spin_polls)))
 

@@ -849,7 +849,8 @@ struct PcgArgs {
   const double* b;
   double *x, *r[2], *p[2], *z, *q, *tmp;
   double* part;  // 3 x gridDim.x
-  int* bar;      // [0] arrivals, [1] error
+  unsigned* bar;    // [0] arrivals, [1] error
+  long long polls;  // bound of a wait
   double* out;   // iterations, |r|, |b|
   double tol;
   int maxit, staged;
@@ -857,20 +858,22 @@ struct PcgArgs {
 constexpr int PCG_THREADS = 512;
 constexpr int PCG_STAGE = 200 * 1024;  // p staged in shared memory up to this many bytes
 
-// Waits until every CTA has arrived `turn` times; false when the wait ran out
-// (bounded, ~2 s) here or elsewhere, which ends the kernel.
-__device__ __forceinline__ bool pcg_barrier(const PcgArgs& g, int turn) {
+constexpr long long PCG_POLLS = 1LL << 25;  // a second or two
+
+// Waits until every CTA has arrived `turn` times (counted modulo 2^32); false
+// when the wait ran out here or elsewhere, which ends the kernel.
+__device__ __forceinline__ bool pcg_barrier(const PcgArgs& g, unsigned turn) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     ok = 1;
     __threadfence();
-    atomicAdd(g.bar, 1);
-    const int target = turn * (int)gridDim.x;
+    atomicAdd(g.bar, 1u);
+    const unsigned target = turn * gridDim.x;
     long long polls = 0;
-    while (*((volatile int*)g.bar) < target) {
-      if (*((volatile int*)(g.bar + 1)) || ++polls > (1LL << 25)) {
-        atomicExch(g.bar + 1, 1);
+    while ((int)(*((volatile unsigned*)g.bar) - target) < 0) {
+      if (*((volatile unsigned*)(g.bar + 1)) || ++polls > g.polls) {
+        atomicExch(g.bar + 1, 1u);
         ok = 0;
         break;
       }
@@ -925,7 +928,8 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) lp_pcg_kernel(PcgArgs g) {
   auto gi = [&](int a, int c) { return c < 3 ? 3 * a + c : 3 * g.nn + 3 * a + c - 3; };
   auto bi = [&](int i) { return i < 3 * g.nn ? 6 * (i / 3) + i % 3 : 6 * ((i - 3 * g.nn) / 3) + 3 + (i - 3 * g.nn) % 3; };
   double alpha = 0.0, rz = 0.0, bn = 1.0, rn = 0.0;
-  int it = 0, turn = 0;
+  int it = 0;
+  unsigned turn = 0;
   for (;; it++) {
     const double *r0 = it ? g.r[(it - 1) & 1] : g.b, *p0 = g.p[it & 1];  // p of the last iteration
     double *r1 = g.r[it & 1], *p1 = g.p[(it + 1) & 1];
@@ -1336,7 +1340,8 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
   a.tmp = V + 6 * (size_t)P;
   a.part = V + 7 * (size_t)P;
   a.out = a.part + 3 * (size_t)grid;
-  a.bar = reinterpret_cast<int*>(a.out + 4);
+  a.bar = reinterpret_cast<unsigned*>(a.out + 4);
+  a.polls = ctx->tri_spin_polls > 0 ? ctx->tri_spin_polls : PCG_POLLS;
   a.tol = tol;
   a.maxit = maxit;
   a.staged = sizeof(double) * (size_t)P <= PCG_STAGE;
