@@ -32,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include "coop.cuh"
 #include "pdl.cuh"
 #include "rsd_internal.cuh"
 
@@ -1317,7 +1318,7 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
                   int* iters, double* resid) {
   cudaStream_t s = ctx->stream;
   const int nn = g.nn, P = 6 * nn;
-  const int grid = ctx->sm_count;  // one CTA per SM: all are resident (cooperative launch)
+  int grid = ctx->sm_count;  // one CTA per SM: all are resident (cooperative launch)
   double* V = (double*)rsd_scratch(ctx, "lp_pcg", sizeof(double) * (7 * (size_t)P + 3 * (size_t)grid + 8));
   if (!V) return RSD_ENOMEM;
   PcgArgs a{};
@@ -1354,7 +1355,10 @@ static int lp_pcg(rsd_ctx* ctx, int mode, const lp_graph& g, const double* A, in
     a.x = x + (size_t)c * P;
     RSD_CUDA(ctx, cudaMemsetAsync(a.bar, 0, 2 * sizeof(int), s));
     void* args[] = {&a};
-    RSD_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)lp_pcg_kernel, dim3(grid), dim3(PCG_THREADS), args, smem, s)); RSD_LAUNCH_NOTE();
+    RSD_CUDA(ctx, rsd_coop_launch(&grid, [&](int g) {
+      return cudaLaunchCooperativeKernel((const void*)lp_pcg_kernel, dim3(g), dim3(PCG_THREADS), args, smem, s);
+    }));
+    RSD_LAUNCH_NOTE();
     double h[5];
     RSD_CUDA(ctx, cudaMemcpyAsync(h, a.out, 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
     RSD_CUDA(ctx, cudaStreamSynchronize(s));
