@@ -28,6 +28,7 @@
 #include "overlap.cuh"
 #include "dsf.cuh"
 #include "f32x2.cuh"
+#include "images.cuh"
 #include "pdl.cuh"
 #include "rsd_internal.cuh"
 
@@ -849,11 +850,6 @@ __device__ __forceinline__ int pack_image(int nx, int ny, int nz, int NR) {
   return (nx + NR) | ((ny + NR) << 8) | ((nz + NR) << 16);
 }
 
-// FP32 column base of the classification (the same sequence for both sets)
-__device__ __forceinline__ void column_base_f(const float* Rf, const float* A, int nx, int ny, float* p) {
-  for (int k = 0; k < 3; k++) p[k] = __fmaf_rn(A[3 + k], (float)ny, __fmaf_rn(A[k], (float)nx, Rf[k]));
-}
-
 // Lists the next images of the set (near: r2 < rc2; far: rc2 <= r2 < rmax2)
 // from the resumable position (col, nz) into list[.][t], at most REAL_CAP;
 // takes every step-th column; returns the count.
@@ -915,10 +911,11 @@ __device__ __forceinline__ void near_moments(const dsf_tables& T, int (*list)[RE
   } while (col < (2 * NR + 1) * (2 * NR + 1));
 }
 
-// The same for the far images, in FP32.
-__device__ __forceinline__ void far_moments(int (*list)[REAL_THREADS], int t, const float* Rf, const float* A, int NR,
-                                            float rc2, float rmax2, float lamf, float cdf, int col, int step,
-                                            float* acc) {
+// The same for the far images, in FP32 (EXACT: from column_base_s).
+template <bool EXACT = false>
+__device__ __forceinline__ void far_moments(int (*list)[REAL_THREADS], int t, const float* Rf, const float* A,
+                                            const dsf* Rs, const dsf* As, int NR, float rc2, float rmax2, float lamf,
+                                            float cdf, int col, int step, float* acc) {
   const float lam2f = lamf * lamf;
 #pragma unroll
   for (int m = 0; m < RSD_NMOM_REAL; m++) acc[m] = 0.f;
@@ -929,7 +926,11 @@ __device__ __forceinline__ void far_moments(int (*list)[REAL_THREADS], int t, co
       const int e = list[q][t];
       const int ix = (e & 255) - NR, iy = ((e >> 8) & 255) - NR, iz = (e >> 16) - NR;
       float p[3], x0, x1, x2;
-      column_base_f(Rf, A, ix, iy, p);
+      if (EXACT) {
+        column_base_s(Rs, As, ix, iy, p);
+      } else {
+        column_base_f(Rf, A, ix, iy, p);
+      }
       const float r2 = image_r2f(p[0], p[1], p[2], A[6], A[7], A[8], iz, &x0, &x1, &x2);
       const float r = sqrtf(r2), ir = 1.f / r;
       rsd_real_image<float>(x0, x1, x2, r, ir, erfcf(lamf * r), cdf * expf(-r2 * lam2f), lamf, acc);
@@ -1020,7 +1021,8 @@ __global__ void __launch_bounds__(REAL_THREADS, 2) ewald_pair_real_mix(int nn, r
   real_pair(L, pos, a, b, g);
   {
     float acc[RSD_NMOM_REAL];
-    far_moments(sh.list, t, g.Rf, g.A, L.NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
+    far_moments<true>(sh.list, t, g.Rf, g.A, g.Rs, g.As, L.NR, rc2, rmax2, (float)L.lam,
+                      (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
 #pragma unroll
     for (int m = 0; m < RSD_NMOM_REAL; m++) sh.far[m][t] = acc[m];
   }
@@ -1066,7 +1068,7 @@ __global__ void __launch_bounds__(REAL_THREADS, MINB) ewald_pair_real_eq(int nn,
   const int NR = L.NR;
   {
     float acc[RSD_NMOM_REAL];
-    far_moments(sh.list, t, g.Rf, g.A, NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
+    far_moments(sh.list, t, g.Rf, g.A, g.Rs, g.As, NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), 0, 1, acc);
 #pragma unroll
     for (int q = 0; q < 60; q++) {
       sh.oh[q][t] = rsd_real_epi_row<float, float, float>(q, acc, sh.cf);
@@ -1204,7 +1206,8 @@ __global__ void __launch_bounds__(REAL_THREADS, 2) ewald_real_slices(int nn, rsd
   const int64_t np = (int64_t)nn * (nn - 1) / 2, o = (int64_t)z * RSD_NMOM_REAL * np + (int64_t)b * (b - 1) / 2 + a;
   {
     float acc[RSD_NMOM_REAL];
-    far_moments(sh.list, t, g.Rf, g.A, L.NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), z, S, acc);
+    far_moments(sh.list, t, g.Rf, g.A, g.Rs, g.As, L.NR, rc2, rmax2, (float)L.lam, (float)(2.0 * RSD_PIP5 * L.lam), z, S,
+                acc);
 #pragma unroll
     for (int m = 0; m < RSD_NMOM_REAL; m++) far[o + m * np] = acc[m];
   }
