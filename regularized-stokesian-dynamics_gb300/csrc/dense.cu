@@ -764,6 +764,9 @@ __global__ void __launch_bounds__(256) potf2_inv_f32(float* __restrict__ A, int6
 // 33 with the rows published twice over, to save the packing of multipliers).
 // What is left is issue (180 instructions a thread for two steps, 40 of them
 // multiply-adds) and the two reciprocals' chain.
+// The reciprocals are those of 2 ulp, which hold up to 2^126: a block whose largest
+// diagonal entry is beyond 2^+-60 is scaled by a power of four first, and its
+// factors scaled back.
 struct gj_regs {
   uint64_t T[8][4];         // row 2 v + p of this thread, column pairs
   uint64_t s0[4], s1[4];    // rows k and k + 1 (after step k) at this thread's columns
@@ -907,6 +910,12 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
   }
   if (t == 0) failed = 0;
   __syncthreads();
+  int h = 0;  // the block is factored times 4^-h
+#pragma unroll
+  for (int e = 0; e < NB / 32; e++)
+    h = max(h, (int)(__float_as_uint(gj_tile[(lane + 32 * e) * (GJ_LD + 1)]) >> 23 & 0xff));
+  h = __reduce_max_sync(0xffffffffu, h) - 127;
+  h = h >= -60 && h <= 60 ? 0 : h >> 1;
   gj_regs g;
 #pragma unroll
   for (int v = 0; v < 4; v++)
@@ -918,6 +927,13 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
       g.T[2 * v][c] = f2_pack(i <= j ? a.x : 0.f, i <= j + 1 ? b.x : 0.f);
       g.T[2 * v + 1][c] = f2_pack(i + 1 <= j ? a.y : 0.f, i <= j ? b.y : 0.f);
     }
+  if (h) {
+    const float f = ldexpf(1.f, -h);
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) g.T[u][c] = f2_mul(f2_mul(g.T[u][c], f2_pack(f, f)), f2_pack(f, f));
+  }
   if (ty == 0) gj_publish<0>(g, row[0], tx);
   __syncthreads();
   gj_load<0, 4>(g, row[0], dd, 0, tx, ty, t);
@@ -965,6 +981,14 @@ __global__ void __launch_bounds__(256) potf2_gj_f32(float* __restrict__ A, int64
     }
   }
   __syncthreads();
+  if (h) {
+    const float fu = ldexpf(1.f, h), fw = ldexpf(1.f, -h);
+    for (int e = t; e < NB * NB; e += 256) {
+      gj_tile[e % NB + e / NB * GJ_LD] *= fu;
+      Wout[e] *= fw;
+    }
+    __syncthreads();
+  }
   if (vec) {
 #pragma unroll
     for (int e = 0; e < 16; e++) {
@@ -1115,11 +1139,13 @@ int smem_potf2(int jb) {
   return (jb * jb + jb) * (int)sizeof(T);
 }
 
-// exported: the factor ends in a matrix that is handed out (the FP32 RPP of
-// rsd_resistance_pp_dev), whose TF32 rounding goes with the last bits of every
-// block; potf2_inv_f32 keeps them what they were.
-void launch_potf2(cudaStream_t s, bool exported, float* A, int64_t lda, int jb, int* info, int j0, float* W) {
-  if (exported)
+// potf2_inv_f32 stays for what is handed out and must not lose to the faster
+// form: the FP32 RPP of rsd_resistance_pp_dev, whose TF32 rounding goes with the
+// last bits of every block, and the ragged block of a factor that the caller gets,
+// whose last columns it takes by IEEE square roots and divisions.  (In
+// potf2_gj_f32 these cost every block 6 us of instruction fetch.)
+void launch_potf2(cudaStream_t s, rsd_factor_use use, float* A, int64_t lda, int jb, int* info, int j0, float* W) {
+  if (use == RSD_FACTOR_RPP || (use == RSD_FACTOR_OUT && jb < NB))
     pdl_launch(potf2_inv_f32, 1, 256, SMEM_POTF2_INV, s, A, lda, jb, info, j0, W);
   else
     pdl_launch(potf2_gj_f32, 1, 256, GJ_SMEM, s, A, lda, jb, info, j0, W);
@@ -1241,7 +1267,7 @@ int trailing_update(rsd_ctx* ctx, int tc, const T* P, int64_t ldp, int kb, int m
 // Events: A (a's near work done), B (the work the next near step reads),
 // M (the previous remainder, which the next diagonal tile reads).
 constexpr int NBO = 512;
-static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
+static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, rsd_factor_use use) {
   cudaStream_t s = ctx->stream, s2 = ctx->side;
   RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
   for (int J0 = 0; J0 < n; J0 += NBO) {
@@ -1253,7 +1279,7 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      launch_potf2(s2, exported, Ajj, lda, jb, st, j0, Wb);
+      launch_potf2(s2, use, Ajj, lda, jb, st, j0, Wb);
       if (rest <= 0) continue;
       // row panel U_jj^-T B = W_jj^T B in place on tensor cores (each output
       // tile reads only its own columns of B)
@@ -1281,7 +1307,7 @@ static int potrf_two_level_sched0(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
   return RSD_OK;
 }
 
-static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
+static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, rsd_factor_use use) {
   cudaStream_t s = ctx->stream, sa = ctx->side, sb = ctx->side2;
   cudaEvent_t evA = ctx->ev_la[0], evB = ctx->ev_la[1], evM = ctx->ev_la[2], evS = ctx->ev_la[3];
   int* err = st + 1;
@@ -1299,7 +1325,7 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
       const int rest = n - j0 - jb;
       float* Apan = d_A + j0 + (int64_t)(j0 + jb) * lda;
       float* Wb = W + (size_t)(j0 / NB) * NB * NB;
-      launch_potf2(sa, exported, Ajj, lda, jb, st, j0, Wb);
+      launch_potf2(sa, use, Ajj, lda, jb, st, j0, Wb);
       if (rest <= 0) continue;
       RSD_CUDA(ctx, cudaStreamWaitEvent(sa, evB, 0));
       const int m_in = J0 + JB - (j0 + jb);  // rows of this outer panel below block k
@@ -1358,9 +1384,9 @@ static int potrf_two_level_sched1(rsd_ctx* ctx, int n, float* d_A, int64_t lda, 
   return RSD_OK;
 }
 
-int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, bool exported) {
-  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W, st, exported)
-                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W, st, exported);
+int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, float* W, int* st, rsd_factor_use use) {
+  return ctx->factor_schedule == 0 ? potrf_two_level_sched0(ctx, n, d_A, lda, tc, W, st, use)
+                                   : potrf_two_level_sched1(ctx, n, d_A, lda, tc, W, st, use);
 }
 
 // Blocked right-looking upper Cholesky with one step of look-ahead: the
@@ -1369,7 +1395,7 @@ int potrf_two_level_f32(rsd_ctx* ctx, int n, float* d_A, int64_t lda, int tc, fl
 // update has landed, while the rest of that update runs on the main stream.
 template <typename T>
 int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc, int* d_status,
-                      bool exported) {
+                      rsd_factor_use use) {
   if (n < 1 || lda < n) return rsd_fail(ctx, RSD_EARG, "potrf: n=%d lda=%lld", n, (long long)lda);
   RSD_TRY(ensure_attrs<T>(ctx));
   RSD_TRY(rsd_side_stream(ctx));
@@ -1388,7 +1414,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
   bool two_level = false;
   if constexpr (F32) two_level = tc && ctx->use_tc && rsd_tc_syrk_ok(d_A, lda, d_A, lda, NB);
   if constexpr (F32) {
-    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W, st, exported));
+    if (two_level) RSD_TRY(potrf_two_level_f32(ctx, n, d_A, lda, tc, W, st, use));
   }
   if (!two_level) {
     RSD_CUDA(ctx, cudaEventRecord(ctx->ev_next, s));
@@ -1402,7 +1428,7 @@ int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const
       {
         // factor + inverse of the diagonal block, then the panel as W_jj^T B
         T* Wb = W + (size_t)b * NB * NB;
-        launch_potf2(s2, exported, Ajj, lda, jb, st, j0, Wb);
+        launch_potf2(s2, use, Ajj, lda, jb, st, j0, Wb);
         if (rest > 0) {
           launch_gemm<T>(s2, gp(jb, rest, jb, 1.0, Wb, NB, 1, Apan, lda, 0, 0.0, T1, NB));
           RSD_CUDA(ctx, cudaMemcpy2DAsync(Apan, lda * sizeof(T), T1, NB * sizeof(T), jb * sizeof(T), rest,
@@ -2063,7 +2089,7 @@ template int rsd_gemv<float>(rsd_ctx*, int, int, int, float, const float*, int64
                              float*, int64_t);
 template int rsd_gemv<double>(rsd_ctx*, int, int, int, double, const double*, int64_t, const double*, int64_t, int,
                               double, double*, int64_t);
-template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*, bool);
+template int rsd_potrf_upper_t<float>(rsd_ctx*, int, float*, int64_t, int*, const char*, int, int*, rsd_factor_use);
 template int rsd_potri_upper_t<float>(rsd_ctx*, int, float*, int64_t, const char*, int, const float*, int*);
 template int rsd_mirror_upper_t<float>(rsd_ctx*, int, float*, int64_t);
 template int rsd_diag_inverses_t<float>(rsd_ctx*, int, const float*, int64_t, const char*, float**);
@@ -2111,7 +2137,7 @@ extern "C" int rsd_potrf_f32_dev(rsd_ctx* ctx, int32_t n, float* d_A, int64_t ld
   RSD_TRY(check_prec(ctx, prec));
   RSD_TRY(rsd_set_device(ctx));
   int inf = 0;
-  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec, nullptr, false));
+  RSD_TRY(rsd_potrf_upper_t<float>(ctx, n, d_A, lda, &inf, "f32dev", prec, nullptr, RSD_FACTOR_OUT));
   *info = inf;
   return RSD_OK;
 }

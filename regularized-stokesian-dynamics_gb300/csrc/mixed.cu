@@ -32,7 +32,7 @@ int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t
              int nrhs, T beta, T* y, int64_t ldy);
 template <typename T>
 int rsd_potrf_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, int* info, const char* tag, int tc,
-                      int* d_status = nullptr, bool exported = false);
+                      int* d_status = nullptr, rsd_factor_use use = RSD_FACTOR_STEP);
 template <typename T>
 int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag, int tc, const T* W = nullptr,
                       int* d_err = nullptr);
@@ -585,7 +585,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   // (about 2^-21, close to FP32; TF32 there takes ~17 iterations).
   int inf = 0;
   RSD_TRY(rsd_potrf_upper_t<float>(ctx, (int)d.np, M32, d.np, &inf, "m32", ctx->use_tc == 3 ? 3 : 1, st,
-                                   rpp_out != nullptr));
+                                   rpp_out ? RSD_FACTOR_RPP : RSD_FACTOR_STEP));
   const float* W128 = rsd_potrf_inverses_s(ctx, (int)d.np, "m32");
   float* W_m = nullptr;
   if (!rpp_out) RSD_TRY(rsd_wide_inverses_s(ctx, (int)d.np, M32, d.np, "m32", W128, &W_m));

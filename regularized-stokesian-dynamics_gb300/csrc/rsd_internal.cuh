@@ -263,6 +263,8 @@ int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t
 int rsd_lub_add_pp_f64(rsd_ctx* ctx, const rsd_lub_sparse* sp, double* A, int64_t lda);
 // Dense linear algebra (dense.cu)
 int rsd_mirror_upper(rsd_ctx* ctx, int n, double* d_A, int64_t lda);
+// What an FP32 factor is for: the step's refinement, the caller, or an RPP that is handed out
+enum rsd_factor_use { RSD_FACTOR_STEP, RSD_FACTOR_OUT, RSD_FACTOR_RPP };
 // FP64 factor, inverse from it and solves (dense64.cu): the diagonal-block inverses of a factorisation are kept
 // in a scratch buffer named by `tag`, so two factorisations can coexist.
 int rsd_potrf_upper_tag(rsd_ctx* ctx, int n, double* d_A, int64_t lda, int* info, const char* tag);
