@@ -105,7 +105,9 @@ int rsd_ctx_set_mixed_lambda_scale(rsd_ctx* ctx, double scale);
 /* Equal radii, mixed-precision assembly: the double-single near images are
  * summed in `passes` passes (1 to 4), each over one part of the moments
  * (fewer live accumulators and a shorter loop per pass; r, erfc and exp are
- * evaluated once per pass).  A performance setting; the sums are the same. */
+ * evaluated once per pass).  1, the default, deals the images of a system of
+ * less than about 190 particles out over more threads instead.  A performance
+ * setting; the sums are the same. */
 int rsd_ctx_set_mixed_real_passes(rsd_ctx* ctx, int32_t passes);
 /* Overlap corrections in the fused step (rsd_stepper_stokesian): the
  * correction_method of per_GRPY_YZD.f90:98-116 (0 none, the default; 1

@@ -2044,11 +2044,12 @@ int rsd_ewald_assemble(rsd_ctx* ctx, int nn, const double* d_pos, const double* 
         for (int k = 0; k < RSD_REAL_EPI_NC; k++) e[61 + k] = (unsigned short)rsd_real_epi_mom(k);
       }
       // Slices of a small system: so many that their CTAs (those above the
-      // diagonal) come to two per SM, what the kernels' registers allow.
+      // diagonal) come to two per SM, what the kernels' registers allow.  Sums in
+      // several passes are asked for by the caller, and taken unsliced.
       int ctas = 0;
       for (unsigned y = 0; y < grd.y; y++) ctas += std::min((4 * (int)y + 3 + 31) / 32, (int)grd.x);
       const int S = std::min(EWALD_SLICES, 2 * ctx->sm_count / ctas);
-      const bool sliced = equal && !exported && S >= 2;
+      const bool sliced = equal && !exported && S >= 2 && ctx->mixed_real_passes == 1;
       if (sliced) RSD_TRY(real_slices(ctx, beside.side, S, grd, blk, nn, L, d_pos, (float)rc2, (float)rmax2));
       int* dh = (int*)rsd_scratch(ctx, "ewald_hlist", sizeof(int) * up.size());
       double* t64 = equal ? nullptr : (double*)rsd_scratch(ctx, "ewald_ktab64", sizeof(double) * (size_t)(K64 > 0 ? K64 : 1) * KW);
