@@ -1322,7 +1322,12 @@ __global__ void __launch_bounds__(P64_THREADS) ewald_pair64(int nn, int64_t npai
     const float R0[3] = {(float)R[0], (float)R[1], (float)R[2]};
     int k[3];
     rsd_skew_shift_f32(A, LIf, R0, k);
-    for (int i = 0; i < 3; i++) R[i] -= k[0] * L.LR[i] + k[1] * L.LR[3 + i] + k[2] * L.LR[6 + i];
+    if (max(abs(k[0]), max(abs(k[1]), abs(k[2]))) < 2000) {  // FP32 holds the fraction to 1e-3 of a cell
+      for (int i = 0; i < 3; i++) R[i] -= k[0] * L.LR[i] + k[1] * L.LR[3 + i] + k[2] * L.LR[6 + i];
+    } else {
+      double dmin;
+      rsd_skew_correction(L.LR, L.LI, R, &dmin);
+    }
   }
   {
     const float Rf[3] = {(float)R[0], (float)R[1], (float)R[2]};

@@ -164,15 +164,7 @@ __global__ void lp_near(int nn, rsd_lat_dev L, const double* __restrict__ pos, c
     bool c = false;
     if (b < nn && b != a) {
       const float R[3] = {(float)(x0 - pos[3 * b]), (float)(x1 - pos[3 * b + 1]), (float)(x2 - pos[3 * b + 2])};
-      int k[3];
-      rsd_skew_shift_f32(LR, LI, R, k);
-      float d2 = 0.f;
-      for (int i = 0; i < 3; i++) {
-        const float e = R[i] - (LR[i] * k[0] + LR[i + 3] * k[1] + LR[i + 6] * k[2]);
-        d2 += e * e;
-      }
-      const float lim = 0.5f * (float)LP_CUT * (ra + (float)radii[b]) * 1.001f + 1e-3f;
-      c = !(d2 > lim * lim);
+      c = rsd_maybe_within_f32(LR, LI, R, 0.5f * (float)LP_CUT * (ra + (float)radii[b]));
     }
     const unsigned m = __ballot_sync(0xffffffffu, c);
     if (c) cand[warp][nc + __popc(m & below)] = b;

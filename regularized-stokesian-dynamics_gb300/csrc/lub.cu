@@ -91,20 +91,9 @@ __device__ void lubcalc_dev(const lub_dev_tab& t, double r, double* o) {
 
 // FP32 screen of a pair: false where it is clearly beyond the cut-off s = 4
 __device__ __forceinline__ bool maybe_near(const float* LR, const float* LI, int is_period, const float R[3], float asum) {
-  float d2;
-  if (is_period) {
-    int k[3];
-    rsd_skew_shift_f32(LR, LI, R, k);
-    d2 = 0.f;
-    for (int i = 0; i < 3; i++) {
-      const float e = R[i] - (LR[i] * k[0] + LR[i + 3] * k[1] + LR[i + 6] * k[2]);
-      d2 += e * e;
-    }
-  } else {
-    d2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
-  }
+  if (is_period) return rsd_maybe_within_f32(LR, LI, R, 2.0f * asum);
   const float lim = 2.0f * asum * 1.001f + 1e-3f;
-  return !(d2 > lim * lim);
+  return !(R[0] * R[0] + R[1] * R[1] + R[2] * R[2] > lim * lim);
 }
 
 __device__ inline bool near_pair(const rsd_lat_dev& L, int is_period, const double* pos, const double* radii, int a,

@@ -211,6 +211,23 @@ __host__ __device__ inline void rsd_skew_shift_f32(const float* LR, const float*
   k[2] += best & 1;
 }
 
+// FP32 screen: false only where the minimum image of R is farther than lim.  The
+// margin holds the roundings of R and of the shift (at most 6 2^-24 of their
+// sizes a component), which reach any size when positions lie many cells apart;
+// NaN passes.
+__host__ __device__ inline bool rsd_maybe_within_f32(const float* LR, const float* LI, const float R[3], float lim) {
+  int k[3];
+  rsd_skew_shift_f32(LR, LI, R, k);
+  float d2 = 0.f, size = 0.f;
+  for (int i = 0; i < 3; i++) {
+    const float s0 = LR[i] * k[0], s1 = LR[i + 3] * k[1], s2 = LR[i + 6] * k[2], e = R[i] - (s0 + s1 + s2);
+    d2 += e * e;
+    size += fabsf(R[i]) + fabsf(s0) + fabsf(s1) + fabsf(s2);
+  }
+  lim = lim * 1.001f + 1e-3f + 1e-6f * size;
+  return !(d2 > lim * lim);
+}
+
 // ------------------------------------------------------------ kernels
 // Ewald (ewald.cu).  RSD_PREC_FP64: d_M is the FP64 grand mobility (ld
 // ldm).  RSD_PREC_MIXED: the same buffer holds it as two FP32 planes, hi at
