@@ -123,10 +123,14 @@ int rsd_ctx_set_correction_method(rsd_ctx* ctx, int32_t method);
  * floor of the residual arithmetic on stiff systems).  When it diverges
  * (its residual grows 1000 times above its best) or ends above 100 times the
  * tolerance, flexible GMRES finishes the solve from zero
- * (rsd_step_info.fallback = 1).  Mode 1 = flexible GMRES alone, with the
+ * (rsd_step_info.fallback = 1).  A residual no larger than 4 2^-53 times the size
+ * of its terms, |Fe| + |f| + |R_lub||U| relative to the right-hand side, is at the
+ * rounding of the velocities themselves and ends either method: gaps below
+ * ~1e-7 leave up to 1e-8 so, with velocities and stresslets as good as ever.
+ * Mode 1 = flexible GMRES alone, with the
  * same preconditioner and FP64 residuals, restarted every `restart`
  * iterations (1..30, 0: 30).  A solve that ends above 100 times the
- * tolerance returns RSD_ENOCONV. */
+ * tolerance and above that rounding returns RSD_ENOCONV. */
 int rsd_ctx_set_refinement(rsd_ctx* ctx, int32_t mode, int32_t restart);
 /* Bounds of the device-side waits (no counterpart in the reference): every
  * mbarrier wait of the tensor-core products, FP32 and FP64, gives up after

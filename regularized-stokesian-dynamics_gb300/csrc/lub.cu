@@ -392,7 +392,9 @@ __device__ inline void pair_pos(int r, int c, bool ab, int* off, double* sgn) {
 // a thread per entry (r, c) of its 11 x 11 blocks: the position in the pair
 // block is fixed per thread, a neighbour costs one multiply-add of each, and
 // the 11 columns are added at the end in a fixed order.  Bound by the FP64
-// pipe and the latency of the neighbour loop.
+// pipe and the latency of the neighbour loop.  ABS: the sum of the terms' sizes,
+// |L| |w| (blocks of several pairs taken whole).
+template <bool ABS>
 __global__ void __launch_bounds__(128) lub_spmv_w(int N, const int* __restrict__ off, const int* __restrict__ off2,
                                                   const int* __restrict__ list2, const int2* __restrict__ pairs,
                                                   const double* __restrict__ blk, const double* __restrict__ self,
@@ -407,16 +409,18 @@ __global__ void __launch_bounds__(128) lub_spmv_w(int N, const int* __restrict__
     double sa, sb;
     pair_pos(r, c, true, &oa, &sa);
     pair_pos(r, c, false, &ob, &sb);
+    auto term = [](double x) { return ABS ? fabs(x) : x; };
+    if (ABS) sa = sb = 1.0;
     const int wbase = c < 3 ? c : (c < 6 ? 3 * N + c - 3 : 6 * N + c - 6), wstep = c < 6 ? 3 : 5;
-    sv[t] = self[(size_t)u * 121 + t] * wc[wbase + wstep * u];
+    sv[t] = term(self[(size_t)u * 121 + t] * wc[wbase + wstep * u]);
     double va = 0.0, vb = 0.0;
     const int p1 = off[u + 1], q1 = off2[u + 1];
 #pragma unroll 4
-    for (int p = off[u]; p < p1; p++) va = fma(blk[(size_t)p * PB + oa], wc[wbase + wstep * pairs[p].y], va);
+    for (int p = off[u]; p < p1; p++) va = fma(term(blk[(size_t)p * PB + oa]), term(wc[wbase + wstep * pairs[p].y]), va);
 #pragma unroll 4
     for (int q = off2[u]; q < q1; q++) {
       const int p = list2[q];
-      vb = fma(blk[(size_t)p * PB + ob], wc[wbase + wstep * pairs[p].x], vb);
+      vb = fma(term(blk[(size_t)p * PB + ob]), term(wc[wbase + wstep * pairs[p].x]), vb);
     }
     pv[t] = sa * va + sb * vb;
   }
@@ -595,8 +599,17 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, in
 // y (11N x nr, grand layout, ld ldy) = L w
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy) {
-  pdl_launch(lub_spmv_w, dim3(sp->nn, nr), 128, 0, ctx->stream, sp->nn, sp->off, sp->off2, sp->list2, sp->pairs, sp->blk,
-                                                        sp->self, sp->scale, w, ldw, y, ldy);
+  pdl_launch(lub_spmv_w<false>, dim3(sp->nn, nr), 128, 0, ctx->stream, sp->nn, sp->off, sp->off2, sp->list2, sp->pairs,
+             sp->blk, sp->self, sp->scale, w, ldw, y, ldy);
+  RSD_CUDA(ctx, cudaGetLastError());
+  return RSD_OK;
+}
+
+// y (11N) = |L| |w|
+int rsd_lub_absmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, const double* w, double* y) {
+  const int64_t n = 11LL * sp->nn;
+  pdl_launch(lub_spmv_w<true>, dim3(sp->nn, 1), 128, 0, ctx->stream, sp->nn, sp->off, sp->off2, sp->list2, sp->pairs,
+             sp->blk, sp->self, sp->scale, w, n, y, n);
   RSD_CUDA(ctx, cudaGetLastError());
   return RSD_OK;
 }

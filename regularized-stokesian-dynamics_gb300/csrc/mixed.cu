@@ -357,6 +357,26 @@ __global__ void __launch_bounds__(256) it_residual(mixed_dims d, const double* _
   }
 }
 
+// Per block of the grid the sums of squares of the sizes of r2's terms, |Fe| + |f_P|
+// + (|L||w|)_P, in La the last.
+__global__ void __launch_bounds__(256) it_scale(int64_t P, const double* __restrict__ Fe, const double* __restrict__ f,
+                                                const double* __restrict__ La, double* __restrict__ part) {
+  pdl_enter();
+  __shared__ double red[256];
+  double a = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < P; i += (int64_t)gridDim.x * 256) {
+    const double v = (Fe ? fabs(Fe[i]) : 0.0) + fabs(f[i]) + La[i];
+    a += v * v;
+  }
+  red[threadIdx.x] = a;
+  __syncthreads();
+  for (int h = 128; h > 0; h >>= 1) {
+    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+}
+
 // y = unperm(x32) (y = M^-1 r1); u32 = r2 - y_P, zero past P
 __global__ void it_velocity(mixed_dims d, int nr, const float* __restrict__ x32, const double* __restrict__ r2,
                             double* __restrict__ y, float* __restrict__ u32) {
@@ -647,11 +667,35 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   };
   // refinement
   const int* tri_err = rsd_uhat_error_flag(ctx);
+  // A solve is accepted within the stagnation band of the tolerance, or where its
+  // residual is no more than the rounding of its own terms: with a gap of 1e-8
+  // L w cancels from 1e8 times the velocities, and no velocities held in FP64
+  // leave less of it.
+  const double accept = 100.0 * tol;
+  // relative residual of column c that the rounding of r2 alone can make up (w
+  // and f of that column as they are): the velocities' 2^-53 times |L||w|, about
+  // as much from its sum and the terms beside it, and twice that for safety
+  auto rounding = [&](int c, double bn, double* out) -> int {
+    double* La = (double*)rsd_scratch(ctx, "mixed_la", sizeof(double) * (size_t)(n + IT_BLOCKS));
+    if (!La) return RSD_ENOMEM;
+    double part[IT_BLOCKS], s2 = 0.0;
+    if (lub)
+      RSD_TRY(rsd_lub_absmv(ctx, lub, w + (size_t)c * n, La));
+    else
+      RSD_CUDA(ctx, cudaMemsetAsync(La, 0, sizeof(double) * n, s));
+    pdl_launch(it_scale, IT_BLOCKS, 256, 0, s, P, have_fe && c == 0 ? Fe : nullptr, f + (size_t)c * n, La, La + n);
+    RSD_CUDA(ctx, cudaMemcpyAsync(part, La + n, sizeof part, cudaMemcpyDeviceToHost, s));
+    RSD_CUDA(ctx, cudaStreamSynchronize(s));
+    for (int k = 0; k < IT_BLOCKS; k++) s2 += part[k];
+    *out = 4.0 * 0x1p-53 * sqrt(s2) / bn;
+    return RSD_OK;
+  };
   // Right-preconditioned flexible GMRES(m) per right-hand side, FP64
   // residuals; the preconditioner is the stationary iteration's correction.
   // Starts from zero; gm_maxit bounds the iterations over all right-hand
-  // sides; returns the iterations and the worst relative residual.
-  auto run_gmres = [&](int gm_maxit, int* its_out, double* res_out) -> int {
+  // sides; returns the iterations, the worst relative residual, and whether
+  // every column is accepted.
+  auto run_gmres = [&](int gm_maxit, int* its_out, double* res_out, bool* ok) -> int {
     const int m = ctx->gmres_restart > 0 ? ctx->gmres_restart : 30;
     const int64_t len = n + P;
     double* KV = (double*)rsd_scratch(ctx, "gm_basis", sizeof(double) * (size_t)(2 * m + 1) * len + 8 * 64);
@@ -728,8 +772,9 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     int total_it = 0;
     double worst = 0.0;
     std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), yv(m), hh(m + 2);
+    *ok = true;
     for (int c = 0; c < nr; c++) {
-      double rel = 0.0;
+      double rel = 0.0, last = 0.0, floor = 0.0;
       for (int cycle = 0;; cycle++) {
         RSD_TRY(residual(c, Vb));
         pdl_launch(gm_nrm2, 1, 256, 0, s, len, Vb, dn);
@@ -742,7 +787,11 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
         const double beta = sqrt(beta2);
         rel = beta / bnorm[c];
         if (!std::isfinite(rel)) return rsd_fail(ctx, RSD_ENAN, "refinement residual is not finite");
-        if (rel <= tol || total_it >= gm_maxit) break;
+        if (rel <= tol) break;
+        const bool spent = total_it >= gm_maxit;
+        if (spent || (cycle > 0 && rel > 0.5 * last)) RSD_TRY(rounding(c, bnorm[c], &floor));
+        if (spent || rel <= floor) break;
+        last = rel;
         pdl_launch(gm_scale, nblk(len), 256, 0, s, len, Vb, dn, Vb);
         std::fill(g.begin(), g.end(), 0.0);
         g[0] = beta;
@@ -801,30 +850,41 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
         pdl_launch(gm_update, nblk(P), 256, 0, s, P, j, Zb + n, len, hbuf, U + (size_t)c * P);
       }
       worst = fmax(worst, rel);
+      *ok = *ok && rel <= fmax(accept, floor);
     }
     *its_out = total_it;
     *res_out = worst;
     return RSD_OK;
   };
-  // A solve is accepted within the stagnation band of the tolerance.
-  const double accept = 100.0 * tol;
   cudaEventRecord(ctx->ev[7], s);
+  bool ok = false;
   if (ctx->refine_gmres) {
     int its = 0;
     double res = 0.0;
-    RSD_TRY(run_gmres(maxit, &its, &res));
+    RSD_TRY(run_gmres(maxit, &its, &res, &ok));
     pdl_launch(outputs, nblk(P), 256, 0, s, P, Q, nr - 1, f, Lw, U, U_par, S_hyd);
     RSD_CUDA(ctx, cudaGetLastError());
     info->iterations = its;
     info->residual = res;
-    if (!(res <= accept))
+    if (!ok)
       return rsd_fail(ctx, RSD_ENOCONV, "refinement did not converge: residual %.3e after %d iterations", res, its);
     return RSD_OK;
   }
   RSD_CUDA(ctx, cudaMemsetAsync(f, 0, sizeof(double) * nr * (n + P), s));  // and U, behind it
   double worst = 0.0, best_res = INFINITY;
   int it = 0;
-  std::vector<double> hist;
+  std::vector<double> hist, rel(nr), bn(nr);
+  auto accepted = [&]() -> int {
+    ok = worst <= accept;
+    if (ok || !std::isfinite(worst)) return RSD_OK;
+    ok = true;
+    for (int c = 0; c < nr && ok; c++) {
+      double floor = 0.0;
+      if (rel[c] > accept) RSD_TRY(rounding(c, bn[c], &floor));
+      ok = rel[c] <= fmax(accept, floor);
+    }
+    return RSD_OK;
+  };
   for (;; it++) {
     pdl_launch(it_begin, nblk(n * nr), 256, 0, s, P, Q, nr, U, ein, f, w, r1, fs);
     // r1 -= M f, double-single products of the two planes, both right-hand
@@ -851,8 +911,9 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
         a2 += hn[2 * (c * IT_BLOCKS + k)];
         b2 += hn[2 * (c * IT_BLOCKS + k) + 1];
       }
-      const double rr = sqrt(a2) / (sqrt(b2) > 0 ? sqrt(b2) : 1.0);
-      worst = std::isfinite(rr) ? fmax(worst, rr) : INFINITY;
+      bn[c] = sqrt(b2) > 0 ? sqrt(b2) : 1.0;
+      rel[c] = sqrt(a2) / bn[c];
+      worst = std::isfinite(rel[c]) ? fmax(worst, rel[c]) : INFINITY;
     }
     if (worst <= tol || it >= maxit) break;
     // Divergence: FP32 factors too far from the FP64 system (a pair so close
@@ -863,11 +924,14 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     // Stagnation: the FP64 residual of a stiff system (many near-contact
     // pairs: forces ~1/gap times the velocities) has a floor of about the
     // residual arithmetic's rounding times |M||f| / |b|, which can sit just
-    // above tol.  Within 100 tol, an iteration that does not halve the best
-    // of the previous two ends the refinement (the solution does not improve
-    // further); the reported residual is the one reached.
+    // above tol.  Within 100 tol, or at that floor, an iteration that does not
+    // halve the best of the previous two ends the refinement (the solution
+    // does not improve further); the reported residual is the one reached.
     hist.push_back(worst);
-    if (it >= 2 && worst <= 100.0 * tol && worst > 0.5 * fmin(hist[it - 1], hist[it - 2])) break;
+    if (it >= 2 && worst > 0.5 * fmin(hist[it - 1], hist[it - 2])) {
+      RSD_TRY(accepted());
+      if (ok) break;
+    }
     RSD_TRY(solve_m(t32, nr, x32, 0));  // y = M^-1 r1
     pdl_launch(it_velocity, nblk(d.np * nr), 256, 0, s, d, nr, x32, r2, y, u32);
     RSD_TRY(solve_r(u32, nr, du32));    // dU = RPP^-1 (r2 - y_P)
@@ -875,13 +939,14 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
     RSD_TRY(solve_m(t32, nr, x32, (int)d.Qp));
     pdl_launch(it_update, nblk(d.np * nr), 256, 0, s, d, nr, x32, y, du32, f, U);  // df = y + M^-1 [dU; 0]
   }
-  if (!(worst <= accept)) {
+  RSD_TRY(accepted());
+  if (!ok) {
     // diverged or stalled above the band: flexible GMRES from zero over the
     // same corrections, which converges where a few modes of the FP32
     // factors are poor
     int its = 0;
     double res = 0.0;
-    RSD_TRY(run_gmres(std::max(3 * maxit, 100), &its, &res));
+    RSD_TRY(run_gmres(std::max(3 * maxit, 100), &its, &res, &ok));
     it += its;
     worst = res;
     info->fallback = 1;
@@ -890,7 +955,7 @@ int rsd_mixed_solve(rsd_ctx* ctx, int nn, double* M, int64_t ld, const rsd_lub_s
   RSD_CUDA(ctx, cudaGetLastError());
   info->iterations = it;
   info->residual = worst;
-  if (!(worst <= accept))
+  if (!ok)
     return rsd_fail(ctx, RSD_ENOCONV, "refinement did not converge: residual %.3e after %d iterations", worst, it);
   return RSD_OK;
 }

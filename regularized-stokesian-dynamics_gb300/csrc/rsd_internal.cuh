@@ -276,6 +276,7 @@ int rsd_lub_build_sparse(rsd_ctx* ctx, cudaStream_t s, const rsd_lubtab* tab, in
                          rsd_lub_sparse* sp);
 int rsd_lub_spmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, int nr, const double* w, int64_t ldw, double* y,
                  int64_t ldy);
+int rsd_lub_absmv(rsd_ctx* ctx, const rsd_lub_sparse* sp, const double* w, double* y);
 int rsd_lub_add_pp_f32(rsd_ctx* ctx, const rsd_lub_sparse* sp, float* A, int64_t lda);
 int rsd_lub_add_pp_f64(rsd_ctx* ctx, const rsd_lub_sparse* sp, double* A, int64_t lda);
 // Dense linear algebra (dense.cu)
