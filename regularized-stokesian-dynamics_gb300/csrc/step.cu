@@ -369,8 +369,12 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
   } else {
     {
       rsd_range r("rsd_solve");
-      RSD_TRY(rsd_mixed_solve(ctx, nn, M, ldm, p->use_lub ? &lub : nullptr, p, ein, d_Fe ? Fe : nullptr, Upar, S, &loc,
-                              (float*)rpp_out, rpp_ld));
+      const int rc = rsd_mixed_solve(ctx, nn, M, ldm, p->use_lub ? &lub : nullptr, p, ein, d_Fe ? Fe : nullptr, Upar, S,
+                                     &loc, (float*)rpp_out, rpp_ld);
+      if (rc != RSD_OK) {
+        if (info) *info = loc;
+        return rc;
+      }
     }
     if (rpp_out) {
       RSD_CUDA(ctx, cudaStreamSynchronize(s));
