@@ -1586,8 +1586,8 @@ int rsd_potri_upper_t(rsd_ctx* ctx, int n, T* d_A, int64_t lda, const char* tag,
 }
 
 // Inverses of the NB2 x NB2 diagonal blocks of an upper factor U, for the
-// wide-block solves: each block copied out (lower part zero) and inverted in
-// place by the blocked triangular inverse.  W2: nblk2 blocks of NB2 x NB2.
+// wide-block solves (wide_init, wide_combine below).  W2: nblk2 blocks of NB2 x
+// NB2.
 constexpr int NB2 = 512;
 // D_b, one NB2 x NB2 block per diagonal block b = blockIdx.z of U (n x n): the
 // inverses W of its NB-wide diagonal blocks, U's entries right of them, zero

@@ -589,8 +589,9 @@ __global__ void __launch_bounds__(256) potf2_inv_f64(double* __restrict__ A, int
 // of the block (factor of stiff pairs at 1e8: 4600 eps of the scaled matrix, 8
 // so).  16 lanes per system; with U's entries divided by the pivot of their step
 // a step is a broadcast and at most W / 16 multiply-adds, and the unknowns are
-// scaled at the end.  Bound by the FP64 pipe (64 cycles per warp instruction and
-// SM quarter): ~7 us for up to 1216 systems of 64, ~22 of 128.
+// scaled at the end.  Bound by the chain of steps and the FP64 pipe (64 cycles per
+// warp instruction and SM quarter): 22.5 us for 64 to 640 systems of 64, 27 for
+// 2100 (from cold; 34 for 2600 with one load of U in flight per thread).
 // The reciprocals of the diagonal come from the 64-wide inverses in Wd.
 constexpr int SUB_SYS = 8, SUB_THREADS = 16 * SUB_SYS;
 template <int W>
@@ -612,9 +613,18 @@ __global__ void __launch_bounds__(SUB_THREADS) subst64(int w, const double* __re
 #pragma unroll
   for (int j = 0; j < R; j++) b[j] = q < nsys && at(l + 16 * j) < w ? Bq[at(l + 16 * j)] : 0.0;
   __syncthreads();
-  for (int e = t; e < W * W; e += SUB_THREADS) {  // U(r, c), r < c, by columns
-    const int r = e % W, c = e / W, k = BACK ? at(c) : r, i = BACK ? at(r) : c;
-    if (r < c) S[k * LD + i] = c < w ? U[r + (int64_t)c * ldu] * rd[k] : 0.0;
+  for (int e0 = t; e0 < W * W; e0 += 16 * SUB_THREADS) {  // U(r, c), r < c, by columns, 16 loads in flight
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+      const int e = e0 + u * SUB_THREADS, r = e % W, c = e / W;
+      v[u] = r < c && c < w ? U[r + (int64_t)c * ldu] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+      const int e = e0 + u * SUB_THREADS, r = e % W, c = e / W, k = BACK ? at(c) : r, i = BACK ? at(r) : c;
+      if (r < c) S[k * LD + i] = v[u] * rd[k];
+    }
   }
   __syncthreads();
 #pragma unroll
