@@ -15,7 +15,8 @@ TOO_LARGE, OUT_OF_MEMORY = 720, 2
 @pytest.fixture(scope="module")
 def check(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("coop") / "coop_check.so")
-    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-I", "/usr/local/cuda/include",
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC,
+                           "-I", "/usr/local/cuda/include",
                            os.path.join(ROOT, "tests", "cpp", "coop_check.cpp"), "-o", so])
     f = ctypes.CDLL(so).coop_check
 

@@ -14,7 +14,8 @@ CSRC = os.path.join(ROOT, "regularized-stokesian-dynamics_gb300", "csrc")
 
 def test_granted_once_per_context_and_kernel(tmp_path):
     so = str(tmp_path / "smem_check.so")
-    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-I", "/usr/local/cuda/include",
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC,
+                           "-I", "/usr/local/cuda/include",
                            os.path.join(ROOT, "tests", "cpp", "smem_check.cpp"), "-o", so])
     assert ctypes.CDLL(so).smem_check() == 0
 
