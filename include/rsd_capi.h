@@ -93,14 +93,17 @@ int rsd_ctx_set_mixed_split(rsd_ctx* ctx, double lam_r_cut, int32_t kshell);
  * with k^2/(4 lammda^2) >= k2_over_4lam2_max are dropped.  Defaults 6.0 and
  * 10 pi: each changes a mobility block by less than ~1e-12 of its largest
  * entry (the reference's cubes reach lammda*r ~ 10 and k^2/(4 lammda^2) ~
- * 85 at zero strain).  The FP64 form always sums the whole cubes. */
+ * 85 at zero strain).  The FP64 form is not concerned: it leaves out only what
+ * FP64 cannot hold (lammda*r beyond 6.8, k^2/(4 lammda^2) beyond 46). */
 int rsd_ctx_set_mixed_truncation(rsd_ctx* ctx, double lam_r_max, double k2_over_4lam2_max);
 /* Ewald splitting parameter of the mixed-precision assembly relative to the
  * reference's lammda = sqrt(pi)/LV^(1/3).  The Ewald sum does not depend on
  * it; a larger value moves work from the real-space images to the cheaper
  * reciprocal vectors, and the image cubes are widened to hold the
  * truncation spheres.  1 keeps the reference's lammda, NR and NI; the
- * default is 1.75.  The FP64 form always uses the reference's values. */
+ * default is 1.75.  The FP64 form is not concerned: it takes 1.45 times the
+ * reference's lammda where the reference's cubes NR, NI hold the sums to FP64
+ * rounding, and the cubes at the reference's lammda where they cut them. */
 int rsd_ctx_set_mixed_lambda_scale(rsd_ctx* ctx, double scale);
 /* Equal radii, mixed-precision assembly: the double-single near images are
  * summed in `passes` passes (1 to 4), each over one part of the moments
