@@ -146,6 +146,11 @@ int rsd_ctx_set_refinement(rsd_ctx* ctx, int32_t mode, int32_t restart);
  * raises an error word; the call returns RSD_ETIMEOUT and the context stays
  * usable.  Values far below the defaults only serve to exercise that path. */
 int rsd_ctx_set_wait_limits(rsd_ctx* ctx, int64_t tc_wait_ns, int64_t tri_spin_polls);
+/* Bound of the context's device scratch memory in bytes (0, the default: the
+ * GPU's; no counterpart in the reference).  A call that needs more returns
+ * RSD_ENOMEM; the FP64 resistance and inverse first take slower forms that work in
+ * place of the matrix, as they do where the GPU's memory is short (N beyond ~9000). */
+int rsd_ctx_set_scratch_limit(rsd_ctx* ctx, int64_t bytes);
 /* Schedule of the mixed form's FP32 Cholesky factorisations on tensor
  * cores: 1 (default) keeps only the next diagonal tile on the chain of
  * diagonal blocks and runs the wide row-panel work on a second stream beside

@@ -105,6 +105,7 @@ _sig("rsd_ctx_set_mixed_lambda_scale", _i, [_vp, _d])
 _sig("rsd_ctx_set_mixed_real_passes", _i, [_vp, _i32])
 _sig("rsd_ctx_set_correction_method", _i, [_vp, _i32])
 _sig("rsd_ctx_set_wait_limits", _i, [_vp, _i64, _i64])
+_sig("rsd_ctx_set_scratch_limit", _i, [_vp, _i64])
 _sig("rsd_ctx_set_factor_schedule", _i, [_vp, _i32])
 _sig("rsd_ctx_set_refinement", _i, [_vp, _i32, _i32])
 _sig("rsd_ctx_set_rpp_solver", _i, [_vp, _i32, _vp, _d, _i32])
@@ -203,6 +204,12 @@ class Context:
         (0: 2^21 and 2^25); a wait that gives up makes the call return
         RSD_ETIMEOUT."""
         self.check(_lib.rsd_ctx_set_wait_limits(self.h, int(tc_wait_ns), int(tri_spin_polls)))
+
+    def set_scratch_limit(self, nbytes=0):
+        """Bound of the context's device scratch memory (0: the GPU's); a call
+        that needs more fails with RSD_ENOMEM, the FP64 resistance and inverse
+        after trying the forms that work in place."""
+        self.check(_lib.rsd_ctx_set_scratch_limit(self.h, int(nbytes)))
 
     def set_factor_schedule(self, schedule=1):
         """Mixed form's FP32 Cholesky schedule: 1 look-ahead on the chain of

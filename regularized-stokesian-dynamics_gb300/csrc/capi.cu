@@ -36,24 +36,36 @@ int rsd_cuda_check(rsd_ctx* ctx, cudaError_t e, const char* what) {
   return rsd_fail(ctx, RSD_ECUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes) {
+void rsd_scratch_free(rsd_ctx* ctx, const char* name) {
+  rsd_buf& b = ctx->bufs[name];
+  if (!b.p) return;
+  cudaStreamSynchronize(ctx->stream);
+  cudaFree(b.p);
+  ctx->scratch_bytes -= b.bytes;
+  b.p = nullptr;
+  b.bytes = 0;
+}
+
+void* rsd_scratch_try(rsd_ctx* ctx, const char* name, size_t bytes) {
   if (bytes == 0) bytes = 1;
   rsd_buf& b = ctx->bufs[name];
   if (b.bytes >= bytes) return b.p;
-  if (b.p) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
-  }
+  rsd_scratch_free(ctx, name);
+  if (ctx->scratch_limit && ctx->scratch_bytes + bytes > ctx->scratch_limit) return nullptr;
   if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
     cudaGetLastError();
-    rsd_fail(ctx, RSD_ENOMEM, "cannot allocate %zu bytes for %s", bytes, name);
     b.p = nullptr;
     return nullptr;
   }
   b.bytes = bytes;
+  ctx->scratch_bytes += bytes;
   return b.p;
+}
+
+void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes) {
+  void* p = rsd_scratch_try(ctx, name, bytes);
+  if (!p) rsd_fail(ctx, RSD_ENOMEM, "cannot allocate %zu bytes for %s", bytes, name);
+  return p;
 }
 
 void* rsd_pinned(rsd_ctx* ctx, size_t bytes) {
@@ -191,6 +203,13 @@ extern "C" int rsd_ctx_set_wait_limits(rsd_ctx* c, int64_t tc_wait_ns, int64_t t
   if (tc_wait_ns < 0 || tri_spin_polls < 0) return rsd_fail(c, RSD_EARG, "wait limits must be >= 0");
   c->tc_wait_ns = tc_wait_ns;
   c->tri_spin_polls = tri_spin_polls;
+  return RSD_OK;
+}
+
+extern "C" int rsd_ctx_set_scratch_limit(rsd_ctx* c, int64_t bytes) {
+  if (!c) return RSD_EARG;
+  if (bytes < 0) return rsd_fail(c, RSD_EARG, "scratch limit must be >= 0");
+  c->scratch_limit = (size_t)bytes;
   return RSD_OK;
 }
 
@@ -712,9 +731,8 @@ static int nogmres_impl(rsd_ctx* ctx, int32_t nn, const double* APP, const doubl
   const int64_t n = 11LL * nn, p = 6LL * nn, q = 5LL * nn;
   double* M = (double*)rsd_scratch(ctx, "M", sizeof(double) * n * n);
   double* Lb = (double*)rsd_scratch(ctx, "L", sizeof(double) * n * n);
-  double* RP = (double*)rsd_scratch(ctx, "nog_RPP", sizeof(double) * p * p);
   double* V = (double*)rsd_scratch(ctx, "nog_vec", sizeof(double) * (8 * p + 4 * q));
-  if (!M || !Lb || !RP || !V) return RSD_ENOMEM;
+  if (!M || !Lb || !V) return RSD_ENOMEM;
   // MobToResist_FTS, through the Schur complement (resist64.cu)
   RSD_TRY(put_block(ctx, M, n, APP, p, p));
   RSD_TRY(put_block(ctx, M + p * n, n, APQ, p, q));
@@ -731,8 +749,9 @@ static int nogmres_impl(rsd_ctx* ctx, int32_t nn, const double* APP, const doubl
   RSD_CUDA(ctx, cudaMemcpyAsync(drfu, rfu, sizeof(double) * p * p, cudaMemcpyHostToDevice, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(drfe, rfe, sizeof(double) * p * q, cudaMemcpyHostToDevice, s));
   RSD_CUDA(ctx, cudaMemcpyAsync(drse, rse, sizeof(double) * q * q, cudaMemcpyHostToDevice, s));
-  RSD_CUDA(ctx, cudaMemcpyAsync(RP, h.Ai, sizeof(double) * p * p, cudaMemcpyDeviceToDevice, s));
-  RSD_TRY(rsd_axpy_block(ctx, p, p, drfu, p, RP, p));
+  double* RP = h.RPP;
+  const int64_t ldr = h.ldp;
+  RSD_TRY(rsd_axpy_block(ctx, p, p, drfu, p, RP, ldr));
   // right-hand sides [Fe + RPQ EIN, RPQ EIN, Fe_inter] in X; Y = [X2, X3, UB]
   double *X = V, *Y = V + 3 * p, *f0 = V + 6 * p, *ein = V + 7 * p, *S = ein + q;
   RSD_CUDA(ctx, cudaMemcpyAsync(ein, EIN, sizeof(double) * q, cudaMemcpyHostToDevice, s));
@@ -744,12 +763,12 @@ static int nogmres_impl(rsd_ctx* ctx, int32_t nn, const double* APP, const doubl
   RSD_TRY(rsd_axpy_block(ctx, p, 1, X + p, p, X, p));
   // RPP factored in place
   int inf_r = 0;
-  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)p, RP, p, &inf_r, "rpp"));
+  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)p, RP, ldr, &inf_r, "rpp"));
   if (inf_r) {
     *info = inf_r;
     return RSD_OK;
   }
-  RSD_TRY(rsd_potrs_upper_tag(ctx, (int)p, RP, p, X, p, 3, "rpp"));
+  RSD_TRY(rsd_potrs_upper_tag(ctx, (int)p, RP, ldr, X, p, 3, "rpp"));
   // S_hyd = RPQ^T X2 - RQQ EIN ; S_FP(part) = RPQ^T X3 ; S_B = RPQ^T UB
   RSD_CUDA(ctx, cudaMemcpyAsync(Y, X + p, sizeof(double) * 2 * p, cudaMemcpyDeviceToDevice, s));
   RSD_CUDA(ctx, cudaMemsetAsync(Y + 2 * p, 0, sizeof(double) * p, s));
@@ -763,9 +782,12 @@ static int nogmres_impl(rsd_ctx* ctx, int32_t nn, const double* APP, const doubl
   RSD_CUDA(ctx, cudaMemcpyAsync(SijN_B, S + 2 * q, sizeof(double) * q, cudaMemcpyDeviceToHost, s));
   // Rheology leaves RPP inverted
   if (RPP) {
-    RSD_TRY(rsd_potri_upper_tag(ctx, (int)p, RP, p, "rpp"));
-    RSD_TRY(rsd_mirror_upper(ctx, (int)p, RP, p));
-    RSD_CUDA(ctx, cudaMemcpyAsync(RPP, RP, sizeof(double) * p * p, cudaMemcpyDeviceToHost, s));
+    RSD_TRY(rsd_potri_upper_tag(ctx, (int)p, RP, ldr, "rpp"));
+    RSD_TRY(rsd_mirror_upper(ctx, (int)p, RP, ldr));
+    if (ldr == p)
+      RSD_CUDA(ctx, cudaMemcpyAsync(RPP, RP, sizeof(double) * p * p, cudaMemcpyDeviceToHost, s));
+    else
+      RSD_TRY(get_block(ctx, RPP, p, p, RP, ldr));
   }
   RSD_TRY(sync(ctx));
   // stresslet dipole of the interparticle forces (Rheology 425-444)

@@ -20,6 +20,7 @@ template <typename T>
 int rsd_gemv(rsd_ctx* ctx, int trans, int m, int k, T alpha, const T* A, int64_t lda, const T* X, int64_t ldx,
              int nrhs, T beta, T* y, int64_t ldy);
 int rsd_potri64(rsd_ctx* ctx, int n, double* d_A, int64_t lda, const rsd_factor64& f);
+int rsd_potri64_space(rsd_ctx* ctx, int n);
 int rsd_potrf64_factor(rsd_ctx* ctx, int n, const char* tag, rsd_factor64* f);
 int rsd_trsv64_fwd(rsd_ctx* ctx, int n, const double* U, int64_t ldu, const double* W, double* X, double* Y,
                    int64_t ldx, int nrhs);
@@ -96,33 +97,41 @@ inline unsigned blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
 
 // Factors M' of the grand mobility in M (the upper triangle of the
-// reference's order is read) and forms A^-1 in full.  A matrix within rounding of
-// a singular one may have a positive definite factor in the one order only: then
-// M itself is factored and inverted, like MATREV, and h holds M^-1 in M.  A
-// positive info is DPOTRF's on M in the reference's order; M is then overwritten.
+// reference's order is read) and forms A^-1 in full, twice: the caller adds the
+// lubrication to the one in RPP.  Two cases are left to M itself, factored and
+// inverted in place like MATREV; h then holds M^-1 in M, and RPP is its PP block:
+// - a matrix within rounding of a singular one, which may have a positive
+//   definite factor in the one order only;
+// - no memory for M' and the rest (2.6 times that of M, which alone fits the GPU
+//   up to N ~ 16000).  The full inverse takes 2.3 times the operations: a step of
+//   10000 particles 45 s through the Schur complement, 102 s so; of 16000 390 s.
+// A positive info is DPOTRF's on M in the reference's order; M is then overwritten.
 int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int* info) {
   const int64_t P = 6LL * nn, Q = 5LL * nn;
   h->P = P;
   h->Q = Q;
   h->Qp = (Q + R64_BLOCK - 1) / R64_BLOCK * R64_BLOCK;
   h->np = h->Qp + P;
-  h->Mp = (double*)rsd_scratch(ctx, "r64_Mp", sizeof(double) * (size_t)h->np * h->np);
-  h->Ai = (double*)rsd_scratch(ctx, "r64_Ai", sizeof(double) * (size_t)P * P);
-  if (!h->Mp || !h->Ai) return RSD_ENOMEM;
+  const size_t pp = sizeof(double) * (size_t)P * P;
+  h->Mp = (double*)rsd_scratch_try(ctx, "r64_Mp", sizeof(double) * (size_t)h->np * h->np);
+  h->Ai = h->Mp ? (double*)rsd_scratch_try(ctx, "r64_Ai", pp) : nullptr;
+  h->RPP = h->Ai ? (double*)rsd_scratch_try(ctx, "r64_RPP", pp) : nullptr;
   cudaStream_t s = ctx->stream;
-  const unsigned nt = (unsigned)((h->np + 31) / 32);
-  pdl_launch(permute_qp, dim3(nt, nt), dim3(32, 8), 0, s, nn, h->Qp, h->np, M, ld, h->Mp);
-  int inf = 0;
-  RSD_TRY(rsd_potrf_upper_tag(ctx, (int)h->np, h->Mp, h->np, &inf, "mob"));
+  int inf = 1;
+  if (h->RPP && rsd_potri64_space(ctx, (int)P)) {
+    const unsigned nt = (unsigned)((h->np + 31) / 32);
+    pdl_launch(permute_qp, dim3(nt, nt), dim3(32, 8), 0, s, nn, h->Qp, h->np, M, ld, h->Mp);
+    RSD_TRY(rsd_potrf_upper_tag(ctx, (int)h->np, h->Mp, h->np, &inf, "mob"));
+  } else {
+    for (const char* name : {"r64_Mp", "r64_Ai", "r64_RPP"}) rsd_scratch_free(ctx, name);
+  }
   if (inf) {
     RSD_TRY(rsd_potrf_upper_tag(ctx, (int)(P + Q), M, ld, info, "mob"));
     if (*info) return RSD_OK;
     RSD_TRY(rsd_potri_upper_tag(ctx, (int)(P + Q), M, ld, "mob"));
     RSD_TRY(rsd_mirror_upper(ctx, (int)(P + Q), M, ld));
-    h->R = M;
-    h->ldr = ld;
-    RSD_CUDA(ctx, cudaMemcpy2DAsync(h->Ai, sizeof(double) * P, M, sizeof(double) * ld, sizeof(double) * P, P,
-                                    cudaMemcpyDeviceToDevice, s));
+    h->R = h->RPP = M;
+    h->ldr = h->ldp = ld;
     return RSD_OK;
   }
   *info = 0;
@@ -130,7 +139,10 @@ int rsd_r64_factor(rsd_ctx* ctx, int nn, double* M, int64_t ld, rsd_r64* h, int*
   pdl_launch(copy_upper64, blocks(P * P), 256, 0, s, P, h->Mp + h->Qp * (h->np + 1), h->np, h->Ai);
   const rsd_factor64 fp{h->f.W + (size_t)(h->Qp / R64_BLOCK) * R64_BLOCK * R64_BLOCK, h->f.dexp + h->Qp};
   RSD_TRY(rsd_potri64(ctx, (int)P, h->Ai, P, fp));
-  return rsd_mirror_upper(ctx, (int)P, h->Ai, P);
+  RSD_TRY(rsd_mirror_upper(ctx, (int)P, h->Ai, P));
+  h->ldp = P;
+  RSD_CUDA(ctx, cudaMemcpyAsync(h->RPP, h->Ai, pp, cudaMemcpyDeviceToDevice, s));
+  return RSD_OK;
 }
 
 // f0 = (M^-1)_PQ ein (length P); z = U_QQ^-T ein (length Qp) is kept in h

@@ -31,6 +31,7 @@ struct rsd_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   std::map<std::string, rsd_buf> bufs;  // grow-only device buffers by name
+  size_t scratch_bytes = 0, scratch_limit = 0;  // their sum, and its bound (0: the GPU's memory)
   cudaEvent_t ev[8] = {};
   double phase_ms[4] = {0, 0, 0, 0};
   int use_tc = 1;         // FP32 factorisations: 0 SIMT, 1 per-factor TF32/3xTF32, 3 all 3xTF32
@@ -93,6 +94,9 @@ int rsd_cuda_check(rsd_ctx* ctx, cudaError_t e, const char* what);
 // Grow-only named device buffer; returns nullptr (and sets ctx->err) on
 // allocation failure.
 void* rsd_scratch(rsd_ctx* ctx, const char* name, size_t bytes);
+// null where the memory cannot be had, without an error; and back to the GPU
+void* rsd_scratch_try(rsd_ctx* ctx, const char* name, size_t bytes);
+void rsd_scratch_free(rsd_ctx* ctx, const char* name);
 int rsd_set_device(rsd_ctx* ctx);
 // Dynamic shared memory above 48 KB is granted per kernel and device: asked for
 // at the kernel's first launch from each context.
@@ -300,9 +304,11 @@ struct rsd_r64 {
   int64_t P = 0, Q = 0, Qp = 0, np = 0;
   double* Mp = nullptr;  // U' in the upper triangle, np x np
   double* Ai = nullptr;  // (M^-1)_PP, full
+  double* RPP = nullptr;  // (M^-1)_PP once more, the caller's to change
+  int64_t ldp = 0;
   rsd_factor64 f;
   double* z = nullptr;
-  const double* R = nullptr;  // M^-1 in full, in place of the factor of M'
+  const double* R = nullptr;  // M^-1 in full (RPP its PP block), in place of the factor of M' and Ai
   int64_t ldr = 0;
   const double* ein = nullptr;
 };

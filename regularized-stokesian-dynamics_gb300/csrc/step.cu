@@ -302,13 +302,13 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     // arrangResist: RPP = (R_inf)_PP + rfu; the products with rfe and rse
     // come from the sparse lubrication operator (the factor has waited for it)
     if (p->use_lub) loc.n_contact = ctx->h_info[RSD_INFO_CONTACTS];
-    double* RPP = (double*)rsd_scratch(ctx, "step_RPP", sizeof(double) * P * P);
+    double* RPP = h.RPP;
+    const int64_t ldp = h.ldp;
     double* f0 = (double*)rsd_scratch(ctx, "step_f0", sizeof(double) * (P + 3 * n));
-    if (!RPP || !f0) return RSD_ENOMEM;
-    RSD_CUDA(ctx, cudaMemcpyAsync(RPP, h.Ai, sizeof(double) * P * P, cudaMemcpyDeviceToDevice, s));
-    if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f64(ctx, &lub, RPP, P));
+    if (!f0) return RSD_ENOMEM;
+    if (p->use_lub) RSD_TRY(rsd_lub_add_pp_f64(ctx, &lub, RPP, ldp));
     if (rpp_out) {
-      RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(double) * rpp_ld, RPP, sizeof(double) * P, sizeof(double) * P, P,
+      RSD_CUDA(ctx, cudaMemcpy2DAsync(rpp_out, sizeof(double) * rpp_ld, RPP, sizeof(double) * ldp, sizeof(double) * P, P,
                                       cudaMemcpyDeviceToDevice, s));
       RSD_CUDA(ctx, cudaStreamSynchronize(s));
       if (info) *info = loc;
@@ -336,7 +336,7 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
       const double tol = ctx->rpp_tol > 0 ? ctx->rpp_tol : 1e-12;
       int it = 0;
       double res = 0.0;
-      RSD_TRY(rsd_lp_pcg_internal(ctx, (rsd_lp*)ctx->rpp_net, ctx->rpp_mode, nn, d_conf, d_radii, &lat, RPP, P, 2, B, X,
+      RSD_TRY(rsd_lp_pcg_internal(ctx, (rsd_lp*)ctx->rpp_net, ctx->rpp_mode, nn, d_conf, d_radii, &lat, RPP, ldp, 2, B, X,
                                   tol, ctx->rpp_maxit > 0 ? ctx->rpp_maxit : 1000, &it, &res));
       loc.rpp_iterations = it;
       if (res <= tol) {
@@ -348,13 +348,13 @@ static int step_impl(rsd_ctx* ctx, const rsd_lubtab* tab, const rsd_step_params*
     }
     if (!solved) {
       int info_r = 0;
-      RSD_TRY(rsd_potrf_upper_tag(ctx, (int)P, RPP, P, &info_r, "rpp"));
+      RSD_TRY(rsd_potrf_upper_tag(ctx, (int)P, RPP, ldp, &info_r, "rpp"));
       if (info_r) {
         loc.info = info_r;
         if (info) *info = loc;
         return info_r;
       }
-      RSD_TRY(rsd_potrs_upper_tag(ctx, (int)P, RPP, P, X, P, 2, "rpp"));
+      RSD_TRY(rsd_potrs_upper_tag(ctx, (int)P, RPP, ldp, X, P, 2, "rpp"));
     }
     // SijN_hyd = RPQ^T RPP^-1 RPQ EIN - RQQ EIN
     RSD_TRY(rsd_r64_stresslet(ctx, &h, X + P, 1, f0, S));
